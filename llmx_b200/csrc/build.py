@@ -48,6 +48,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "attention_split": ["attention_split.cu"],     # softmax attention with key and value widths of their own, windows and chunks
     "moe": ["moe.cu"],                        # experts chosen by a table: routing on the device, grouped products
     "latent_attention": ["latent_attention.cu"],   # attention over a cache of latents
+    "latent_prompt_tc": ["latent_prompt_tc.cu"],    # the same for requests of many rows: keys and values made once a step
     "selftest": ["selftest.cu"],              # the bounded wait made to run out on purpose (tests)
     "runtime": ["runtime/runtime.cpp", "runtime/engine.cpp", "runtime/loader.cpp"],       # host code: the parts' forward passes (no kernels of its own)
 }

@@ -144,6 +144,9 @@ _SIGNATURES = {
     ("latent_attention", "llmx_latent_query"): [_p, _i, _p, _i, _p, _p, _i, _i, _f, _p, _i, _i, _i, _i, _i, _f, _p],
     ("latent_attention", "llmx_latent_scores"): [_p, _p, _i, _p, _p, _i, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p],
     ("latent_attention", "llmx_latent_merge"): [_p, _p, _i, _p, _i, _i, _i, _i, _i, _p],
+    ("latent_prompt_tc", "llmx_latent_expand"): [_p, ctypes.c_longlong, _p, _p, _i, _p, _p, _i, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i,
+                                                 _i, _p, _p],
+    ("latent_prompt_tc", "llmx_latent_prompt"): [_p, _i, _p, _i, _p, _p, _i, _p, _i, _i, _f, _p, _i, _i, _i, _i, _i, _f, _p, _p],
     ("gemm_plain", "llmx_gemm_plain"): [_p, _i, _p, _i, _p, _i, _i, _i, _i, _p],
     ("attention_plain", "llmx_attention_plain"): [_p, _i, _p, _i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _p],
 }
@@ -1150,4 +1153,53 @@ def latent_attention_tiled(q: torch.Tensor, cache: torch.Tensor, w_uk: torch.Ten
                                                          1 if plain_cores else 0, _stream()), "latent_scores")
     _check(_fn("latent_attention", "llmx_latent_merge")(_ptr(part), _ptr(w_uv), _code(w_uv), _ptr(out), rows, heads, value_dim, latent,
                                                         int(splits), _stream()), "latent_merge")
+    return out
+
+
+# What `latent_attention_prompt` keeps of a (token, head): three parts each of 128 key and 128 value values, 64 rotated ones.
+LATENT_EXPANDED = 832
+
+
+def latent_prompt_fits(key_dim: int, rot: int, value_dim: int, latent: int, page_size: int, w_dtype, cache_dtype) -> bool:
+    """Whether `latent_attention_prompt` takes these sizes and types."""
+    return (key_dim == 128 and value_dim == 128 and 0 <= rot <= 64 and rot % 8 == 0 and latent % 64 == 0 and page_size % 16 == 0
+            and w_dtype == torch.bfloat16 and cache_dtype == torch.bfloat16)
+
+
+def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, w_uk: torch.Tensor, w_uv: torch.Tensor, out: torch.Tensor,
+                            freq: torch.Tensor, row_request: torch.Tensor, positions: torch.Tensor, block_tables: torch.Tensor,
+                            requests: torch.Tensor, n_requests: int, max_tokens: int, tiles: torch.Tensor, n_tiles: int, tokens: int,
+                            group_heads: int, heads: int, key_dim: int, rot: int, value_dim: int, latent: int, page_size: int,
+                            window: Optional[int], scale: float, halves: bool = False, magnitude: float = 1.0) -> torch.Tensor:
+    """`latent_attention` for requests of many rows (csrc/latent_prompt_tc.cu): keys and values of `group_heads` heads at a
+    time are made in a workspace of `tokens` tokens, then read by tiles of 128 rows on the tensor cores.  `requests` int32
+    [n_requests, 4] (first row, rows, first workspace token, workspace tokens) and `tiles` int32 [n_tiles, 4] (first row,
+    rows, first workspace token of the request, first row of the request) on the device; only the tiles' rows of `out` are
+    written."""
+    from .runtime import error_word
+    _cuda(cache, w_uk, w_uv, out, freq, row_request, positions, block_tables, requests, tiles)
+    rows = q.shape[0]
+    _need(q.is_cuda and q.dtype == torch.float32 and q.shape[1] == heads * (key_dim + rot) and q.stride(1) == 1,
+          "latent_attention: queries float32 [rows, heads * (key_dim + rot)]")
+    _need(latent_prompt_fits(key_dim, rot, value_dim, latent, page_size, w_uk.dtype, cache.dtype),
+          "latent_attention_prompt: sizes or types that this form does not take")
+    _need(tuple(w_uk.shape) == (heads * key_dim, latent) and tuple(w_uv.shape) == (heads * value_dim, latent)
+          and w_uk.dtype == w_uv.dtype == out.dtype, "latent_attention: key and value maps do not fit")
+    _need(tuple(out.shape) == (rows, heads * value_dim) and cache.shape[-1] == latent + rot, "latent_attention: output or cache rows do not fit")
+    for t in (row_request, positions, block_tables, requests, tiles):
+        _need(t.dtype == torch.int32, "latent_attention: metadata must be int32")
+    _need(requests.numel() >= 4 * n_requests > 0 and tiles.numel() >= 4 * n_tiles > 0 and 0 < max_tokens <= tokens and group_heads > 0,
+          "latent_attention_prompt: requests or tiles do not fit")
+    err = _ptr(error_word(q.device))
+    expanded = torch.empty((min(group_heads, heads), tokens, LATENT_EXPANDED), dtype=torch.bfloat16, device=q.device)
+    for h in range(0, heads, group_heads):
+        n = min(group_heads, heads - h)
+        _check(_fn("latent_prompt_tc", "llmx_latent_expand")(
+            _ptr(cache), cache.numel() // cache.shape[-1], _ptr(w_uk), _ptr(w_uv), heads, _ptr(expanded), _ptr(requests), int(n_requests),
+            int(max_tokens), _ptr(row_request), _ptr(positions), _ptr(block_tables), block_tables.shape[1], int(tokens), h, n, latent, rot,
+            page_size, int(window or 0), err, _stream()), "latent_expand")
+        _check(_fn("latent_prompt_tc", "llmx_latent_prompt")(
+            _ptr(expanded), int(tokens), _ptr(q), q.stride(0) if rows > 1 else q.shape[1], _ptr(out), _ptr(tiles), int(n_tiles), _ptr(freq),
+            freq.numel(), 1 if halves else 0, float(magnitude), _ptr(positions), heads, h, n, rot, int(window or 0), float(scale), err,
+            _stream()), "latent_prompt")
     return out

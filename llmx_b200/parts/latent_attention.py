@@ -8,9 +8,10 @@ a query latent of `q_rank` and a key/value latent of C = `kv_rank` values:
     o = softmax over the keys lo..p (lo = 0, or p - window + 1 under a sliding window) of s, times v
     residual += o Wo^T
 Only [c | r] is cached, one vector per token (a cache entry of one plane).  The rotation pairs neighbours
-(2i, 2i + 1) of the first `rot_dims` values of the rotated part by the angle p * base^(-2i / rot_dims).  The kernels
-(csrc/latent_attention.cu) never make keys or values of cached tokens: the query goes through Wuk once, the weighted
-sum of latents through Wuv once.
+(2i, 2i + 1) of the first `rot_dims` values of the rotated part by the angle p * base^(-2i / rot_dims).  The general
+kernels (csrc/latent_attention.cu) never make keys or values of cached tokens: the query goes through Wuk once, the
+weighted sum of latents through Wuv once.  For requests with many rows a step makes them once, in a workspace, and the
+rows' attention over them runs on the tensor cores (csrc/latent_prompt_tc.cu).
 
 Options for designs that vary it:
     q_rank None        no query latent: q = h Wq^T straight from the input (tensor role `q` instead of dq, dq.norm, uq)
@@ -35,16 +36,31 @@ from .linear import Linear, add_product, stored_product
 from .rope import blended_frequencies, power_frequencies
 
 
-class _TilePlan(PartPlan):
-    """The row tiles of a step for the tiled kernels: (first row, rows) per tile, rows of one request each.  They follow
-    the step's row counts alone, so a recorded step's plan never changes."""
+# Requests that bring at least this many rows, and one for this many of the keys they see, have their keys and values made
+# (csrc/latent_prompt_tc.cu): making them costs the same for one row as for many.  Measured, us, that form / the general one, 16
+# heads of 128 + 64 over latents of 512: after nothing 16 rows 45 / 53, 32 rows 46 / 68, 512 rows 75 / 394; after 1,000 tokens 16
+# rows 98 / 80, 32 rows 102 / 131, 512 rows 137 / 840; after 8,000 tokens 32 rows 538 / 364, 64 rows 539 / 640, 512 rows 574 / 3,973.
+PROMPT_ROWS, PROMPT_KEYS_A_ROW = 32, 128
+# The workspace of made keys and values: heads are taken in groups that fit these bytes, or what the general form's queries
+# and sums over the same rows would take if that is more.
+PROMPT_BYTES = 256 << 20
 
-    def __init__(self, tiles):
-        self.tiles = np.asarray(tiles, dtype=np.int32).reshape(-1)
-        self.ints = int(self.tiles.size)
+
+class _TilePlan(PartPlan):
+    """How a step's rows are cut for the kernels.  A run is a stretch of neighbouring rows for the tiled kernels: (first row,
+    rows, first int, tiles, key ranges), its ints (first row in the stretch, rows) per tile, rows of one request each.
+    `whole` is the run of all rows.  `wide`, where some requests have many rows: (first int of those requests, how many, the
+    largest share of the workspace, first int of their tiles, how many, workspace tokens, heads a group); `runs` are then the
+    stretches between them.  All follows the step's row counts and the context it has room for, so a recorded step's plan
+    never changes."""
+
+    def __init__(self, whole, runs, wide, ints):
+        self.whole, self.runs, self.wide = whole, runs, wide
+        self.values = np.asarray(ints, dtype=np.int32)
+        self.ints = int(self.values.size)
 
     def fill(self, histories, out: np.ndarray) -> None:
-        out[:self.ints] = self.tiles
+        out[:self.ints] = self.values
 
 
 class LatentAttention(Part):
@@ -133,11 +149,60 @@ class LatentAttention(Part):
         splits = max(1, min(-(-2 * self._sms // blocks), keys // 128))
         return tiles, splits
 
+    def _wide(self, counts, contexts):
+        """The requests whose keys and values are made: (ints of the requests, ints of their tiles, largest share of the
+        workspace, workspace tokens, heads a group), or None when there are none or their workspace would not fit."""
+        requests, tiles, start, tokens, rows = [], [], 0, 0, 0
+        for n, context in zip(counts, contexts):
+            keys = context if self.window is None else min(context, self.window + n - 1)
+            if n >= PROMPT_ROWS and n * PROMPT_KEYS_A_ROW >= keys:
+                share = -(-(keys + 63) // 128) * 128             # the first key lies up to 63 tokens into its share
+                requests.append((start, n, tokens, share))
+                tiles += [(start + i, min(128, n - i), tokens, start) for i in reversed(range(0, n, 128))]
+                tokens, rows = tokens + share, rows + n
+            start += n
+        if not requests:
+            return None
+        room = max(PROMPT_BYTES, rows * self.heads * (2 * self.kv_rank + self.rot_dim + 2) * 4)
+        group = min(self.heads, room // (tokens * ops.LATENT_EXPANDED * 2))
+        if group < 1:
+            return None
+        return requests, tiles, max(r[3] for r in requests), tokens, group
+
     def plan_step(self, shape: StepShape) -> Optional[PartPlan]:
         if getattr(self, "precision", None) is None or self.precision.invariant:
             return None
-        context = shape.room if shape.room > 0 else max(h + c for h, c in zip(shape.histories, shape.counts))
-        return _TilePlan(self._tiling(shape.counts, context)[0])
+        counts = shape.counts
+        contexts = [shape.room] * len(counts) if shape.room > 0 else [h + c for h, c in zip(shape.histories, counts)]
+        ints = []
+
+        def run(first, some):
+            tiles, splits = self._tiling(some, max(contexts))
+            at = len(ints)
+            ints.extend(x for t in tiles for x in t)
+            return first, sum(some), at, len(tiles), splits
+
+        whole, runs, wide = run(0, counts), [], None
+        if self.key_dim == 128 and self.value_dim == 128 and self.w_uk.dtype is torch.bfloat16:
+            wide = self._wide(counts, contexts)
+        if wide is not None:
+            requests, tiles, share, tokens, group = wide
+            made = {r[0] for r in requests}
+            first = at = 0
+            small = []
+            for n in counts:
+                if at not in made:
+                    small.append(n)
+                else:
+                    if small:
+                        runs.append(run(first, small))
+                    first, small = at + n, []
+                at += n
+            if small:
+                runs.append(run(first, small))
+            wide = (len(ints), len(requests), share, len(ints) + 4 * len(requests), len(tiles), tokens, group)
+            ints += [x for r in requests + tiles for x in r]
+        return _TilePlan(whole, runs, wide, ints)
 
     def forward(self, h: torch.Tensor, step: StepBatch, cache_entry: int, residual: torch.Tensor,
                 write_cache: bool = True) -> None:
@@ -163,14 +228,24 @@ class LatentAttention(Part):
             gate_at = latents + self.q_width
         o = torch.empty((rows, self.v_width), dtype=self.precision.act, device=h.device)
         # The tiled kernels hold a cache row in a warp's registers: rows of up to 768 values.
-        tiles = None if self.precision.invariant or self.kv_rank + self.rot_dim > 768 else step.plan_ints(self)
-        if tiles is not None:
+        ints = None if self.precision.invariant or self.kv_rank + self.rot_dim > 768 else step.plan_ints(self)
+        if ints is not None:
+            plan = step.plan.plan_of(self)
+            sizes = (self.heads, self.key_dim, self.rot_dim, self.value_dim, self.kv_rank, group.page_size, self.window, self.scale)
+            runs = [plan.whole]
+            if plan.wide is not None and not self.plain_cores and ops.latent_prompt_fits(
+                    self.key_dim, self.rot_dim, self.value_dim, self.kv_rank, group.page_size, self.w_uk.dtype, cache.dtype):
+                at, n_requests, share, tiles_at, n_tiles, tokens, heads = plan.wide
+                ops.latent_attention_prompt(q, cache, self.w_uk, self.w_uv, o, self.freq, step.row_request, step.positions,
+                                            group.block_tables, ints[at:at + 4 * n_requests], n_requests, share,
+                                            ints[tiles_at:tiles_at + 4 * n_tiles], n_tiles, tokens, heads, *sizes, halves=halves, magnitude=mag)
+                runs = plan.runs
             # The tiled kernels: 16 (row, head) pairs share the keys they read; key ranges fill the device when rows are few.
-            host_tiles, splits = self._tiling(step.host_row_count, step.max_context)
-            ops.latent_attention_tiled(q, cache, self.w_uk, self.w_uv, o, self.freq, step.row_request, step.positions,
-                                       group.block_tables, tiles, len(host_tiles), splits, self.heads, self.key_dim, self.rot_dim,
-                                       self.value_dim, self.kv_rank, group.page_size, self.window, self.scale, plain_cores=self.plain_cores,
-                                       halves=halves, magnitude=mag)
+            for first, n, at, n_tiles, splits in runs:
+                rows_of = slice(first, first + n)
+                ops.latent_attention_tiled(q[rows_of], cache, self.w_uk, self.w_uv, o[rows_of], self.freq, step.row_request[rows_of],
+                                           step.positions[rows_of], group.block_tables, ints[at:at + 2 * n_tiles], n_tiles, splits,
+                                           *sizes, plain_cores=self.plain_cores, halves=halves, magnitude=mag)
         else:
             # One block per (row, head): the schedule follows the sizes alone (an invariant path, or a step without a plan).
             ops.latent_attention(q, cache, self.w_uk, self.w_uv, o, self.freq, step.row_request, step.positions, group.block_tables,

@@ -723,3 +723,77 @@ def test_random_weights_are_the_same_on_the_device_and_on_the_host():
         host, device = RandomSource(specs, 7, dtype=dtype, device="cpu"), RandomSource(specs, 7, dtype=dtype, device=DEV)
         for name in specs:
             assert torch.equal(host.tensor(name), device.tensor(name).cpu()), (name, dtype)
+
+
+# ---- latent attention of requests with many rows: keys and values made once a step ----------------------------------------------
+LATENT_STEPS = {
+    "one_tile": ([32], [0]), "edges_of_a_tile": ([128, 127, 129], [0, 0, 0]), "odd_after_odd": ([65, 33], [63, 1]),
+    "many_keys": ([40], [700]), "few_rows_between": ([3, 200, 1, 31, 64, 2], [50, 17, 130, 0, 64, 9]), "two_tiles_after_a_stage": ([256], [64]),
+}
+
+
+@pytest.mark.parametrize("name", list(LATENT_STEPS))
+@pytest.mark.parametrize("heads,rot,latent,window,halves", [(3, 64, 512, 100, False), (5, 8, 64, None, True), (2, 0, 192, 1, False), (1, 48, 128, 64, True)])
+def test_latent_prompt_equals_the_general_form(name, heads, rot, latent, window, halves):
+    """Every row of a planned step against the same attention in 64 bits over the same queries, cache and maps, by the form for
+    many rows and by the general one.  Both round the result to bfloat16 (2^-9 of it) after 32-bit sums of a few hundred to
+    a thousand terms, whose error is relative to the values' size (about 2^-20 of it): the bound below is twice these."""
+    from llmx_b200 import ops
+    from llmx_b200.parts.base import Precision, StepShape
+    from llmx_b200.parts.latent_attention import LatentAttention
+    counts, histories = LATENT_STEPS[name]
+    g = torch.Generator(device="cuda").manual_seed(7)
+    page, rows, scale, mag = 16, sum(counts), 0.11, 1.25
+    part = LatentAttention(64, heads, 128, rot, 128, None, latent, scale, 1e4, rot, 1e-6, window, pairing="halves" if halves else "neighbours")
+    part.precision, part._sms = Precision.of("bfloat16"), 148
+    part.w_uk, part.w_uv = (torch.randn(heads * 128, latent, device="cuda", generator=g).mul_(latent ** -0.5).bfloat16() for _ in range(2))
+    freq = torch.from_numpy(part.frequencies()[0]).cuda()
+    plan = part.plan_step(StepShape(counts, histories))
+    assert plan.wide is not None and sum(r[1] for r in plan.runs) == sum(n for n in counts if n < 32)
+    ints = torch.tensor(plan.values, device="cuda")
+    needs = [-(-(h + n) // page) for h, n in zip(histories, counts)]
+    order = torch.randperm(sum(needs), generator=torch.Generator().manual_seed(3)).tolist()
+    tables, at = torch.full((len(counts), max(needs)), -1, dtype=torch.int32), 0
+    for r, k in enumerate(needs):
+        tables[r, :k] = torch.tensor(order[at:at + k])
+        at += k
+        if window is not None:                                   # pages below every row's window have been given back
+            tables[r, :max(0, histories[r] - window + 1) // page] = -1
+    cache = torch.randn(sum(needs), 1, 1, page, latent + rot, device="cuda", generator=g).bfloat16()
+    q = torch.randn(rows, heads * (128 + rot), device="cuda", generator=g)
+    request = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(counts)])
+    position = torch.cat([torch.arange(h, h + n, dtype=torch.int32) for h, n in zip(histories, counts)])
+    meta = request.cuda(), position.cuda(), tables.cuda()
+    sizes = (heads, 128, rot, 128, latent, page, window, scale)
+    out = torch.zeros(rows, heads * 128, device="cuda", dtype=torch.bfloat16)
+    first, n_req, share, tiles_at, n_tiles, tokens, group = plan.wide
+    ops.latent_attention_prompt(q, cache, part.w_uk, part.w_uv, out, freq, *meta, ints[first:], n_req, share, ints[tiles_at:], n_tiles, tokens,
+                                max(1, min(group, heads - 1)), *sizes, halves=halves, magnitude=mag)
+    for start, n, at, n_tiles, splits in plan.runs:
+        s = slice(start, start + n)
+        ops.latent_attention_tiled(q[s], cache, part.w_uk, part.w_uv, out[s], freq, meta[0][s], meta[1][s], meta[2], ints[at:], n_tiles, splits, *sizes,
+                                   halves=halves, magnitude=mag)
+    general = torch.zeros_like(out)
+    ops.latent_attention(q, cache, part.w_uk, part.w_uv, general, freq, *meta, *sizes, halves=halves, magnitude=mag)
+    from llmx_b200.runtime import check_errors
+    check_errors()
+    uk, uv = (w.double().view(heads, 128, latent) for w in (part.w_uk, part.w_uv))
+    flat = cache.view(-1, latent + rot).double()
+    for r in range(rows):
+        p, table = int(position[r]), meta[2][int(request[r])].long()
+        t = torch.arange(max(0, p - window + 1) if window else 0, p + 1, device="cuda")
+        c = flat[table[t // page] * page + t % page]
+        qh = q[r].double().view(heads, 128 + rot)
+        x = qh[:, 128:].clone()
+        a, b = (x[:, :rot // 2], x[:, rot // 2:]) if halves else (x[:, 0::2], x[:, 1::2])
+        angle = (p * freq).double()                              # the angle is the 32-bit product
+        turned = torch.cat([a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()], 1)
+        if not halves:
+            turned = turned.view(heads, 2, rot // 2).transpose(1, 2).reshape(heads, rot)
+        s = torch.einsum("hd,hdc,tc->ht", qh[:, :128], uk, c[:, :latent]) + mag * turned @ c[:, latent:].T
+        values = torch.einsum("hvc,tc->htv", uv, c[:, :latent])
+        want = torch.einsum("ht,htv->hv", torch.softmax(s * scale, 1), values).reshape(-1)
+        bound = 2 * (2.0 ** -9 * want.abs() + 2.0 ** -20 * (1.0 + s.abs().max() * scale) * values.abs().max())
+        for how, got in (("many rows", out), ("general", general)):
+            worst = ((got[r].double() - want).abs() / bound).max()
+            assert worst <= 1.0, (how, r, p, float(worst))
