@@ -151,14 +151,33 @@ recurrence_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     }
 }
 
-// The wide form for long runs of rows: sixteen columns of one head a block, and the rows' q, k, v and gates brought to shared
-// memory sixteen rows at a time by cp.async (the next sixteen in flight meanwhile), so that a row waits for shared memory
-// and for the row before it, not for the L2 cache.  With a delta rule a warp owns one column: every row waits for a sum over
-// the warp's lanes.  Without one a warp owns two columns (a row's q, k and gates are read once for both) and the
-// read-outs of eight rows are summed over the lanes together.
-constexpr int WIDE_COLS = 16, WIDE_CH = 16, WIDE_SUMS = 8;
-constexpr int wide_columns_a_warp(int mode) { return mode == M_DELTA || mode == M_DELTA_VEC ? 1 : 2; }
-constexpr int wide_threads(int mode) { return 32 * WIDE_COLS / wide_columns_a_warp(mode); }
+// The wide form for long runs of rows: 16 or 32 columns of one head a block.  A group of LANES lanes shares CPL columns: a lane
+// reads PER values of a row's q and k (and gates) from shared memory once and uses them for its share of all the columns.
+// (Shared memory gives a lane 4 bytes a cycle: one column a group of eight lanes was bound by that, 162 cycles a row and
+// warp.)  A lane's values are pairs in 64-bit registers, two multiply-adds an instruction.  Four more warps bring the rows' q, k, v and gates to shared memory by cp.async, sixteen rows
+// a buffer (four a warp), two or three buffers, handed over by named barriers: the workers address no global memory for
+// their inputs.
+//
+// With a delta rule a row waits for the sum k . S over the group's lanes, and the next row for that row.  Four rows t are
+// therefore taken at a time: p_t = k_t . S (after the decays of the rows up to t) against the state before the four, whose
+// sums over the lanes go side by side, and what the rows between add to it, (k_t . k_s) u_s, comes from the six products
+// of the four keys with one another -- the same for all columns, made by the warp that copied the four rows:
+//     x_t = p_t;  for s < t:  x_t = a_s x_t + (k_t . k_s) u_s         (channel decays: inside p_t and the products)
+//     u_t = beta_t (v_t - a_t x_t)
+// The state then takes the four rows in order.  The read-outs, which nothing waits for, are summed over the lanes eight rows
+// at a time.
+//
+// 16 heads of 128 x 128, 2,048 rows of one request, us before (a warp two columns, or with a correction one, copies by all
+// threads) and now: constant decay 245 -> 166, delta rule 673 -> 259, scaled 265 -> 172, delta rule with channel decays 715 -> 307,
+// channel decays alone 298 -> 186; 32 heads: 362 -> 235, 949 -> 362 and (channel decays) 1,037 -> 449; eight requests of 190 rows:
+// 122 -> 110, 329 -> 159 and 339 -> 192.  A row's multiply-adds are 48 to 64 cycles of a warp, its reads of shared memory and
+// shuffles 50 to 90 cycles of the SM; the rest is the chain of the four rows' corrections (delta rule) and the hand-over.
+constexpr int WIDE_CH = 16, WIDE_SUMS = 8;
+constexpr int WIDE_COPY_WARPS = 4, WIDE_COPY_ROWS = WIDE_CH / WIDE_COPY_WARPS;
+constexpr int WIDE_GRAM = 8 * WIDE_COPY_WARPS;          // floats a buffer has for its keys' products: six (of eight) for four rows
+
+__device__ __forceinline__ void barrier_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void barrier_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
 __device__ __forceinline__ void cp_async_4(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -168,220 +187,369 @@ __device__ __forceinline__ void cp_async_16f(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-// A lane holds the PER neighbouring values d = PER * lane .. of its column; a row's vectors are padded with zeros to PER * 32
-// values, so that a lane's share is whole 16-byte (or 8-byte) reads from shared memory without a condition.
-template <int PER>
-__device__ __forceinline__ void read_run(const float* p, int lane, float (&out)[PER]) {
-    static_assert(PER == 1 || PER == 2 || PER % 4 == 0, "a lane's share of a row");
-    if constexpr (PER == 1) {
-        out[0] = p[lane];
-    } else if constexpr (PER == 2) {
-        const float2 x = *reinterpret_cast<const float2*>(p + lane * 2);
-        out[0] = x.x, out[1] = x.y;
-    } else {
+// Two 32-bit numbers in a 64-bit register, and operations on both.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float pair_sum(f32x2 v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return lo + hi;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// A lane holds PER values of its column, d = 4 (lane + LANES i) + 0 .. 3; a row's vectors are padded with zeros to LANES PER values,
+// so that a lane's share is whole 16-byte reads from shared memory without a condition (neighbouring lanes read a run).
+template <int PER, int LANES>
+__device__ __forceinline__ void read_share(const float* p, int sub, f32x2 (&out)[PER / 2]) {
 #pragma unroll
-        for (int i = 0; i < PER; i += 4) {
-            const float4 x = *reinterpret_cast<const float4*>(p + lane * PER + i);
-            out[i] = x.x, out[i + 1] = x.y, out[i + 2] = x.z, out[i + 3] = x.w;
-        }
+    for (int i = 0; i < PER / 4; ++i) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(p + 4 * (sub + LANES * i));
+        out[2 * i] = x.x, out[2 * i + 1] = x.y;
     }
 }
 
-template <int PER, int MODE>
-__global__ void __launch_bounds__(wide_threads(MODE))
+// The sum of a lane's share of a dot product, in two chains.
+template <int N>
+__device__ __forceinline__ float share_dot(const f32x2 (&a)[N], const f32x2 (&b)[N]) {
+    f32x2 s0 = mul2(a[0], b[0]), s1 = mul2(a[1], b[1]);
+#pragma unroll
+    for (int i = 2; i < N; i += 2) {
+        s0 = fma2(a[i], b[i], s0);
+        s1 = fma2(a[i + 1], b[i + 1], s1);
+    }
+    return pair_sum(add2(s0, s1));
+}
+
+template <int PER, int LANES, int CPL, int COLS, int MODE>
+__global__ void __launch_bounds__(COLS / CPL * LANES + 32 * WIDE_COPY_WARPS, 1)
 recurrence_wide_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, int q_stride,
                        int k_stride, int v_stride, const float* __restrict__ decay, const float* __restrict__ gate,
                        const float* __restrict__ beta, int gate_stride, int beta_stride, const float* __restrict__ skip,
                        float* __restrict__ state, long long slot_floats,
                        const int* __restrict__ row_start, const int* __restrict__ row_count,
                        const int* __restrict__ history, const int* __restrict__ slot_in,
-                       const int* __restrict__ slot_out, float* __restrict__ out, int heads, int qk_heads, int D, int V) {
+                       const int* __restrict__ slot_out, float* __restrict__ out, int heads, int qk_heads, int D, int V, int stages) {
     pdl_trigger();
     pdl_wait();
-    extern __shared__ __align__(16) float stage[];   // [2][WIDE_CH][row_floats]: q (Dp), k (Dp), [gates per channel (Dp)], v (the block's columns), gate, beta, pad
-    constexpr bool VEC = has_channel_gate(MODE);
-    constexpr int CPW = wide_columns_a_warp(MODE), THREADS = wide_threads(MODE);
+    extern __shared__ __align__(16) float stage[];   // [stages]{[WIDE_CH][row_floats]: q (Dp), k (Dp), [gates per channel (Dp)], v (the block's columns), gate, beta, pad; gram}
+    constexpr bool VEC = has_channel_gate(MODE), CORRECTED = MODE == M_DELTA || MODE == M_DELTA_VEC;
     constexpr int NV = VEC ? 3 : 2;                  // vectors of D values a row brings
-    const int Dp = PER * 32;                         // a row's q and k padded to the lanes' runs (the pad is cleared once and never written by the copies)
-    const int row_floats = NV * Dp + WIDE_COLS + 4;  // a multiple of 4: every row starts on 16 bytes
+    constexpr int WORKERS = COLS / CPL * LANES, THREADS = WORKERS + 32 * WIDE_COPY_WARPS;
+    constexpr int BLK = PER == 16 ? 1 : 4;           // rows taken at a time (four of 16 values a lane: too many registers)
+    constexpr int Dp = PER * LANES;                  // the vectors' padded length (the pad is cleared once and never written by the copies)
+    constexpr int row_floats = NV * Dp + COLS + 4;   // a multiple of 4: every row starts on 16 bytes
+    constexpr int stage_floats = WIDE_CH * row_floats + WIDE_GRAM;
+    constexpr int P2 = PER / 2;
+    constexpr int FULL = 1, EMPTY = 4;               // named barriers: buffer s is filled (FULL + s), is free again (EMPTY + s)
     const int r = blockIdx.x;
-    const int blocks_per_head = (V + WIDE_COLS - 1) / WIDE_COLS;
+    const int blocks_per_head = (V + COLS - 1) / COLS;
     const int h = blockIdx.y / blocks_per_head;
-    const int first_col = (blockIdx.y % blocks_per_head) * WIDE_COLS;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = first_col + warp * CPW;          // the warp's first column; columns past V shadow the last one and store nothing
+    const int first_col = (blockIdx.y % blocks_per_head) * COLS;
     const int n = row_count[r];
     if (n <= 0) return;
     const int a0 = row_start[r];
-    const int hq = h / (heads / qk_heads);
-    float S[CPW][PER];
-    const bool fresh = history[r] == 0;
-#pragma unroll
-    for (int w = 0; w < CPW; ++w) {
-        const float* sin_ = state + (size_t)slot_in[r] * slot_floats + ((size_t)h * V + min(col + w, V - 1)) * D;
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            const int d = lane * PER + i;
-            S[w][i] = (!fresh && d < D) ? sin_[d] : 0.0f;
-        }
-    }
-    const float dec = MODE == M_CONST ? decay[h] : VEC ? 1.0f : 0.0f;
-    const float sk = MODE == M_SCALED && skip != nullptr ? skip[h] : 0.0f;
-    // What this thread copies of every chunk is the same from chunk to chunk, so its places are worked out once:
-    // pieces of 16 bytes of q and k when rows allow it (else single values), and the chunk's small values one by one.
-    const bool vec = D % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)k & 15) == 0 &&
-                     (!VEC || (gate_stride % 4 == 0 && ((uintptr_t)gate & 15) == 0));
-    const int unit = vec ? 4 : 1;
-    const int per_vec = D / unit;
-    const int per_row = NV * per_vec;                // copies a row's q and k (and channel gates) take
-    constexpr int MAX_COPIES = NV * PER * 32 * WIDE_CH / THREADS;     // at most, with single values
-    auto issue = [&](int chunk, int which) {
-        float* buf = stage + (size_t)which * WIDE_CH * row_floats;
-        const int t0 = chunk * WIDE_CH, rows = min(WIDE_CH, n - t0);
-        const int copies = rows * per_row;
-        int p = threadIdx.x, t = p / per_row, e = p % per_row;
-        const int dt = THREADS / per_row, de = THREADS % per_row;
-#pragma unroll 4
-        for (int i = 0; i < MAX_COPIES; ++i) {
-            if (p >= copies) break;
-            const size_t row = (size_t)(a0 + t0 + t);
-            const int which_vec = (e >= per_vec) + (e >= 2 * per_vec);       // 0: q, 1: k, 2: the gates per channel
-            const int off = (e - which_vec * per_vec) * unit;
-            const float* src = which_vec == 0 ? q + row * q_stride + (size_t)hq * D + off
-                             : which_vec == 1 ? k + row * k_stride + (size_t)hq * D + off
-                                              : gate + row * gate_stride + (size_t)h * D + off;
-            float* dst = buf + (size_t)t * row_floats + which_vec * Dp + off;
-            if (vec) cp_async_16f(dst, src);
-            else cp_async_4(dst, src);
-            p += THREADS;
-            t += dt;
-            e += de;
-            if (e >= per_row) {
-                e -= per_row;
-                ++t;
-            }
-        }
-        for (int i = threadIdx.x; i < WIDE_CH * (WIDE_COLS + 2); i += THREADS) {
-            const int small_t = i / (WIDE_COLS + 2), small_e = i % (WIDE_COLS + 2);
-            if (small_t >= rows || !(small_e < WIDE_COLS || (small_e == WIDE_COLS ? (MODE == M_DELTA || MODE == M_SCALED) : has_beta(MODE)))) continue;
-            const size_t row = (size_t)(a0 + t0 + small_t);
-            const float* src = small_e < WIDE_COLS ? v + row * v_stride + (size_t)h * V + min(first_col + small_e, V - 1)
-                             : small_e == WIDE_COLS ? gate + row * gate_stride + h : beta + row * beta_stride + h;
-            cp_async_4(buf + (size_t)small_t * row_floats + NV * Dp + small_e, src);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
+    const int chunks = (n + WIDE_CH - 1) / WIDE_CH;
     if (D < Dp) {
-        for (int i = threadIdx.x; i < 2 * WIDE_CH * row_floats; i += THREADS) stage[i] = 0.0f;
+        for (int i = threadIdx.x; i < stages * stage_floats; i += THREADS) stage[i] = 0.0f;
         __syncthreads();
     }
-    const int chunks = (n + WIDE_CH - 1) / WIDE_CH;
-    issue(0, 0);
-    for (int c = 0; c < chunks; ++c) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                             // chunk c has landed; everyone has left the other buffer
-        if (c + 1 < chunks) issue(c + 1, (c + 1) & 1);
-        const float* buf = stage + (size_t)(c & 1) * WIDE_CH * row_floats;
-        const int rows = min(WIDE_CH, n - c * WIDE_CH);
-        if constexpr (MODE != M_DELTA && MODE != M_DELTA_VEC) {
-            // A whole group of rows has no condition within it, so that the reads of its rows run ahead of their sums.
-            auto group = [&](int t0, auto whole) {
-                float acc[WIDE_SUMS * CPW];          // [row][column]
+
+    if (threadIdx.x >= WORKERS) {
+        // ---- a copying warp: four rows of every chunk, pieces of 16 bytes where addresses and widths allow it, else single
+        // values.  A lane has one piece of a vector (more with wide vectors), of all four rows, and one of the rows' small pieces.
+        const int lane = threadIdx.x & 31, first = (threadIdx.x - WORKERS) / 32 * WIDE_COPY_ROWS;
+        const bool vec = D % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)k & 15) == 0 &&
+                         (!VEC || (gate_stride % 4 == 0 && ((uintptr_t)gate & 15) == 0));
+        const bool vec_v = V % 4 == 0 && v_stride % 4 == 0 && ((uintptr_t)v & 15) == 0 && first_col + COLS <= V;
+        const size_t row0 = (size_t)(a0 + first);
+        const int hq = h / (heads / qk_heads);
+        const float* src[3] = {q + row0 * q_stride + (size_t)hq * D, k + row0 * k_stride + (size_t)hq * D,
+                               VEC ? gate + row0 * gate_stride + (size_t)h * D : nullptr};
+        const int strides[3] = {q_stride, k_stride, gate_stride};
+        const float* src_v = v + row0 * v_stride + (size_t)h * V;
+        const float* src_gate = MODE == M_DELTA || MODE == M_SCALED ? gate + row0 * gate_stride + h : nullptr;
+        const float* src_beta = has_beta(MODE) ? beta + row0 * beta_stride + h : nullptr;
+        auto issue = [&](int chunk, float* buf) {
+            const int rows = min(WIDE_COPY_ROWS, n - chunk * WIDE_CH - first);      // negative where the last chunk ends before this warp's rows
+            buf += first * row_floats;
+            const size_t t0 = (size_t)chunk * WIDE_CH;
 #pragma unroll
-                for (int i = 0; i < WIDE_SUMS; ++i) {
+            for (int w = 0; w < NV; ++w) {
+                const float* from = src[w] + t0 * strides[w];
 #pragma unroll
-                    for (int w = 0; w < CPW; ++w) acc[i * CPW + w] = 0.0f;
-                    if (!whole.value && t0 + i >= rows) continue;
-                    const float* rowp = buf + (size_t)(t0 + i) * row_floats;
-                    float kk[PER], qq[PER], gg[PER];
-                    read_run<PER>(rowp, lane, qq);
-                    read_run<PER>(rowp + Dp, lane, kk);
-                    if (VEC) read_run<PER>(rowp + 2 * Dp, lane, gg);
-                    float u[CPW];
+                for (int t = 0; t < WIDE_COPY_ROWS; ++t) {
+                    if (t >= rows) break;
+                    float* to = buf + t * row_floats + w * Dp;
+                    if (vec) {
 #pragma unroll
-                    for (int w = 0; w < CPW; ++w) u[w] = rowp[NV * Dp + warp * CPW + w];
-                    const float a = MODE == M_SCALED ? rowp[NV * Dp + WIDE_COLS] : dec;
-                    if (MODE == M_SCALED) {
-                        const float bt = rowp[NV * Dp + WIDE_COLS + 1];
+                        for (int e = 0; e < Dp; e += 128)
+                            if (e + 4 * lane < D) cp_async_16f(to + e + 4 * lane, from + e + 4 * lane);
+                    } else {
+                        for (int e = lane; e < D; e += 32) cp_async_4(to + e, from + e);
+                    }
+                    from += strides[w];
+                }
+            }
+            const float* from = src_v + t0 * v_stride;
+            if (vec_v) {
+                constexpr int PIECES = COLS / 4;     // of a row: 32 lanes have four rows' at once
+                static_assert(WIDE_COPY_ROWS * PIECES <= 32, "a lane a piece");
+                const int t = lane / PIECES, e = 4 * (lane % PIECES);
+                if (t < rows) cp_async_16f(buf + t * row_floats + NV * Dp + e, from + (size_t)t * v_stride + first_col + e);
+            } else {
+                for (int i = lane; i < WIDE_COPY_ROWS * COLS; i += 32)
+                    if (i / COLS < rows)
+                        cp_async_4(buf + i / COLS * row_floats + NV * Dp + i % COLS, from + (size_t)(i / COLS) * v_stride + min(first_col + i % COLS, V - 1));
+            }
+            if (src_gate != nullptr && lane < rows) cp_async_4(buf + lane * row_floats + NV * Dp + COLS, src_gate + (t0 + lane) * gate_stride);
+            if (src_beta != nullptr && lane >= 16 && lane - 16 < rows)
+                cp_async_4(buf + (lane - 16) * row_floats + NV * Dp + COLS + 1, src_beta + (t0 + lane - 16) * beta_stride);
+        };
+        for (int c = 0; c < stages - 1; ++c) {
+            if (c < chunks) issue(c, stage + (size_t)c * stage_floats);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        int at = 0;                                  // c % stages
+        for (int c = 0; c < chunks; ++c) {
+            if (stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();                            // this warp's rows of chunk c have landed
+            float* buf = stage + (size_t)at * stage_floats;
+            if constexpr (CORRECTED && BLK == 4) {
+                // k_t . k_s for s < t, with channel decays (k_t g_t .. g_{s+1}) . k_s.  Rows that a last chunk does not have
+                // give numbers that nobody reads.
+                static_assert(WIDE_COPY_ROWS == BLK, "a copying warp's rows are the rows taken together");
+                float g[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                        for (int w = 0; w < CPW; ++w) u[w] *= bt;
+                for (int e = 0; e < Dp; e += 128) {
+                    const int d = e + 4 * lane;
+                    if (d >= Dp) continue;
+                    const float* rowp = buf + first * row_floats + d;
+                    float4 kr[4], gr[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        kr[t] = *reinterpret_cast<const float4*>(rowp + t * row_floats + Dp);
+                        if (VEC) gr[t] = *reinterpret_cast<const float4*>(rowp + t * row_floats + 2 * Dp);
                     }
 #pragma unroll
-                    for (int d = 0; d < PER; ++d)
+                    for (int t = 1; t < 4; ++t) {
+                        float4 w = kr[t];
 #pragma unroll
-                        for (int w = 0; w < CPW; ++w) {
-                            S[w][d] = fmaf(VEC ? gg[d] : a, S[w][d], kk[d] * u[w]);
-                            acc[i * CPW + w] = fmaf(S[w][d], qq[d], acc[i * CPW + w]);
+                        for (int s = 2; s >= 0; --s) {
+                            if (s >= t) continue;
+                            if (VEC) w.x *= gr[s + 1].x, w.y *= gr[s + 1].y, w.z *= gr[s + 1].z, w.w *= gr[s + 1].w;
+                            float& sum = g[t * (t - 1) / 2 + s];
+                            sum = fmaf(w.x, kr[s].x, fmaf(w.y, kr[s].y, fmaf(w.z, kr[s].z, fmaf(w.w, kr[s].w, sum))));
                         }
+                    }
                 }
-                // At each step a lane gives half of the sums it holds to its partner and takes the partner's share of the other
-                // half; when one is left, the lanes that hold the same one add theirs up.
-                int held = WIDE_SUMS * CPW, index = 0;
+                // Sums over the lanes: each gives half of the sums it holds to its partner and takes the partner's share of the
+                // other half until one is left; the lanes that hold the same one add theirs up.
+                int index = 0;
 #pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) {
+                for (int o = 16, held = 8; o >= 1; o >>= 1) {
                     if (held == 1) {
-                        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+                        g[0] += __shfl_xor_sync(0xffffffffu, g[0], o);
                         continue;
                     }
                     held >>= 1;
                     const bool high = lane & o;
                     if (high) index += held;
 #pragma unroll
-                    for (int i = 0; i < WIDE_SUMS * CPW / 2; ++i) {
+                    for (int i = 0; i < 4; ++i) {
                         if (i >= held) continue;
-                        const float keep = high ? acc[i + held] : acc[i], give = high ? acc[i] : acc[i + held];
-                        acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                        const float keep = high ? g[i + held] : g[i], give = high ? g[i] : g[i + held];
+                        g[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                     }
                 }
-                const int t = t0 + index / CPW, w = index % CPW;
-                if (lane % (32 / (WIDE_SUMS * CPW)) == 0 && t < rows && col + w < V) {
-                    float sum = acc[0];
-                    if (MODE == M_SCALED) sum = fmaf(sk, buf[(size_t)t * row_floats + NV * Dp + warp * CPW + w], sum);
-                    out[(size_t)(a0 + c * WIDE_CH + t) * ((size_t)heads * V) + (size_t)h * V + col + w] = sum;
-                }
-            };
-            for (int t0 = 0; t0 < rows; t0 += WIDE_SUMS) {
-                if (t0 + WIDE_SUMS <= rows) group(t0, std::true_type{});
-                else group(t0, std::false_type{});
+                if (lane % 4 == 0) buf[WIDE_CH * row_floats + 2 * first + index] = g[0];
             }
-        } else {
-            for (int t = 0; t < rows; ++t) {
-                const float* rowp = buf + (size_t)t * row_floats;
-                float kk[PER], qq[PER];
-                read_run<PER>(rowp, lane, qq);
-                read_run<PER>(rowp + Dp, lane, kk);
-                float u = rowp[NV * Dp + warp];
-                const float a = VEC ? 1.0f : rowp[NV * Dp + WIDE_COLS];
-                if (VEC) {
-                    float gg[PER];
-                    read_run<PER>(rowp + 2 * Dp, lane, gg);
-#pragma unroll
-                    for (int i = 0; i < PER; ++i) S[0][i] *= gg[i];     // past D everything is zero and stays so
-                }
-                float dot = 0.0f;
-#pragma unroll
-                for (int i = 0; i < PER; ++i) dot = fmaf(S[0][i], kk[i], dot);
-                dot = warp_sum(dot);
-                u = rowp[NV * Dp + WIDE_COLS + 1] * (u - a * dot);
-                float acc = 0.0f;
-#pragma unroll
-                for (int i = 0; i < PER; ++i) {
-                    S[0][i] = fmaf(a, S[0][i], kk[i] * u);
-                    acc = fmaf(S[0][i], qq[i], acc);
-                }
-                acc = warp_sum(acc);
-                if (col < V && lane == 0) out[(size_t)(a0 + c * WIDE_CH + t) * ((size_t)heads * V) + (size_t)h * V + col] = acc;
+            __threadfence_block();
+            barrier_arrive(FULL + at, THREADS);
+            const int next = c + stages - 1, next_at = at == 0 ? stages - 1 : at - 1;      // next % stages
+            if (next < chunks) {
+                if (c > 0) barrier_sync(EMPTY + next_at, THREADS);        // the workers have left chunk c - 1
+                issue(next, stage + (size_t)next_at * stage_floats);
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            at = at + 1 == stages ? 0 : at + 1;
+        }
+        return;
+    }
+
+    // ---- the workers
+    const int sub = threadIdx.x % LANES, mine = threadIdx.x / LANES * CPL;      // the group's first column in the block
+    const int col = first_col + mine;                // columns past V shadow the last one and store nothing
+    f32x2 S[CPL][P2];
+#pragma unroll
+    for (int w = 0; w < CPL; ++w) {
+        const bool fresh = history[r] == 0;
+        const float* from = state + (size_t)slot_in[r] * slot_floats + ((size_t)h * V + min(col + w, V - 1)) * D;
+#pragma unroll
+        for (int i = 0; i < P2; ++i) {
+            const int d = 4 * (sub + LANES * (i / 2)) + 2 * (i % 2);
+            S[w][i] = pair(!fresh && d < D ? from[d] : 0.0f, !fresh && d + 1 < D ? from[d + 1] : 0.0f);
         }
     }
+    const float dec = MODE == M_CONST ? decay[h] : 1.0f;
+    const float sk = MODE == M_SCALED && skip != nullptr ? skip[h] : 0.0f;
+    for (int c = 0, at = 0; c < chunks; ++c, at = at + 1 == stages ? 0 : at + 1) {
+        const float* buf = stage + (size_t)at * stage_floats;
+        const int rows = min(WIDE_CH, n - c * WIDE_CH);
+        barrier_sync(FULL + at, THREADS);
+        // N rows from t0 on, their corrections together; leaves the lane's shares of the read-outs in acc.
+        auto take = [&](int t0, auto count, float* acc) {
+            constexpr int N = decltype(count)::value;
+            const float* rowp = buf + (size_t)t0 * row_floats;
+            f32x2 kk[N][P2], gg[VEC ? N : 1][P2];
+            float u[N][CPL], a[N];
 #pragma unroll
-    for (int w = 0; w < CPW; ++w) {
+            for (int i = 0; i < N; ++i) {
+                read_share<PER, LANES>(rowp + i * row_floats + Dp, sub, kk[i]);
+                if constexpr (VEC) read_share<PER, LANES>(rowp + i * row_floats + 2 * Dp, sub, gg[i]);
+                const float* smalls = rowp + i * row_floats + NV * Dp;
+                a[i] = MODE == M_DELTA || MODE == M_SCALED ? smalls[COLS] : dec;
+                if constexpr (!CORRECTED)
+#pragma unroll
+                    for (int w = 0; w < CPL; ++w) u[i][w] = MODE == M_SCALED ? smalls[COLS + 1] * smalls[mine + w] : smalls[mine + w];
+            }
+            if constexpr (CORRECTED) {
+                static_assert(CPL <= 2, "a half of the group a column");
+                float x[N][CPL];
+#pragma unroll
+                for (int w = 0; w < CPL; ++w) {
+                    f32x2 decayed[P2];                   // channel decays: the state before the rows, decayed up to row i
+#pragma unroll
+                    for (int d = 0; d < P2; ++d) decayed[d] = S[w][d];
+#pragma unroll
+                    for (int i = 0; i < N; ++i) {
+                        if constexpr (VEC)
+#pragma unroll
+                            for (int d = 0; d < P2; ++d) decayed[d] = mul2(decayed[d], gg[i][d]);    // past D everything is zero and stays so
+                        x[i][w] = share_dot(decayed, kk[i]);
+                    }
+                }
+                // The sums over the group's lanes; with two columns each half of the lanes ends with one column's.
+                const bool second = CPL == 2 && (sub & (LANES / 2));
+                float own[N];
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    own[i] = x[i][0];
+                    if constexpr (CPL == 2) {
+                        const float give = second ? x[i][0] : x[i][1];
+                        own[i] = (second ? x[i][1] : x[i][0]) + __shfl_xor_sync(0xffffffffu, give, LANES / 2);
+                    }
+                }
+#pragma unroll
+                for (int o = LANES / CPL / 2; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < N; ++i) own[i] += __shfl_xor_sync(0xffffffffu, own[i], o);
+                const float* gram = buf + WIDE_CH * row_floats + 2 * t0;
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    const float* smalls = rowp + i * row_floats + NV * Dp;
+                    float y = own[i];
+#pragma unroll
+                    for (int j = 0; j < i; ++j) y = fmaf(gram[i * (i - 1) / 2 + j], own[j], VEC ? y : a[j] * y);
+                    own[i] = smalls[COLS + 1] * (smalls[mine + (second ? 1 : 0)] - a[i] * y);          // u_i from here on
+                }
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    u[i][0] = own[i];
+                    if constexpr (CPL == 2) {
+                        const float other = __shfl_xor_sync(0xffffffffu, own[i], LANES / 2);
+                        u[i][0] = second ? other : own[i];
+                        u[i][1] = second ? own[i] : other;
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const f32x2 a2 = pair(a[i], a[i]);
+                f32x2 qq[P2];
+                read_share<PER, LANES>(rowp + i * row_floats, sub, qq);
+#pragma unroll
+                for (int w = 0; w < CPL; ++w) {
+                    const f32x2 u2 = pair(u[i][w], u[i][w]);
+#pragma unroll
+                    for (int d = 0; d < P2; ++d) S[w][d] = fma2(VEC ? gg[VEC ? i : 0][d] : a2, S[w][d], mul2(kk[i][d], u2));
+                    acc[i * CPL + w] = share_dot(S[w], qq);
+                }
+            }
+        };
+        auto store = [&](int t, int w, float sum) {
+            if (MODE == M_SCALED) sum = fmaf(sk, buf[(size_t)t * row_floats + NV * Dp + mine + w], sum);
+            if (col + w < V) out[(size_t)(a0 + c * WIDE_CH + t) * ((size_t)heads * V) + (size_t)h * V + col + w] = sum;
+        };
+        int t0 = 0;
+        for (; t0 + WIDE_SUMS <= rows; t0 += WIDE_SUMS) {
+            constexpr int SUMS = WIDE_SUMS * CPL;        // [row][column]
+            static_assert(SUMS <= LANES, "a lane a sum");
+            float acc[SUMS];
+#pragma unroll
+            for (int i = 0; i < WIDE_SUMS; i += BLK) take(t0 + i, std::integral_constant<int, BLK>{}, acc + i * CPL);
+            // At each step a lane gives half of the sums it holds to its partner and takes the partner's share of the other
+            // half; when one is left, the lanes that hold the same one add theirs up.
+            int held = SUMS, index = 0;
+#pragma unroll
+            for (int o = LANES / 2; o >= 1; o >>= 1) {
+                if (held == 1) {
+                    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+                    continue;
+                }
+                held >>= 1;
+                const bool high = sub & o;
+                if (high) index += held;
+#pragma unroll
+                for (int i = 0; i < SUMS / 2; ++i) {
+                    if (i >= held) continue;
+                    const float keep = high ? acc[i + held] : acc[i], give = high ? acc[i] : acc[i + held];
+                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            }
+            if (sub % (LANES / SUMS) == 0) store(t0 + index / CPL, index % CPL, acc[0]);
+        }
+        for (; t0 < rows; ++t0) {                    // a request's last rows, one by one
+            float acc[CPL];
+            take(t0, std::integral_constant<int, 1>{}, acc);
+#pragma unroll
+            for (int w = 0; w < CPL; ++w) {
+#pragma unroll
+                for (int o = LANES / 2; o >= 1; o >>= 1) acc[w] += __shfl_xor_sync(0xffffffffu, acc[w], o);
+                if (sub == 0) store(t0, w, acc[w]);
+            }
+        }
+        if (c + stages < chunks) barrier_arrive(EMPTY + at, THREADS);
+    }
+#pragma unroll
+    for (int w = 0; w < CPL; ++w) {
         if (col + w >= V) continue;
-        float* sout = state + (size_t)slot_out[r] * slot_floats + ((size_t)h * V + col + w) * D;
+        float* to = state + (size_t)slot_out[r] * slot_floats + ((size_t)h * V + col + w) * D;
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            const int d = lane * PER + i;
-            if (d < D) sout[d] = S[w][i];
+        for (int i = 0; i < P2; ++i) {
+            const int d = 4 * (sub + LANES * (i / 2)) + 2 * (i % 2);
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(S[w][i]));
+            if (d < D) to[d] = lo;
+            if (d + 1 < D) to[d + 1] = hi;
         }
     }
 }
@@ -534,24 +702,39 @@ int launch_recurrence(int D, bool wide, int requests, cudaStream_t stream, const
         return launch_status();                                                                                           \
     } while (0)
     if (wide) {
-#define LLMX_WIDE(P)                                                                                                      \
+#define LLMX_WIDE_COLS(P, L, W, C)                                                                                                \
     do {                                                                                                                  \
-        const long long by = (long long)heads * ((V + WIDE_COLS - 1) / WIDE_COLS);                                        \
+        const long long by = (long long)heads * ((V + C - 1) / C);                                                        \
         if (by > 65535) return LLMX_ERR_UNSUPPORTED;                                                                      \
-        const size_t smem = (size_t)2 * WIDE_CH * ((has_channel_gate(MODE) ? 3 : 2) * P * 32 + WIDE_COLS + 4) * sizeof(float);   \
+        const size_t buffer = ((size_t)WIDE_CH * ((has_channel_gate(MODE) ? 3 : 2) * P * L + C + 4) + WIDE_GRAM) * sizeof(float); \
+        const int stages = 3 * buffer <= 200 * 1024 ? 3 : 2;                                                              \
+        const size_t smem = stages * buffer;                                                                              \
         if (smem > 200 * 1024) return LLMX_ERR_UNSUPPORTED;                                                               \
         if (smem > 48 * 1024)                                                                                             \
-            cudaFuncSetAttribute(recurrence_wide_kernel<P, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        launch_kernel(recurrence_wide_kernel<P, MODE>, dim3(requests, (unsigned)by), dim3(wide_threads(MODE)), smem, stream, q, \
-                      k, v, q_stride, k_stride, v_stride, decay, gate, beta, gate_stride, beta_stride, skip, state,      \
-                      slot_floats, row_start, row_count, history, slot_in, slot_out, out, heads, qk_heads, D, V);       \
+            cudaFuncSetAttribute(recurrence_wide_kernel<P, L, W, C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        launch_kernel(recurrence_wide_kernel<P, L, W, C, MODE>, dim3(requests, (unsigned)by), dim3(C / W * L + 32 * WIDE_COPY_WARPS), \
+                      smem, stream, q, k, v, q_stride, k_stride, v_stride, decay, gate, beta, gate_stride, beta_stride, skip, state, \
+                      slot_floats, row_start, row_count, history, slot_in, slot_out, out, heads, qk_heads, D, V, stages); \
         return launch_status();                                                                                           \
     } while (0)
-        if (D <= 32) LLMX_WIDE(1);
-        if (D <= 64) LLMX_WIDE(2);
-        if (D <= 128) LLMX_WIDE(4);
-        if (D <= 256) LLMX_WIDE(8);
-        if (D <= 512) LLMX_WIDE(16);
+        // 32 columns a block (its rows are copied half as often) once blocks of 16 would be more than the 148 SMs take at once.
+#define LLMX_WIDE(P, L, W)                                                                                                \
+    do {                                                                                                                  \
+        if ((long long)requests * heads * ((V + 15) / 16) > 148) LLMX_WIDE_COLS(P, L, W, 32);                             \
+        LLMX_WIDE_COLS(P, L, W, 16);                                                                                      \
+    } while (0)
+        // Values a lane, lanes, columns a group: without a correction more lanes and columns (nothing waits for the sums).
+        constexpr bool corrected = MODE == M_DELTA || MODE == M_DELTA_VEC;
+        if (D <= 32) LLMX_WIDE(4, 8, 1);
+        if (D <= 64) LLMX_WIDE(4, 16, 2);
+        if (D <= 128) {
+            if constexpr (corrected) LLMX_WIDE(8, 16, 2);
+            else LLMX_WIDE(4, 32, 4);
+        }
+        if (D <= 256) LLMX_WIDE_COLS(8, 32, 2, 16);
+        if (D <= 512) LLMX_WIDE_COLS(16, 32, 1, 16);
+#undef LLMX_WIDE_COLS
+#undef LLMX_WIDE_COLS
 #undef LLMX_WIDE
     } else {
         if (D <= 16) LLMX_REC(2, 8);

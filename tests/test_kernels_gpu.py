@@ -797,3 +797,64 @@ def test_latent_prompt_equals_the_general_form(name, heads, rot, latent, window,
         for how, got in (("many rows", out), ("general", general)):
             worst = ((got[r].double() - want).abs() / bound).max()
             assert worst <= 1.0, (how, r, p, float(worst))
+
+
+# ---- matrix-state recurrences over long runs of rows ----------------------------------------------------------------------------
+@pytest.mark.parametrize("mode", ["constant", "delta", "scaled", "delta_channels", "channels"])
+@pytest.mark.parametrize("heads,qk_heads,D,V,counts", [
+    (2, 1, 4, 1, [9, 1]), (3, 3, 32, 17, [16, 23]), (4, 2, 36, 33, [40]), (2, 2, 64, 15, [31, 12, 64]), (40, 20, 64, 64, [17]), (1, 1, 66, 7, [25]),
+    (2, 1, 128, 16, [33, 8]), (20, 10, 128, 130, [21, 48]), (1, 1, 130, 20, [18]), (2, 1, 256, 40, [35]), (1, 1, 512, 9, [20])])
+def test_recurrence_over_many_rows(mode, heads, qk_heads, D, V, counts):
+    """The wide form against the recurrence in 64 bits, from a state and from nothing: vector widths on both sides of every
+    lane layout, columns that do not fill a block, 16 and 32 columns a block, runs that end within a chunk, a group of eight
+    and a group of four rows.  32-bit sums of D terms and decays below one: an error of a few times sqrt(D) 2^-24 of the
+    largest result."""
+    import types
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(D + V)
+    rows, R = sum(counts), len(counts)
+    unit = lambda: torch.nn.functional.normalize(torch.randn(rows, qk_heads, D, generator=g), dim=-1)
+    # q, k and v inside one wider matrix, as the projections hold them.
+    wide = torch.cat([unit().reshape(rows, -1), unit().reshape(rows, -1), torch.randn(rows, heads * V, generator=g)], 1).to(DEV)
+    qk = qk_heads * D
+    q, k, v = wide[:, :qk], wide[:, qk:2 * qk], wide[:, 2 * qk:]
+    per = D if mode in ("delta_channels", "channels") else 1
+    gate = (0.7 + 0.3 * torch.rand(rows, heads * per, generator=g)).to(DEV)
+    beta, skip = torch.rand(rows, heads, generator=g).to(DEV), torch.randn(heads, generator=g).to(DEV)
+    decay = (0.9 + 0.1 * torch.rand(heads, generator=g)).to(DEV)
+    state = torch.randn(2 * R + 1, heads, V, D, generator=g).to(DEV)
+    history = [0 if r == 1 else 5 for r in range(R)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    step = types.SimpleNamespace(row_start=i32([sum(counts[:r]) for r in range(R)]), row_count=i32(counts), history=i32(history),
+                                 state_slots=i32(list(range(R))), state_slots_out=i32([R + 1 + r for r in range(R)]), requests=R,
+                                 max_row_count=max(counts), rows=rows)
+    before = state.double().clone()
+    out = torch.full((rows, heads * V), 7.0, device=DEV)
+    code = ["constant", "delta", "scaled", "delta_channels", "channels"].index(mode)
+    fn, P = ops._fn("recurrence", "llmx_linear_recurrence"), ops._ptr
+    ops._check(fn(P(q), P(k), P(v), q.stride(0), k.stride(0), v.stride(0), code, P(decay), P(gate), P(beta), gate.stride(0), beta.stride(0),
+                  P(skip) if mode == "scaled" else None, P(state), heads * V * D, P(step.row_start), P(step.row_count), P(step.history),
+                  P(step.state_slots), P(step.state_slots_out), P(out), R, heads, qk_heads, D, V, max(counts), ops._stream()), "recurrence")
+    share = heads // qk_heads
+    at = 0
+    for r, n in enumerate(counts):
+        S = torch.zeros_like(before[r]) if history[r] == 0 else before[r].clone()          # [heads, V, D]
+        want = []
+        for t in range(at, at + n):
+            kt, qt = (x[t].double().view(qk_heads, D).repeat_interleave(share, 0) for x in (k, q))
+            vt, gt, bt = v[t].double().view(heads, V), gate[t].double().view(heads, 1, per), beta[t].double().view(heads, 1)
+            S = S * (decay.double().view(heads, 1, 1) if mode == "constant" else gt)
+            u = vt
+            if mode in ("delta", "delta_channels"):
+                u = bt * (vt - torch.einsum("hvd,hd->hv", S, kt))
+            if mode == "scaled":
+                u = bt * vt
+            S = S + u[:, :, None] * kt[:, None, :]
+            o = torch.einsum("hvd,hd->hv", S, qt)
+            want.append((o + skip.double().view(heads, 1) * vt if mode == "scaled" else o).reshape(-1))
+        want = torch.stack(want)
+        bound = 8 * D ** 0.5 * 2.0 ** -24
+        assert (out[at:at + n].double() - want).abs().max() <= bound * max(1.0, float(want.abs().max())), (r, "rows")
+        assert (state[R + 1 + r].double() - S).abs().max() <= bound * max(1.0, float(S.abs().max())), (r, "state")
+        at += n
+    assert torch.equal(state[:R + 1].double(), before[:R + 1])
