@@ -16,10 +16,10 @@
 // The products run one block a (tile of an expert's pairs, tile of output columns): rows are gathered through the
 // list, the expert's weights are read once a tile.  Two forms: on the CUDA cores with explicit fmaf and k in
 // increasing order (32-bit weights and rows: the true 32-bit path; also bfloat16 shapes the tensor-core form does not
-// take), and on the tensor cores (mma.sync m16n8k16, bfloat16 in, 32-bit sums) for bfloat16 with K a multiple of 32.
+// take), and on the tensor cores (tcgen05.mma, bfloat16 in, 32-bit sums) for bfloat16 with K a multiple of 32.
 // A third form serves steps of a few pairs (decoding), where the products are the experts' weights streamed once.
 // The CUDA-core form checks its tiles' size against what the routing wrote (tiles[1]).
-#include "common.cuh"
+#include "tc_common.cuh"
 #include <math.h>
 
 namespace {
@@ -160,148 +160,183 @@ moe_cores_kernel(const T* __restrict__ a, int a_div, const T* __restrict__ w, co
 }
 
 // ---- the product on the tensor cores -------------------------------------------------------------------------------
-// A block of eight warps: a tile of 128 pairs (the routing cut the lists into tiles of 128 for this form) x 128 weight
-// rows, K in steps of 32 through four stages of cp.async copies (16-byte pieces; rows that do not exist are filled with
-// zeros by the copy itself).  The 128 weight rows are two halves of 64: gated, the gate rows and the up rows of the
-// same 64 output columns, so that a thread holds both of an output and writes the gated unit; else 128 output columns.
-// The weights are the A operand of mma.sync m16n8k16 and the gathered rows the B operand, both read by ldmatrix from
-// rows padded by 8 values (no two of a read's eight rows in one bank).  Warp (wm, wn), wm < 4, wn < 2: weight rows
-// 16 wm .. of both halves x pairs 64 wn .. 64 wn + 63.
-constexpr int TC_ROWS = 128, TC_HALF = 64, TC_K = 32, TC_PAD = 8, TC_STAGES = 4, TC_LD = TC_K + TC_PAD;
-constexpr int TC_STAGE_ELEMS = (2 * TC_HALF + TC_ROWS) * TC_LD;
-constexpr size_t TC_SMEM = (size_t)TC_STAGES * TC_STAGE_ELEMS * 2;
+// A block: a tile of up to 256 of an expert's pairs x 256 weight rows, as tcgen05.mma with the weights as the A operand
+// (M = 128, twice) and the gathered rows as B (N = the tile's pairs, rounded up to 16).  The two halves of 128 weight rows
+// are, gated, the gate rows and the up rows of the same 128 output columns, so that a thread holds both of an output and
+// writes the gated unit; else 256 output columns.  The halves' sums fill tensor memory (2 x 256 columns).
+//   warp 0       the weights: K in steps of 64 through three stages, two TMA boxes a step
+//   warp 1       the products, issued by one thread
+//   warps 2-9    the pairs' rows of a step, gathered by cp.async in pieces of 16 bytes laid out as the 128-byte swizzle wants
+//                them (a TMA gather of four rows an instruction took three times as long as the products); then the epilogue: a
+//                thread has an output column (of each half) and half of the pairs, so that a warp writes 32 neighbouring
+//                columns of a pair at a time
+// An expert's list is cut into ceil(pairs / 256) equal tiles: its weights are read that often, and no tile is left with a few
+// pairs.  Of the routing's tiles of 128 pairs the expert's first ones stand for these, the others' blocks return.  Tiles are
+// the grid's fast dimension, so tiles of one expert read the same weights at the same time.
+// 2,048 rows x 2 of 16 experts, 2,048 -> 2 x 1,536 and back: 259 -> 134 us and 141 -> 73 us against the same tiles on
+// mma.sync; 1,201 rows x 2 of 16, 4,096 -> 2 x 3,072 and back: 718 -> 253 us and 374 -> 121 us, where reading the weights
+// once takes 123 and 62 us: bound by how soon a step's rows and weights arrive (three stages in flight) and by the last
+// wave's blocks.
+constexpr int TC_LIST_TILE = 128;                                            // pairs a tile of the routing holds for this form
+constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_STAGES = 3;
+constexpr int TC_W_BYTES = TC_M * TC_K * 2;                                  // one half's weights of a stage
+constexpr int TC_STAGE_BYTES = 2 * TC_W_BYTES + TC_ROWS * TC_K * 2;
+constexpr int TC_ROW_WARPS = 8, TC_THREADS = 64 + TC_ROW_WARPS * 32;
+constexpr size_t TC_SMEM = (size_t)TC_STAGES * TC_STAGE_BYTES + 1024;
+enum : int { ERR_MOE_PRODUCER = 441, ERR_MOE_MMA = 442, ERR_MOE_EPILOGUE = 443 };
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ void cp_async_16_or_zeros(void* dst, const void* src, bool real) {
+__device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst, const void* src, bool real) {
     const int bytes = real ? 16 : 0;                 // fewer source bytes than 16: the rest of the piece is zeros
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
 template <bool GATED, typename OutT>
-__global__ void __launch_bounds__(256)
-moe_tc_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv_bfloat16* __restrict__ w,
+__global__ void __launch_bounds__(TC_THREADS, 1)
+moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUtensorMap w_map, int a_div,
               const int* __restrict__ lists, const int* __restrict__ counts, const int* __restrict__ tiles, int pairs,
-              OutT* __restrict__ out, int N, int K, Glu glu) {
-    pdl_trigger();
+              OutT* __restrict__ out, int N, int K, Glu glu, int* error_word) {
     pdl_wait();
-    if ((int)blockIdx.x >= tiles[0] || tiles[1] != TC_ROWS) return;
-    extern __shared__ __align__(16) unsigned char tc_smem[];
-    __nv_bfloat16* stages = reinterpret_cast<__nv_bfloat16*>(tc_smem);
+    if ((int)blockIdx.x >= tiles[0] || tiles[1] != TC_LIST_TILE) return;
+    const int e = tiles[2 + 2 * blockIdx.x], count = counts[e];
+    const int parts = (count + TC_ROWS - 1) / TC_ROWS, part = tiles[3 + 2 * blockIdx.x] / TC_LIST_TILE;
+    if (part >= parts) return;
+    // Equal parts, multiples of 16 of at most 256 pairs: the last one is never empty, (parts - 1) * 256 being below the count.
+    const int step = ((count + parts - 1) / parts + 15) & ~15, at = part * step;
+    extern __shared__ uint8_t tc_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full[TC_STAGES], empty[TC_STAGES], done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_word;
     __shared__ int src_pair[TC_ROWS];
-    const int e = tiles[2 + 2 * blockIdx.x], at = tiles[3 + 2 * blockIdx.x];
-    const int n_here = min(TC_ROWS, counts[e] - at);
-    const int* list = lists + (size_t)e * pairs + at;
-    if (threadIdx.x < TC_ROWS) src_pair[threadIdx.x] = (int)threadIdx.x < n_here ? list[threadIdx.x] : -1;
-    __syncthreads();
-    const int out_cols = GATED ? TC_HALF : 2 * TC_HALF;           // output columns a block makes
-    const int col0 = blockIdx.y * out_cols;
-    const __nv_bfloat16* wbase = w + (size_t)e * (GATED ? 2 : 1) * N * K;
-    // What this thread copies a stage: pieces t and t + 256 of the weights (row piece / 4, 8 values at 8 * (piece % 4)),
-    // and the same of the gathered rows.  The rows' addresses do not change from stage to stage.
-    const __nv_bfloat16* wsrc[2];
-    const __nv_bfloat16* bsrc[2];
-    bool wreal[2], breal[2];
-    int dst_off[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int piece = threadIdx.x + 256 * i;
-        const int row = piece >> 2, kp = piece & 3;
-        const int half = row >> 6, rr = row & 63;
-        const int col = col0 + (GATED ? rr : row);                // the output column this weight row belongs to
-        wreal[i] = col < N;
-        const size_t wrow = GATED ? (size_t)half * N + col : (size_t)col;
-        wsrc[i] = wreal[i] ? wbase + wrow * K + 8 * kp : wbase;
-        const int p = src_pair[row];
-        breal[i] = p >= 0;
-        bsrc[i] = breal[i] ? a + (size_t)(p / a_div) * K + 8 * kp : a;
-        dst_off[i] = row * TC_LD + 8 * kp;
-    }
-    auto load = [&](int kt, int stage) {
-        __nv_bfloat16* ws = stages + (size_t)stage * TC_STAGE_ELEMS;
-        __nv_bfloat16* bs = ws + 2 * TC_HALF * TC_LD;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            cp_async_16_or_zeros(ws + dst_off[i], wsrc[i] + (size_t)kt * TC_K, wreal[i]);
-            cp_async_16_or_zeros(bs + dst_off[i], bsrc[i] + (size_t)kt * TC_K, breal[i]);
-        }
-    };
+    volatile int* abort_flag = &abort_word;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = warp & 3, wn = warp >> 2;
-    const int gid = lane >> 2, tig = lane & 3;
-    float acc[2][8][4];
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int t = 0; t < 8; ++t) acc[h][t][0] = acc[h][t][1] = acc[h][t][2] = acc[h][t][3] = 0.0f;
-    const int KT = K / TC_K;
-#pragma unroll
-    for (int s = 0; s < TC_STAGES - 1; ++s) {
-        if (s < KT) load(s, s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    // ldmatrix addresses inside a stage: A (weights): row lane % 16, k offset 8 * (lane / 16); B (pairs): two tiles of 8
-    // pairs a read: pair (lane % 8) + 8 * (lane / 16), k offset 8 * ((lane / 8) % 2).
-    const int a_row = lane & 15, a_k = (lane >> 4) * 8;
-    const int b_row = (lane & 7) + ((lane >> 4) << 3), b_k = ((lane >> 3) & 1) * 8;
-    for (int kt = 0; kt < KT; ++kt) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(TC_STAGES - 2) : "memory");
-        __syncthreads();                             // stage kt has landed; everyone has left the stage that is filled next
-        if (kt + TC_STAGES - 1 < KT) load(kt + TC_STAGES - 1, (kt + TC_STAGES - 1) % TC_STAGES);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const __nv_bfloat16* ws = stages + (size_t)(kt % TC_STAGES) * TC_STAGE_ELEMS;
-        const __nv_bfloat16* bs = ws + 2 * TC_HALF * TC_LD;
-#pragma unroll
-        for (int ks = 0; ks < TC_K; ks += 16) {
-            uint32_t af[2][4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const __nv_bfloat16* p = ws + (size_t)(h * TC_HALF + 16 * wm + a_row) * TC_LD + ks + a_k;
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(af[h][0]), "=r"(af[h][1]), "=r"(af[h][2]), "=r"(af[h][3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
-            }
-            // All of the step's fragments are asked for before the first product, so that the reads overlap the products
-            // of the step before (the statements keep their order; a warp's products do not wait for one another).
-            uint32_t b[4][4];
-#pragma unroll
-            for (int t2 = 0; t2 < 4; ++t2) {
-                const __nv_bfloat16* p = bs + (size_t)(64 * wn + 16 * t2 + b_row) * TC_LD + ks + b_k;
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(b[t2][0]), "=r"(b[t2][1]), "=r"(b[t2][2]), "=r"(b[t2][3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
-            }
-#pragma unroll
-            for (int t2 = 0; t2 < 4; ++t2)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    mma_bf16(acc[h][2 * t2], af[h], b[t2][0], b[t2][1]);
-                    mma_bf16(acc[h][2 * t2 + 1], af[h], b[t2][2], b[t2][3]);
-                }
+    const int n_here = min(step, count - at);
+    const int n16 = (n_here + 15) & ~15;
+    const int* list = lists + (size_t)e * pairs + at;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < TC_STAGES; ++i) {
+            tc::mbar_init(&full[i], 1 + TC_ROW_WARPS);
+            tc::mbar_init(&empty[i], 1);
         }
+        tc::mbar_init(&done, 1);
+        abort_word = 0;
+        tc::fence_barrier_init();
+        tc::tma_prefetch_desc(&w_map);
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // d[0], d[1]: weight row 16 wm + gid of a half, pairs 64 wn + 8 t + 2 tig, + 1;  d[2], d[3]: weight row + 8.
-#pragma unroll
-    for (int t = 0; t < 8; ++t)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int p = src_pair[64 * wn + 8 * t + 2 * tig + (i & 1)];
-            const int rr = 16 * wm + gid + (i >> 1) * 8;
-            if (p < 0) continue;
-            if (GATED) {
-                const int c = col0 + rr;
-                if (c < N) out[(size_t)p * N + c] = from_float<OutT>(glu_f(glu, acc[0][t][i], acc[1][t][i]));
-            } else {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int c = col0 + h * TC_HALF + rr;
-                    if (c < N) out[(size_t)p * N + c] = from_float<OutT>(acc[h][t][i]);
-                }
+    if (warp == 1) {
+        tc::tmem_alloc(&tmem_slot, 2 * TC_ROWS);
+        tc::tmem_relinquish();
+    }
+    if (threadIdx.x < TC_ROWS) src_pair[threadIdx.x] = (int)threadIdx.x < n_here ? list[threadIdx.x] : -1;
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    pdl_trigger();
+    const uint32_t tmem_base = tmem_slot;
+    const int col0 = blockIdx.y * (GATED ? TC_M : 2 * TC_M);
+    const int steps = (K + TC_K - 1) / TC_K;
+
+    if (warp == 0) {
+        const int w_row = e * (GATED ? 2 * N : N) + col0;
+        if (tc::elect_one()) {
+            for (int s = 0; s < steps; ++s) {
+                const int st = s % TC_STAGES;
+                if (!tc::mbar_wait(&empty[st], ((s / TC_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_MOE_PRODUCER)) break;
+                uint8_t* base = smem + st * TC_STAGE_BYTES;
+                tc::mbar_expect_tx(&full[st], 2 * TC_W_BYTES);
+                tc::tma_load_2d(base, &w_map, s * TC_K, w_row, &full[st]);
+                tc::tma_load_2d(base + TC_W_BYTES, &w_map, s * TC_K, w_row + (GATED ? N : TC_M), &full[st]);
             }
         }
+    } else if (warp == 1) {
+        if (tc::elect_one()) {
+            const uint32_t idesc = tc::instr_desc_bf16(TC_M, n16);
+            bool ok = true;
+            for (int s = 0; s < steps; ++s) {
+                const int st = s % TC_STAGES;
+                ok = tc::mbar_wait(&full[st], (s / TC_STAGES) & 1u, abort_flag, error_word, ERR_MOE_MMA);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const uint32_t w_addr = tc::smem_u32(smem + st * TC_STAGE_BYTES), b_addr = w_addr + 2 * TC_W_BYTES;
+#pragma unroll
+                for (int kk = 0; kk < TC_K / 16; ++kk)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        tc::mma_bf16_ss(tmem_base + h * TC_ROWS, tc::smem_desc_k_sw128(w_addr + h * TC_W_BYTES + kk * 32),
+                                        tc::smem_desc_k_sw128(b_addr + kk * 32), idesc, (s > 0 || kk > 0) ? 1u : 0u);
+                tc::mma_commit(&empty[st]);
+            }
+            if (ok) tc::mma_commit(&done);
+        }
+    } else {
+        // Piece `piece` of every 32nd of the pairs' rows; a place without a pair gets zeros.
+        const int piece = threadIdx.x & 7, first = (threadIdx.x - 64) >> 3;
+        long long at16[TC_ROWS / 32];                    // where the piece of the step 0 lies, in pieces of 16 bytes
+#pragma unroll
+        for (int i = 0; i < TC_ROWS / 32; ++i) {
+            const int p = src_pair[first + 32 * i];
+            at16[i] = p < 0 ? -1 : (long long)(p / a_div) * (K / 8) + piece;
+        }
+        const uint4* src = reinterpret_cast<const uint4*>(a);
+        const uint32_t place = tc::smem_u32(smem) + 2 * TC_W_BYTES + first * 128 + ((piece ^ (first & 7)) << 4);
+        // A stage's rows are handed over two steps later, when they have landed: a fence makes them visible to the products.
+        auto hand_over = [&](int s) {
+            tc::fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&full[s % TC_STAGES]);
+        };
+        bool ok = true;
+        for (int s = 0; s < steps; ++s) {
+            const int st = s % TC_STAGES;
+            ok = tc::mbar_wait(&empty[st], ((s / TC_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_MOE_PRODUCER);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const bool real = 64 * s + 8 * piece < K;
+#pragma unroll
+            for (int i = 0; i < TC_ROWS / 32; ++i)
+                if (32 * i < n16 && first + 32 * i < n16)
+                    cp_async_16_or_zeros(place + st * TC_STAGE_BYTES + i * 32 * 128, src + (real && at16[i] >= 0 ? at16[i] + 8 * s : 0), real && at16[i] >= 0);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (s >= 2) {
+                asm volatile("cp.async.wait_group 2;" ::: "memory");
+                hand_over(s - 2);
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (ok)
+            for (int s = max(0, steps - 2); s < steps; ++s) hand_over(s);
+        ok = ok && tc::mbar_wait(&done, 0, abort_flag, error_word, ERR_MOE_EPILOGUE);
+        tc::tc_fence_after();
+        // A warp may touch the tensor-memory lanes 32 (warp % 4) .. + 31; of two warps with the same lanes each takes every
+        // other run of 16 pairs.
+        const int quarter = warp & 3, c = col0 + 32 * quarter + lane;
+        const uint32_t lanes = tmem_base + ((uint32_t)(32 * quarter) << 16);
+        for (int p0 = 16 * ((warp - 2) >> 2); ok && p0 < n16; p0 += 32) {
+            uint32_t v[2][16];
+            tc::tmem_ld_32x16(lanes + p0, v[0]);
+            tc::tmem_ld_32x16(lanes + TC_ROWS + p0, v[1]);
+            tc::tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int p = src_pair[p0 + i];
+                if (p < 0) break;                            // the tile's pairs come first
+                OutT* row = out + (size_t)p * N;
+                const float x0 = __uint_as_float(v[0][i]), x1 = __uint_as_float(v[1][i]);
+                if (GATED) {
+                    if (c < N) row[c] = from_float<OutT>(glu_f(glu, x0, x1));
+                } else {
+                    if (c < N) row[c] = from_float<OutT>(x0);
+                    if (c + TC_M < N) row[c + TC_M] = from_float<OutT>(x1);
+                }
+            }
+        }
+        tc::tc_fence_before();
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(tmem_base, 2 * TC_ROWS);
+    }
 }
 
 // ---- steps of a few pairs -------------------------------------------------------------------------------------------
@@ -670,17 +705,17 @@ LLMX_EXPORT int llmx_moe_combine_weighted(const float* y, float* x, const float*
 }
 
 // The pairs a tile holds for the products' two forms: the routing cuts the lists for the form that will run.
-LLMX_EXPORT int llmx_moe_tile_rows(int tensor_cores) { return tensor_cores ? TC_ROWS : TILE_ROWS; }
+LLMX_EXPORT int llmx_moe_tile_rows(int tensor_cores) { return tensor_cores ? TC_LIST_TILE : TILE_ROWS; }
 
 // Whether the tensor-core form takes a product of these sizes and type.
-LLMX_EXPORT int llmx_moe_tensor_cores_fit(int dtype, int K) { return dtype == LLMX_BF16 && K > 0 && K % TC_K == 0; }
+LLMX_EXPORT int llmx_moe_tensor_cores_fit(int dtype, int K) { return dtype == LLMX_BF16 && K > 0 && K % 32 == 0; }
 
 // token_ids int32 [rows]; table int32 [vocab, top]; lists int32 [experts, rows * top]; counts int32 [experts]; tiles int32
 // [2 + 2 * (ceil(rows * top / tile_rows) + experts)].
 LLMX_EXPORT int llmx_moe_route(const int* token_ids, const int* table, int top, int rows, int experts, int vocab, int* lists,
                                int* counts, int* tiles, int tile_rows, cudaStream_t stream) {
     if (rows <= 0) return 0;
-    if (top <= 0 || experts <= 0 || experts > 65535 || (tile_rows != TILE_ROWS && tile_rows != TC_ROWS)) return LLMX_ERR_BAD_ARGUMENT;
+    if (top <= 0 || experts <= 0 || experts > 65535 || (tile_rows != TILE_ROWS && tile_rows != TC_LIST_TILE)) return LLMX_ERR_BAD_ARGUMENT;
     launch_kernel(route_kernel, dim3(experts), dim3(256), 0, stream, token_ids, table, top, rows, experts, vocab, lists, counts);
     int status = launch_status();
     if (status) return status;
@@ -693,23 +728,26 @@ LLMX_EXPORT int llmx_moe_route(const int* token_ids, const int* table, int top, 
 // the lists into tiles of `llmx_moe_tile_rows(tensor_cores)` pairs.
 LLMX_EXPORT int llmx_moe_product(const void* a, int a_div, const void* w, int dtype, const int* lists, const int* counts,
                                  const int* tiles, int pairs, int experts, void* out, int out_dtype, int N, int K,
-                                 int gated, int clamped, float limit, float alpha, int tensor_cores, cudaStream_t stream) {
+                                 int gated, int clamped, float limit, float alpha, int tensor_cores, int* error_word,
+                                 cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (N <= 0 || K <= 0 || a_div <= 0) return LLMX_ERR_BAD_ARGUMENT;
     if (!gated && out_dtype != LLMX_F32) return LLMX_ERR_UNSUPPORTED;
     const Glu glu = {clamped, limit, alpha};
     if (tensor_cores) {
         if (!llmx_moe_tensor_cores_fit(dtype, K) || ((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return LLMX_ERR_UNSUPPORTED;
-        const int out_cols = gated ? TC_HALF : 2 * TC_HALF;
-        dim3 grid(max_tiles(pairs, experts, TC_ROWS), (N + out_cols - 1) / out_cols);
-        if (grid.y > 65535) return LLMX_ERR_UNSUPPORTED;
+        const int out_cols = gated ? TC_M : 2 * TC_M;
         const __nv_bfloat16* ab = (const __nv_bfloat16*)a;
-        const __nv_bfloat16* wb = (const __nv_bfloat16*)w;
+        const long long w_rows = (long long)experts * (gated ? 2 : 1) * N;
+        dim3 grid(max_tiles(pairs, experts, TC_LIST_TILE), (N + out_cols - 1) / out_cols);
+        if (grid.y > 65535 || w_rows >= (1ll << 31)) return LLMX_ERR_UNSUPPORTED;
+        CUtensorMap w_map;
+        if (int bad = llmx_make_map_bf16_2d(&w_map, w, (uint64_t)w_rows, (uint64_t)K, TC_M, TC_K)) return bad;
 #define LLMX_MOE_TC(G, O)                                                                                              \
     do {                                                                                                                \
         cudaFuncSetAttribute(moe_tc_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);          \
-        launch_kernel(moe_tc_kernel<G, O>, dim3(grid), dim3(256), TC_SMEM, stream, ab, a_div, wb, lists, counts, tiles, \
-                      pairs, (O*)out, N, K, glu);                                                                          \
+        launch_kernel(moe_tc_kernel<G, O>, dim3(grid), dim3(TC_THREADS), TC_SMEM, stream, ab, w_map, a_div, lists,      \
+                      counts, tiles, pairs, (O*)out, N, K, glu, error_word);                                              \
     } while (0)
         if (gated && out_dtype == LLMX_BF16) LLMX_MOE_TC(true, __nv_bfloat16);
         else if (gated) LLMX_MOE_TC(true, float);

@@ -128,7 +128,7 @@ _SIGNATURES = {
                                                   _f, _p, _i, _p, _i, _i, _f, _f, _f, _p, _i, _p],
     ("moe", "llmx_moe_route"): [_p, _p, _i, _i, _i, _i, _p, _p, _p, _i, _p],
     ("moe", "llmx_moe_product_few"): [_p, _i, _p, _p, _p, _i, _i, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _p],
-    ("moe", "llmx_moe_product"): [_p, _i, _p, _i, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _i, _p],
+    ("moe", "llmx_moe_product"): [_p, _i, _p, _i, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _i, _p, _p],
     ("moe", "llmx_moe_combine"): [_p, _p, _i, _i, _i, _f, _p],
     ("moe", "llmx_moe_router"): [_p, _i, _p, _p, _i, _i, _i, _i, _i, _i, _p, _i, _i, _f, _p, _p, _p, _p],
     ("moe", "llmx_moe_combine_weighted"): [_p, _p, _p, _p, _i, _p, _i, _p, _p, _i, _i, _i, _f, _p],
@@ -995,6 +995,7 @@ def moe_product(a: torch.Tensor, a_div: int, w: torch.Tensor, lists: torch.Tenso
     then up rows), K] of a's type.  gated: out = silu(gate) * up in out's type, or with `clamp` = (limit, alpha)
     min(gate, limit) sigmoid(alpha min(gate, limit)) (clamp(up, -limit, limit) + 1); else float32.  `tensor_cores` as the
     routing was told.  Pairs in no list (an expert without weights) keep what `out` held."""
+    from .runtime import error_word
     clamped, limit, alpha = _clamp(clamp)
     _cuda(a, w, lists, counts, tiles, out)
     experts, wn, K = w.shape
@@ -1003,7 +1004,7 @@ def moe_product(a: torch.Tensor, a_div: int, w: torch.Tensor, lists: torch.Tenso
     _need(tuple(out.shape) == (pairs, N), "moe_product: output shape does not fit")
     _check(_fn("moe", "llmx_moe_product")(_ptr(a), int(a_div), _ptr(w), _code(w), _ptr(lists), _ptr(counts), _ptr(tiles), pairs,
                                           experts, _ptr(out), _code(out), N, K, 1 if gated else 0, clamped, limit, alpha,
-                                          1 if tensor_cores else 0, _stream()), "moe_product")
+                                          1 if tensor_cores else 0, _ptr(error_word(a.device)), _stream()), "moe_product")
     return out
 
 

@@ -858,3 +858,39 @@ def test_recurrence_over_many_rows(mode, heads, qk_heads, D, V, counts):
         assert (state[R + 1 + r].double() - S).abs().max() <= bound * max(1.0, float(S.abs().max())), (r, "state")
         at += n
     assert torch.equal(state[:R + 1].double(), before[:R + 1])
+
+
+# ---- the experts' products on the tensor cores ----------------------------------------------------------------------------------
+@pytest.mark.parametrize("counts", [[1, 0, 15, 16, 17], [255, 256, 257], [127, 128, 129, 512, 513], [272, 3]])
+@pytest.mark.parametrize("K,N,clamp", [(32, 8, None), (160, 130, None), (96, 256, (1.5, 1.7))])
+def test_expert_products_at_the_edges_of_their_tiles(counts, K, N, clamp):
+    """Experts whose pairs end just below, at and above a tile, part of a tile or several equal ones, widths that end within a
+    block of columns or a step of K: both products against the same in 64 bits.  The gated one is rounded to bfloat16 (2^-9),
+    and 32-bit sums of K terms of about one are off by less than sqrt(K) 2^-22."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(K + N)
+    experts, rows = len(counts), sum(counts)
+    choice = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(counts)])[torch.randperm(rows, generator=g)].view(rows, 1).to(DEV)
+    h = _bf16(torch.randn(rows, K, generator=g)).to(DEV)
+    w_gu = _bf16(torch.randn(experts, 2 * N, K, generator=g) * K ** -0.5).to(DEV)
+    w = _bf16(torch.randn(experts, N, K, generator=g) * K ** -0.5).to(DEV)
+    lists = torch.empty((experts, rows), dtype=torch.int32, device=DEV)
+    held = torch.empty((experts,), dtype=torch.int32, device=DEV)
+    tiles = torch.empty((ops.moe_tiles_len(rows, experts),), dtype=torch.int32, device=DEV)
+    ops.moe_route(None, choice, experts, lists, held, tiles, tensor_cores=True)
+    assert held.tolist() == counts
+    act = torch.full((rows, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.moe_product(h, 1, w_gu, lists, held, tiles, rows, act, gated=True, tensor_cores=True, clamp=clamp)
+    y = torch.full((rows, N), 7.0, dtype=torch.float32, device=DEV)
+    ops.moe_product(h, 1, w, lists, held, tiles, rows, y, gated=False, tensor_cores=True)
+    e = choice[:, 0].long()
+    both = torch.einsum("rk,rnk->rn", h.double(), w_gu.double()[e])
+    gate, up = both[:, :N], both[:, N:]
+    if clamp is None:
+        want = gate * torch.sigmoid(gate) * up
+    else:
+        gate, up = gate.clamp(max=clamp[0]), up.clamp(-clamp[0], clamp[0])
+        want = gate * torch.sigmoid(clamp[1] * gate) * (up + 1.0)
+    slack = K ** 0.5 * 2.0 ** -22
+    assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 8 * slack).all()
+    assert (y.double() - torch.einsum("rk,rnk->rn", h.double(), w.double()[e])).abs().max() <= 4 * slack
