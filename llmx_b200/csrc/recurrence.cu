@@ -640,6 +640,145 @@ conv_prepare_kernel(const float* __restrict__ proj, int stride, int first, int c
     }
 }
 
+// The same where channels come in fours: a thread owns four neighbouring channels (16-byte reads and writes) of a run of rows,
+// whose last taps - 1 inputs it keeps, so an input is read once for all the outputs it enters; the D / 4 lanes of a head sum
+// its squares by shuffles.  A block has up to 1,024 channels of `run` rows, or those channels of a request's kept inputs, or
+// the gates of the rows: a few rows (decoding) spread over as many blocks as the channels make, where one block a row
+// took them 256 at a time, each waiting for the one before: 8 rows of
+// 4,096 channels 28 -> 5.6 us, 4 rows of 8,192 and 6,144 channels 45 -> 5.9 us.
+constexpr int CONV_THREADS = 256, CONV_RUN = 16, CONV_TAPS = 4;
+
+__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float silu_f(float y) { return y / (1.0f + expf(-y)); }
+
+__global__ void __launch_bounds__(CONV_THREADS)
+conv_prepare_four_kernel(const float* __restrict__ proj, int stride, int first, int channels, int q_channels, int k_channels,
+                         const float* __restrict__ taps_w, const float* __restrict__ taps_b, int taps,
+                         float* __restrict__ ready, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                         int b_off, int a_off, int gate_kind, const float* __restrict__ decay_in, int decay_stride,
+                         float* __restrict__ gates, int gates_stride, int heads, int D, float q_factor,
+                         float* __restrict__ state, long long slot_floats, long long conv_off,
+                         const int* __restrict__ row_request, const int* __restrict__ row_start,
+                         const int* __restrict__ row_count, const int* __restrict__ history, const int* __restrict__ slot_in,
+                         const int* __restrict__ slot_out, int rows, int run, int row_blocks, int conv_blocks) {
+    pdl_trigger();
+    const int keep = taps - 1;
+    const int c = ((int)blockIdx.y * CONV_THREADS + (int)threadIdx.x) * 4;
+    const bool conv = (int)blockIdx.y < conv_blocks, mine = conv && c < channels;
+    // The filter's weights are written by no kernel: they are read before the wait.  w[j]: tap j of the four channels.
+    float4 w[CONV_TAPS], bias = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int j = 0; j < CONV_TAPS; ++j) w[j] = bias;
+    if (mine) {
+        float* wv = reinterpret_cast<float*>(w);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int j = 0; j < CONV_TAPS; ++j)
+                if (j < taps) wv[4 * j + u] = taps_w[(size_t)(c + u) * taps + j];
+        if (taps_b) bias = load_four(taps_b + c);
+    }
+    pdl_wait();
+    if ((int)blockIdx.x >= row_blocks) {
+        // The inputs the next step's filter will need.
+        if (!mine) return;
+        const int r = blockIdx.x - row_blocks;
+        const int n = row_count[r], a0 = row_start[r], hist = history[r];
+        if (n <= 0) return;
+        const float* old = state + (size_t)slot_in[r] * slot_floats + conv_off;
+        float* fresh = state + (size_t)slot_out[r] * slot_floats + conv_off;
+        for (int s = 0; s < keep; ++s) {             // slot_in and slot_out differ: the rows' blocks read the old inputs meanwhile
+            const int ii = n - keep + s;
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (ii >= 0) x = load_four(proj + (size_t)(a0 + ii) * stride + first + c);
+            else if (hist + ii >= 0) x = load_four(old + (size_t)(keep + ii) * channels + c);
+            *reinterpret_cast<float4*>(fresh + (size_t)s * channels + c) = x;
+        }
+        return;
+    }
+    const int row0 = blockIdx.x * run, row_end = min(rows, row0 + run);
+    if (!conv) {
+        // Gates: `per` a row, in blocks of four a thread.
+        const int per = gate_kind == 2 ? heads * D : heads;
+        const int g0 = ((int)blockIdx.y - conv_blocks) * CONV_THREADS * 4;
+        const int here = min(per - g0, CONV_THREADS * 4);
+        for (int i = threadIdx.x; i < (row_end - row0) * here; i += CONV_THREADS) {
+            const int row = row0 + i / here, g = g0 + i % here;
+            float* grow = gates + (size_t)row * gates_stride;
+            const float* prow = proj + (size_t)row * stride;
+            if (gate_kind == 2) {
+                const float z = decay_in[(size_t)row * decay_stride + g] + dt_bias[g];
+                grow[heads + g] = expf(-expf(a_log[g / D]) * softplus_f(z));
+                if (g < heads) grow[g] = 1.0f / (1.0f + expf(-prow[b_off + g]));
+                continue;
+            }
+            const float z = prow[a_off + g] + dt_bias[g];
+            if (gate_kind == 1) {
+                const float dt = z > 20.0f ? z : log1pf(expf(z));      // the same function beyond 20 up to rounding: no clamp of dt itself
+                grow[g] = expf(-expf(a_log[g]) * dt);
+                grow[heads + g] = dt;
+            } else {
+                grow[g] = expf(-expf(a_log[g]) * softplus_f(z));
+                grow[heads + g] = 1.0f / (1.0f + expf(-prow[b_off + g]));
+            }
+        }
+        return;
+    }
+    const bool unit = c < q_channels + k_channels;   // the same for all lanes of a head: heads are whole
+    const float factor = c < q_channels ? q_factor : 1.0f;
+    float4 x[CONV_TAPS];                             // x[j]: the input under tap j
+    float4 next = mine ? load_four(proj + (size_t)row0 * stride + first + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int left = 0;                                    // rows of the request at hand that are still to come
+#pragma unroll
+    for (int j = 0; j < CONV_TAPS; ++j) x[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int row = row0; row < row_end; ++row) {
+        const float4 now = next;
+        if (mine && row + 1 < row_end) next = load_four(proj + (size_t)(row + 1) * stride + first + c);
+        if (left == 0) {
+            // The first row of the block or of a request: the inputs before it, from earlier rows or the state.
+            const int r = row_request[row];
+            const int i0 = row - row_start[r], hist = history[r];
+            left = row_count[r] - i0;
+            if (mine) {
+                const float* old = state + (size_t)slot_in[r] * slot_floats + conv_off;
+#pragma unroll
+                for (int j = 0; j < CONV_TAPS; ++j) {
+                    const int ii = i0 - keep + j;        // tap j's input of this row, as this row's place in the request has it
+                    if (j >= keep) continue;
+                    x[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (ii >= 0) x[j] = load_four(proj + (size_t)(row_start[r] + ii) * stride + first + c);
+                    else if (hist + ii >= 0) x[j] = load_four(old + (size_t)(keep + ii) * channels + c);
+                }
+            }
+        }
+        --left;
+        float4 y = bias;
+#pragma unroll
+        for (int j = 0; j < CONV_TAPS; ++j) {
+            if (j >= taps) continue;
+            const float4 v = j == keep ? now : x[j];
+            y.x = fmaf(w[j].x, v.x, y.x);
+            y.y = fmaf(w[j].y, v.y, y.y);
+            y.z = fmaf(w[j].z, v.z, y.z);
+            y.w = fmaf(w[j].w, v.w, y.w);
+        }
+#pragma unroll
+        for (int j = 0; j + 1 < CONV_TAPS; ++j)
+            if (j < keep) x[j] = j + 1 == keep ? now : x[j + 1];
+        y = make_float4(silu_f(y.x), silu_f(y.y), silu_f(y.z), silu_f(y.w));
+        // Every lane takes part in the shuffles; only heads that are made unit vectors use the sum.
+        float s = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, y.w * y.w)));
+        if (q_channels + k_channels > 0) {
+            for (int o = D / 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (unit) {
+                const float f = factor / sqrtf(s + 1e-6f);
+                y.x *= f, y.y *= f, y.z *= f, y.w *= f;
+            }
+        }
+        if (mine) *reinterpret_cast<float4*>(ready + (size_t)row * channels + c) = y;
+    }
+}
+
 // Decays per key channel through a low-rank pair, in 32-bit: z = low W2^T + bias, decay = sigmoid(z)^(1 / tau); `low` is the
 // pair's inner values (a run of columns of the projections), `w2t` W2 transposed [rank][channels].  In passing the same
 // channels of q (columns q_off .. of the projections) are multiplied by `q_factor`.  A thread a channel, DECAY_ROWS rows.
@@ -800,6 +939,24 @@ LLMX_EXPORT int llmx_conv_prepare(const float* proj, int stride, int first, int 
         return LLMX_ERR_BAD_ARGUMENT;
     const size_t smem = (size_t)channels * sizeof(float);
     if (smem > 200 * 1024) return LLMX_ERR_UNSUPPORTED;
+    // Fours: a head's lanes are a power of two of a warp's (without unit heads any width does), and every run of channels
+    // starts on 16 bytes.
+    const bool units = q_channels + k_channels > 0;
+    if (taps <= CONV_TAPS && channels % 4 == 0 && stride % 4 == 0 && first % 4 == 0 && slot_floats % 4 == 0 && conv_off % 4 == 0 &&
+        (!units || (D % 4 == 0 && D <= 128 && ((D / 4) & (D / 4 - 1)) == 0)) &&
+        (((uintptr_t)proj | (uintptr_t)ready | (uintptr_t)state | (uintptr_t)taps_b) & 15) == 0) {
+        const int per = gate_kind == 2 ? heads * D : heads, block = CONV_THREADS * 4;
+        const int conv_blocks = (channels + block - 1) / block, gate_blocks = (per + block - 1) / block;
+        // One row a block while that leaves the SMs' 296 places unfilled, longer runs of rows beyond.
+        int run = (int)((long long)rows * conv_blocks / 592);
+        run = run < 1 ? 1 : run > CONV_RUN ? CONV_RUN : run;
+        const int row_blocks = (rows + run - 1) / run;
+        launch_kernel(conv_prepare_four_kernel, dim3(row_blocks + requests, conv_blocks + gate_blocks), dim3(CONV_THREADS), 0, stream, proj,
+                      stride, first, channels, q_channels, k_channels, taps_w, taps_b, taps, ready, a_log, dt_bias, b_off, a_off,
+                      gate_kind, decay_in, decay_stride, gates, gates_stride, heads, D, q_factor, state, slot_floats, conv_off,
+                      row_request, row_start, row_count, history, slot_in, slot_out, rows, run, row_blocks, conv_blocks);
+        return launch_status();
+    }
     if (smem > 48 * 1024) cudaFuncSetAttribute(conv_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     launch_kernel(conv_prepare_kernel, dim3(rows + requests), dim3(256), smem, stream, proj, stride, first, channels,
                   q_channels, k_channels, taps_w, taps_b, taps, ready, a_log, dt_bias, b_off, a_off, gate_kind, decay_in,

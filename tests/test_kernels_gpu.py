@@ -894,3 +894,95 @@ def test_expert_products_at_the_edges_of_their_tiles(counts, K, N, clamp):
     slack = K ** 0.5 * 2.0 ** -22
     assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 8 * slack).all()
     assert (y.double() - torch.einsum("rk,rnk->rn", h.double(), w.double()[e])).abs().max() <= 4 * slack
+
+
+# ---- small kernels of a few rows ---------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("kind", ["delta", "step", "delta_channel"])
+@pytest.mark.parametrize("heads,D,taps,q_heads,more,counts", [
+    (2, 4, 2, 1, 8, [1, 3]), (3, 64, 4, 2, 1100, [1] * 9), (2, 128, 3, 2, 260, [5, 1, 40]), (16, 128, 4, 8, 2048, [700, 3, 650]), (4, 12, 4, 0, 20, [33])])
+def test_filter_of_channels_in_fours(kind, heads, D, taps, q_heads, more, counts):
+    """The short filter, unit heads, gates and kept inputs against the same in 64 bits: one row a block and runs of rows that
+    cross requests, first rows with and without a history, channels that end within a block.  32-bit throughout."""
+    import types
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(D + taps)
+    rows, R, q_ch, k_ch = sum(counts), len(counts), q_heads * D, q_heads * D
+    channels, first = q_ch + k_ch + more, 4
+    stride = first + channels + 2 * heads + (-(first + channels + 2 * heads)) % 4
+    proj = torch.randn(rows, stride, generator=g).to(DEV)
+    w, bias = (torch.randn(channels, taps, generator=g) * 0.4).to(DEV), (torch.randn(channels, generator=g) * 0.1).to(DEV)
+    per = heads * D if kind == "delta_channel" else heads
+    a_log, dt_bias = (torch.randn(heads, generator=g) * 0.5).to(DEV), (torch.randn(per, generator=g) * 0.5).to(DEV)
+    decay_in = torch.randn(rows, per, generator=g).to(DEV) if kind == "delta_channel" else None
+    state = torch.randn(2 * R, 8 + (taps - 1) * channels, generator=g)
+    state = torch.cat([state, torch.zeros(2 * R, -state.shape[1] % 4)], 1).to(DEV)
+    before, off = state.clone(), 8
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    history = [0 if r % 2 == 0 else 1 + r for r in range(R)]
+    starts = [sum(counts[:r]) for r in range(R)]
+    step = types.SimpleNamespace(row_request=i32([r for r, n in enumerate(counts) for _ in range(n)]), row_start=i32(starts), row_count=i32(counts),
+                                 history=i32(history), state_slots=i32(list(range(R))), state_slots_out=i32([R + r for r in range(R)]), requests=R)
+    ready = torch.full((rows, channels), 7.0, device=DEV)
+    gates = torch.full((rows, heads + per), 7.0, device=DEV)
+    b_off, a_off, q_factor = first + channels, first + channels + heads, 0.3
+    ops.conv_prepare(proj, channels, q_ch, k_ch, w, ready, a_log, dt_bias, b_off, a_off, gates, heads, D, q_factor, state, off, step, first=first,
+                     bias=bias, gate_kind=kind, decay_in=decay_in)
+    for r, n in enumerate(counts):
+        rows_r = slice(starts[r], starts[r] + n)
+        u = proj[rows_r, first:first + channels].double()
+        old = before[r, off:off + (taps - 1) * channels].double().view(taps - 1, channels).clone()
+        for s in range(taps - 1):
+            if history[r] - (taps - 1) + s < 0:
+                old[s] = 0.0
+        seen = torch.cat([old, u])
+        y = bias.double() + sum(w[:, j].double() * seen[j:j + n] for j in range(taps))
+        y = y * torch.sigmoid(y)
+        for lo, factor in ((0, q_factor), (q_ch, 1.0)):
+            if q_ch:
+                part = y[:, lo:lo + q_ch].reshape(n, q_heads, D)
+                y[:, lo:lo + q_ch] = (part * factor / (part.square().sum(-1, keepdim=True) + 1e-6).sqrt()).reshape(n, q_ch)
+        assert (ready[rows_r].double() - y).abs().max() <= 2e-6 * max(1.0, float(y.abs().max())), r
+        assert torch.equal(state[R + r, off:off + (taps - 1) * channels].view(taps - 1, channels).double(), seen[n:]), (r, "kept inputs")
+        z = (decay_in[rows_r] if kind == "delta_channel" else proj[rows_r, a_off:a_off + heads]).double() + dt_bias.double()
+        dt = torch.nn.functional.softplus(z, threshold=60.0)
+        decay = torch.exp(-torch.exp(a_log.double()).repeat_interleave(per // heads) * dt)
+        beta = torch.sigmoid(proj[rows_r, b_off:b_off + heads].double())
+        want = {"delta": [decay, beta], "step": [decay, dt], "delta_channel": [beta, decay]}[kind]
+        assert (gates[rows_r].double() - torch.cat(want, 1)).abs().max() <= 2e-6 * max(1.0, float(dt.abs().max())), r
+    assert torch.equal(state[:R], before[:R])
+
+
+@pytest.mark.parametrize("rows,heads,D,R,V,C,splits", [(1, 2, 40, 8, 50, 264, 1), (5, 3, 128, 64, 128, 512, 3), (64, 2, 136, 0, 33, 768, 5), (2, 1, 7, 4, 1, 8, 40)])
+def test_latent_maps_of_a_few_rows(rows, heads, D, R, V, C, splits):
+    """The query and merge steps with bfloat16 maps against the same in 64 bits; ranges without keys (maximum minus infinity, sums
+    never made) among the merged ones.  32-bit sums of D or C terms, the merged result rounded to bfloat16 (2^-9)."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(C + rows)
+    uk, uv = _bf16(torch.randn(heads * D, C, generator=g) * C ** -0.5).to(DEV), _bf16(torch.randn(heads * V, C, generator=g) * C ** -0.5).to(DEV)
+    q = torch.randn(rows, heads * (D + R) + 3, generator=g).to(DEV)[:, :heads * (D + R)]
+    freq = torch.rand(R // 2, generator=g).to(DEV)
+    pos = torch.arange(3, 3 + rows, dtype=torch.int32, device=DEV)
+    qk = torch.full((rows, heads, C + R), 7.0, device=DEV)
+    P = ops._ptr
+    ops._check(ops._fn("latent_attention", "llmx_latent_query")(P(q), q.stride(0), P(uk), 1, P(qk), P(freq), R // 2, 1, 1.5, P(pos), rows, heads, D, R, C,
+                                                                0.25, ops._stream()), "query")
+    qh = q.double().view(rows, heads, D + R)
+    want = torch.einsum("rhd,hdc->rhc", qh[:, :, :D], uk.double().view(heads, D, C)) * 0.25
+    assert (qk[:, :, :C].double() - want).abs().max() <= 2.0 ** -20 * D ** 0.5 * float(want.abs().max() + 1)
+    angle = (pos[:, None].float() * freq).double()[:, None, :]
+    a, b = qh[:, :, D:D + R // 2], qh[:, :, D + R // 2:]
+    turned = torch.cat([a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()], 2) * 1.5 * 0.25
+    assert R == 0 or (qk[:, :, C:].double() - turned).abs().max() <= 1e-5
+    part = torch.randn(rows, heads, splits, C + 2, generator=g).to(DEV)
+    part[..., C + 1] = part[..., C + 1].abs() + 0.5
+    if splits > 1:
+        part[:, :, 1] = float("nan")
+        part[:, :, 1, C] = -float("inf")
+    out = torch.zeros(rows, heads * V, dtype=torch.bfloat16, device=DEV)
+    ops._check(ops._fn("latent_attention", "llmx_latent_merge")(P(part), P(uv), 1, P(out), rows, heads, V, C, splits, ops._stream()), "merge")
+    live = [s for s in range(splits) if s != 1 or splits == 1]
+    p = part[:, :, live].double()
+    e = torch.exp(p[..., C] - p[..., C].amax(2, keepdim=True))
+    lat = (p[..., :C] * e[..., None]).sum(2) / (p[..., C + 1] * e).sum(2, keepdim=True)
+    want = torch.einsum("rhc,hvc->rhv", lat, uv.double().view(heads, V, C)).reshape(rows, -1)
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * float(lat.abs().max())).all()
