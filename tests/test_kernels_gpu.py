@@ -986,3 +986,33 @@ def test_latent_maps_of_a_few_rows(rows, heads, D, R, V, C, splits):
     lat = (p[..., :C] * e[..., None]).sum(2) / (p[..., C + 1] * e).sum(2, keepdim=True)
     want = torch.einsum("rhc,hvc->rhv", lat, uv.double().view(heads, V, C)).reshape(rows, -1)
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * float(lat.abs().max())).all()
+
+
+@pytest.mark.parametrize("rows,width", [(1, 4), (3, 100), (8, 2048), (70, 4096), (2, 8192), (2, 8196)])
+def test_norms_of_rows_in_fours(rows, width):
+    """Centred, gated and paired norms of rows that a block holds in groups of four (and one width beyond): against 64 bits, 32-bit
+    results within a few roundings, bfloat16 ones within one."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(width)
+    t = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    x, w, gate, wb = t(rows, width) + 0.5, 1 + 0.1 * t(width), t(rows, width + 4)[:, :width], 1 + 0.1 * t(width)
+    rms = lambda v: v / (v.square().mean(-1, keepdim=True) + 1e-5).sqrt()
+    for dtype, tol in ((torch.float32, 4e-6), (torch.bfloat16, 2.0 ** -8)):
+        y, zero = torch.empty(rows, width, dtype=dtype, device=DEV), torch.full((4 * 700,), 3.0, device=DEV)
+        ops.layernorm(x, w, 1e-5, y, zero=zero)
+        d = x.double() - x.double().mean(-1, keepdim=True)
+        want = rms(d) * w.double()
+        assert ((y.double() - want).abs() <= tol * (want.abs() + 0.1)).all() and not zero.any()
+        for kind in (0, 1):
+            for gate_first in (0, 1):
+                P = ops._ptr
+                ops._check(ops._fn("rowwise", "llmx_gated_rmsnorm")(P(x), P(gate), gate.stride(0), P(w), width, P(y), ops._code(y), rows, 1, width, 1e-5, kind,
+                                                                    gate_first, ops._stream()), "gated")
+                a = torch.sigmoid(gate.double()) * (gate.double() if kind else 1.0)
+                want = rms(x.double() * a) * w.double() if gate_first else rms(x.double()) * w.double() * a
+                assert ((y.double() - want).abs() <= tol * (want.abs() + 0.1)).all(), (kind, gate_first)
+    a, b, s = t(rows, width), t(rows, width), t(rows, width)
+    want = s.double() + 0.5 * (rms(a.double()) * w.double() + rms(b.double()) * wb.double())
+    P = ops._ptr
+    ops._check(ops._fn("rowwise", "llmx_pair_norm_add")(P(a), P(b), P(w), P(wb), P(s), rows, width, 1e-5, 0.5, ops._stream()), "pair")
+    assert (s.double() - want).abs().max() <= 4e-6 * float(want.abs().max())
