@@ -76,6 +76,16 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, float a, float b, flo
     *reinterpret_cast<uint2*>(dst) = v;
 }
 
+// A thread's share of a row of n4 groups of four: groups threadIdx.x, + blockDim.x, ..., zeros past the end.
+template <int N>
+__device__ __forceinline__ void load_row4(float4 (&v)[N], const float4* src, int n4) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        v[k] = i < n4 ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
 // `zero` (optional): a float buffer of `zero_count` values (a multiple of 4, 16-byte aligned) that the launch
 // clears with blocks of its own (those beyond `rows`): the output of the product that follows, when that product
 // adds its pieces with atomics.
@@ -84,27 +94,24 @@ __global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __r
                                    const int* __restrict__ row_index, int rows, int width, float eps,
                                    float* __restrict__ zero, long long zero_count) {
     pdl_trigger();
-    pdl_wait();
     __shared__ float scratch[32];
-    const int r = blockIdx.x;
+    const int r = blockIdx.x, n4 = width >> 2;
+    // No kernel writes the weights: they are read before the wait (with a few rows the norm's time is that of its reads:
+    // four rows of 4,096 4.3 -> 2.7 us; a decode step of one Qwen3-0.6B request 863 -> 750 us).
+    float4 ww[NORM_VEC_MAX];
+    if (r < rows) load_row4(ww, reinterpret_cast<const float4*>(w), n4);
+    pdl_wait();
     if (r >= rows) {
         // Blocks beyond the rows only clear: with a few rows, a few blocks would store for longer than the norm takes.
         float4* z = reinterpret_cast<float4*>(zero);
-        const long long n4 = zero_count >> 2;
+        const long long z4 = zero_count >> 2;
         const long long blocks = gridDim.x - rows;
-        for (long long i = (long long)(r - rows) * blockDim.x + threadIdx.x; i < n4; i += blocks * blockDim.x)
+        for (long long i = (long long)(r - rows) * blockDim.x + threadIdx.x; i < z4; i += blocks * blockDim.x)
             z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    const float4* src = reinterpret_cast<const float4*>(x + (size_t)(row_index ? row_index[r] : r) * width);
-    const float4* wv = reinterpret_cast<const float4*>(w);
-    const int n4 = width >> 2;
     float4 v[NORM_VEC_MAX];
-#pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) {
-        const int i = threadIdx.x + k * blockDim.x;
-        v[k] = i < n4 ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    load_row4(v, reinterpret_cast<const float4*>(x + (size_t)(row_index ? row_index[r] : r) * width), n4);
     float s = 0.0f;
 #pragma unroll
     for (int k = 0; k < NORM_VEC_MAX; ++k) {
@@ -120,8 +127,7 @@ __global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __r
     for (int k = 0; k < NORM_VEC_MAX; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         if (i < n4) {
-            const float4 ww = wv[i];
-            store4(dst + 4 * i, v[k].x * (rr * ww.x), v[k].y * (rr * ww.y), v[k].z * (rr * ww.z), v[k].w * (rr * ww.w));
+            store4(dst + 4 * i, v[k].x * (rr * ww[k].x), v[k].y * (rr * ww[k].y), v[k].z * (rr * ww[k].z), v[k].w * (rr * ww[k].w));
         }
     }
 }
@@ -684,6 +690,46 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const float* __res
     }
 }
 
+// The same for rows of whole groups of four values, up to 8,192 of them, without a bias and written to `y`: 16-byte reads, and the
+// weights, which no kernel writes, before the wait.  Eight rows of 2,048: 10.2 -> 3.1 us.
+template <typename OutT>
+__global__ void __launch_bounds__(256)
+layernorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, OutT* __restrict__ y, const int* __restrict__ row_index,
+                     int rows, int width, float eps, float* __restrict__ zero, long long zero_count) {
+    pdl_trigger();
+    __shared__ float scratch[32];
+    const int r = blockIdx.x, n4 = width >> 2;
+    float4 ww[NORM_VEC_MAX], v[NORM_VEC_MAX];
+    if (r < rows) load_row4(ww, reinterpret_cast<const float4*>(w), n4);
+    pdl_wait();
+    if (r >= rows) {
+        float4* z = reinterpret_cast<float4*>(zero);
+        const long long z4 = zero_count >> 2, blocks = gridDim.x - rows;
+        for (long long i = (long long)(r - rows) * blockDim.x + threadIdx.x; i < z4; i += blocks * blockDim.x)
+            z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    load_row4(v, reinterpret_cast<const float4*>(x + (size_t)(row_index ? row_index[r] : r) * width), n4);
+    float s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NORM_VEC_MAX; ++k) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+    const float n = (float)width;            // divided by, as above
+    const float mean = block_sum(s, scratch) / n;
+    float q = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+        if ((int)(threadIdx.x + k * blockDim.x) >= n4) continue;
+        v[k] = make_float4(v[k].x - mean, v[k].y - mean, v[k].z - mean, v[k].w - mean);
+        q = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, q))));
+    }
+    const float rr = 1.0f / sqrtf(block_sum(q, scratch) / n + eps);
+#pragma unroll
+    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) store4(y + (size_t)r * width + 4 * i, v[k].x * rr * ww[k].x, v[k].y * rr * ww[k].y, v[k].z * rr * ww[k].z, v[k].w * rr * ww[k].w);
+    }
+}
+
 // The centred norm in its general form: y = ((x + in_bias) - mean) / sqrt(var + eps) * w + b.  `in_bias` and `b` may be
 // null.  With `add_to` (float [rows, width]) nothing is written to `y`; instead add_to += mult * y in 32-bit: the norm
 // after a sublayer and the sublayer's weighted entry into the residual stream in one pass.
@@ -693,6 +739,19 @@ LLMX_EXPORT int llmx_layernorm_affine(const float* x, const float* in_bias, cons
     if (rows <= 0) return 0;
     if (width <= 0 || (!y && !add_to)) return LLMX_ERR_BAD_ARGUMENT;
     if (zero && (zero_count % 4 || ((uintptr_t)zero & 15))) return LLMX_ERR_BAD_ARGUMENT;
+    if (!in_bias && !b && !add_to && width % 4 == 0 && width <= 4 * NORM_VEC_MAX * 256 && !(((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15)) {
+        const int n4 = width / 4;
+        int threads = ((n4 + 1) / 2 + 31) / 32 * 32;         // two groups of four a thread; the block width follows the row width alone
+        threads = threads > 256 ? 256 : threads;
+        long long zero_blocks = zero ? (zero_count / 4 + 4 * threads - 1) / (4 * threads) : 0;
+        zero_blocks = zero_blocks > 1024 ? 1024 : zero_blocks;
+        const dim3 grid((unsigned)(rows + zero_blocks));
+        if (out_dtype == LLMX_BF16)
+            launch_kernel(layernorm_vec_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream, x, w, (__nv_bfloat16*)y, row_index, rows, width, eps, zero, zero_count);
+        else
+            launch_kernel(layernorm_vec_kernel<float>, grid, dim3(threads), 0, stream, x, w, (float*)y, row_index, rows, width, eps, zero, zero_count);
+        return launch_status();
+    }
     // The block width follows the row width alone, so a row's sums have one order whatever the batch.
     int threads = (width + LN_MAX - 1) / LN_MAX;
     threads = (threads + 31) / 32 * 32;
@@ -1067,6 +1126,49 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const float* _
     }
 }
 
+// The same for groups of whole fours, up to 8,192 values: the group and its gates in registers, 16-byte accesses, the weights
+// before the wait.  Eight rows of one group of 2,048: 9.9 -> 4.3 us.
+template <typename OutT>
+__global__ void __launch_bounds__(256)
+gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_stride, const float* __restrict__ w,
+                         int w_len, OutT* __restrict__ y, int groups, int group, float eps, int gate_kind, int gate_first) {
+    pdl_trigger();
+    __shared__ float scratch[32];
+    const int r = blockIdx.x, j = blockIdx.y, n4 = group >> 2;
+    const size_t base = ((size_t)r * groups + j) * group;
+    float4 ww[NORM_VEC_MAX], v[NORM_VEC_MAX], g[NORM_VEC_MAX];
+    if (w) {
+        load_row4(ww, reinterpret_cast<const float4*>(w + (size_t)j * group % w_len), n4);
+    } else {
+#pragma unroll
+        for (int k = 0; k < NORM_VEC_MAX; ++k) ww[k] = make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+    pdl_wait();
+    load_row4(v, reinterpret_cast<const float4*>(o + base), n4);
+    load_row4(g, reinterpret_cast<const float4*>(gate + (size_t)r * gate_stride + (size_t)j * group), n4);
+    auto act = [&](float z) {
+        const float sg = 1.0f / (1.0f + expf(-z));
+        return gate_kind == 0 ? sg : z * sg;
+    };
+    float s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+        if ((int)(threadIdx.x + k * blockDim.x) >= n4) continue;
+        g[k] = make_float4(act(g[k].x), act(g[k].y), act(g[k].z), act(g[k].w));
+        if (gate_first) v[k] = make_float4(v[k].x * g[k].x, v[k].y * g[k].y, v[k].z * g[k].z, v[k].w * g[k].w);
+        s = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, s))));
+    }
+    const float rr = 1.0f / sqrtf(block_sum(s, scratch) / (float)group + eps);
+#pragma unroll
+    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i >= n4) continue;
+        if (gate_first) g[k] = make_float4(1.f, 1.f, 1.f, 1.f);
+        store4(y + base + 4 * i, v[k].x * rr * ww[k].x * g[k].x, v[k].y * rr * ww[k].y * g[k].y, v[k].z * rr * ww[k].z * g[k].z,
+               v[k].w * rr * ww[k].w * g[k].w);
+    }
+}
+
 // `gate_first` 0: y = o / rms(o) * w * act(gate).  1: the gate comes before the norm: z = o * act(gate), y = z / rms(z) * w.
 LLMX_EXPORT int llmx_gated_rmsnorm(const float* o, const float* gate, int gate_stride, const float* w, int w_len, void* y,
                                    int out_dtype, int rows, int groups, int group, float eps, int gate_kind, int gate_first,
@@ -1093,6 +1195,14 @@ LLMX_EXPORT int llmx_gated_rmsnorm(const float* o, const float* gate, int gate_s
     int threads = (group + 3) / 4;
     threads = (threads + 31) / 32 * 32;
     threads = threads < 32 ? 32 : threads > 256 ? 256 : threads;
+    if (group % 4 == 0 && group <= 4 * NORM_VEC_MAX * 256 && gate_stride % 4 == 0 && (!w || (w_len % group == 0)) &&
+        !(((uintptr_t)o | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)y) & 15)) {
+        if (out_dtype == LLMX_BF16)
+            launch_kernel(gated_rmsnorm_vec_kernel<__nv_bfloat16>, dim3(rows, groups), dim3(threads), 0, stream, o, gate, gate_stride, w, w_len, (__nv_bfloat16*)y, groups, group, eps, gate_kind, gate_first);
+        else
+            launch_kernel(gated_rmsnorm_vec_kernel<float>, dim3(rows, groups), dim3(threads), 0, stream, o, gate, gate_stride, w, w_len, (float*)y, groups, group, eps, gate_kind, gate_first);
+        return launch_status();
+    }
     if (out_dtype == LLMX_BF16)
         launch_kernel(gated_rmsnorm_kernel<__nv_bfloat16>, dim3(rows, groups), dim3(threads), 0, stream, o, gate, gate_stride, w, w_len, (__nv_bfloat16*)y, groups, group, eps, gate_kind, gate_first);
     else
@@ -1122,10 +1232,56 @@ pair_norm_add_kernel(const float* __restrict__ a, const float* __restrict__ b, c
         x[base + i] += factor * (a[base + i] * ra * wa[i] + b[base + i] * rb * wb[i]);
 }
 
+// The same for rows of whole groups of four, up to 8,192 values, both rows in registers.  Four rows of 4,096: 18 -> 6 us.
+constexpr int PAIR_MAX = 4, PAIR_THREADS = 512;
+__global__ void __launch_bounds__(PAIR_THREADS)
+pair_norm_add_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ wa,
+                         const float* __restrict__ wb, float* __restrict__ x, int width, float eps, float factor) {
+    pdl_trigger();
+    __shared__ float scratch[2][PAIR_THREADS / 32];
+    const int n4 = width >> 2, warp = threadIdx.x >> 5;
+    const size_t base = (size_t)blockIdx.x * width;
+    float4 va[PAIR_MAX], vb[PAIR_MAX], ua[PAIR_MAX], ub[PAIR_MAX], vx[PAIR_MAX];
+    load_row4(ua, reinterpret_cast<const float4*>(wa), n4);
+    load_row4(ub, reinterpret_cast<const float4*>(wb), n4);
+    pdl_wait();
+    load_row4(va, reinterpret_cast<const float4*>(a + base), n4);
+    load_row4(vb, reinterpret_cast<const float4*>(b + base), n4);
+    load_row4(vx, reinterpret_cast<const float4*>(x + base), n4);
+    float sa = 0.0f, sb = 0.0f;
+#pragma unroll
+    for (int k = 0; k < PAIR_MAX; ++k) {
+        sa = fmaf(va[k].x, va[k].x, fmaf(va[k].y, va[k].y, fmaf(va[k].z, va[k].z, fmaf(va[k].w, va[k].w, sa))));
+        sb = fmaf(vb[k].x, vb[k].x, fmaf(vb[k].y, vb[k].y, fmaf(vb[k].z, vb[k].z, fmaf(vb[k].w, vb[k].w, sb))));
+    }
+    sa = warp_sum(sa);
+    sb = warp_sum(sb);
+    if ((threadIdx.x & 31) == 0) scratch[0][warp] = sa, scratch[1][warp] = sb;
+    __syncthreads();
+    sa = sb = 0.0f;
+#pragma unroll
+    for (int g = 0; g < PAIR_THREADS / 32; ++g) sa += scratch[0][g], sb += scratch[1][g];
+    const float ra = 1.0f / sqrtf(sa / (float)width + eps), rb = 1.0f / sqrtf(sb / (float)width + eps);
+#pragma unroll
+    for (int k = 0; k < PAIR_MAX; ++k) {
+        const int i = threadIdx.x + k * PAIR_THREADS;
+        if (i >= n4) continue;
+        store4(x + base + 4 * i, vx[k].x + factor * (va[k].x * ra * ua[k].x + vb[k].x * rb * ub[k].x),
+               vx[k].y + factor * (va[k].y * ra * ua[k].y + vb[k].y * rb * ub[k].y),
+               vx[k].z + factor * (va[k].z * ra * ua[k].z + vb[k].z * rb * ub[k].z),
+               vx[k].w + factor * (va[k].w * ra * ua[k].w + vb[k].w * rb * ub[k].w));
+    }
+}
+
 LLMX_EXPORT int llmx_pair_norm_add(const float* a, const float* b, const float* wa, const float* wb, float* x, int rows,
                                    int width, float eps, float factor, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (width <= 0) return LLMX_ERR_BAD_ARGUMENT;
+    if (width % 4 == 0 && width <= 4 * PAIR_MAX * PAIR_THREADS &&
+        !(((uintptr_t)a | (uintptr_t)b | (uintptr_t)wa | (uintptr_t)wb | (uintptr_t)x) & 15)) {
+        launch_kernel(pair_norm_add_vec_kernel, dim3(rows), dim3(PAIR_THREADS), 0, stream, a, b, wa, wb, x, width, eps, factor);
+        return launch_status();
+    }
     launch_kernel(pair_norm_add_kernel, dim3(rows), dim3(256), 0, stream, a, b, wa, wb, x, width, eps, factor);
     return launch_status();
 }

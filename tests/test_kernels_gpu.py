@@ -1016,3 +1016,17 @@ def test_norms_of_rows_in_fours(rows, width):
     P = ops._ptr
     ops._check(ops._fn("rowwise", "llmx_pair_norm_add")(P(a), P(b), P(w), P(wb), P(s), rows, width, 1e-5, 0.5, ops._stream()), "pair")
     assert (s.double() - want).abs().max() <= 4e-6 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 65, 36), (4, 4096, 256), (3, 130, 1000)])
+def test_plain_product_of_a_few_rows_is_the_tiled_one_bit_for_bit(dtype, M, N, K):
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(K)
+    a, w, c = torch.randn(70, K, generator=g).to(dtype).to(DEV), torch.randn(N, K, generator=g).to(dtype).to(DEV), torch.randn(70, N, generator=g).to(DEV)
+    for accumulate in (0, 1):
+        few, many = c[:M].clone(), c.clone()
+        for out, rows in ((few, M), (many, 70)):
+            ops._check(ops._fn("gemm_plain", "llmx_gemm_plain")(ops._ptr(a), ops._code(a), ops._ptr(w), ops._code(w), ops._ptr(out), rows, N, K, accumulate,
+                                                                ops._stream()), "plain")
+        assert torch.equal(few, many[:M])
