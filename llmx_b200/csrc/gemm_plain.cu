@@ -64,12 +64,85 @@ __global__ void __launch_bounds__(256) gemm_plain_kernel(const AT* __restrict__ 
         }
     }
 }
+
+// A few rows: a thread an output column, its weight row in pieces of four values, FEW_AHEAD pieces in flight before the
+// first is used; A's rows lie in shared memory.  k runs in increasing order, as above, so a row's result is the same bit for
+// bit whichever form runs.  Four rows, 4,096 columns over 256: 29 -> 9 us.
+constexpr int FEW_ROWS = 8, FEW_COLS = 64, FEW_AHEAD = 8, FEW_BYTES = 40 * 1024;
+
+__device__ __forceinline__ void four(const float* p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+}
+__device__ __forceinline__ void four(const __nv_bfloat16* p, float (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
+template <typename AT, typename WT>
+__global__ void __launch_bounds__(FEW_COLS) gemm_plain_few_kernel(const AT* __restrict__ A, const WT* __restrict__ W, float* __restrict__ C,
+                                                                  int M, int N, int K, int accumulate) {
+    pdl_trigger();
+    extern __shared__ __align__(16) float rows[];        // [M][K]
+    const int n = blockIdx.x * FEW_COLS + threadIdx.x;
+    const WT* w = W + (size_t)min(n, N - 1) * K;
+    float acc[FEW_ROWS] = {}, ahead[FEW_AHEAD][4];
+    // No kernel writes the weights: the first pieces are asked for before the wait.
+#pragma unroll
+    for (int i = 0; i < FEW_AHEAD; ++i)
+        if (4 * i < K) four(w + 4 * i, ahead[i]);
+    pdl_wait();
+    for (int i = threadIdx.x; i < M * K; i += FEW_COLS) rows[i] = to_float(A[i]);
+    __syncthreads();
+    for (int k0 = 0; k0 < K; k0 += 4 * FEW_AHEAD) {
+        float now[FEW_AHEAD][4];
+#pragma unroll
+        for (int i = 0; i < FEW_AHEAD; ++i) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) now[i][u] = ahead[i][u];
+            const int next = k0 + 4 * (FEW_AHEAD + i);
+            if (next < K) four(w + next, ahead[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < FEW_AHEAD; ++i) {
+            if (k0 + 4 * i >= K) continue;
+#pragma unroll
+            for (int m = 0; m < FEW_ROWS; ++m) {
+                if (m >= M) continue;
+                const float4 a = *reinterpret_cast<const float4*>(rows + m * K + k0 + 4 * i);
+                acc[m] = fmaf(a.x, now[i][0], acc[m]);
+                acc[m] = fmaf(a.y, now[i][1], acc[m]);
+                acc[m] = fmaf(a.z, now[i][2], acc[m]);
+                acc[m] = fmaf(a.w, now[i][3], acc[m]);
+            }
+        }
+    }
+    if (n >= N) return;
+#pragma unroll
+    for (int m = 0; m < FEW_ROWS; ++m) {
+        if (m >= M) continue;
+        float* c = C + (size_t)m * N + n;
+        *c = accumulate ? *c + acc[m] : acc[m];
+    }
+}
 }  // namespace
 
 LLMX_EXPORT int llmx_gemm_plain(const void* A, int a_dtype, const void* W, int w_dtype, float* C, int M, int N, int K,
                                 int accumulate, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return LLMX_ERR_BAD_ARGUMENT;
+    const size_t few_bytes = (size_t)M * K * sizeof(float);
+    if (M <= FEW_ROWS && K % 4 == 0 && few_bytes <= FEW_BYTES && !((uintptr_t)W & 15) && a_dtype == w_dtype) {
+        const dim3 few((N + FEW_COLS - 1) / FEW_COLS);
+        if (a_dtype == LLMX_F32)
+            launch_kernel(gemm_plain_few_kernel<float, float>, few, dim3(FEW_COLS), few_bytes, stream, (const float*)A, (const float*)W, C, M, N, K, accumulate);
+        else if (a_dtype == LLMX_BF16)
+            launch_kernel(gemm_plain_few_kernel<__nv_bfloat16, __nv_bfloat16>, few, dim3(FEW_COLS), few_bytes, stream, (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, C, M, N, K, accumulate);
+        else
+            return LLMX_ERR_UNSUPPORTED;
+        return launch_status();
+    }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return LLMX_ERR_UNSUPPORTED;
     if (a_dtype == LLMX_F32 && w_dtype == LLMX_F32)
