@@ -3,7 +3,9 @@
 // reciprocal (a few units in the last place, far below the bfloat16 rounding that follows): with short inner widths the
 // epilogue, not the products, sets the kernel's time.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace {
 
@@ -24,6 +26,31 @@ __device__ __forceinline__ float act_gated(const ActEpilogue& a, float g, float 
         return __fdividef(g, 1.0f + __expf(-a.alpha * g)) * (u + 1.0f);
     }
     return __fdividef(g, 1.0f + __expf(-g)) * u;
+}
+
+// 32 tokens of one output column: out[j * stride] = act(g[j], u[j]) for j < left.  All values are made before any is stored, and
+// a full run of tokens has no condition: with the condition around each store the compiler put each value's chain (exponential,
+// reciprocal) behind its own branch, and a tile's epilogue took 13 us where its products over 1,024 take 4 (1,722 tokens x 2 x
+// 3,072 over 1,024: 47.6 -> 24.6 us).
+template <int N>
+__device__ __forceinline__ void store_gated(const ActEpilogue& a, const uint32_t (&g)[N], const uint32_t (&u)[N], __nv_bfloat16* out,
+                                            size_t stride, int left) {
+    __nv_bfloat16 v[N];
+    if (a.kind == ACT_CLAMPED) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j] = __float2bfloat16_rn(act_gated({ACT_CLAMPED, a.limit, a.alpha}, __uint_as_float(g[j]), __uint_as_float(u[j])));
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j] = __float2bfloat16_rn(act_gated({ACT_SWIGLU, 0.0f, 0.0f}, __uint_as_float(g[j]), __uint_as_float(u[j])));
+    }
+    if (left >= N) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) out[(size_t)j * stride] = v[j];
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (j < left) out[(size_t)j * stride] = v[j];
+    }
 }
 
 __device__ __forceinline__ float act_single(float x) {

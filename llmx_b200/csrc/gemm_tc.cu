@@ -323,12 +323,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         tc::tmem_wait_ld();
                         if (n < N) {
                             __nv_bfloat16* C = (__nv_bfloat16*)C_ + (size_t)(w.mt * BN + c) * N + n;
-                            const int m_left = M - (w.mt * BN + c);
-#pragma unroll
-                            for (int j = 0; j < CH; ++j) {
-                                const float act = act_gated(ae, __uint_as_float(r[j]), __uint_as_float(u[j]));
-                                if (j < m_left) C[(size_t)j * N] = __float2bfloat16_rn(act);
-                            }
+                            store_gated(ae, r, u, C, (size_t)N, M - (w.mt * BN + c));
                         }
                     } else {
                         tc::tmem_wait_ld();

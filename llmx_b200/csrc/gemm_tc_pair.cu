@@ -310,12 +310,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
                         tc::tmem_wait_ld();
                         if (n < N) {
                             __nv_bfloat16* out = (__nv_bfloat16*)C_ + (size_t)(w.mt * BN + c) * N + n;
-                            const int m_left = M - (w.mt * BN + c);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                const float act = act_gated(ae, __uint_as_float(r[j]), __uint_as_float(u[j]));
-                                if (j < m_left) out[(size_t)j * N] = __float2bfloat16_rn(act);
-                            }
+                            store_gated(ae, r, u, out, (size_t)N, M - (w.mt * BN + c));
                         }
                         continue;
                     }
