@@ -31,44 +31,70 @@ struct Glu {
     float limit, alpha;
 };
 __device__ __forceinline__ float glu_f(const Glu& a, float g, float u) {
-    if (!a.clamped) return g / (1.0f + expf(-g)) * u;
+    if (!a.clamped) return quotient(g, 1.0f + expf(-g)) * u;
     g = fminf(g, a.limit);
     u = fminf(fmaxf(u, -a.limit), a.limit);
-    return g / (1.0f + expf(-a.alpha * g)) * (u + 1.0f);
+    return quotient(g, 1.0f + expf(-a.alpha * g)) * (u + 1.0f);
 }
 
-__global__ void __launch_bounds__(256)
+// A block's threads look up ROUTE_AHEAD pairs each before any is counted; the places follow the pairs' order: a ballot within a
+// warp, a scan over the (turn, warp) counts of the chunk by the first warp.  4,096 pairs: 23.6 -> 6.1 us.
+constexpr int ROUTE_THREADS = 1024, ROUTE_WARPS = ROUTE_THREADS / 32, ROUTE_AHEAD = 4;
+
+__global__ void __launch_bounds__(ROUTE_THREADS)
 route_kernel(const int* __restrict__ token_ids, const int* __restrict__ table, int top, int rows, int experts, int vocab,
              int* __restrict__ lists, int* __restrict__ counts) {
     pdl_trigger();
     pdl_wait();
-    __shared__ int warp_count[8];
-    __shared__ int base;
+    __shared__ int place[ROUTE_AHEAD * ROUTE_WARPS];     // counts, then the places where the turns' and warps' pairs begin
+    __shared__ int total;
     const int e = blockIdx.x;
     const int pairs = rows * top;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();
-    for (int p0 = 0; p0 < pairs; p0 += 256) {
-        const int p = p0 + threadIdx.x;
-        bool mine = false;
-        if (p < pairs) {
-            const int tok = token_ids ? token_ids[p / top] : p / top;      // no ids: the table has a row for each row of the step
-            mine = tok >= 0 && tok < vocab && table[(size_t)tok * top + p % top] == e;
+    int base = 0;
+    for (int p0 = 0; p0 < pairs; p0 += ROUTE_THREADS * ROUTE_AHEAD) {
+        int tok[ROUTE_AHEAD];
+        bool mine[ROUTE_AHEAD];
+#pragma unroll
+        for (int i = 0; i < ROUTE_AHEAD; ++i) {
+            const int p = p0 + i * ROUTE_THREADS + threadIdx.x;
+            tok[i] = p >= pairs ? -1 : token_ids ? token_ids[p / top] : p / top;      // no ids: the table has a row for each row of the step
         }
-        const unsigned ballot = __ballot_sync(0xffffffffu, mine);
-        if (lane == 0) warp_count[warp] = __popc(ballot);
-        __syncthreads();
-        int before = base;
-        for (int w = 0; w < warp; ++w) before += warp_count[w];
-        if (mine) lists[(size_t)e * pairs + before + __popc(ballot & ((1u << lane) - 1u))] = p;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int total = 0;
-            for (int w = 0; w < 8; ++w) total += warp_count[w];
-            base += total;
+#pragma unroll
+        for (int i = 0; i < ROUTE_AHEAD; ++i) {
+            const int p = p0 + i * ROUTE_THREADS + threadIdx.x;
+            mine[i] = tok[i] >= 0 && tok[i] < vocab && table[(size_t)tok[i] * top + p % top] == e;
+        }
+        unsigned ballot[ROUTE_AHEAD];
+#pragma unroll
+        for (int i = 0; i < ROUTE_AHEAD; ++i) {
+            ballot[i] = __ballot_sync(0xffffffffu, mine[i]);
+            if (lane == 0) place[i * ROUTE_WARPS + warp] = __popc(ballot[i]);
         }
         __syncthreads();
+        if (warp == 0) {
+            int at = base;
+#pragma unroll
+            for (int i = 0; i < ROUTE_AHEAD; ++i) {
+                const int n = place[i * ROUTE_WARPS + lane];
+                int upto = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += below;
+                }
+                place[i * ROUTE_WARPS + lane] = at + upto - n;
+                at += __shfl_sync(0xffffffffu, upto, 31);
+            }
+            if (lane == 0) total = at;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ROUTE_AHEAD; ++i)
+            if (mine[i])
+                lists[(size_t)e * pairs + place[i * ROUTE_WARPS + warp] + __popc(ballot[i] & ((1u << lane) - 1u))] = p0 + i * ROUTE_THREADS + threadIdx.x;
+        base = total;
+        __syncthreads();                                 // the counts may be written again
     }
     if (threadIdx.x == 0) counts[e] = base;
 }
@@ -164,7 +190,8 @@ moe_cores_kernel(const T* __restrict__ a, int a_div, const T* __restrict__ w, co
 // (M = 128, twice) and the gathered rows as B (N = the tile's pairs, rounded up to 16).  The two halves of 128 weight rows
 // are, gated, the gate rows and the up rows of the same 128 output columns, so that a thread holds both of an output and
 // writes the gated unit; else 256 output columns.  The halves' sums fill tensor memory (2 x 256 columns).
-//   warp 0       the weights: K in steps of 64 through three stages, two TMA boxes a step
+//   warp 0       the weights: K in steps of 64 through three to five stages (as many as the tile's pairs leave room for), two
+//                TMA boxes a step
 //   warp 1       the products, issued by one thread
 //   warps 2-9    the pairs' rows of a step, gathered by cp.async in pieces of 16 bytes laid out as the 128-byte swizzle wants
 //                them (a TMA gather of four rows an instruction took three times as long as the products); then the epilogue: a
@@ -173,16 +200,16 @@ moe_cores_kernel(const T* __restrict__ a, int a_div, const T* __restrict__ w, co
 // An expert's list is cut into ceil(pairs / 256) equal tiles: its weights are read that often, and no tile is left with a few
 // pairs.  Of the routing's tiles of 128 pairs the expert's first ones stand for these, the others' blocks return.  Tiles are
 // the grid's fast dimension, so tiles of one expert read the same weights at the same time.
-// 2,048 rows x 2 of 16 experts, 2,048 -> 2 x 1,536 and back: 259 -> 134 us and 141 -> 73 us against the same tiles on
-// mma.sync; 1,201 rows x 2 of 16, 4,096 -> 2 x 3,072 and back: 718 -> 253 us and 374 -> 121 us, where reading the weights
-// once takes 123 and 62 us: bound by how soon a step's rows and weights arrive (three stages in flight) and by the last
-// wave's blocks.
+// 2,048 rows x 2 of 16 experts, 2,048 -> 2 x 1,536 and back: 259 -> 99 us and 141 -> 51 us against tiles of 128 pairs on
+// mma.sync; 1,201 rows x 2 of 16, 4,096 -> 2 x 3,072 and back: 718 -> 189 us and 374 -> 87 us, where reading the weights
+// once takes 123 and 62 us: bound by how soon a step's rows and weights arrive and by the last wave's blocks.  (Handing the
+// rows over two steps late with three stages made every product wait for the one before: 134, 73, 253 and 121 us.)
 constexpr int TC_LIST_TILE = 128;                                            // pairs a tile of the routing holds for this form
-constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_STAGES = 3;
+constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_MAX_STAGES = 5;
 constexpr int TC_W_BYTES = TC_M * TC_K * 2;                                  // one half's weights of a stage
-constexpr int TC_STAGE_BYTES = 2 * TC_W_BYTES + TC_ROWS * TC_K * 2;
+constexpr int TC_ROOM = 224 * 1024;                                          // shared memory of the stages
 constexpr int TC_ROW_WARPS = 8, TC_THREADS = 64 + TC_ROW_WARPS * 32;
-constexpr size_t TC_SMEM = (size_t)TC_STAGES * TC_STAGE_BYTES + 1024;
+constexpr size_t TC_SMEM = TC_ROOM + 1024;
 enum : int { ERR_MOE_PRODUCER = 441, ERR_MOE_MMA = 442, ERR_MOE_EPILOGUE = 443 };
 
 __device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst, const void* src, bool real) {
@@ -204,7 +231,7 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
     const int step = ((count + parts - 1) / parts + 15) & ~15, at = part * step;
     extern __shared__ uint8_t tc_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[TC_STAGES], empty[TC_STAGES], done;
+    __shared__ uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES], done;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     __shared__ int src_pair[TC_ROWS];
@@ -212,9 +239,10 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_here = min(step, count - at);
     const int n16 = (n_here + 15) & ~15;
+    const int stage_bytes = 2 * TC_W_BYTES + n16 * TC_K * 2, stages = min(TC_MAX_STAGES, TC_ROOM / stage_bytes);
     const int* list = lists + (size_t)e * pairs + at;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < TC_STAGES; ++i) {
+        for (int i = 0; i < TC_MAX_STAGES; ++i) {
             tc::mbar_init(&full[i], 1 + TC_ROW_WARPS);
             tc::mbar_init(&empty[i], 1);
         }
@@ -239,25 +267,26 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
     if (warp == 0) {
         const int w_row = e * (GATED ? 2 * N : N) + col0;
         if (tc::elect_one()) {
+            uint32_t st = 0, phase = 1;
             for (int s = 0; s < steps; ++s) {
-                const int st = s % TC_STAGES;
-                if (!tc::mbar_wait(&empty[st], ((s / TC_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_MOE_PRODUCER)) break;
-                uint8_t* base = smem + st * TC_STAGE_BYTES;
+                if (!tc::mbar_wait(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER)) break;
+                uint8_t* base = smem + st * stage_bytes;
                 tc::mbar_expect_tx(&full[st], 2 * TC_W_BYTES);
                 tc::tma_load_2d(base, &w_map, s * TC_K, w_row, &full[st]);
                 tc::tma_load_2d(base + TC_W_BYTES, &w_map, s * TC_K, w_row + (GATED ? N : TC_M), &full[st]);
+                if ((int)++st == stages) { st = 0; phase ^= 1; }
             }
         }
     } else if (warp == 1) {
         if (tc::elect_one()) {
             const uint32_t idesc = tc::instr_desc_bf16(TC_M, n16);
             bool ok = true;
+            uint32_t st = 0, phase = 0;
             for (int s = 0; s < steps; ++s) {
-                const int st = s % TC_STAGES;
-                ok = tc::mbar_wait(&full[st], (s / TC_STAGES) & 1u, abort_flag, error_word, ERR_MOE_MMA);
+                ok = tc::mbar_wait(&full[st], phase, abort_flag, error_word, ERR_MOE_MMA);
                 if (!ok) break;
                 tc::tc_fence_after();
-                const uint32_t w_addr = tc::smem_u32(smem + st * TC_STAGE_BYTES), b_addr = w_addr + 2 * TC_W_BYTES;
+                const uint32_t w_addr = tc::smem_u32(smem + st * stage_bytes), b_addr = w_addr + 2 * TC_W_BYTES;
 #pragma unroll
                 for (int kk = 0; kk < TC_K / 16; ++kk)
 #pragma unroll
@@ -265,6 +294,7 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
                         tc::mma_bf16_ss(tmem_base + h * TC_ROWS, tc::smem_desc_k_sw128(w_addr + h * TC_W_BYTES + kk * 32),
                                         tc::smem_desc_k_sw128(b_addr + kk * 32), idesc, (s > 0 || kk > 0) ? 1u : 0u);
                 tc::mma_commit(&empty[st]);
+                if ((int)++st == stages) { st = 0; phase ^= 1; }
             }
             if (ok) tc::mma_commit(&done);
         }
@@ -279,32 +309,38 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
         }
         const uint4* src = reinterpret_cast<const uint4*>(a);
         const uint32_t place = tc::smem_u32(smem) + 2 * TC_W_BYTES + first * 128 + ((piece ^ (first & 7)) << 4);
-        // A stage's rows are handed over two steps later, when they have landed: a fence makes them visible to the products.
-        auto hand_over = [&](int s) {
+        // A stage's rows are handed over `stages` - 2 steps later, when they have landed (a fence makes them visible to the
+        // products): the stage whose turn it is then has been free for a step, so that no product waits for the one before.
+        const int lag = stages - 2;
+        uint32_t st = 0, phase = 1, ready = 0;
+        auto hand_over = [&]() {
             tc::fence_proxy_async();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&full[s % TC_STAGES]);
+            if (lane == 0) tc::mbar_arrive(&full[ready]);
+            if ((int)++ready == stages) ready = 0;
         };
         bool ok = true;
         for (int s = 0; s < steps; ++s) {
-            const int st = s % TC_STAGES;
-            ok = tc::mbar_wait(&empty[st], ((s / TC_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_MOE_PRODUCER);
+            ok = tc::mbar_wait(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             const bool real = 64 * s + 8 * piece < K;
 #pragma unroll
             for (int i = 0; i < TC_ROWS / 32; ++i)
                 if (32 * i < n16 && first + 32 * i < n16)
-                    cp_async_16_or_zeros(place + st * TC_STAGE_BYTES + i * 32 * 128, src + (real && at16[i] >= 0 ? at16[i] + 8 * s : 0), real && at16[i] >= 0);
+                    cp_async_16_or_zeros(place + st * stage_bytes + i * 32 * 128, src + (real && at16[i] >= 0 ? at16[i] + 8 * s : 0), real && at16[i] >= 0);
             asm volatile("cp.async.commit_group;" ::: "memory");
-            if (s >= 2) {
-                asm volatile("cp.async.wait_group 2;" ::: "memory");
-                hand_over(s - 2);
+            if ((int)++st == stages) { st = 0; phase ^= 1; }
+            if (s >= lag) {
+                if (lag == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else if (lag == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+                else asm volatile("cp.async.wait_group 3;" ::: "memory");
+                hand_over();
             }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (ok)
-            for (int s = max(0, steps - 2); s < steps; ++s) hand_over(s);
+            for (int s = max(0, steps - lag); s < steps; ++s) hand_over();
         ok = ok && tc::mbar_wait(&done, 0, abort_flag, error_word, ERR_MOE_EPILOGUE);
         tc::tc_fence_after();
         // A warp may touch the tensor-memory lanes 32 (warp % 4) .. + 31; of two warps with the same lanes each takes every
@@ -316,18 +352,21 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
             tc::tmem_ld_32x16(lanes + p0, v[0]);
             tc::tmem_ld_32x16(lanes + TC_ROWS + p0, v[1]);
             tc::tmem_wait_ld();
+            // All values are made before any is stored: with the conditions around each, their chains ran one after another.
+            OutT x0[16], x1[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float a0 = __uint_as_float(v[0][i]), a1 = __uint_as_float(v[1][i]);
+                x0[i] = from_float<OutT>(GATED ? glu_f(glu, a0, a1) : a0);
+                x1[i] = from_float<OutT>(a1);
+            }
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int p = src_pair[p0 + i];
                 if (p < 0) break;                            // the tile's pairs come first
                 OutT* row = out + (size_t)p * N;
-                const float x0 = __uint_as_float(v[0][i]), x1 = __uint_as_float(v[1][i]);
-                if (GATED) {
-                    if (c < N) row[c] = from_float<OutT>(glu_f(glu, x0, x1));
-                } else {
-                    if (c < N) row[c] = from_float<OutT>(x0);
-                    if (c + TC_M < N) row[c + TC_M] = from_float<OutT>(x1);
-                }
+                if (c < N) row[c] = x0[i];
+                if (!GATED && c + TC_M < N) row[c + TC_M] = x1[i];
             }
         }
         tc::tc_fence_before();
@@ -392,6 +431,25 @@ moe_few_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv_bfloat
         if (GATED) s1 = warp_sum(s1);
         if (lane == 0) out[(size_t)p * N + c] = from_float<OutT>(GATED ? glu_f(glu, s0, s1) : s0);
     }
+}
+
+// Rows of whole groups of four values: a block a row and 1,024 of its values.  2,048 rows of 2,048, top 2: 25.6 -> 8.3 us.
+__global__ void __launch_bounds__(256)
+combine_vec_kernel(const float4* __restrict__ y, float4* __restrict__ x, int top, int n4, float weight) {
+    pdl_trigger();
+    pdl_wait();
+    const int c = blockIdx.y * 256 + threadIdx.x;
+    if (c >= n4) return;
+    const size_t row = blockIdx.x;
+    const float4* from = y + row * top * n4 + c;
+    float4* to = x + row * n4 + c;
+    float4 t = *to, s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int k = 0; k < top; ++k) {
+        const float4 v = from[(size_t)k * n4];
+        s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+    }
+    *to = make_float4(fmaf(weight, s.x, t.x), fmaf(weight, s.y, t.y), fmaf(weight, s.z, t.z), fmaf(weight, s.w, t.w));
 }
 
 __global__ void combine_kernel(const float* __restrict__ y, float* __restrict__ x, int top, int width, float weight,
@@ -716,7 +774,7 @@ LLMX_EXPORT int llmx_moe_route(const int* token_ids, const int* table, int top, 
                                int* counts, int* tiles, int tile_rows, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (top <= 0 || experts <= 0 || experts > 65535 || (tile_rows != TILE_ROWS && tile_rows != TC_LIST_TILE)) return LLMX_ERR_BAD_ARGUMENT;
-    launch_kernel(route_kernel, dim3(experts), dim3(256), 0, stream, token_ids, table, top, rows, experts, vocab, lists, counts);
+    launch_kernel(route_kernel, dim3(experts), dim3(ROUTE_THREADS), 0, stream, token_ids, table, top, rows, experts, vocab, lists, counts);
     int status = launch_status();
     if (status) return status;
     launch_kernel(tiles_kernel, dim3(1), dim3(32), 0, stream, (const int*)counts, experts, tiles, tile_rows);
@@ -798,6 +856,10 @@ LLMX_EXPORT int llmx_moe_product_few(const void* a, int a_div, const void* w, co
 // x [rows, width] += weight * sum over k of y [rows * top, width], k in increasing order.
 LLMX_EXPORT int llmx_moe_combine(const float* y, float* x, int rows, int top, int width, float weight, cudaStream_t stream) {
     if (rows <= 0) return 0;
+    if (width > 0 && width % 4 == 0 && width <= 4 * 256 * 65535 && !(((uintptr_t)y | (uintptr_t)x) & 15)) {
+        launch_kernel(combine_vec_kernel, dim3(rows, (width / 4 + 255) / 256), dim3(256), 0, stream, (const float4*)y, (float4*)x, top, width / 4, weight);
+        return launch_status();
+    }
     const long long n = (long long)rows * width;
     launch_kernel(combine_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, y, x, top, width, weight, n);
     return launch_status();

@@ -1030,3 +1030,33 @@ def test_plain_product_of_a_few_rows_is_the_tiled_one_bit_for_bit(dtype, M, N, K
             ops._check(ops._fn("gemm_plain", "llmx_gemm_plain")(ops._ptr(a), ops._code(a), ops._ptr(w), ops._code(w), ops._ptr(out), rows, N, K, accumulate,
                                                                 ops._stream()), "plain")
         assert torch.equal(few, many[:M])
+
+
+def test_gated_unit_at_extreme_inputs():
+    """silu(gate) * up of an expert over gates from subnormal exponentials to infinities, 32-bit output: the division's branchless form
+    within two units in the last place of 64 bits wherever those are normal numbers, and the same infinities and NaNs."""
+    from llmx_b200 import ops
+    gates = torch.tensor([0.0, -0.0, 1e-3, -1.0, 1.0, -20.0, -69.0, -70.0, -86.0, -88.0, -88.5, -90.0, -104.0, -1e4, 60.0, 2e38, float("inf"), float("-inf"),
+                          float("nan"), 5.5])
+    n = gates.numel()
+    h = torch.zeros(n, 32, dtype=torch.bfloat16)
+    h[:, 0], h[:, 1] = gates.bfloat16(), 1.5
+    gates = h[:, 0].double()
+    w = torch.zeros(1, 2 * 8, 32, dtype=torch.bfloat16)
+    w[0, :8, 0], w[0, 8:, 1] = 1.0, 1.0
+    choice = torch.zeros(n, 1, dtype=torch.int32, device=DEV)
+    lists, held = torch.empty((1, n), dtype=torch.int32, device=DEV), torch.empty((1,), dtype=torch.int32, device=DEV)
+    tiles = torch.empty((ops.moe_tiles_len(n, 1),), dtype=torch.int32, device=DEV)
+    finite = torch.isfinite(gates)
+    for rows in (finite, ~finite):           # a product row with an infinity has no number elsewhere: 0 * inf
+        x = torch.where(rows[:, None], h, torch.zeros_like(h)).to(DEV)
+        ops.moe_route(None, choice, 1, lists, held, tiles, tensor_cores=True)
+        out = torch.zeros(n, 8, device=DEV)
+        ops.moe_product(x, 1, w.to(DEV), lists, held, tiles, n, out, gated=True, tensor_cores=True)
+        got = out[:, 0].cpu().double()[rows]
+        if rows is finite:
+            want = 1.5 * gates[rows] / (1.0 + torch.exp(-gates[rows]))
+            normal = want.abs() > 2e-37
+            assert ((got - want).abs()[normal] <= 2.0 ** -21 * want.abs()[normal]).all() and (got[~normal].abs() <= 2.1e-37).all()
+        else:
+            assert torch.isnan(got[1:]).all() and (torch.isinf(got[0]) or torch.isnan(got[0]))
