@@ -86,10 +86,21 @@ __device__ __forceinline__ void load_row4(float4 (&v)[N], const float4* src, int
     }
 }
 
+// Calls launch(pieces) with the groups of four a thread holds, 1, 2, 4 or 8, as a constant: what it does not hold costs it no
+// registers (with eight for all, 2,048 rows of 2,048 gated took 23 us where two take 10).
+template <typename F>
+static void by_pieces(int n4, int threads, F&& launch) {
+    const int n = (n4 + threads - 1) / threads;
+    if (n <= 1) launch(std::integral_constant<int, 1>{});
+    else if (n <= 2) launch(std::integral_constant<int, 2>{});
+    else if (n <= 4) launch(std::integral_constant<int, 4>{});
+    else launch(std::integral_constant<int, 8>{});
+}
+
 // `zero` (optional): a float buffer of `zero_count` values (a multiple of 4, 16-byte aligned) that the launch
 // clears with blocks of its own (those beyond `rows`): the output of the product that follows, when that product
 // adds its pieces with atomics.
-template <typename OutT>
+template <typename OutT, int PIECES>
 __global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, OutT* __restrict__ y,
                                    const int* __restrict__ row_index, int rows, int width, float eps,
                                    float* __restrict__ zero, long long zero_count) {
@@ -98,7 +109,7 @@ __global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __r
     const int r = blockIdx.x, n4 = width >> 2;
     // No kernel writes the weights: they are read before the wait (with a few rows the norm's time is that of its reads:
     // four rows of 4,096 4.3 -> 2.7 us; a decode step of one Qwen3-0.6B request 863 -> 750 us).
-    float4 ww[NORM_VEC_MAX];
+    float4 ww[PIECES];
     if (r < rows) load_row4(ww, reinterpret_cast<const float4*>(w), n4);
     pdl_wait();
     if (r >= rows) {
@@ -110,11 +121,11 @@ __global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __r
             z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    float4 v[NORM_VEC_MAX];
+    float4 v[PIECES];
     load_row4(v, reinterpret_cast<const float4*>(x + (size_t)(row_index ? row_index[r] : r) * width), n4);
     float s = 0.0f;
 #pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+    for (int k = 0; k < PIECES; ++k) {
         s = fmaf(v[k].x, v[k].x, s);
         s = fmaf(v[k].y, v[k].y, s);
         s = fmaf(v[k].z, v[k].z, s);
@@ -124,7 +135,7 @@ __global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __r
     const float rr = 1.0f / sqrtf(s / (float)width + eps);
     OutT* dst = y + (size_t)r * width;
 #pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+    for (int k = 0; k < PIECES; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         if (i < n4) {
             store4(dst + 4 * i, v[k].x * (rr * ww[k].x), v[k].y * (rr * ww[k].y), v[k].z * (rr * ww[k].z), v[k].w * (rr * ww[k].w));
@@ -146,10 +157,13 @@ LLMX_EXPORT int llmx_rmsnorm(const float* x, const float* w, void* y, int out_dt
         long long zero_blocks = zero ? (zero_count / 4 + 4 * threads - 1) / (4 * threads) : 0;
         zero_blocks = zero_blocks > 1024 ? 1024 : zero_blocks;
         const dim3 grid((unsigned)(rows + zero_blocks));
-        if (out_dtype == LLMX_BF16)
-            launch_kernel(rmsnorm_vec_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream, x, w, (__nv_bfloat16*)y, row_index, rows, width, eps, zero, zero_count);
-        else
-            launch_kernel(rmsnorm_vec_kernel<float>, grid, dim3(threads), 0, stream, x, w, (float*)y, row_index, rows, width, eps, zero, zero_count);
+        by_pieces(n4, threads, [&](auto pieces) {
+            constexpr int P = decltype(pieces)::value;
+            if (out_dtype == LLMX_BF16)
+                launch_kernel(rmsnorm_vec_kernel<__nv_bfloat16, P>, grid, dim3(threads), 0, stream, x, w, (__nv_bfloat16*)y, row_index, rows, width, eps, zero, zero_count);
+            else
+                launch_kernel(rmsnorm_vec_kernel<float, P>, grid, dim3(threads), 0, stream, x, w, (float*)y, row_index, rows, width, eps, zero, zero_count);
+        });
         return launch_status();
     }
     if (zero && cudaMemsetAsync(zero, 0, (size_t)zero_count * sizeof(float), stream) != cudaSuccess) return launch_status();
@@ -692,14 +706,14 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const float* __res
 
 // The same for rows of whole groups of four values, up to 8,192 of them, without a bias and written to `y`: 16-byte reads, and the
 // weights, which no kernel writes, before the wait.  Eight rows of 2,048: 10.2 -> 3.1 us.
-template <typename OutT>
+template <typename OutT, int PIECES>
 __global__ void __launch_bounds__(256)
 layernorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, OutT* __restrict__ y, const int* __restrict__ row_index,
                      int rows, int width, float eps, float* __restrict__ zero, long long zero_count) {
     pdl_trigger();
     __shared__ float scratch[32];
     const int r = blockIdx.x, n4 = width >> 2;
-    float4 ww[NORM_VEC_MAX], v[NORM_VEC_MAX];
+    float4 ww[PIECES], v[PIECES];
     if (r < rows) load_row4(ww, reinterpret_cast<const float4*>(w), n4);
     pdl_wait();
     if (r >= rows) {
@@ -712,19 +726,19 @@ layernorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, O
     load_row4(v, reinterpret_cast<const float4*>(x + (size_t)(row_index ? row_index[r] : r) * width), n4);
     float s = 0.0f;
 #pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+    for (int k = 0; k < PIECES; ++k) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
     const float n = (float)width;            // divided by, as above
     const float mean = block_sum(s, scratch) / n;
     float q = 0.0f;
 #pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+    for (int k = 0; k < PIECES; ++k) {
         if ((int)(threadIdx.x + k * blockDim.x) >= n4) continue;
         v[k] = make_float4(v[k].x - mean, v[k].y - mean, v[k].z - mean, v[k].w - mean);
         q = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, q))));
     }
     const float rr = 1.0f / sqrtf(block_sum(q, scratch) / n + eps);
 #pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+    for (int k = 0; k < PIECES; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         if (i < n4) store4(y + (size_t)r * width + 4 * i, v[k].x * rr * ww[k].x, v[k].y * rr * ww[k].y, v[k].z * rr * ww[k].z, v[k].w * rr * ww[k].w);
     }
@@ -746,10 +760,13 @@ LLMX_EXPORT int llmx_layernorm_affine(const float* x, const float* in_bias, cons
         long long zero_blocks = zero ? (zero_count / 4 + 4 * threads - 1) / (4 * threads) : 0;
         zero_blocks = zero_blocks > 1024 ? 1024 : zero_blocks;
         const dim3 grid((unsigned)(rows + zero_blocks));
-        if (out_dtype == LLMX_BF16)
-            launch_kernel(layernorm_vec_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream, x, w, (__nv_bfloat16*)y, row_index, rows, width, eps, zero, zero_count);
-        else
-            launch_kernel(layernorm_vec_kernel<float>, grid, dim3(threads), 0, stream, x, w, (float*)y, row_index, rows, width, eps, zero, zero_count);
+        by_pieces(n4, threads, [&](auto pieces) {
+            constexpr int P = decltype(pieces)::value;
+            if (out_dtype == LLMX_BF16)
+                launch_kernel(layernorm_vec_kernel<__nv_bfloat16, P>, grid, dim3(threads), 0, stream, x, w, (__nv_bfloat16*)y, row_index, rows, width, eps, zero, zero_count);
+            else
+                launch_kernel(layernorm_vec_kernel<float, P>, grid, dim3(threads), 0, stream, x, w, (float*)y, row_index, rows, width, eps, zero, zero_count);
+        });
         return launch_status();
     }
     // The block width follows the row width alone, so a row's sums have one order whatever the batch.
@@ -1036,10 +1053,25 @@ __global__ void silu_columns_kernel(float* __restrict__ x, int stride, int c0, i
     *p = v / (1.0f + expf(-v));
 }
 
+// Columns in groups of four: a block a row and 1,024 of its columns.  2,048 rows of 6,144 columns: 52 -> 17 us.
+__global__ void __launch_bounds__(256) silu_columns_vec_kernel(float* __restrict__ x, int stride, int c0, int n4) {
+    pdl_trigger();
+    pdl_wait();
+    const int c = blockIdx.y * 256 + threadIdx.x;
+    if (c >= n4) return;
+    float4* p = reinterpret_cast<float4*>(x + (size_t)blockIdx.x * stride + c0) + c;
+    const float4 v = *p;
+    *p = make_float4(quotient(v.x, 1.0f + expf(-v.x)), quotient(v.y, 1.0f + expf(-v.y)), quotient(v.z, 1.0f + expf(-v.z)), quotient(v.w, 1.0f + expf(-v.w)));
+}
+
 LLMX_EXPORT int llmx_silu_columns(float* x, int rows, int stride, int c0, int n, cudaStream_t stream) {
     const long long total = (long long)rows * n;
     if (total <= 0) return 0;
     if (c0 < 0 || c0 + n > stride) return LLMX_ERR_BAD_ARGUMENT;
+    if (n % 4 == 0 && c0 % 4 == 0 && stride % 4 == 0 && n <= 4 * 256 * 65535 && !((uintptr_t)x & 15)) {
+        launch_kernel(silu_columns_vec_kernel, dim3(rows, (n / 4 + 255) / 256), dim3(256), 0, stream, x, stride, c0, n / 4);
+        return launch_status();
+    }
     launch_kernel(silu_columns_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, x, stride, c0, n, total);
     return launch_status();
 }
@@ -1128,7 +1160,7 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const float* _
 
 // The same for groups of whole fours, up to 8,192 values: the group and its gates in registers, 16-byte accesses, the weights
 // before the wait.  Eight rows of one group of 2,048: 9.9 -> 4.3 us.
-template <typename OutT>
+template <typename OutT, int PIECES>
 __global__ void __launch_bounds__(256)
 gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_stride, const float* __restrict__ w,
                          int w_len, OutT* __restrict__ y, int groups, int group, float eps, int gate_kind, int gate_first) {
@@ -1136,12 +1168,12 @@ gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ 
     __shared__ float scratch[32];
     const int r = blockIdx.x, j = blockIdx.y, n4 = group >> 2;
     const size_t base = ((size_t)r * groups + j) * group;
-    float4 ww[NORM_VEC_MAX], v[NORM_VEC_MAX], g[NORM_VEC_MAX];
+    float4 ww[PIECES], v[PIECES], g[PIECES];
     if (w) {
         load_row4(ww, reinterpret_cast<const float4*>(w + (size_t)j * group % w_len), n4);
     } else {
 #pragma unroll
-        for (int k = 0; k < NORM_VEC_MAX; ++k) ww[k] = make_float4(1.f, 1.f, 1.f, 1.f);
+        for (int k = 0; k < PIECES; ++k) ww[k] = make_float4(1.f, 1.f, 1.f, 1.f);
     }
     pdl_wait();
     load_row4(v, reinterpret_cast<const float4*>(o + base), n4);
@@ -1152,7 +1184,7 @@ gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ 
     };
     float s = 0.0f;
 #pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+    for (int k = 0; k < PIECES; ++k) {
         if ((int)(threadIdx.x + k * blockDim.x) >= n4) continue;
         g[k] = make_float4(act(g[k].x), act(g[k].y), act(g[k].z), act(g[k].w));
         if (gate_first) v[k] = make_float4(v[k].x * g[k].x, v[k].y * g[k].y, v[k].z * g[k].z, v[k].w * g[k].w);
@@ -1160,7 +1192,7 @@ gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ 
     }
     const float rr = 1.0f / sqrtf(block_sum(s, scratch) / (float)group + eps);
 #pragma unroll
-    for (int k = 0; k < NORM_VEC_MAX; ++k) {
+    for (int k = 0; k < PIECES; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         if (i >= n4) continue;
         if (gate_first) g[k] = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -1197,10 +1229,13 @@ LLMX_EXPORT int llmx_gated_rmsnorm(const float* o, const float* gate, int gate_s
     threads = threads < 32 ? 32 : threads > 256 ? 256 : threads;
     if (group % 4 == 0 && group <= 4 * NORM_VEC_MAX * 256 && gate_stride % 4 == 0 && (!w || (w_len % group == 0)) &&
         !(((uintptr_t)o | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)y) & 15)) {
-        if (out_dtype == LLMX_BF16)
-            launch_kernel(gated_rmsnorm_vec_kernel<__nv_bfloat16>, dim3(rows, groups), dim3(threads), 0, stream, o, gate, gate_stride, w, w_len, (__nv_bfloat16*)y, groups, group, eps, gate_kind, gate_first);
-        else
-            launch_kernel(gated_rmsnorm_vec_kernel<float>, dim3(rows, groups), dim3(threads), 0, stream, o, gate, gate_stride, w, w_len, (float*)y, groups, group, eps, gate_kind, gate_first);
+        by_pieces(group / 4, threads, [&](auto pieces) {
+            constexpr int P = decltype(pieces)::value;
+            if (out_dtype == LLMX_BF16)
+                launch_kernel(gated_rmsnorm_vec_kernel<__nv_bfloat16, P>, dim3(rows, groups), dim3(threads), 0, stream, o, gate, gate_stride, w, w_len, (__nv_bfloat16*)y, groups, group, eps, gate_kind, gate_first);
+            else
+                launch_kernel(gated_rmsnorm_vec_kernel<float, P>, dim3(rows, groups), dim3(threads), 0, stream, o, gate, gate_stride, w, w_len, (float*)y, groups, group, eps, gate_kind, gate_first);
+        });
         return launch_status();
     }
     if (out_dtype == LLMX_BF16)
@@ -1234,6 +1269,7 @@ pair_norm_add_kernel(const float* __restrict__ a, const float* __restrict__ b, c
 
 // The same for rows of whole groups of four, up to 8,192 values, both rows in registers.  Four rows of 4,096: 18 -> 6 us.
 constexpr int PAIR_MAX = 4, PAIR_THREADS = 512;
+template <int PIECES>
 __global__ void __launch_bounds__(PAIR_THREADS)
 pair_norm_add_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ wa,
                          const float* __restrict__ wb, float* __restrict__ x, int width, float eps, float factor) {
@@ -1241,7 +1277,7 @@ pair_norm_add_vec_kernel(const float* __restrict__ a, const float* __restrict__ 
     __shared__ float scratch[2][PAIR_THREADS / 32];
     const int n4 = width >> 2, warp = threadIdx.x >> 5;
     const size_t base = (size_t)blockIdx.x * width;
-    float4 va[PAIR_MAX], vb[PAIR_MAX], ua[PAIR_MAX], ub[PAIR_MAX], vx[PAIR_MAX];
+    float4 va[PIECES], vb[PIECES], ua[PIECES], ub[PIECES], vx[PIECES];
     load_row4(ua, reinterpret_cast<const float4*>(wa), n4);
     load_row4(ub, reinterpret_cast<const float4*>(wb), n4);
     pdl_wait();
@@ -1250,7 +1286,7 @@ pair_norm_add_vec_kernel(const float* __restrict__ a, const float* __restrict__ 
     load_row4(vx, reinterpret_cast<const float4*>(x + base), n4);
     float sa = 0.0f, sb = 0.0f;
 #pragma unroll
-    for (int k = 0; k < PAIR_MAX; ++k) {
+    for (int k = 0; k < PIECES; ++k) {
         sa = fmaf(va[k].x, va[k].x, fmaf(va[k].y, va[k].y, fmaf(va[k].z, va[k].z, fmaf(va[k].w, va[k].w, sa))));
         sb = fmaf(vb[k].x, vb[k].x, fmaf(vb[k].y, vb[k].y, fmaf(vb[k].z, vb[k].z, fmaf(vb[k].w, vb[k].w, sb))));
     }
@@ -1259,12 +1295,11 @@ pair_norm_add_vec_kernel(const float* __restrict__ a, const float* __restrict__ 
     if ((threadIdx.x & 31) == 0) scratch[0][warp] = sa, scratch[1][warp] = sb;
     __syncthreads();
     sa = sb = 0.0f;
-#pragma unroll
-    for (int g = 0; g < PAIR_THREADS / 32; ++g) sa += scratch[0][g], sb += scratch[1][g];
+    for (int g = 0; g < (int)blockDim.x / 32; ++g) sa += scratch[0][g], sb += scratch[1][g];
     const float ra = 1.0f / sqrtf(sa / (float)width + eps), rb = 1.0f / sqrtf(sb / (float)width + eps);
 #pragma unroll
-    for (int k = 0; k < PAIR_MAX; ++k) {
-        const int i = threadIdx.x + k * PAIR_THREADS;
+    for (int k = 0; k < PIECES; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
         if (i >= n4) continue;
         store4(x + base + 4 * i, vx[k].x + factor * (va[k].x * ra * ua[k].x + vb[k].x * rb * ub[k].x),
                vx[k].y + factor * (va[k].y * ra * ua[k].y + vb[k].y * rb * ub[k].y),
@@ -1279,7 +1314,14 @@ LLMX_EXPORT int llmx_pair_norm_add(const float* a, const float* b, const float* 
     if (width <= 0) return LLMX_ERR_BAD_ARGUMENT;
     if (width % 4 == 0 && width <= 4 * PAIR_MAX * PAIR_THREADS &&
         !(((uintptr_t)a | (uintptr_t)b | (uintptr_t)wa | (uintptr_t)wb | (uintptr_t)x) & 15)) {
-        launch_kernel(pair_norm_add_vec_kernel, dim3(rows), dim3(PAIR_THREADS), 0, stream, a, b, wa, wb, x, width, eps, factor);
+        // Two pieces a thread, so that a row of a prompt portion takes no more threads than it has work for.
+        int threads = ((width / 4 + 1) / 2 + 31) / 32 * 32;
+        threads = threads > PAIR_THREADS ? PAIR_THREADS : threads;
+        by_pieces(width / 4, threads, [&](auto pieces) {
+            constexpr int P = decltype(pieces)::value;
+            if constexpr (P <= PAIR_MAX)
+                launch_kernel(pair_norm_add_vec_kernel<P>, dim3(rows), dim3(threads), 0, stream, a, b, wa, wb, x, width, eps, factor);
+        });
         return launch_status();
     }
     launch_kernel(pair_norm_add_kernel, dim3(rows), dim3(256), 0, stream, a, b, wa, wb, x, width, eps, factor);
