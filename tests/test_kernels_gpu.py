@@ -1020,16 +1020,20 @@ def test_norms_of_rows_in_fours(rows, width):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 65, 36), (4, 4096, 256), (3, 130, 1000)])
-def test_plain_product_of_a_few_rows_is_the_tiled_one_bit_for_bit(dtype, M, N, K):
+def test_plain_products_of_few_and_many_rows_are_the_tiled_one_bit_for_bit(dtype, M, N, K):
     from llmx_b200 import ops
     g = torch.Generator().manual_seed(K)
-    a, w, c = torch.randn(70, K, generator=g).to(dtype).to(DEV), torch.randn(N, K, generator=g).to(dtype).to(DEV), torch.randn(70, N, generator=g).to(DEV)
+    a, w, c = torch.randn(130, K, generator=g).to(dtype).to(DEV), torch.randn(N, K, generator=g).to(dtype).to(DEV), torch.randn(130, N, generator=g).to(DEV)
     for accumulate in (0, 1):
-        few, many = c[:M].clone(), c.clone()
-        for out, rows in ((few, M), (many, 70)):
-            ops._check(ops._fn("gemm_plain", "llmx_gemm_plain")(ops._ptr(a), ops._code(a), ops._ptr(w), ops._code(w), ops._ptr(out), rows, N, K, accumulate,
-                                                                ops._stream()), "plain")
-        assert torch.equal(few, many[:M])
+        tiled, few, many = c[:40].clone(), c[:M].clone(), c.clone()
+        for out in (tiled, few, many):
+            ops._check(ops._fn("gemm_plain", "llmx_gemm_plain")(ops._ptr(a), ops._code(a), ops._ptr(w), ops._code(w), ops._ptr(out), out.shape[0], N, K,
+                                                                accumulate, ops._stream()), "plain")
+        assert torch.equal(few, tiled[:M]) and torch.equal(tiled, many[:40])
+        # K multiply-adds and at most one addition, each rounded once to 2^-24 of a partial sum: (K + 1) 2^-24 of the terms' sizes.
+        start = c.double() if accumulate else torch.zeros_like(c, dtype=torch.float64)
+        want, sizes = a.double() @ w.double().T + start, a.double().abs() @ w.double().abs().T + start.abs()
+        assert ((many.double() - want).abs() <= (K + 1) * 2.0 ** -24 * sizes).all()
 
 
 def test_gated_unit_at_extreme_inputs():
