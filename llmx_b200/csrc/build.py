@@ -46,6 +46,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "sampling": ["sampling.cu"],
     "recurrence": ["recurrence.cu"],          # matrix-state recurrences (decayed linear attention, gated delta rule, selective state space) and the short convolution
     "attention_split": ["attention_split.cu"],     # softmax attention with key and value widths of their own, windows and chunks
+    "attention_rows_tc": ["attention_rows_tc.cu"],     # the same for many rows, widths of 128
     "moe": ["moe.cu"],                        # experts chosen by a table: routing on the device, grouped products
     "latent_attention": ["latent_attention.cu"],   # attention over a cache of latents
     "latent_prompt_tc": ["latent_prompt_tc.cu"],    # the same for requests of many rows: keys and values made once a step

@@ -32,7 +32,7 @@
 //
 // Shapes: D = V = 128, R a multiple of 8 up to 64, C a multiple of 64, pages of a multiple of 16 tokens, bfloat16 cache
 // and maps.  Every wait on an mbarrier is bounded (tc_common.cuh).
-#include "attn_common.cuh"
+#include "attn_parts.cuh"
 #include <math.h>
 
 namespace {
@@ -57,34 +57,8 @@ constexpr uint32_t IDESC_QK = tc::instr_desc_bf16(ROWS, KEYS);
 constexpr uint32_t IDESC_PV = tc::instr_desc_bf16(ROWS, D) | (1u << 16);       // values: the MN-major operand
 constexpr uint32_t IDESC_EXPAND = tc::instr_desc_bf16(ROWS, D);
 
-// Shared-memory operand, MN-major, 128-byte swizzle: 64 elements of the MN dimension contiguous, the next 64 `block` bytes on.
-__device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr, uint32_t block) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(block >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-
-__device__ __forceinline__ float exp2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
 __device__ __forceinline__ void tmem_st_32x1(uint32_t addr, uint32_t v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr), "r"(v) : "memory");
-}
-
-// Three 8-bit pieces of a float's significand, cut off (not rounded) so that each remainder is exact: a pair of numbers
-// becomes three pairs of bfloat16, the first number in the low half.
-__device__ __forceinline__ void split3_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-    hi = __byte_perm(ua, ub, 0x7632);
-    const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
-    const uint32_t va = __float_as_uint(ra), vb = __float_as_uint(rb);
-    mid = __byte_perm(va, vb, 0x7632);
-    lo = __byte_perm(__float_as_uint(ra - __uint_as_float(va & 0xffff0000u)), __float_as_uint(rb - __uint_as_float(vb & 0xffff0000u)), 0x7632);
 }
 
 // The keys a request's rows see, from its first row's window to its last row's own; the workspace starts at the stage
@@ -209,7 +183,7 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid
                     uint32_t p[3][4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        split3_pair(__uint_as_float(v[i + 2 * u]), __uint_as_float(v[i + 2 * u + 1]), p[0][u], p[1][u], p[2][u]);
+                        attn::split3_pair(__uint_as_float(v[i + 2 * u]), __uint_as_float(v[i + 2 * u + 1]), p[0][u], p[1][u], p[2][u]);
 #pragma unroll
                     for (int q = 0; q < 3; ++q)
                         *reinterpret_cast<uint4*>(part + q * D + i) = real ? make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]) : zero;
@@ -330,7 +304,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
 #pragma unroll
                     for (int kk = 0; kk < KEYS / 16; ++kk)
                         tc::mma_bf16_ts(to, ts + PA[p] * P_PART + kk * 8,
-                                        smem_desc_mn_sw128(v_addr + 2 * PB[p] * BLOCK_BYTES + kk * 16 * 128, BLOCK_BYTES), IDESC_PV,
+                                        attn::smem_desc_mn_sw128(v_addr + 2 * PB[p] * BLOCK_BYTES + kk * 16 * 128, BLOCK_BYTES), IDESC_PV,
                                         (p > 0 || kk > 0) ? 1u : 0u);
                 tc::mma_commit(&v_empty[st]);
                 tc::mma_commit(o_full);
@@ -350,7 +324,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
                 const float2 x = *reinterpret_cast<const float2*>(src + c + 2 * u);
-                split3_pair(valid ? x.x * scale_log2 : 0.0f, valid ? x.y * scale_log2 : 0.0f, p[0][u], p[1][u], p[2][u]);
+                attn::split3_pair(valid ? x.x * scale_log2 : 0.0f, valid ? x.y * scale_log2 : 0.0f, p[0][u], p[1][u], p[2][u]);
             }
 #pragma unroll
             for (int k = 0; k < 3; ++k) tc::tmem_st_32x16(lanes + TMEM_Q + k * Q_PART + c / 2, p[k]);
@@ -370,7 +344,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
 #pragma unroll 1
         for (int e = 0; e < 64; e += 2) {
             uint32_t hi, mid, lo;
-            split3_pair(turned(e), turned(e + 1), hi, mid, lo);
+            attn::split3_pair(turned(e), turned(e + 1), hi, mid, lo);
             __syncwarp();
             tmem_st_32x1(lanes + TMEM_Q + Q_ROT + e / 2, hi);
             tmem_st_32x1(lanes + TMEM_Q + Q_PART + Q_ROT + e / 2, mid);
@@ -419,7 +393,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
 #pragma unroll
             for (int k = 0; k < KEYS; k += 8)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) mx[u] = max3(mx[u], __uint_as_float(sc[k + 2 * u]), __uint_as_float(sc[k + 2 * u + 1]));
+                for (int u = 0; u < 4; ++u) mx[u] = attn::max3(mx[u], __uint_as_float(sc[k + 2 * u]), __uint_as_float(sc[k + 2 * u + 1]));
             const float cand = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
             const bool raise = j > 0 && __any_sync(0xffffffffu, cand > m_used + RAISE);
             const float factor = !raise || cand == -INFINITY ? 1.0f : exp2f(m_used - cand);
@@ -431,9 +405,9 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
                 uint32_t p[3][16];
 #pragma unroll
                 for (int u = 0; u < 16; ++u) {
-                    const float a = exp2_approx(__uint_as_float(sc[c + 2 * u]) - base), b = exp2_approx(__uint_as_float(sc[c + 2 * u + 1]) - base);
+                    const float a = attn::exp2_approx(__uint_as_float(sc[c + 2 * u]) - base), b = attn::exp2_approx(__uint_as_float(sc[c + 2 * u + 1]) - base);
                     sum[u & 3] += a + b;
-                    split3_pair(a, b, p[0][u], p[1][u], p[2][u]);
+                    attn::split3_pair(a, b, p[0][u], p[1][u], p[2][u]);
                 }
 #pragma unroll
                 for (int k = 0; k < 3; ++k) tc::tmem_st_32x16(lanes + TMEM_S + k * P_PART + c / 2, p[k]);

@@ -126,6 +126,7 @@ _SIGNATURES = {
     ("attention_split", "llmx_attention_tiled_fits"): [_i, _i, _i, _i, _i],
     ("attention_split", "llmx_attention_tiled"): [_p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f,
                                                   _f, _p, _i, _p, _i, _i, _f, _f, _f, _p, _i, _p],
+    ("attention_rows_tc", "llmx_attention_rows_tc"): [_p, _p, ctypes.c_longlong, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p],
     ("moe", "llmx_moe_route"): [_p, _p, _i, _i, _i, _i, _p, _p, _p, _i, _p],
     ("moe", "llmx_moe_product_few"): [_p, _i, _p, _p, _p, _i, _i, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _p],
     ("moe", "llmx_moe_product"): [_p, _i, _p, _i, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _i, _p, _p],
@@ -824,6 +825,10 @@ class SoftmaxExtras:
     def maps(self) -> int:
         return 1 if self.difference is None else 2
 
+    @property
+    def plain(self) -> bool:
+        return not self.softcap and self.sink is None and self.vfreq is None and self.difference is None and self.gate is None
+
     def with_gate(self, gate: torch.Tensor) -> "SoftmaxExtras":
         return SoftmaxExtras(self.softcap, self.sink, self.vfreq, self.v_neighbours, self.difference, gate)
 
@@ -910,7 +915,9 @@ def attention_tiled(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, ste
                     extras: Optional["SoftmaxExtras"] = None) -> torch.Tensor:
     """`attention_split` on the tensor cores (csrc/attention_split.cu): bfloat16 q [rows, heads * D], out [rows, heads * V]
     and cache; 64 rows that share their keys a block, keys in tiles of 64; softmax weights enter the second product
-    as sums of three bfloat16 values.  `step`: the StepBatch (row ranges and histories are read on the device)."""
+    as sums of three bfloat16 values.  With widths of 128, pages of whole sixteens and a plain softmax, 128 rows a block by
+    tcgen05 (csrc/attention_rows_tc.cu).  `step`: the StepBatch (row ranges and histories are read on the device)."""
+    from .runtime import error_word
     _cuda(q, cache, out, block_tables)
     rows = q.shape[0]
     _need(q.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16, "attention_tiled: bfloat16 queries, output and cache")
@@ -919,6 +926,13 @@ def attention_tiled(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, ste
     _need(cache.dim() == 5 and cache.shape[1] == 1 and cache.shape[2] == kv_heads and cache.shape[4] == maps * key_dim + value_dim,
           "attention: cache layout does not fit")
     _need(block_tables.dtype == torch.int32 and block_tables.dim() == 2 and rows == step.rows, "attention: metadata does not fit")
+    if (key_dim == 128 and value_dim == 128 and cache.shape[3] % 16 == 0 and scale > 0 and heads // kv_heads <= 128 and (extras or NO_EXTRAS).plain
+            and cache.numel() // 256 < 2 ** 31):
+        _check(_fn("attention_rows_tc", "llmx_attention_rows_tc")(
+            _ptr(q), _ptr(cache), cache.numel() // 256, _ptr(out), _ptr(step.row_start), _ptr(step.row_count), _ptr(step.history),
+            _ptr(block_tables), block_tables.shape[1], rows, step.requests, heads, kv_heads, cache.shape[3], int(window or 0),
+            int(chunk or 0), float(scale), _ptr(error_word(q.device)), _stream()), "attention_rows_tc")
+        return out
     _check(_fn("attention_split", "llmx_attention_tiled")(
         _ptr(q), _ptr(cache), _ptr(out), _ptr(step.row_start), _ptr(step.row_count), _ptr(step.history), _ptr(block_tables),
         block_tables.shape[1], rows, step.requests, heads * maps, kv_heads, key_dim, value_dim, cache.shape[3], int(window or 0),

@@ -1064,3 +1064,49 @@ def test_gated_unit_at_extreme_inputs():
             assert ((got - want).abs()[normal] <= 2.0 ** -21 * want.abs()[normal]).all() and (got[~normal].abs() <= 2.1e-37).all()
         else:
             assert torch.isnan(got[1:]).all() and (torch.isinf(got[0]) or torch.isnan(got[0]))
+
+
+@pytest.mark.parametrize("heads,kv_heads,page,window,chunk", [(4, 1, 16, None, None), (3, 1, 32, 70, None), (32, 2, 48, None, 96), (2, 2, 16, 1, None), (10, 2, 16, 64, 200)])
+@pytest.mark.parametrize("counts,histories", [([5], [0]), ([128, 1, 33], [0, 63, 64]), ([65, 7], [700, 130]), ([300], [1])])
+def test_attention_of_rows_that_share_their_keys(heads, kv_heads, page, window, chunk, counts, histories):
+    """The tcgen05 form of the tiled attention against 64 bits: runs of rows below, at and above a tile, padded head groups, windows
+    and chunks that begin within a stage; every slot of the cache that no row may see holds NaN, pages below a window are
+    given back.  Weights keep 24 bits, so the result's own rounding (2^-9) decides."""
+    import types
+    from llmx_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(heads + page)
+    rows, scale = sum(counts), 0.1
+    needs = [-(-(h + n) // page) for h, n in zip(histories, counts)]
+    order = torch.randperm(sum(needs), generator=torch.Generator().manual_seed(1)).tolist()
+    tables, at = torch.full((len(counts), max(needs)), -1, dtype=torch.int32), 0
+    cache = torch.full((sum(needs) + 1, 1, kv_heads, page, 256), float("nan"), device="cuda", dtype=torch.bfloat16)
+    lowest = lambda p: max(max(0, p - window + 1) if window else 0, p // chunk * chunk if chunk else 0)
+    kv = []
+    for r, (n, h) in enumerate(zip(counts, histories)):
+        mine = order[at:at + needs[r]]
+        at += needs[r]
+        tables[r, :needs[r]] = torch.tensor(mine)
+        rows_r = torch.randn(h + n, kv_heads, 256, device="cuda", generator=g).bfloat16()
+        kv.append(rows_r.double())
+        lo = lowest(h)
+        t = torch.arange(lo, h + n, device="cuda")
+        cache[torch.tensor(mine, device="cuda")[t // page], 0, :, t % page] = rows_r[lo:]
+        tables[r, :lo // page] = -1
+    q = torch.randn(rows, heads * 128, device="cuda", generator=g).bfloat16()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    step = types.SimpleNamespace(row_start=i32([sum(counts[:r]) for r in range(len(counts))]), row_count=i32(counts), history=i32(histories), requests=len(counts),
+                                 rows=rows)
+    out = torch.zeros(rows, heads * 128, device="cuda", dtype=torch.bfloat16)
+    ops.attention_tiled(q, cache, out, step, tables.cuda(), heads, kv_heads, 128, 128, window, chunk, scale)
+    from llmx_b200.runtime import check_errors
+    check_errors()
+    row = 0
+    for r, (n, h) in enumerate(zip(counts, histories)):
+        k, v = (x.repeat_interleave(heads // kv_heads, 1) for x in kv[r].split(128, 2))
+        for p in range(h, h + n):
+            lo = lowest(p)
+            s = torch.einsum("hd,thd->ht", q[row].double().view(heads, 128), k[lo:p + 1]) * scale
+            want = torch.einsum("ht,thd->hd", torch.softmax(s, 1), v[lo:p + 1]).reshape(-1)
+            bound = 2.0 ** -8 * want.abs() + 2.0 ** -19 * (1.0 + s.abs().max()) * v[lo:p + 1].abs().max()
+            assert ((out[row].double() - want).abs() <= bound).all(), (r, p)
+            row += 1
