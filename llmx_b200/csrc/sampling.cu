@@ -17,7 +17,9 @@
 // each scans its slice of the vocabulary, their counts and sums meet in the first block's shared memory, which
 // decides (one block alone issues instructions for 150,000 scores at about 25 us a pass, whatever its loads do).
 // The top-k threshold is found by radix selection over the 32-bit order-preserving image of the score (counting
-// tokens).  When the kept set then fits shared memory (top-k of at most 1,024, the usual case) it is gathered
+// tokens): the pass that finds the best token also counts the leading eight bits, the next one lists each block's tokens at or
+// above the bin that holds the k-th, and what follows reads that list (a few hundred tokens) instead of the row.  32 rows of
+// 151,936, top-k 40: 50 -> 35 us.  When the kept set then fits shared memory (top-k of at most 1,024, the usual case) it is gathered
 // there, ranked, and the nucleus, min-p and the draw are one thread's walk over it with double sums, exactly the
 // reference's walk.  Without top-k (or a larger one) nothing is gathered: thresholds by radix selection over the
 // vocabulary, summing weights.
@@ -32,6 +34,8 @@ constexpr int TIES = 32;          // tokens with exactly the same score that are
 constexpr int MAX_CLUSTER = 8;    // blocks that share a row
 constexpr int NO_ID = 0x7fffffff;
 constexpr int STRIPES_BYTES = 256 * 32 * (8 + 4);
+constexpr int LISTED = 8192;      // tokens a block's list holds (ids and scores, where the stripes lie later)
+static_assert(LISTED * 8 <= STRIPES_BYTES, "the list lies in the stripes' memory");
 
 struct RowParams {
     float temperature, top_p, min_p, r;
@@ -131,7 +135,7 @@ struct Shared {
     uint32_t u32[4];
     double f64[4];
     int i32[8];
-    int n_hits, n_kept, walked;
+    int n_hits, n_kept, walked, n_listed;
     int hit_list[TIES];
     int c_id[KMAX], o_id[KMAX];
     uint32_t c_bits[KMAX], l_bits[KMAX];
@@ -198,6 +202,19 @@ __device__ __forceinline__ void scan_slice(const Row& c, F&& f) {
             f(id, ok ? row[id] : 0.0f, ok);
         }
     }
+}
+
+// The same over the block's list of `listed` tokens, or over its slice when there is no list (`listed` negative).  f may not use
+// warp-wide operations.
+template <typename F>
+__device__ __forceinline__ void scan_listed(const Row& c, int listed, F&& f) {
+    if (listed < 0) {
+        scan_slice(c, f);
+        return;
+    }
+    const int* ids = reinterpret_cast<const int*>(c.stripes);
+    const float* scores = reinterpret_cast<const float*>(ids + LISTED);
+    for (int i = threadIdx.x; i < listed; i += THREADS) f(ids[i], scores[i], true);
 }
 
 // Which tokens take part: all but the masked one; then the top-k set; then the nucleus.
@@ -279,9 +296,9 @@ __device__ __forceinline__ int find_bin(Amount&& amount, T above, Reached&& reac
 // are and the leader picks among them; more ties than the list holds are walked by the leader alone, chunk by chunk.
 // Every thread of the cluster returns the same id.
 template <int LEVEL>
-__device__ int nth_with_bits(const Row& c, uint32_t bits, int nth, const Sets& sets, float best_score, float temp) {
+__device__ int nth_with_bits(const Row& c, uint32_t bits, int nth, const Sets& sets, float best_score, float temp, int listed = -1) {
     Shared& sh = *c.sh;
-    scan_slice(c, [&](int id, float s, bool ok) {
+    scan_listed(c, listed, [&](int id, float s, bool ok) {
         if (!ok) return;
         const uint32_t b = order_bits(s);
         if (b != bits || !in_level<LEVEL>(sets, id, b, s, best_score, temp)) return;
@@ -342,53 +359,79 @@ __device__ int nth_with_bits(const Row& c, uint32_t bits, int nth, const Sets& s
     return lead_load(&sh.i32[5]);
 }
 
+// Counts of bins while scanning: most scores share their leading bits, so a thread keeps the count of the bin it met last and
+// adds it to the block's bins only when the bin changes.
+struct RunCount {
+    int bin = -1;
+    unsigned n = 0;
+    __device__ __forceinline__ void add(unsigned* count, int b) {
+        if (b != bin) {
+            flush(count);
+            bin = b;
+            n = 0;
+        }
+        ++n;
+    }
+    __device__ __forceinline__ void flush(unsigned* count) const {
+        if (n) atomicAdd(&count[bin], n);
+    }
+};
+
+// The leader's first warp: the bin of its counts that holds the `remaining`-th token from the top, and what is then left to find.
+__device__ __forceinline__ void find_count_bin(Shared& sh, int remaining) {
+    int above = 0;
+    int bin = find_bin<int>([&](int i) { return (int)sh.gcount[i]; }, 0,
+                            [&](int before, int after) { return after >= remaining && after > before; }, above);
+    if (bin < 0) { bin = 0; above = 0; for (int i = 1; i < 256; ++i) above += (int)sh.gcount[i]; }
+    if (threadIdx.x == 0) {
+        sh.u32[0] = (uint32_t)bin;
+        sh.i32[0] = remaining - above;
+        sh.i32[2] = sh.gmin_id[bin];
+    }
+}
+
 // Radix selection by count: the bits of the k-th best token (k >= 1) among the tokens that are not masked, how many
 // tokens with exactly those bits are among the k best, and the lowest id with those bits (the last round notes each
 // bin's, so that the usual case -- one token of the tie is taken -- needs no pass of its own).  A round: every block
 // counts its slice's tokens by the next eight bits, adds its bins to the leader's, and the leader finds the bin that
-// holds the k-th.
-__device__ void select_by_count(const Row& c, int k, const Sets& sets, uint32_t& out_bits, int& out_equal_taken,
-                                int& out_first_id) {
+// holds the k-th.  The first round was `best_token`'s.  The second lists the block's tokens at or above the first round's bin;
+// `listed` is their number, or -1 when they are more than the list holds (every block for itself).
+__device__ void select_by_count(const Row& c, const Sets& sets, uint32_t& out_bits, int& out_equal_taken, int& out_first_id, int& listed) {
     Shared& sh = *c.sh;
-    uint32_t prefix = 0, mask = 0;
-    int remaining = k;
-    for (int shift = 24; shift >= 0; shift -= 8) {
+    uint32_t prefix = lead_load(&sh.u32[0]) << 24, mask = 255u << 24;
+    int remaining = lead_load(&sh.i32[0]);
+    int* ids = reinterpret_cast<int*>(c.stripes);
+    float* scores = reinterpret_cast<float*>(ids + LISTED);
+    listed = -1;
+    for (int shift = 16; shift >= 0; shift -= 8) {
         for (int i = threadIdx.x; i < 256; i += THREADS) { sh.count[i] = 0; sh.min_id[i] = NO_ID; }
+        if (threadIdx.x == 0) sh.n_listed = 0;
         __syncthreads();
-        // Most scores share their leading bits: a thread keeps the count of the bin it met last and adds it to the
-        // block's bins only when the bin changes.
-        int run_bin = -1;
-        unsigned run = 0;
-        scan_slice(c, [&](int id, float s, bool ok) {
+        RunCount run;
+        scan_listed(c, listed, [&](int id, float s, bool ok) {
             const uint32_t b = order_bits(s);
-            if (!(ok && id != sets.skip && (b & mask) == prefix)) return;
+            if (!ok || id == sets.skip || b < prefix) return;
+            if (shift == 16) {
+                const int slot = atomicAdd(&sh.n_listed, 1);
+                if (slot < LISTED) {
+                    ids[slot] = id;
+                    scores[slot] = s;
+                }
+            }
+            if ((b & mask) != prefix) return;
             const int bin = (b >> shift) & 255u;
             if (shift == 0) atomicMin(&sh.min_id[bin], id);
-            if (bin != run_bin) {
-                if (run) atomicAdd(&sh.count[run_bin], run);
-                run_bin = bin;
-                run = 0;
-            }
-            ++run;
+            run.add(sh.count, bin);
         });
-        if (run) atomicAdd(&sh.count[run_bin], run);
+        run.flush(sh.count);
         __syncthreads();
+        if (shift == 16 && sh.n_listed <= LISTED) listed = sh.n_listed;
         if (threadIdx.x < 256 && sh.count[threadIdx.x]) {
             lead_add(&sh.gcount[threadIdx.x], sh.count[threadIdx.x]);
             if (shift == 0) lead_min(&sh.gmin_id[threadIdx.x], sh.min_id[threadIdx.x]);
         }
         leader_turn(c, [&] {
-            if (threadIdx.x < 32) {
-                int above = 0;
-                int bin = find_bin<int>([&](int i) { return (int)sh.gcount[i]; }, 0,
-                                        [&](int before, int after) { return after >= remaining && after > before; }, above);
-                if (bin < 0) { bin = 0; above = 0; for (int i = 1; i < 256; ++i) above += (int)sh.gcount[i]; }
-                if (threadIdx.x == 0) {
-                    sh.u32[0] = (uint32_t)bin;
-                    sh.i32[0] = remaining - above;
-                    sh.i32[2] = sh.gmin_id[bin];
-                }
-            }
+            if (threadIdx.x < 32) find_count_bin(sh, remaining);
             __syncthreads();
             if (threadIdx.x < 256) { sh.gcount[threadIdx.x] = 0; sh.gmin_id[threadIdx.x] = NO_ID; }      // for the next round
         });
@@ -511,15 +554,24 @@ __device__ void select_by_weight(const Row& c, double fraction, bool strict, con
 }
 
 // The best token: largest score, ties to the lowest id; a NaN only as the first token taking part
-// (src/inference/sampler.hpp:88-132).  Every thread of the cluster returns the same id.
-__device__ int best_token(const Row& c, int skip) {
+// (src/inference/sampler.hpp:88-132).  Every thread of the cluster returns the same id.  With k > 0 the same pass is the first
+// round of `select_by_count` for the k-th best: the leader leaves its bin in u32[0] and what is left to find in i32[0].
+__device__ int best_token(const Row& c, int skip, int k = 0) {
     Shared& sh = *c.sh;
+    if (k > 0) {
+        for (int i = threadIdx.x; i < 256; i += THREADS) sh.count[i] = 0;
+        __syncthreads();
+    }
+    RunCount run;
     const int first = skip == 0 ? 1 : 0;
     float bs = -INFINITY;
     int bi = first;
     scan_slice(c, [&](int id, float s, bool ok) {
-        if (ok && id != skip && (s > bs || (s == bs && id < bi))) { bs = s; bi = id; }
+        if (!ok || id == skip) return;
+        if (s > bs || (s == bs && id < bi)) { bs = s; bi = id; }
+        if (k > 0) run.add(sh.count, order_bits(s) >> 24);
     });
+    if (k > 0) run.flush(sh.count);
     for (int o = 16; o > 0; o >>= 1) {
         const float os = __shfl_xor_sync(0xffffffffu, bs, o);
         const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
@@ -533,7 +585,13 @@ __device__ int best_token(const Row& c, int skip) {
         lead_store(&sh.part_score[c.rank], bs);
         lead_store(&sh.part_id[c.rank], bi);
     }
+    if (k > 0 && threadIdx.x < 256 && sh.count[threadIdx.x]) lead_add(&sh.gcount[threadIdx.x], sh.count[threadIdx.x]);
     leader_turn(c, [&] {
+        if (k > 0) {
+            if (threadIdx.x < 32) find_count_bin(sh, k);
+            __syncthreads();
+            if (threadIdx.x < 256) sh.gcount[threadIdx.x] = 0;
+        }
         if (threadIdx.x == 0) {
             float s = sh.part_score[0];
             int i = sh.part_id[0];
@@ -583,7 +641,9 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(const float* __restrict
     sets.topk_last_id = sets.nuc_last_id = n;
     sets.min_p = 0.0f;
 
-    const int best = best_token(c, sets.skip);
+    const int m = sets.skip >= 0 ? n - 1 : n;
+    const int keep = (p.top_k > 0 && p.top_k < m) ? p.top_k : m;
+    const int best = best_token(c, sets.skip, p.temperature > 0.0f && keep < m ? keep : 0);
     const float best_score = row[best];
     sets.best = best;
     if (!(p.temperature > 0.0f)) {
@@ -592,15 +652,14 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(const float* __restrict
         return;
     }
     const float temp = p.temperature;
-    const int m = sets.skip >= 0 ? n - 1 : n;
-    const int keep = (p.top_k > 0 && p.top_k < m) ? p.top_k : m;
 
     // ---- top-k: the bits of the k-th best and the last id taken among its ties
+    int listed = -1;
     if (keep < m) {
         uint32_t bits;
         int taken, first;
-        select_by_count(c, keep, sets, bits, taken, first);
-        const int last = taken == 1 ? first : nth_with_bits<0>(c, bits, taken - 1, sets, best_score, temp);
+        select_by_count(c, sets, bits, taken, first, listed);
+        const int last = taken == 1 ? first : nth_with_bits<0>(c, bits, taken - 1, sets, best_score, temp, listed);
         sets.has_topk = true;
         sets.topk_bits = bits;
         sets.topk_last_id = last < 0 ? n : last;
@@ -615,7 +674,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(const float* __restrict
         __shared__ int n_mine, my_base;
         if (threadIdx.x == 0) n_mine = 0;
         __syncthreads();
-        scan_slice(c, [&](int id, float s, bool ok) {
+        scan_listed(c, listed, [&](int id, float s, bool ok) {
             if (!ok) return;
             const uint32_t b = order_bits(s);
             if (!in_kept(sets, id, b)) return;
