@@ -645,13 +645,15 @@ conv_prepare_kernel(const float* __restrict__ proj, int stride, int first, int c
 // its squares by shuffles.  A block has up to 1,024 channels of `run` rows, or those channels of a request's kept inputs, or
 // the gates of the rows: a few rows (decoding) spread over as many blocks as the channels make, where one block a row
 // took them 256 at a time, each waiting for the one before: 8 rows of
-// 4,096 channels 28 -> 5.6 us, 4 rows of 8,192 and 6,144 channels 45 -> 5.9 us.
-constexpr int CONV_THREADS = 256, CONV_RUN = 16, CONV_TAPS = 4;
+// 4,096 channels 28 -> 5.6 us, 4 rows of 8,192 and 6,144 channels 45 -> 5.9 us; 2,048 rows of 4,096 channels 51 -> 31 us, with
+// a decay per key channel 76 -> 60, 1,201 rows of 8,192 with such decays 129 -> 73 us (bound by its exponentials and
+// logarithms: 40 % of the issue slots with three blocks an SM).
+constexpr int CONV_THREADS = 256, CONV_RUN = 16, CONV_TAPS = 4, CONV_AHEAD = 2;
 
 __device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float silu_f(float y) { return y / (1.0f + expf(-y)); }
+__device__ __forceinline__ float silu_f(float y) { return quotient(y, 1.0f + expf(-y)); }
 
-__global__ void __launch_bounds__(CONV_THREADS)
+__global__ void __launch_bounds__(CONV_THREADS, 3)
 conv_prepare_four_kernel(const float* __restrict__ proj, int stride, int first, int channels, int q_channels, int k_channels,
                          const float* __restrict__ taps_w, const float* __restrict__ taps_b, int taps,
                          float* __restrict__ ready, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
@@ -660,11 +662,13 @@ conv_prepare_four_kernel(const float* __restrict__ proj, int stride, int first, 
                          float* __restrict__ state, long long slot_floats, long long conv_off,
                          const int* __restrict__ row_request, const int* __restrict__ row_start,
                          const int* __restrict__ row_count, const int* __restrict__ history, const int* __restrict__ slot_in,
-                         const int* __restrict__ slot_out, int rows, int run, int row_blocks, int conv_blocks) {
+                         const int* __restrict__ slot_out, int rows, int run, int row_blocks, int gate_blocks) {
     pdl_trigger();
     const int keep = taps - 1;
-    const int c = ((int)blockIdx.y * CONV_THREADS + (int)threadIdx.x) * 4;
-    const bool conv = (int)blockIdx.y < conv_blocks, mine = conv && c < channels;
+    // The gates' blocks come first: they are the longest.
+    const bool conv = (int)blockIdx.y >= gate_blocks;
+    const int c = (((int)blockIdx.y - gate_blocks) * CONV_THREADS + (int)threadIdx.x) * 4;
+    const bool mine = conv && c < channels;
     // The filter's weights are written by no kernel: they are read before the wait.  w[j]: tap j of the four channels.
     float4 w[CONV_TAPS], bias = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
@@ -698,28 +702,27 @@ conv_prepare_four_kernel(const float* __restrict__ proj, int stride, int first, 
     }
     const int row0 = blockIdx.x * run, row_end = min(rows, row0 + run);
     if (!conv) {
-        // Gates: `per` a row, in blocks of four a thread.
+        // Gates: `per` a row, a thread one of them for all of the block's rows.
         const int per = gate_kind == 2 ? heads * D : heads;
-        const int g0 = ((int)blockIdx.y - conv_blocks) * CONV_THREADS * 4;
-        const int here = min(per - g0, CONV_THREADS * 4);
-        for (int i = threadIdx.x; i < (row_end - row0) * here; i += CONV_THREADS) {
-            const int row = row0 + i / here, g = g0 + i % here;
+        const int g = (int)blockIdx.y * CONV_THREADS + (int)threadIdx.x;
+        if (g >= per) return;
+        const float rate = -expf(a_log[gate_kind == 2 ? g / D : g]), bias_g = dt_bias[g];
+#pragma unroll 4
+        for (int row = row0; row < row_end; ++row) {
             float* grow = gates + (size_t)row * gates_stride;
             const float* prow = proj + (size_t)row * stride;
+            const float z = (gate_kind == 2 ? decay_in[(size_t)row * decay_stride + g] : prow[a_off + g]) + bias_g;
+            const float beta = gate_kind != 1 && g < heads ? quotient(1.0f, 1.0f + expf(-prow[b_off + g])) : 0.0f;
             if (gate_kind == 2) {
-                const float z = decay_in[(size_t)row * decay_stride + g] + dt_bias[g];
-                grow[heads + g] = expf(-expf(a_log[g / D]) * softplus_f(z));
-                if (g < heads) grow[g] = 1.0f / (1.0f + expf(-prow[b_off + g]));
-                continue;
-            }
-            const float z = prow[a_off + g] + dt_bias[g];
-            if (gate_kind == 1) {
+                grow[heads + g] = expf(rate * softplus_f(z));
+                if (g < heads) grow[g] = beta;
+            } else if (gate_kind == 1) {
                 const float dt = z > 20.0f ? z : log1pf(expf(z));      // the same function beyond 20 up to rounding: no clamp of dt itself
-                grow[g] = expf(-expf(a_log[g]) * dt);
+                grow[g] = expf(rate * dt);
                 grow[heads + g] = dt;
             } else {
-                grow[g] = expf(-expf(a_log[g]) * softplus_f(z));
-                grow[heads + g] = 1.0f / (1.0f + expf(-prow[b_off + g]));
+                grow[g] = expf(rate * softplus_f(z));
+                grow[heads + g] = beta;
             }
         }
         return;
@@ -727,13 +730,20 @@ conv_prepare_four_kernel(const float* __restrict__ proj, int stride, int first, 
     const bool unit = c < q_channels + k_channels;   // the same for all lanes of a head: heads are whole
     const float factor = c < q_channels ? q_factor : 1.0f;
     float4 x[CONV_TAPS];                             // x[j]: the input under tap j
-    float4 next = mine ? load_four(proj + (size_t)row0 * stride + first + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 ahead[CONV_AHEAD];                        // the next rows' inputs
+#pragma unroll
+    for (int i = 0; i < CONV_AHEAD; ++i)
+        ahead[i] = mine && row0 + i < row_end ? load_four(proj + (size_t)(row0 + i) * stride + first + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     int left = 0;                                    // rows of the request at hand that are still to come
 #pragma unroll
     for (int j = 0; j < CONV_TAPS; ++j) x[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int row = row0; row < row_end; ++row) {
-        const float4 now = next;
-        if (mine && row + 1 < row_end) next = load_four(proj + (size_t)(row + 1) * stride + first + c);
+    for (int row1 = row0; row1 < row_end; row1 += CONV_AHEAD)
+#pragma unroll
+    for (int turn = 0; turn < CONV_AHEAD; ++turn) {
+        const int row = row1 + turn;
+        if (row >= row_end) break;
+        const float4 now = ahead[turn];
+        if (mine && row + CONV_AHEAD < row_end) ahead[turn] = load_four(proj + (size_t)(row + CONV_AHEAD) * stride + first + c);
         if (left == 0) {
             // The first row of the block or of a request: the inputs before it, from earlier rows or the state.
             const int r = row_request[row];
@@ -946,15 +956,15 @@ LLMX_EXPORT int llmx_conv_prepare(const float* proj, int stride, int first, int 
         (!units || (D % 4 == 0 && D <= 128 && ((D / 4) & (D / 4 - 1)) == 0)) &&
         (((uintptr_t)proj | (uintptr_t)ready | (uintptr_t)state | (uintptr_t)taps_b) & 15) == 0) {
         const int per = gate_kind == 2 ? heads * D : heads, block = CONV_THREADS * 4;
-        const int conv_blocks = (channels + block - 1) / block, gate_blocks = (per + block - 1) / block;
+        const int conv_blocks = (channels + block - 1) / block, gate_blocks = (per + CONV_THREADS - 1) / CONV_THREADS;
         // One row a block while that leaves the SMs' 296 places unfilled, longer runs of rows beyond.
         int run = (int)((long long)rows * conv_blocks / 592);
         run = run < 1 ? 1 : run > CONV_RUN ? CONV_RUN : run;
         const int row_blocks = (rows + run - 1) / run;
-        launch_kernel(conv_prepare_four_kernel, dim3(row_blocks + requests, conv_blocks + gate_blocks), dim3(CONV_THREADS), 0, stream, proj,
+        launch_kernel(conv_prepare_four_kernel, dim3(row_blocks + requests, gate_blocks + conv_blocks), dim3(CONV_THREADS), 0, stream, proj,
                       stride, first, channels, q_channels, k_channels, taps_w, taps_b, taps, ready, a_log, dt_bias, b_off, a_off,
                       gate_kind, decay_in, decay_stride, gates, gates_stride, heads, D, q_factor, state, slot_floats, conv_off,
-                      row_request, row_start, row_count, history, slot_in, slot_out, rows, run, row_blocks, conv_blocks);
+                      row_request, row_start, row_count, history, slot_in, slot_out, rows, run, row_blocks, gate_blocks);
         return launch_status();
     }
     if (smem > 48 * 1024) cudaFuncSetAttribute(conv_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
