@@ -61,6 +61,13 @@ __device__ __forceinline__ void tmem_st_32x1(uint32_t addr, uint32_t v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr), "r"(v) : "memory");
 }
 
+// Whether all 128 row threads say so (a barrier among them).
+__device__ __forceinline__ bool all_rows(bool mine) {
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(all) : "r"(mine ? 1u : 0u) : "memory");
+    return all != 0;
+}
+
 // The keys a request's rows see, from its first row's window to its last row's own; the workspace starts at the stage
 // boundary below.
 __device__ __forceinline__ int first_key(int pos_first, int window) {
@@ -69,14 +76,17 @@ __device__ __forceinline__ int first_key(int pos_first, int window) {
 
 // requests[4 i ..]: first row, rows, first workspace token, workspace tokens (a multiple of 128) of request i.
 // 128 keys x one head: two accumulators of 128 x 128 (key, value) over C in steps of 64 columns.  Bound by the writes to the
-// workspace (1,664 bytes a token and head); two blocks an SM, so one's writes run beside the other's products.
+// workspace (1,664 bytes a token and head); two blocks an SM, so one's writes run beside the other's products.  The parts are laid
+// out in shared memory (the operands' stages are free then) and leave by TMA, whole 128-byte lines: 2,048 tokens of 16
+// heads 52 -> 21 us, 5,003 tokens 135 -> 57, against 16-byte stores of 32 rows at a time.
 constexpr int EXPAND_STAGE = 3 * ROWS * 128;                // 128 keys, 128 + 128 rows of the maps, 64 columns each
 constexpr int EXPAND_STAGES = 2;
+static_assert(EXPAND_STAGES * EXPAND_STAGE >= 6 * ROWS * 128, "the parts of 128 keys or values");
 constexpr int EXPAND_SMEM = EXPAND_STAGES * EXPAND_STAGE + 1024 + 256;
 
 __global__ void __launch_bounds__(PROMPT_THREADS, 2)
 latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap uk_map,
-                     const __grid_constant__ CUtensorMap uv_map, const __nv_bfloat16* __restrict__ cache,
+                     const __grid_constant__ CUtensorMap uv_map, const __grid_constant__ CUtensorMap expanded_map, const __nv_bfloat16* __restrict__ cache,
                      __nv_bfloat16* __restrict__ expanded, const int* __restrict__ requests,
                      const int* __restrict__ row_request, const int* __restrict__ positions,
                      const int* __restrict__ block_tables, int table_stride, int tokens, int head0, int C, int R,
@@ -170,24 +180,41 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid
             cache + ((size_t)(real ? table[t / page_size] : 0) * page_size + t % page_size) * (C + R) + C);
 #pragma unroll
         for (int i = 0; i < 8; ++i) rot[i] = real && i * 8 < R ? src[i] : zero;
-        if (tc::mbar_wait(done, 0, abort_flag, error_word, ERR_LAT_EXPAND)) {
+        // The four warps of rows go on together or not at all: they meet at barriers below.
+        if (all_rows(tc::mbar_wait(done, 0, abort_flag, error_word, ERR_LAT_EXPAND))) {
             tc::tc_fence_after();
 #pragma unroll 1
-            for (int c = 0; c < 2 * D; c += 32) {              // 32 values of the key, then of the value
-                uint32_t v[32];
-                tc::tmem_ld_32x32(tmem_base + c + ((uint32_t)(quarter * 32) << 16), v);
-                tc::tmem_wait_ld();
-                __nv_bfloat16* part = dst + (c < D ? c : K_BLOCKS * 64 + c - D);
+            for (int which = 0; which < 2; ++which) {          // the keys' parts, then the values'
+#pragma unroll 1
+                for (int c = 0; c < D; c += 32) {
+                    uint32_t v[32];
+                    tc::tmem_ld_32x32(tmem_base + which * D + c + ((uint32_t)(quarter * 32) << 16), v);
+                    tc::tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    uint32_t p[3][4];
+                    for (int i = 0; i < 32; i += 8) {
+                        uint32_t p[3][4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        attn::split3_pair(__uint_as_float(v[i + 2 * u]), __uint_as_float(v[i + 2 * u + 1]), p[0][u], p[1][u], p[2][u]);
+                        for (int u = 0; u < 4; ++u)
+                            attn::split3_pair(__uint_as_float(v[i + 2 * u]), __uint_as_float(v[i + 2 * u + 1]), p[0][u], p[1][u], p[2][u]);
 #pragma unroll
-                    for (int q = 0; q < 3; ++q)
-                        *reinterpret_cast<uint4*>(part + q * D + i) = real ? make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]) : zero;
+                        for (int q = 0; q < 3; ++q)
+                            *reinterpret_cast<uint4*>(smem + (2 * q + (c >> 6)) * ROWS * 128 + attn::swz(row, ((c & 63) + i) >> 3)) =
+                                real ? make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]) : zero;
+                    }
                 }
+                tc::fence_proxy_async();
+                asm volatile("bar.sync 1, 128;" ::: "memory");                 // the four warps of rows
+                if (threadIdx.x == 64) {
+                    for (int b = 0; b < 12; ++b)
+                        asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];"
+                                     ::"l"(&expanded_map), "r"(tc::smem_u32(smem + (b >> 1) * ROWS * 128 + (b & 1) * BLOCK_BYTES)), "r"(0),
+                                     "r"(rq[2] + (int)blockIdx.x * ROWS + (b & 1) * KEYS), "r"((which ? K_BLOCKS : 0) + (b >> 1)), "r"((int)blockIdx.y),
+                                     "r"(0) : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    if (which == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    else asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");                 // the copies have read what the next half overwrites
             }
         }
         tc::tc_fence_before();
@@ -476,13 +503,14 @@ LLMX_EXPORT int llmx_latent_expand(const void* cache, long long pool_tokens, con
         pool_tokens <= 0 || tokens <= 0 || tokens % ROWS || max_tokens <= 0 || max_tokens % ROWS || head0 < 0 || head0 + n_heads > all_heads ||
         (((uintptr_t)cache | (uintptr_t)w_uk | (uintptr_t)w_uv | (uintptr_t)expanded) & 15))
         return LLMX_ERR_UNSUPPORTED;
-    CUtensorMap cache_map, uk_map, uv_map;
+    CUtensorMap cache_map, uk_map, uv_map, expanded_map;
+    if (int e = make_expanded_map(&expanded_map, expanded, (uint64_t)tokens, (uint64_t)n_heads)) return e;
     if (int e = llmx_make_map_bf16_2d(&cache_map, cache, (uint64_t)pool_tokens, (uint64_t)(C + R), 16, 64)) return e;
     if (int e = llmx_make_map_bf16_2d(&uk_map, w_uk, (uint64_t)all_heads * D, (uint64_t)C, D, 64)) return e;
     if (int e = llmx_make_map_bf16_2d(&uv_map, w_uv, (uint64_t)all_heads * D, (uint64_t)C, D, 64)) return e;
     if (int e = allow_smem(latent_expand_kernel, EXPAND_SMEM)) return e;
     launch_kernel(latent_expand_kernel, dim3(max_tokens / ROWS, n_heads, n_req), dim3(PROMPT_THREADS), (size_t)EXPAND_SMEM, stream, cache_map,
-                  uk_map, uv_map, (const __nv_bfloat16*)cache, (__nv_bfloat16*)expanded, requests, row_request, positions, block_tables,
+                  uk_map, uv_map, expanded_map, (const __nv_bfloat16*)cache, (__nv_bfloat16*)expanded, requests, row_request, positions, block_tables,
                   table_stride, tokens, head0, C, R, page_size, window, error_word);
     return launch_status();
 }
