@@ -21,6 +21,7 @@
 // The CUDA-core form checks its tiles' size against what the routing wrote (tiles[1]).
 #include "tc_common.cuh"
 #include <math.h>
+#include <type_traits>
 
 namespace {
 constexpr int TILE_ROWS = 32;     // pairs a tile holds
@@ -433,6 +434,139 @@ moe_few_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv_bfloat
     }
 }
 
+// The same for steps of up to FEW_PAIRS pairs whose weight rows fit shared memory several times (K up to FEW_K): the experts
+// that the pairs name, each once, as a stream.  A block an SM takes an equal run of the items (expert, two weight rows: the
+// gate and up rows of a column, or two columns); one thread brings them by bulk copies of whole rows into a ring of up to
+// 192 KB, so that the memory always has requests, and up to sixteen warps take the ring's places in turn: dot products with
+// the rows of all pairs that name the expert (which the L1 cache holds), the lanes' sums met by shuffles in a fixed order.
+// The warps' number divides the ring's places, so that a place is always the same warp's: a waiter tells uses of a place
+// apart by parity only, and a warp that came to a place before its last use had landed would take it for the next.
+// Eight pairs that name six experts, gate and up of K 4,096 and N 3,072: 70 -> 57 us, down 38.7 -> 32; two pairs 38.8 -> 22
+// and 15.4 -> 12.6 us.  Bound by the dot products more than by the memory where an expert's rows meet several pairs: sixteen
+// pairs on twelve experts took 204 us (eight warps) against the kernel above's 118, so the line lies at eight.
+constexpr int FEW_PAIRS = 8, FEW_WARPS = 16, FEW_THREADS = 32 * FEW_WARPS + 32, FEW_PLACES = 32, FEW_K = 12288, FEW_RING = 192 * 1024;
+enum : int { ERR_FEW_PRODUCER = 451, ERR_FEW_CONSUMER = 452 };
+
+template <bool GATED, typename OutT>
+__global__ void __launch_bounds__(FEW_THREADS, 1)
+moe_few_stream_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv_bfloat16* __restrict__ w,
+                      const int* __restrict__ token_ids, const int* __restrict__ table, int top, int vocab, int experts, int pairs,
+                      OutT* __restrict__ out, int N, int K, Glu glu, int places, int* error_word) {
+    const int workers = (int)blockDim.x / 32 - 1;
+    extern __shared__ __align__(128) unsigned char ring[];
+    __shared__ uint64_t full[FEW_PLACES], empty[FEW_PLACES];
+    __shared__ int abort_word;
+    // The experts that the pairs name, in the order of the first pair of each, and which pairs name each.
+    __shared__ int expert_of[FEW_PAIRS], named;
+    __shared__ unsigned pairs_of[FEW_PAIRS];
+    volatile int* abort_flag = &abort_word;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < places; ++i) {
+            tc::mbar_init(&full[i], 1);
+            tc::mbar_init(&empty[i], 1);
+        }
+        abort_word = 0;
+        tc::fence_barrier_init();
+    }
+    pdl_trigger();
+    pdl_wait();
+    if (warp == 0) {
+        int mine = -1;
+        if (lane < pairs) {
+            const int tok = token_ids ? token_ids[lane / top] : lane / top;
+            const int e = (tok >= 0 && tok < vocab) ? table[(size_t)tok * top + lane % top] : -1;
+            if (e >= 0 && e < experts) mine = e;
+        }
+        const unsigned who = __match_any_sync(0xffffffffu, mine), before = (1u << lane) - 1;
+        const bool first = mine >= 0 && !(who & before);
+        const unsigned firsts = __ballot_sync(0xffffffffu, first);
+        if (first) {
+            expert_of[__popc(firsts & before)] = mine;
+            pairs_of[__popc(firsts & before)] = who;
+        }
+        if (lane == 0) named = __popc(firsts);
+    }
+    __syncthreads();
+    const int per_expert = GATED ? N : (N + 1) / 2;
+    const int items = named * per_expert;
+    const int per = (items + gridDim.x - 1) / gridDim.x;
+    const int begin = blockIdx.x * per, count = min(items, begin + per) - begin;
+    const size_t row_bytes = (size_t)K * 2;
+
+    if (warp == workers) {
+        if (tc::elect_one()) {
+            int st = 0;
+            uint32_t phase = 1;
+            for (int n = 0; n < count; ++n) {
+                if (!tc::mbar_wait(&empty[st], phase, abort_flag, error_word, ERR_FEW_PRODUCER)) break;
+                const int it = begin + n, e = expert_of[it / per_expert];
+                const int c = it % per_expert * (GATED ? 1 : 2);
+                const __nv_bfloat16* w0 = w + ((size_t)e * (GATED ? 2 : 1) * N + c) * K;
+                const __nv_bfloat16* w1 = GATED ? w0 + (size_t)N * K : c + 1 < N ? w0 + K : w0;
+                unsigned char* dst = ring + (size_t)st * 2 * row_bytes;
+                tc::mbar_expect_tx(&full[st], (uint32_t)(2 * row_bytes));
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 ::"r"(tc::smem_u32(dst + i * row_bytes)), "l"(i ? w1 : w0), "r"((uint32_t)row_bytes), "r"(tc::smem_u32(&full[st])) : "memory");
+                if (++st == places) { st = 0; phase ^= 1; }
+            }
+        }
+        return;
+    }
+    for (int n = warp; n < count; n += workers) {
+        const int st = n % places;
+        if (!tc::mbar_wait(&full[st], (n / places) & 1u, abort_flag, error_word, ERR_FEW_CONSUMER)) break;
+        const uint4* w0 = reinterpret_cast<const uint4*>(ring + (size_t)st * 2 * row_bytes);
+        const uint4* w1 = reinterpret_cast<const uint4*>(ring + (size_t)st * 2 * row_bytes + row_bytes);
+        const int it = begin + n;
+        const int c = it % per_expert * (GATED ? 1 : 2);
+        unsigned left = pairs_of[it / per_expert];
+        auto rows = [&](auto number) {                   // the next pairs of the expert
+            constexpr int R = decltype(number)::value;
+            int p[R];
+            const uint4* x[R];
+            float s0[R], s1[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                p[r] = __ffs(left) - 1;
+                left &= left - 1;
+                x[r] = reinterpret_cast<const uint4*>(a + (size_t)(p[r] / a_div) * K);
+                s0[r] = s1[r] = 0.0f;
+            }
+#pragma unroll 4
+            for (int i = lane; i < K / 8; i += 32) {
+                const uint4 a0 = w0[i], a1 = w1[i];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint4 xv = x[r][i];
+                    fma8(s0[r], a0, xv);
+                    fma8(s1[r], a1, xv);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                s0[r] = warp_sum(s0[r]);
+                s1[r] = warp_sum(s1[r]);
+                if (lane == 0) {
+                    OutT* row = out + (size_t)p[r] * N;
+                    row[c] = from_float<OutT>(GATED ? glu_f(glu, s0[r], s1[r]) : s0[r]);
+                    if (!GATED && c + 1 < N) row[c + 1] = from_float<OutT>(s1[r]);
+                }
+            }
+        };
+        while (left) {
+            const int k = __popc(left);
+            if (k >= 4) rows(std::integral_constant<int, 4>{});
+            else if (k >= 2) rows(std::integral_constant<int, 2>{});
+            else rows(std::integral_constant<int, 1>{});
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&empty[st]);
+    }
+}
+
 // Rows of whole groups of four values: a block a row and 1,024 of its values.  2,048 rows of 2,048, top 2: 25.6 -> 8.3 us.
 __global__ void __launch_bounds__(256)
 combine_vec_kernel(const float4* __restrict__ y, float4* __restrict__ x, int top, int n4, float weight) {
@@ -831,13 +965,34 @@ LLMX_EXPORT int llmx_moe_product(const void* a, int a_div, const void* w, int dt
 // multiple of 8; the pair's expert is read from the table.
 LLMX_EXPORT int llmx_moe_product_few(const void* a, int a_div, const void* w, const int* token_ids, const int* table,
                                      int top, int vocab, int pairs, int experts, void* out, int out_dtype, int N, int K,
-                                     int gated, int clamped, float limit, float alpha, cudaStream_t stream) {
+                                     int gated, int clamped, float limit, float alpha, int* error_word, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (N <= 0 || K <= 0 || K % 8 || a_div <= 0 || top <= 0 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return LLMX_ERR_UNSUPPORTED;
     if (!gated && out_dtype != LLMX_F32) return LLMX_ERR_UNSUPPORTED;
     const Glu glu = {clamped, limit, alpha};
     const size_t smem = (size_t)K * 2;
     if (smem > 200 * 1024) return LLMX_ERR_UNSUPPORTED;
+    const long long items = (long long)pairs * (gated ? N : (N + 1) / 2);
+    if (pairs <= FEW_PAIRS && K <= FEW_K && items < (1ll << 31)) {
+        int places = FEW_RING / (4 * K);
+        places = places > FEW_PLACES ? FEW_PLACES : places;
+        int workers = FEW_WARPS;                             // at least four: four places fit whatever K is
+        while (places % workers) --workers;
+        if (workers < 4) workers = 4, places = places / 4 * 4;
+        const size_t ring = (size_t)places * 4 * K;
+        const dim3 stream_grid((unsigned)(items < 148 ? items : 148));
+#define LLMX_FEW(G, O)                                                                                                  \
+    do {                                                                                                                \
+        cudaFuncSetAttribute(moe_few_stream_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_RING);        \
+        launch_kernel(moe_few_stream_kernel<G, O>, stream_grid, dim3(32 * workers + 32), ring, stream, (const __nv_bfloat16*)a, a_div, \
+                      (const __nv_bfloat16*)w, token_ids, table, top, vocab, experts, pairs, (O*)out, N, K, glu, places, error_word); \
+    } while (0)
+        if (gated && out_dtype == LLMX_BF16) LLMX_FEW(true, __nv_bfloat16);
+        else if (gated) LLMX_FEW(true, float);
+        else LLMX_FEW(false, float);
+#undef LLMX_FEW
+        return launch_status();
+    }
     dim3 grid(pairs, (N + GV_COLS - 1) / GV_COLS);
     if (grid.y > 65535) return LLMX_ERR_UNSUPPORTED;
 #define LLMX_FEW(G, O)                                                                                                  \

@@ -896,6 +896,37 @@ def test_expert_products_at_the_edges_of_their_tiles(counts, K, N, clamp):
     assert (y.double() - torch.einsum("rk,rnk->rn", h.double(), w.double()[e])).abs().max() <= 4 * slack
 
 
+@pytest.mark.parametrize("rows,top,K,N,experts", [(1, 1, 8, 1, 3), (1, 8, 16, 7, 8), (8, 1, 1032, 300, 1), (3, 2, 4096, 333, 5), (4, 2, 12288, 95, 4), (9, 1, 264, 21, 2),
+                                                  (2, 2, 12296, 5, 3), (7, 1, 2048, 2001, 4)])
+def test_expert_products_of_a_few_pairs(rows, top, K, N, experts):
+    """One to nine pairs (the stream of weight rows takes up to eight), one to all of them naming an expert, one pair naming none,
+    rings of thirty-two places down to four, an odd column left over, more columns than blocks: both products against the same
+    in 64 bits, with the bounds of the tiles' test."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(K + N)
+    pairs = rows * top
+    choice = torch.randint(0, experts, (rows, top), generator=g, dtype=torch.int32)
+    if pairs > 2:
+        choice.view(-1)[pairs // 2] = -1
+    h = _bf16(torch.randn(rows, K, generator=g)).to(DEV)
+    w_gu = _bf16(torch.randn(experts, 2 * N, K, generator=g) * K ** -0.5).to(DEV)
+    act = torch.full((pairs, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.moe_product_few(h, top, w_gu, None, choice.to(DEV), pairs, act, gated=True)
+    y = torch.full((pairs, N), 7.0, dtype=torch.float32, device=DEV)
+    w = w_gu[:, :N].contiguous()
+    ops.moe_product_few(h, top, w, None, choice.to(DEV), pairs, y, gated=False)
+    for p in range(pairs):
+        e = int(choice.view(-1)[p])
+        if e < 0:
+            assert (act[p] == 7.0).all() and (y[p] == 7.0).all()
+            continue
+        both = w_gu[e].double() @ h[p // top].double()
+        want = both[:N] * torch.sigmoid(both[:N]) * both[N:]
+        slack = K ** 0.5 * 2.0 ** -22
+        assert ((act[p].double() - want).abs() <= 2.0 ** -8 * want.abs() + 8 * slack).all()
+        assert (y[p].double() - both[:N]).abs().max() <= 4 * slack
+
+
 # ---- small kernels of a few rows ---------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("kind", ["delta", "step", "delta_channel"])
 @pytest.mark.parametrize("heads,D,taps,q_heads,more,counts", [
