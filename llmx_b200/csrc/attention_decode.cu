@@ -284,7 +284,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap cache_map, const __nv_bfl
         for (int it = 0; it < iters; ++it) {
             const int stage = it % STAGES;
             const uint32_t phase = (uint32_t)(it / STAGES) & 1u;
-            if (!tc::mbar_wait(&full_bar[stage], phase, abort_flag, error_word, ERR_DEC_CONSUMER)) break;
+            if (!tc::mbar_wait_warp(&full_bar[stage], phase, abort_flag, error_word, ERR_DEC_CONSUMER)) break;
             if ((it & 1) != group) {
                 if (lane == 0) tc::mbar_arrive(&empty_bar[stage]);
                 continue;

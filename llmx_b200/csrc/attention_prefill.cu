@@ -156,7 +156,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap cache_map, const __nv_bf
     for (int it = 0; it < iters; ++it) {
         const int stage = it % STAGES;
         const uint32_t phase = (uint32_t)(it / STAGES) & 1u;
-        if (!tc::mbar_wait(&full_bar[stage], phase, abort_flag, error_word, ERR_PRE_CONSUMER)) break;
+        if (!tc::mbar_wait_warp(&full_bar[stage], phase, abort_flag, error_word, ERR_PRE_CONSUMER)) break;
         const int key0 = kv_begin + it * KEYS;
         if (warp_active && key0 <= warp_max_pos && key0 + KEYS > warp_lo) {
             const uint32_t sbase = tc::smem_u32(tiles + stage * cfg::STAGE_BYTES);

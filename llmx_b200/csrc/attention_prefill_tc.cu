@@ -382,7 +382,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const int lo = window > 0 ? max(0, pos - window + 1) : 0;
             float m_used = -INFINITY, l_run = 0.0f;
             for (int j = 0; j < iters; ++j) {
-                ok = tc::mbar_wait(&s_full[t], s_done & 1u, abort_flag, error_word, ERR_TCA_SOFTMAX);
+                ok = tc::mbar_wait_warp(&s_full[t], s_done & 1u, abort_flag, error_word, ERR_TCA_SOFTMAX);
                 if (!ok) break;
                 ++s_done;
                 tc::tc_fence_after();
@@ -461,7 +461,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 if (lane == 0) tc::mbar_arrive(&p_full[t]);
             }
             // ---- O / l once the last P V has run
-            if (ok) ok = tc::mbar_wait(&s_full[t], s_done & 1u, abort_flag, error_word, ERR_TCA_SOFTMAX);
+            if (ok) ok = tc::mbar_wait_warp(&s_full[t], s_done & 1u, abort_flag, error_word, ERR_TCA_SOFTMAX);
             if (ok) {
                 ++s_done;
                 tc::tc_fence_after();

@@ -97,8 +97,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap cache_map, const __nv_
         for (int j = 0; j < n_iter && ok; ++j) {
             const int st = j & 1, t = begin + j * KEYS + RUN * (lane >> 2);
             const int page = lane < 16 && t < key_end ? max(table[t / page_size], 0) : 0;
-            ok = tc::mbar_wait(&empty[st], ((j >> 1) & 1u) ^ 1u, abort_flag, error_word, ERR_ROWS_PRODUCER);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = tc::mbar_wait_warp(&empty[st], ((j >> 1) & 1u) ^ 1u, abort_flag, error_word, ERR_ROWS_PRODUCER);
             if (!ok) break;
             if (lane == 0) tc::mbar_expect_tx(&full[st], STAGE_BYTES);
             __syncwarp();
@@ -159,8 +158,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap cache_map, const __nv_
             const int key0 = begin + j * KEYS;
             if (key0 < key_lo || key0 + KEYS > key_end) {
                 // Slots of the stage that no row may see: a zero weight must meet a finite value.  Thread t has key t % 64, half t / 64.
-                ok = tc::mbar_wait(&full[j & 1], (j >> 1) & 1u, abort_flag, error_word, ERR_ROWS_SOFTMAX);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = tc::mbar_wait_warp(&full[j & 1], (j >> 1) & 1u, abort_flag, error_word, ERR_ROWS_SOFTMAX);
                 if (!ok) break;
                 const int t = row % KEYS, key = key0 + t;
                 if (key < key_lo || key >= key_end) {
@@ -170,7 +168,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap cache_map, const __nv_
                 }
                 tc::fence_proxy_async();
             }
-            ok = tc::mbar_wait(s_full, j & 1u, abort_flag, error_word, ERR_ROWS_SOFTMAX);
+            ok = tc::mbar_wait_warp(s_full, j & 1u, abort_flag, error_word, ERR_ROWS_SOFTMAX);
             if (!ok) break;
             tc::tc_fence_after();
             uint32_t sc[KEYS];
@@ -227,7 +225,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap cache_map, const __nv_
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(p_full);
         }
-        if (ok) ok = tc::mbar_wait(s_full, n_iter & 1u, abort_flag, error_word, ERR_ROWS_SOFTMAX);
+        if (ok) ok = tc::mbar_wait_warp(s_full, n_iter & 1u, abort_flag, error_word, ERR_ROWS_SOFTMAX);
         if (ok) {
             tc::tc_fence_after();
             const float inv = 1.0f / l_run;

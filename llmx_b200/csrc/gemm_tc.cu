@@ -302,7 +302,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const bool atomic = STREAMK || mode == MODE_ATOMIC || mode == MODE_ACCUMULATE;
         pdl_wait();     // the output may be read or cleared by the kernel before
         while (ok && sched.next(w)) {
-            ok = tc::mbar_wait(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_EPILOGUE);
+            ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_EPILOGUE);
             if (!ok) break;
             tc::tc_fence_after();
             const int n = w.nt * BM + quarter * 32 + lane;

@@ -291,7 +291,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
         bool ok = true;
         const bool atomic = mode == MODE_ACCUMULATE || splits > 1;
         while (ok && sched.next(w)) {
-            ok = tc::mbar_wait(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_PAIR_EPILOGUE);
+            ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_PAIR_EPILOGUE);
             if (!ok) break;
             tc::tc_fence_after();
             const int n = (w.wt * 2 + (int)rank) * BM + quarter * 32 + lane;

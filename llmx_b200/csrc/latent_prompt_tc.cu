@@ -141,8 +141,7 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid
         bool ok = true;
         for (int s = 0; s < n_steps; ++s) {
             const int st = s % EXPAND_STAGES;
-            ok = tc::mbar_wait(&empty[st], ((s / EXPAND_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_LAT_EXPAND);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = tc::mbar_wait_warp(&empty[st], ((s / EXPAND_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_LAT_EXPAND);
             if (!ok) break;
             uint8_t* base = smem + st * EXPAND_STAGE;
             if (lane == 0) tc::mbar_expect_tx(&full[st], EXPAND_STAGE);
@@ -388,7 +387,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
         for (int d = 0; d < D; ++d) o[d] = 0.0f;
         // What stage j made of the output joins the row's sums.
         auto take_output = [&](int j) -> bool {
-            if (!tc::mbar_wait(o_full, j & 1u, abort_flag, error_word, ERR_LAT_ROWS)) return false;
+            if (!tc::mbar_wait_warp(o_full, j & 1u, abort_flag, error_word, ERR_LAT_ROWS)) return false;
             tc::tc_fence_after();
 #pragma unroll
             for (int c = 0; c < D; c += 32) {
@@ -403,7 +402,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
         bool ok = true;
         for (int j = 0; j < n_iter; ++j) {
             ok = j == 0 || take_output(j - 1);
-            ok = ok && tc::mbar_wait(s_full, j & 1u, abort_flag, error_word, ERR_LAT_ROWS);
+            ok = ok && tc::mbar_wait_warp(s_full, j & 1u, abort_flag, error_word, ERR_LAT_ROWS);
             if (!ok) break;
             tc::tc_fence_after();
             const int key0 = begin + j * KEYS;

@@ -322,8 +322,7 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
         };
         bool ok = true;
         for (int s = 0; s < steps; ++s) {
-            ok = tc::mbar_wait(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = tc::mbar_wait_warp(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER);
             if (!ok) break;
             const bool real = 64 * s + 8 * piece < K;
 #pragma unroll
@@ -342,7 +341,7 @@ moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUten
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (ok)
             for (int s = max(0, steps - lag); s < steps; ++s) hand_over();
-        ok = ok && tc::mbar_wait(&done, 0, abort_flag, error_word, ERR_MOE_EPILOGUE);
+        ok = ok && tc::mbar_wait_warp(&done, 0, abort_flag, error_word, ERR_MOE_EPILOGUE);
         tc::tc_fence_after();
         // A warp may touch the tensor-memory lanes 32 (warp % 4) .. + 31; of two warps with the same lanes each takes every
         // other run of 16 pairs.
@@ -517,7 +516,7 @@ moe_few_stream_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv
     }
     for (int n = warp; n < count; n += workers) {
         const int st = n % places;
-        if (!tc::mbar_wait(&full[st], (n / places) & 1u, abort_flag, error_word, ERR_FEW_CONSUMER)) break;
+        if (!tc::mbar_wait_warp(&full[st], (n / places) & 1u, abort_flag, error_word, ERR_FEW_CONSUMER)) break;
         const uint4* w0 = reinterpret_cast<const uint4*>(ring + (size_t)st * 2 * row_bytes);
         const uint4* w1 = reinterpret_cast<const uint4*>(ring + (size_t)st * 2 * row_bytes + row_bytes);
         const int it = begin + n;

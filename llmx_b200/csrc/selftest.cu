@@ -28,11 +28,35 @@ __global__ void wait_selftest_kernel(unsigned long long limit_ns, int* error_wor
     // What a kernel's other warps do after a failed wait: every later wait returns at once.
     if (threadIdx.x == 32) out[1] = tc::mbar_wait_limit(&bar, 0, &abort_flag, error_word, ERR_SELFTEST_WAIT, limit_ns) ? 1 : 2;
 }
+
+// A warp's wait whose lanes would not agree: the even lanes' barrier has completed, nobody arrives at the odd lanes'.  All
+// lanes must come back with the same answer, or the warp-wide instruction after it would wait for lanes that went elsewhere.
+__global__ void warp_wait_selftest_kernel(unsigned long long limit_ns, int* error_word, int* out) {
+    __shared__ uint64_t bars[2];
+    __shared__ int abort_flag;
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&bars[0], 1);
+        tc::mbar_init(&bars[1], 1);
+        tc::fence_barrier_init();
+        tc::mbar_arrive(&bars[0]);
+        abort_flag = 0;
+    }
+    __syncwarp();
+    const bool ok = tc::mbar_wait_warp_limit(&bars[threadIdx.x & 1], 0, &abort_flag, error_word, ERR_SELFTEST_WAIT, limit_ns);
+    out[threadIdx.x] = ok ? 1 : 2;
+}
 }  // namespace
 
 // limit_ns: 1,000 .. 100,000,000 (a tenth of a second at most).  out: two device ints.
 LLMX_EXPORT int llmx_wait_selftest(unsigned long long limit_ns, int* error_word, int* out, cudaStream_t stream) {
     if (!error_word || !out || limit_ns < 1000ull || limit_ns > 100000000ull) return LLMX_ERR_BAD_ARGUMENT;
     wait_selftest_kernel<<<1, 64, 0, stream>>>(limit_ns, error_word, out);
+    return launch_status();
+}
+
+// The same for a warp's wait; out: 32 device ints, what each lane's wait returned.
+LLMX_EXPORT int llmx_warp_wait_selftest(unsigned long long limit_ns, int* error_word, int* out, cudaStream_t stream) {
+    if (!error_word || !out || limit_ns < 1000ull || limit_ns > 100000000ull) return LLMX_ERR_BAD_ARGUMENT;
+    warp_wait_selftest_kernel<<<1, 32, 0, stream>>>(limit_ns, error_word, out);
     return launch_status();
 }

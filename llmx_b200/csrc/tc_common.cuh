@@ -84,6 +84,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return mbar_wait_limit(bar, parity, abort_flag, error_word, code, WAIT_LIMIT_NS);
 }
 
+// For a whole warp that goes on to warp-wide instructions (tensor-memory loads and stores, shuffles, votes): all 32 lanes
+// wait, and all get the same answer.  A lane that gave up by itself, at the limit's edge or because it saw the abort flag, would
+// leave the others waiting for it in the next such instruction for good.
+__device__ __forceinline__ bool mbar_wait_warp_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* error_word,
+                                                     int code, unsigned long long limit_ns) {
+    return __all_sync(0xffffffffu, mbar_wait_limit(bar, parity, abort_flag, error_word, code, limit_ns));
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* error_word,
+                                               int code) {
+    return mbar_wait_warp_limit(bar, parity, abort_flag, error_word, code, WAIT_LIMIT_NS);
+}
+
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(

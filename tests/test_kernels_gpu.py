@@ -713,6 +713,25 @@ def test_a_wait_that_nothing_satisfies_gives_up_and_is_reported():
     assert fn(10, word.data_ptr(), out.data_ptr(), None) == 10001          # limits outside 1 us .. 0.1 s are refused
 
 
+def test_lanes_of_a_warps_wait_never_disagree():
+    """Half of a warp's lanes wait on a barrier that has completed, half on one that nobody arrives at: all lanes get the same
+    answer (csrc/selftest.cu), so that none is left waiting in the warp-wide instructions that follow such waits."""
+    import ctypes
+    from llmx_b200 import ops_tc, runtime
+    from llmx_b200.csrc import build
+    fn = build.load("selftest").llmx_warp_wait_selftest
+    fn.argtypes = [ctypes.c_ulonglong, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    fn.restype = ctypes.c_int
+    torch.cuda.synchronize()
+    ops_tc.check_errors()
+    word = runtime.error_word(DEV)
+    out = torch.zeros(32, dtype=torch.int32, device=DEV)
+    assert fn(1_000_000, word.data_ptr(), out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert out.tolist() == [2] * 32
+    with pytest.raises(runtime.KernelError, match="nobody arrives"):
+        ops_tc.check_errors()
+
+
 def test_random_weights_are_the_same_on_the_device_and_on_the_host():
     """"Seed 0" names one model: the random-weights mode makes the same bits on the GPU (benchmarks, `Engine.from_config`)
     as on the CPU (model folders, the tests' plain implementation)."""
