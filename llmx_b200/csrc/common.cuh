@@ -51,19 +51,21 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 }
 
 // a / b for b >= 1 (or infinite, or not a number) without a branch: the reciprocal refined by a Newton step, the quotient by its
-// remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990): within one unit in the last
-// place.  Where the refinement meets an infinity its first guess is the answer.  (A division with a branch puts each
-// of a thread's values behind its own: chains that could run side by side run one after another.)
+// remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990): correctly rounded, a zero's
+// sign included, wherever the remainder is a normal number (|a| >= 2^-100), below that within one unit in the last place.  So
+// x / (1 + exp(-x)) has the division's bits for every x.  Where the refinement meets an infinity its first guess is the answer.
+// (A division with a branch puts each of a thread's values behind its own: chains that could run side by side run one
+// after another.)
 __device__ __forceinline__ float quotient(float a, float b) {
     const float s = b > 0x1p100f ? 0x1p-64f : 1.0f;          // the reciprocal of what is left is no subnormal number
-    a *= s;
+    const float a_s = a * s;
     b *= s;
     float r0;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(b));
     const float r = fmaf(fmaf(-b, r0, 1.0f), r0, r0);
-    const float q0 = a * r;
-    const float q = fmaf(fmaf(-b, q0, a), r, q0);
-    return fabsf(q) <= 3.402823466e38f ? q : a * r0;
+    const float q0 = a_s * r;
+    const float q = fmaf(fmaf(-b, q0, a_s), r, q0);
+    return fabsf(q) <= 3.402823466e38f ? copysignf(q, a) : a_s * r0;
 }
 
 static inline int launch_status() { return (int)cudaGetLastError(); }

@@ -1,4 +1,6 @@
-// A self-test of the kernels' bounded waits: a wait that nothing will ever satisfy runs out after the limit it is
+// Self-tests of what the kernels share: the bounded waits (tc_common.cuh) and the division without a branch (common.cuh).
+//
+// The bounded waits: a wait that nothing will ever satisfy runs out after the limit it is
 // given, records its code in the error word, and the block goes on to its end.
 //
 // Every wait on an mbarrier in the tensor-core and attention kernels goes through tc::mbar_wait_limit (two seconds
@@ -45,6 +47,11 @@ __global__ void warp_wait_selftest_kernel(unsigned long long limit_ns, int* erro
     const bool ok = tc::mbar_wait_warp_limit(&bars[threadIdx.x & 1], 0, &abort_flag, error_word, ERR_SELFTEST_WAIT, limit_ns);
     out[threadIdx.x] = ok ? 1 : 2;
 }
+
+__global__ void quotient_selftest_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, long long n) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = quotient(a[i], b[i]);
+}
 }  // namespace
 
 // limit_ns: 1,000 .. 100,000,000 (a tenth of a second at most).  out: two device ints.
@@ -58,5 +65,12 @@ LLMX_EXPORT int llmx_wait_selftest(unsigned long long limit_ns, int* error_word,
 LLMX_EXPORT int llmx_warp_wait_selftest(unsigned long long limit_ns, int* error_word, int* out, cudaStream_t stream) {
     if (!error_word || !out || limit_ns < 1000ull || limit_ns > 100000000ull) return LLMX_ERR_BAD_ARGUMENT;
     warp_wait_selftest_kernel<<<1, 32, 0, stream>>>(limit_ns, error_word, out);
+    return launch_status();
+}
+
+// out[i] = a[i] / b[i] for b[i] >= 1 as the kernels divide.
+LLMX_EXPORT int llmx_quotient_selftest(const float* a, const float* b, float* out, long long n, cudaStream_t stream) {
+    if (!a || !b || !out || n <= 0 || n > (1ll << 32)) return LLMX_ERR_BAD_ARGUMENT;
+    quotient_selftest_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(a, b, out, n);
     return launch_status();
 }

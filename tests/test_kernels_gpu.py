@@ -1086,34 +1086,93 @@ def test_plain_products_of_few_and_many_rows_are_the_tiled_one_bit_for_bit(dtype
         assert ((many.double() - want).abs() <= (K + 1) * 2.0 ** -24 * sizes).all()
 
 
-def test_gated_unit_at_extreme_inputs():
-    """silu(gate) * up of an expert over gates from subnormal exponentials to infinities, 32-bit output: the division's branchless form
-    within two units in the last place of 64 bits wherever those are normal numbers, and the same infinities and NaNs."""
+def _same_bits(got, want):
+    return torch.equal(torch.where(torch.isnan(got), torch.full_like(got, 7.0), got).view(torch.int32),
+                       torch.where(torch.isnan(want), torch.full_like(want, 7.0), want).view(torch.int32))
+
+
+def test_division_without_a_branch_is_the_division():
+    """`quotient` (csrc/common.cuh) against the IEEE division of the same numbers, bit for bit: x / (1 + exp(-x)) over every 251st
+    float of both signs, all divisors of one binade, the divisor with all bits set under all dividends, and random pairs of any
+    exponents from 2^-100 on; below that (subnormal remainders) one unit in the last place."""
+    import ctypes
+    from llmx_b200.csrc import build
+    fn = build.load("selftest").llmx_quotient_selftest
+    fn.argtypes, fn.restype = [ctypes.c_void_p] * 3 + [ctypes.c_longlong, ctypes.c_void_p], ctypes.c_int
+
+    def quotient(a, b):
+        out = torch.empty_like(a)
+        assert fn(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), torch.cuda.current_stream().cuda_stream) == 0
+        return out
+
+    g = torch.Generator(device=DEV).manual_seed(5)
+    floats = lambda bits: bits.to(torch.int64).to(torch.int32).view(torch.float32).clone()
+    signed = lambda bits: torch.where(bits >= 2 ** 31, bits - 2 ** 32, bits)
+    x = floats(signed(torch.arange(0, 2 ** 32, 251, device=DEV, dtype=torch.int64)))
+    x = torch.cat([x, torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), -69.4, -88.7, -88.8, -90.0, -104.0, 1e-45, -1e-45], device=DEV)])
+    b = 1.0 + torch.exp(-x)
+    assert _same_bits(quotient(x, b), x / b)
+    assert _same_bits(quotient(torch.ones_like(b), b), torch.ones_like(b) / b)
+    mantissa = torch.arange(2 ** 23, device=DEV, dtype=torch.int64)
+    one = 127 << 23
+    random = lambda: torch.randint(0, 2 ** 23, (2 ** 23,), device=DEV, generator=g)
+    exponent = lambda lo, hi: torch.randint(lo, hi, (2 ** 23,), device=DEV, generator=g) << 23
+    for a_bits, b_bits in ((one + random(), one + mantissa), (one + mantissa, exponent(127, 254) + 2 ** 23 - 1), (exponent(27, 255) + random(), exponent(127, 255) + random())):
+        a, b = floats(a_bits), floats(b_bits)
+        for a in (a, -a):
+            assert _same_bits(quotient(a, b), a / b)
+    a, b = floats(exponent(0, 27) + random()), floats(exponent(127, 255) + random())
+    assert ((quotient(a, b).view(torch.int32) - (a / b).view(torch.int32)).abs() <= 1).all()
+
+
+def test_silu_of_columns_has_one_result_wherever_the_columns_lie():
+    """Runs of columns in fours and runs that are not take different kernels: the same bits from both, and silu's values at zeros of
+    both signs, infinities and where the exponential leaves the normal numbers."""
     from llmx_b200 import ops
-    gates = torch.tensor([0.0, -0.0, 1e-3, -1.0, 1.0, -20.0, -69.0, -70.0, -86.0, -88.0, -88.5, -90.0, -104.0, -1e4, 60.0, 2e38, float("inf"), float("-inf"),
-                          float("nan"), 5.5])
+    g = torch.Generator(device=DEV).manual_seed(2)
+    x = torch.cat([torch.randn(5, 40, device=DEV, generator=g) * s for s in (1.0, 30.0, 1e-30, 1e30)])
+    x[0, :12] = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), -69.4, -88.7, -88.8, -90.0, -104.0, 1e-45, -3e38], device=DEV)
+    fours, single = x.clone(), torch.cat([torch.zeros(20, 1, device=DEV), x], 1)
+    ops.silu_columns_(fours, 0, 40)
+    ops.silu_columns_(single, 1, 40)
+    assert _same_bits(fours, single[:, 1:].contiguous()) and (single[:, 0] == 0).all()
+    got = fours[0, :5].tolist()
+    assert got[0] == 0.0 and math.copysign(1.0, got[0]) == 1.0 and got[1] == 0.0 and math.copysign(1.0, got[1]) == -1.0
+    assert got[2] == math.inf and math.isnan(got[3]) and math.isnan(got[4])          # -inf / inf is no number
+    want = x.double() / (1.0 + torch.exp(-x.double()))
+    # exp within two units in the last place, the sum and the division half a unit each: below 2^-21 of the value where 1 + exp(-x) is finite.
+    plain = torch.isfinite(want) & (x > -88.0) & (x.abs() > 1e-37)
+    assert ((fours.double() - want).abs()[plain] <= 2.0 ** -21 * want.abs()[plain]).all()
+
+
+def test_gated_unit_at_extreme_inputs():
+    """silu(gate) * up of an expert over gates from subnormal exponentials to infinities, 32-bit output.  Gates that are numbers:
+    exp within two units in the last place, the sum, the division and the product half a unit each, together below 2^-21 of the 64-bit value
+    wherever that is a normal number.  A gate beyond the largest float (the product overflows, the up row's does not) gives its
+    sign's limit: plus infinity, and no number for minus infinity over infinity."""
+    from llmx_b200 import ops
+    gates = torch.tensor([0.0, -0.0, 1e-3, -1.0, 1.0, -20.0, -69.0, -70.0, -86.0, -88.0, -88.5, -90.0, -104.0, -1e4, 60.0, 2e38, 5.5, 3e38, -3e38])
     n = gates.numel()
     h = torch.zeros(n, 32, dtype=torch.bfloat16)
     h[:, 0], h[:, 1] = gates.bfloat16(), 1.5
     gates = h[:, 0].double()
-    w = torch.zeros(1, 2 * 8, 32, dtype=torch.bfloat16)
-    w[0, :8, 0], w[0, 8:, 1] = 1.0, 1.0
     choice = torch.zeros(n, 1, dtype=torch.int32, device=DEV)
     lists, held = torch.empty((1, n), dtype=torch.int32, device=DEV), torch.empty((1,), dtype=torch.int32, device=DEV)
     tiles = torch.empty((ops.moe_tiles_len(n, 1),), dtype=torch.int32, device=DEV)
-    finite = torch.isfinite(gates)
-    for rows in (finite, ~finite):           # a product row with an infinity has no number elsewhere: 0 * inf
-        x = torch.where(rows[:, None], h, torch.zeros_like(h)).to(DEV)
-        ops.moe_route(None, choice, 1, lists, held, tiles, tensor_cores=True)
+    for factor, cores in ((1.0, True), (1.0, False), (2.0, False)):      # twice 2e38 and 3e38: beyond the largest float
+        dtype = torch.bfloat16 if cores else torch.float32
+        w = torch.zeros(1, 2 * 8, 32, dtype=dtype)
+        w[0, :8, 0], w[0, 8:, 1] = factor, 1.0
         out = torch.zeros(n, 8, device=DEV)
-        ops.moe_product(x, 1, w.to(DEV), lists, held, tiles, n, out, gated=True, tensor_cores=True)
-        got = out[:, 0].cpu().double()[rows]
-        if rows is finite:
-            want = 1.5 * gates[rows] / (1.0 + torch.exp(-gates[rows]))
-            normal = want.abs() > 2e-37
-            assert ((got - want).abs()[normal] <= 2.0 ** -21 * want.abs()[normal]).all() and (got[~normal].abs() <= 2.1e-37).all()
-        else:
-            assert torch.isnan(got[1:]).all() and (torch.isinf(got[0]) or torch.isnan(got[0]))
+        ops.moe_route(None, choice, 1, lists, held, tiles, tensor_cores=cores)
+        ops.moe_product(h.to(dtype).to(DEV), 1, w.to(DEV), lists, held, tiles, n, out, gated=True, tensor_cores=cores)
+        got = out[:, 0].cpu().double()
+        z = factor * gates
+        finite = z.abs() < 3.4e38
+        want = 1.5 * z / (1.0 + torch.exp(-z))
+        normal = finite & (want.abs() > 2e-37) & (want.abs() < 3.4e38)
+        assert ((got - want).abs()[normal] <= 2.0 ** -21 * want.abs()[normal]).all() and (got[finite & (want.abs() <= 2e-37)].abs() <= 2.1e-37).all()
+        assert (got[(z > 3.4e38) | (want > 3.4e38)] == math.inf).all() and torch.isnan(got[z < -3.4e38]).all()
 
 
 @pytest.mark.parametrize("heads,kv_heads,page,window,chunk", [(4, 1, 16, None, None), (3, 1, 32, 70, None), (32, 2, 48, None, 96), (2, 2, 16, 1, None), (10, 2, 16, 64, 200)])
