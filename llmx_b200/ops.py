@@ -154,6 +154,13 @@ _SIGNATURES = {
 _fns = {}
 
 
+def _row_stride(t: torch.Tensor) -> int:
+    """The distance between a matrix's rows.  With one row nothing is that far apart, but the kernels also choose their form by it,
+    and a row must get the same form alone as among others: the stride of the matrix it is a view of, unless that is no
+    stride rows of this width can have."""
+    return t.stride(0) if t.shape[0] > 1 or t.stride(0) >= t.shape[1] else t.shape[1]
+
+
 _timed_calls = None       # while `kernel_times` is open: [(exported function, start event, end event)]
 
 
@@ -483,7 +490,7 @@ def sigmoid_gate_(o: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     rows, width = o.shape
     _need(o.is_contiguous() and gate.dtype == torch.float32 and tuple(gate.shape) == (rows, width) and gate.stride(1) == 1,
           "sigmoid_gate: contiguous rows and a float32 gate of the same shape")
-    _check(_fn("rowwise", "llmx_sigmoid_gate")(_ptr(o), _code(o), _ptr(gate), gate.stride(0) if rows > 1 else width, rows, width,
+    _check(_fn("rowwise", "llmx_sigmoid_gate")(_ptr(o), _code(o), _ptr(gate), _row_stride(gate), rows, width,
                                                _stream()), "sigmoid_gate")
     return o
 
@@ -520,7 +527,7 @@ def gated_rmsnorm(o: torch.Tensor, gate: torch.Tensor, weight: Optional[torch.Te
     _need(tuple(out.shape) == (rows, width) and tuple(gate.shape) == (rows, width) and gate.stride(1) == 1, "gated_rmsnorm: shapes do not fit")
     _need(group > 0 and width % group == 0 and (weight is None or weight.numel() in (group, width)), "gated_rmsnorm: the group must divide the row; weight of a group or of the row")
     _need(gate_kind in ("sigmoid", "silu"), "gated_rmsnorm: gate must be sigmoid or silu")
-    _check(_fn("rowwise", "llmx_gated_rmsnorm")(_ptr(o), _ptr(gate), gate.stride(0) if rows > 1 else width, _ptr(weight),
+    _check(_fn("rowwise", "llmx_gated_rmsnorm")(_ptr(o), _ptr(gate), _row_stride(gate), _ptr(weight),
                                                 0 if weight is None else weight.numel(), _ptr(out), _code(out), rows, width // group, group,
                                                 float(eps), 0 if gate_kind == "sigmoid" else 1, 1 if gate_first else 0, _stream()),
            "gated_rmsnorm")
@@ -622,7 +629,7 @@ def softcap_(x: torch.Tensor, cap: float) -> torch.Tensor:
 
 def _strided_rows(t: torch.Tensor, what: str) -> int:
     _need(t.is_cuda and t.dtype == torch.float32 and t.dim() == 2 and t.stride(1) == 1, f"{what}: float32 rows, contiguous within a row")
-    return t.stride(0) if t.shape[0] > 1 else t.shape[1]
+    return _row_stride(t)
 
 
 def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, step, out: torch.Tensor,
@@ -797,7 +804,7 @@ def qkv_finish(proj: torch.Tensor, heads: int, kv_heads: int, key_dim: int, valu
               and slots.dtype == torch.int32 and slots.numel() >= rows, "qkv_finish: cache layout or slots do not fit")
     _need(freq is None or (freq.dtype == torch.float32 and 2 * freq.numel() <= key_dim), "qkv_finish: frequencies float32 [<= D / 2]")
     _check(_fn("attention_split", "llmx_qkv_finish")(
-        _ptr(proj), proj.stride(0) if rows > 1 else proj.shape[1], _ptr(bias), _ptr(taps_w), taps, _ptr(state),
+        _ptr(proj), _row_stride(proj), _ptr(bias), _ptr(taps_w), taps, _ptr(state),
         0 if state is None else state.shape[1], int(conv_off), _ptr(step.row_request), _ptr(step.row_start), _ptr(step.row_count),
         _ptr(step.history), _ptr(step.state_slots), _ptr(step.state_slots_out), _ptr(q_weight), _ptr(k_weight),
         ("none", "before", "after", "whole").index(norm), float(eps), _ptr(freq), 0 if freq is None else freq.numel(), 1 if neighbours else 0,
@@ -1099,7 +1106,7 @@ def latent_write(down: torch.Tensor, q_rank: int, q_weight: Optional[torch.Tenso
     _need(cache.shape[-1] == latent + rot, "latent_write: cache rows do not fit")
     _need(positions.dtype == torch.int32 and slots.dtype == torch.int32 and positions.numel() >= rows and slots.numel() >= rows,
           "latent_write: positions and slots must be int32 per row")
-    _check(_fn("latent_attention", "llmx_latent_write")(_ptr(down), down.stride(0) if rows > 1 else down.shape[1], int(q_rank), _ptr(q_weight), _ptr(cq),
+    _check(_fn("latent_attention", "llmx_latent_write")(_ptr(down), _row_stride(down), int(q_rank), _ptr(q_weight), _ptr(cq),
                                                         _code(cq) if cq is not None else F32, _ptr(weight), float(eps), _ptr(freq),
                                                         freq.numel(), 1 if halves else 0, float(magnitude), _ptr(positions), _ptr(slots),
                                                         _ptr(cache), _code(cache), rows, latent, rot, _stream()), "latent_write")
@@ -1123,7 +1130,7 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, w_uk: torch.Tensor, w
     for t in (row_request, positions, block_tables):
         _need(t.dtype == torch.int32, "latent_attention: metadata must be int32")
     _check(_fn("latent_attention", "llmx_latent_attention")(
-        _ptr(q), q.stride(0) if rows > 1 else q.shape[1], _ptr(cache), _code(cache), _ptr(w_uk), _ptr(w_uv), _code(w_uk), _ptr(out),
+        _ptr(q), _row_stride(q), _ptr(cache), _code(cache), _ptr(w_uk), _ptr(w_uv), _code(w_uk), _ptr(out),
         _ptr(freq), freq.numel(), 1 if halves else 0, float(magnitude), _ptr(row_request), _ptr(positions), _ptr(block_tables), block_tables.shape[1], rows, heads, key_dim, rot, value_dim,
         latent, page_size, int(window or 0), float(scale), _stream()), "latent_attention")
     return out
@@ -1159,7 +1166,7 @@ def latent_attention_tiled(q: torch.Tensor, cache: torch.Tensor, w_uk: torch.Ten
     _need(tiles.numel() >= 2 * n_tiles and n_tiles > 0 and splits > 0, "latent_attention: tiles do not fit")
     qk = torch.empty((rows, heads, latent + rot), dtype=torch.float32, device=q.device)
     part = torch.empty((rows, heads, splits, latent + 2), dtype=torch.float32, device=q.device)
-    _check(_fn("latent_attention", "llmx_latent_query")(_ptr(q), q.stride(0) if rows > 1 else q.shape[1], _ptr(w_uk), _code(w_uk), _ptr(qk),
+    _check(_fn("latent_attention", "llmx_latent_query")(_ptr(q), _row_stride(q), _ptr(w_uk), _code(w_uk), _ptr(qk),
                                                         _ptr(freq), freq.numel(), 1 if halves else 0, float(magnitude),
                                                         _ptr(positions), rows, heads, key_dim, rot, latent, float(scale), _stream()),
            "latent_query")
@@ -1215,7 +1222,7 @@ def latent_attention_prompt(q: torch.Tensor, cache: torch.Tensor, w_uk: torch.Te
             int(max_tokens), _ptr(row_request), _ptr(positions), _ptr(block_tables), block_tables.shape[1], int(tokens), h, n, latent, rot,
             page_size, int(window or 0), err, _stream()), "latent_expand")
         _check(_fn("latent_prompt_tc", "llmx_latent_prompt")(
-            _ptr(expanded), int(tokens), _ptr(q), q.stride(0) if rows > 1 else q.shape[1], _ptr(out), _ptr(tiles), int(n_tiles), _ptr(freq),
+            _ptr(expanded), int(tokens), _ptr(q), _row_stride(q), _ptr(out), _ptr(tiles), int(n_tiles), _ptr(freq),
             freq.numel(), 1 if halves else 0, float(magnitude), _ptr(positions), heads, h, n, rot, int(window or 0), float(scale), err,
             _stream()), "latent_prompt")
     return out

@@ -1068,6 +1068,21 @@ def test_norms_of_rows_in_fours(rows, width):
     assert (s.double() - want).abs().max() <= 4e-6 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("gate_first", [False, True])
+@pytest.mark.parametrize("groups,group", [(1, 1000), (3, 100), (2, 600)])
+def test_a_row_of_a_gated_norm_is_the_same_alone_and_among_others(groups, group, gate_first):
+    """The gate lies in rows of a wider matrix whose width is no multiple of four: one row alone takes the form that several take,
+    and gives the same bits."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(group)
+    width, rows = groups * group, 40
+    o, wide, w = torch.randn(rows, width, generator=g).to(DEV), torch.randn(rows, width + 3, generator=g).to(DEV), torch.randn(group, generator=g).to(DEV)
+    make = lambda s: ops.gated_rmsnorm(o[s], wide[s, :width], w, 1e-6, group, "silu", torch.empty(s.stop - s.start, width, device=DEV), gate_first=gate_first)
+    among = make(slice(0, rows))
+    for r in range(rows):
+        assert torch.equal(make(slice(r, r + 1))[0], among[r]), r
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 65, 36), (4, 4096, 256), (3, 130, 1000)])
 def test_plain_products_of_few_and_many_rows_are_the_tiled_one_bit_for_bit(dtype, M, N, K):
