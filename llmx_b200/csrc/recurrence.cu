@@ -916,7 +916,9 @@ LLMX_EXPORT int llmx_linear_recurrence(const float* q, const float* k, const flo
     if (heads <= 0 || qk_heads <= 0 || heads % qk_heads || D <= 0 || V <= 0 || D > 512) return LLMX_ERR_UNSUPPORTED;
     if (mode < 0 || mode > 4 || (mode == M_CONST ? decay == nullptr : (gate == nullptr || (beta == nullptr && has_beta(mode)))))
         return LLMX_ERR_BAD_ARGUMENT;
-    const bool wide = max_rows > 8;            // `max_rows`: the most rows one request brings (a matter of speed only)
+    // `max_rows`: the most rows one request brings.  Beyond eight the wide form runs, whose sums go in another order: a row's last
+    // bits then depend on how its request was cut and on what else is in the step.  A caller that wants neither says 1.
+    const bool wide = max_rows > 8;
 #define LLMX_MODE(M)                                                                                                      \
     return launch_recurrence<M>(D, wide, requests, stream, q, k, v, q_stride, k_stride, v_stride, decay, gate, beta,      \
                                 gate_stride, beta_stride, skip, state, slot_floats, row_start, row_count, history, slot_in, \

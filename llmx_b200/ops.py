@@ -635,7 +635,7 @@ def _strided_rows(t: torch.Tensor, what: str) -> int:
 def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, step, out: torch.Tensor,
                       heads: int, qk_heads: int, key_dim: int, value_dim: int, decay: Optional[torch.Tensor] = None,
                       gate: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None, form: Optional[str] = None,
-                      skip: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      skip: Optional[torch.Tensor] = None, invariant: bool = False) -> torch.Tensor:
     """Per (request, head): S <- a S + k u^T, o = S^T q over the step's rows in order, S [D, V] float32 carried in the
     request's state slot.  `form` (default: "decay" with `decay`, else "delta"):
       "decay"          a = decay_h [heads], u = v
@@ -644,7 +644,9 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
       "delta_channel"  S <- diag(gate) S first, gate [rows, heads * D]; then u = beta (v - S^T k), S <- S + k u^T
       "channel"        S <- diag(gate) S + k v^T, gate [rows, heads * D] (no beta)
     q, k [rows, qk_heads * D], v [rows, heads * V]: float32 views whose rows may be strided.  state [slots, floats]: the
-    recurrence's values first, [H][V][D].  `step`: the StepBatch (row ranges, histories and slots are read on the device)."""
+    recurrence's values first, [H][V][D].  `step`: the StepBatch (row ranges, histories and slots are read on the device).
+    Steps in which some request brings more than eight rows run a form whose sums go in another order (csrc/recurrence.cu); with
+    `invariant` none does, so that a row's bits depend neither on how its request was cut nor on what else is in the step."""
     rows = q.shape[0]
     qs, ks, vs = _strided_rows(q, "recurrence q"), _strided_rows(k, "recurrence k"), _strided_rows(v, "recurrence v")
     _need(q.shape[1] == qk_heads * key_dim and k.shape[1] == qk_heads * key_dim and v.shape[1] == heads * value_dim
@@ -669,7 +671,7 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
     _check(_fn("recurrence", "llmx_linear_recurrence")(
         _ptr(q), _ptr(k), _ptr(v), qs, ks, vs, mode, _ptr(decay), _ptr(gate), _ptr(beta), gs, bs, _ptr(skip), _ptr(state),
         state.shape[1], _ptr(step.row_start), _ptr(step.row_count), _ptr(step.history), _ptr(step.state_slots),
-        _ptr(step.state_slots_out), _ptr(out), step.requests, heads, qk_heads, key_dim, value_dim, int(step.max_row_count),
+        _ptr(step.state_slots_out), _ptr(out), step.requests, heads, qk_heads, key_dim, value_dim, 1 if invariant else int(step.max_row_count),
         _stream()), "linear_recurrence")
     return out
 

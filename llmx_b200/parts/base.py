@@ -54,8 +54,8 @@ class Precision:
     Softmax, norms, rotation angles and the residual sum are 32-bit on both.
 
     `invariant`: every kernel and schedule is chosen by the part's own sizes alone, never by the step's rows: whole
-    product tiles with k in one piece and the plain attention kernel.  A row's logits then do not depend on what it
-    was batched with, bit for bit (the reference's rule, src/backends/backend.hpp:141-150), at the price of speed;
+    product tiles with k in one piece, the plain attention kernel, recurrences in the form that takes a row after the other
+    whatever the rows.  A row's logits then do not depend on what it was batched with, bit for bit (the reference's rule, src/backends/backend.hpp:141-150), at the price of speed;
     without it the bfloat16 path picks product schedules by the step's total rows and adds partial sums with
     atomics, so a row's last bits move with the batch and from run to run.
     """

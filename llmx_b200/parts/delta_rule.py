@@ -125,13 +125,13 @@ class GatedDeltaRule(Part):
                              self.key_dim, self.key_dim ** -0.5, state, self.state_floats, step, gate_kind="delta_channel",
                              decay_in=decay_in)
             ops.linear_recurrence(ready[:, :qk], ready[:, qk:2 * qk], ready[:, 2 * qk:], state, step, o, H, self.kv_heads,
-                                  self.key_dim, self.value_dim, gate=gates[:, H:], beta=gates[:, :H], form="delta_channel")
+                                  self.key_dim, self.value_dim, gate=gates[:, H:], beta=gates[:, :H], form="delta_channel", invariant=self.precision.invariant)
         else:
             gates = torch.empty((rows, 2 * H), dtype=torch.float32, device=h.device)
             ops.conv_prepare(proj, self.channels, qk, qk, self.taps_w, ready, self.a_log, self.dt_bias, b_off, a_off, gates, H,
                              self.key_dim, self.key_dim ** -0.5, state, self.state_floats, step)
             ops.linear_recurrence(ready[:, :qk], ready[:, qk:2 * qk], ready[:, 2 * qk:], state, step, o, H, self.kv_heads,
-                                  self.key_dim, self.value_dim, gate=gates[:, :H], beta=gates[:, H:])
+                                  self.key_dim, self.value_dim, gate=gates[:, :H], beta=gates[:, H:], invariant=self.precision.invariant)
         gate = self.g2(proj[:, g_off:g_off + self.gate_rank].contiguous()) if self.gate_rank else proj[:, g_off:g_off + vw]
         y = torch.empty((rows, vw), dtype=self.precision.act, device=h.device)
         ops.gated_rmsnorm(o, gate, self.norm_weight, self.norm_eps, self.value_dim, self.gate, y)

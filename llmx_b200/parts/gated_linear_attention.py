@@ -79,7 +79,7 @@ class GatedLinearAttention(Part):
         ops.channel_decay_(proj, g_off + vw, self.a2t, self.a2_bias, self.tau, decay, 0, self.key_dim ** -0.5)
         o = torch.empty((rows, vw), dtype=torch.float32, device=h.device)
         ops.linear_recurrence(proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:g_off], step.state(cache_entry), step, o, self.heads,
-                              self.heads, self.key_dim, self.value_dim, gate=decay, form="channel")
+                              self.heads, self.key_dim, self.value_dim, gate=decay, form="channel", invariant=self.precision.invariant)
         y = torch.empty((rows, vw), dtype=self.precision.act, device=h.device)
         ops.gated_rmsnorm(o, proj[:, g_off:g_off + vw], self.norm_weight, self.norm_eps, self.value_dim, "silu", y)
         add_product(self, self.o, y, residual)

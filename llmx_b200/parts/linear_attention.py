@@ -94,7 +94,7 @@ class DecayedLinearAttention(Part):
             ops.rotate_heads_(proj, self.heads, self.heads, self.key_dim, self.rot_dims, self.freq, step.positions, 1.0, self.key_factor)
         o = torch.empty((rows, vw), dtype=torch.float32, device=h.device)
         ops.linear_recurrence(proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + vw], step.state(cache_entry), step, o,
-                              self.heads, self.heads, self.key_dim, self.value_dim, decay=self.decay)
+                              self.heads, self.heads, self.key_dim, self.value_dim, decay=self.decay, invariant=self.precision.invariant)
         y = torch.empty((rows, vw), dtype=self.precision.act, device=h.device)
         group = vw if self.norm_kind == "row" else self.value_dim
         ops.gated_rmsnorm(o, proj[:, 2 * qk + vw:], self.norm_weight, self.norm_eps, group, self.gate, y)

@@ -88,7 +88,7 @@ class SelectiveStateSpace(Part):
                          self.state_dim, 1.0, state, self.state_floats, step, first=inner, bias=self.taps_b, gate_kind="step")
         y = torch.empty((rows, inner), dtype=torch.float32, device=h.device)
         ops.linear_recurrence(ready[:, inner + bc:], ready[:, inner:inner + bc], ready[:, :inner], state, step, y, H, self.groups,
-                              self.state_dim, self.value_dim, gate=gates[:, :H], beta=gates[:, H:], form="scaled", skip=self.skip)
+                              self.state_dim, self.value_dim, gate=gates[:, :H], beta=gates[:, H:], form="scaled", skip=self.skip, invariant=self.precision.invariant)
         out = torch.empty((rows, inner), dtype=self.precision.act, device=h.device)
         ops.gated_rmsnorm(y, proj[:, :inner], self.norm_weight, self.norm_eps, inner // self.norm_groups, "silu", out, gate_first=True)
         self.o(out, out=residual, accumulate=True)
