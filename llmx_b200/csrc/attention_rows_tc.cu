@@ -197,8 +197,8 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap cache_map, const __nv_
                 uint32_t p[3][16];
 #pragma unroll
                 for (int u = 0; u < 16; ++u) {
-                    const float a = attn::exp2_approx(fmaf(__uint_as_float(sc[c + 2 * u]), scale_log2, -base));
-                    const float b = attn::exp2_approx(fmaf(__uint_as_float(sc[c + 2 * u + 1]), scale_log2, -base));
+                    const float a = exp2f(fmaf(__uint_as_float(sc[c + 2 * u]), scale_log2, -base));
+                    const float b = exp2f(fmaf(__uint_as_float(sc[c + 2 * u + 1]), scale_log2, -base));
                     sum[u & 3] += a + b;
                     attn::split3_pair(a, b, p[0][u], p[1][u], p[2][u]);
                 }

@@ -1,4 +1,8 @@
 // Pieces of the attention kernels whose 32-bit factors meet the tensor cores as three bfloat16 parts.
+//
+// Their softmax weights are exp2f of a score's distance from the row's maximum (within two units in the last place, like the expf
+// of the general forms), subnormal weights among them: the instruction that flushes those gave 0 where the general forms
+// give 2^-126 and less (a value of 2^120 makes the difference visible), and was 8 % faster over [key ; value] rows.
 #pragma once
 #include "attn_common.cuh"
 
@@ -9,12 +13,6 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr, uint32_t b
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(block >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
-// 2^x in one instruction; minus infinity gives 0.
-__device__ __forceinline__ float exp2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));

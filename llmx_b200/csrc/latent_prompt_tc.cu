@@ -431,7 +431,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap expanded_map, const flo
                 uint32_t p[3][16];
 #pragma unroll
                 for (int u = 0; u < 16; ++u) {
-                    const float a = attn::exp2_approx(__uint_as_float(sc[c + 2 * u]) - base), b = attn::exp2_approx(__uint_as_float(sc[c + 2 * u + 1]) - base);
+                    const float a = exp2f(__uint_as_float(sc[c + 2 * u]) - base), b = exp2f(__uint_as_float(sc[c + 2 * u + 1]) - base);
                     sum[u & 3] += a + b;
                     attn::split3_pair(a, b, p[0][u], p[1][u], p[2][u]);
                 }

@@ -1234,3 +1234,36 @@ def test_attention_of_rows_that_share_their_keys(heads, kv_heads, page, window, 
             bound = 2.0 ** -8 * want.abs() + 2.0 ** -19 * (1.0 + s.abs().max()) * v[lo:p + 1].abs().max()
             assert ((out[row].double() - want).abs() <= bound).all(), (r, p)
             row += 1
+
+
+@pytest.mark.parametrize("bits", [3, 64, 120, 126.3, 128.5, 131])
+def test_softmax_weights_below_the_normal_numbers_count(bits):
+    """Two keys, the second 2^-bits of the first in weight, its value 2^120, the first's zero: the result is that product, also where
+    the weight is no normal number any more (below 2^-126 it keeps what a bfloat16 holds of it, multiples of 2^-133), by the tcgen05
+    forms over [key ; value] rows and over latents.  The score is a 32-bit product, its exponent's error below 2^-16 of the weight."""
+    import types
+    from llmx_b200 import ops
+    from llmx_b200.runtime import check_errors
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    score = torch.tensor(-bits * math.log(2.0)).bfloat16().item()
+    want = 2.0 ** 120 * math.exp(score) / (1.0 + math.exp(score))
+    bound = 2.0 ** -8 * want + 2.0 ** -16 * want + (2.0 ** -133 * 2.0 ** 120 if bits > 125 else 0.0)
+    cache = torch.zeros(1, 1, 1, 16, 256, device="cuda", dtype=torch.bfloat16)
+    cache[0, 0, 0, 1, 0], cache[0, 0, 0, 1, 128:] = score, 2.0 ** 120
+    q = torch.zeros(2, 128, device="cuda", dtype=torch.bfloat16)
+    q[:, 0] = 1.0
+    step = types.SimpleNamespace(row_start=i32([0]), row_count=i32([2]), history=i32([0]), requests=1, rows=2)
+    rows = torch.zeros(2, 128, device="cuda", dtype=torch.bfloat16)
+    ops.attention_tiled(q, cache, rows, step, i32([[0]]), 1, 1, 128, 128, None, None, 1.0)
+    latent = torch.zeros(1, 1, 1, 16, 64 + 8, device="cuda", dtype=torch.bfloat16)
+    latent[0, 0, 0, 1, 0], latent[0, 0, 0, 1, 64] = 2.0 ** 60, score
+    w_uk, w_uv = torch.zeros(128, 64, device="cuda", dtype=torch.bfloat16), torch.zeros(128, 64, device="cuda", dtype=torch.bfloat16)
+    w_uv[:, 0] = 2.0 ** 60
+    ql = torch.zeros(2, 128 + 8, device="cuda")
+    ql[:, 128] = 1.0
+    made = torch.zeros(2, 128, device="cuda", dtype=torch.bfloat16)
+    ops.latent_attention_prompt(ql, latent, w_uk, w_uv, made, torch.zeros(0, device="cuda"), i32([0, 0]), i32([0, 1]), i32([[0]]), i32([0, 2, 0, 128]), 1, 128,
+                                i32([0, 2, 0, 0]), 1, 128, 1, 1, 128, 8, 128, 64, 16, None, 1.0)
+    check_errors()
+    for how, out in (("rows", rows), ("latents", made)):
+        assert (out[0] == 0).all() and ((out[1].double() - want).abs() <= bound).all(), (how, out[1, 0].item(), want)
