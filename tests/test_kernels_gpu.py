@@ -1267,3 +1267,41 @@ def test_softmax_weights_below_the_normal_numbers_count(bits):
     check_errors()
     for how, out in (("rows", rows), ("latents", made)):
         assert (out[0] == 0).all() and ((out[1].double() - want).abs() <= bound).all(), (how, out[1, 0].item(), want)
+
+
+@pytest.mark.parametrize("mean", [0.0, 1.0])
+@pytest.mark.parametrize("keys", [300, 2048, 8192])
+def test_attention_over_many_keys_rounds_as_the_exact_one(keys, mean):
+    """How many results round to another bfloat16 than the 64-bit ones, by the tcgen05 form and by the form on mma.sync (which the
+    kernel's entry runs whatever the widths).  A stage of 64 keys is cut off at each of its twelve additions, the stages are
+    joined by rounded ones, so with values of one sign the error stays below 12 x 2^-23 of the result however many keys there are:
+    12 x 2^-23 / 2^-8 = 4e-4 of the results at most lie that close to a bfloat16's edge.  With values of both signs the sums are larger
+    than the result: no more than the other form, whose accumulators run through all keys."""
+    import types
+    from llmx_b200 import ops
+    from llmx_b200.runtime import check_errors
+    g = torch.Generator(device="cuda").manual_seed(keys)
+    rows, heads, kv_heads, scale = 64, 16, 4, 128 ** -0.5
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    cache = torch.randn(-(-keys // 16), 1, kv_heads, 16, 256, device="cuda", generator=g)
+    cache[..., 128:] += mean
+    cache = cache.bfloat16()
+    q = torch.randn(rows, heads * 128, device="cuda", generator=g).bfloat16()
+    tables = torch.arange(cache.shape[0], dtype=torch.int32, device="cuda")[None].contiguous()
+    step = types.SimpleNamespace(row_start=i32([0]), row_count=i32([rows]), history=i32([keys - rows]), requests=1, rows=rows)
+    out, other = (torch.zeros(rows, heads * 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    ops.attention_tiled(q, cache, out, step, tables, heads, kv_heads, 128, 128, None, None, scale)
+    P = ops._ptr
+    ops._check(ops._fn("attention_split", "llmx_attention_tiled")(
+        P(q), P(cache), P(other), P(step.row_start), P(step.row_count), P(step.history), P(tables), tables.shape[1], rows, 1, heads, kv_heads, 128, 128, 16, 0, 0,
+        scale, *ops.NO_EXTRAS.checked(heads, 128, rows), ops._stream()), "attention_tiled")
+    check_errors()
+    kv = cache[:, 0].transpose(1, 2).reshape(-1, kv_heads, 256)[:keys].double()
+    unseen = torch.arange(keys, device="cuda")[None] > torch.arange(keys - rows, keys, device="cuda")[:, None]
+    want = torch.empty(rows, heads, 128, device="cuda", dtype=torch.float64)
+    for h in range(heads):
+        k, v = kv[:, h // (heads // kv_heads)].split(128, 1)
+        want[:, h] = torch.softmax((q.view(rows, heads, 128)[:, h].double() @ k.T * scale).masked_fill(unseen, -math.inf), 1) @ v
+    nearest = want.float().bfloat16().view(rows, -1)
+    share, before = ((x != nearest).double().mean().item() for x in (out, other))
+    assert share <= (4e-4 if mean else max(before, 4e-4)), (share, before)
