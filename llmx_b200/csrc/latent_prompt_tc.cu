@@ -22,13 +22,14 @@
 // parts lie in tensor memory (288 columns), beside the scores / weights (96 columns: three parts of 64 weights over the
 // scores they came from) and a stage's output (128 columns): all 512 columns, so one block per SM and one tile in flight.
 //
-// The tensor core cuts off what an addition shifts out of its accumulator.  A stage's output therefore starts from nothing
+// The tensor core cuts off what an addition shifts out of its accumulator.  A stage's output (and 64 columns of an expanded key or
+// value, below) therefore starts from nothing
 // and joins the row's sums, which its thread holds in registers, by a rounded addition, while the next stage's scores are
 // made; added up over the stages in tensor memory, 3,500 keys cost five times the values (0.8 % against 0.15 %) that
 // round to another bfloat16 than the exact ones.
 //
-// Both kernels together, 2,048 rows after nothing: 16 heads 241 us, 32 heads 410 us; 32 heads, 2,048 rows after 4,096 tokens
-// under a window of 4,096: 1,142 us.  The general form: 2,639, 5,142 and 14,510 us.
+// Both kernels together, 2,048 rows after nothing: 16 heads 247 us, 32 heads 402 us; 32 heads, 2,048 rows after 4,096 tokens
+// under a window of 4,096: 1,068 us.  The general form: 2,639, 5,142 and 14,506 us.
 //
 // Shapes: D = V = 128, R a multiple of 8 up to 64, C a multiple of 64, pages of a multiple of 16 tokens, bfloat16 cache
 // and maps.  Every wait on an mbarrier is bounded (tc_common.cuh).
@@ -61,10 +62,11 @@ __device__ __forceinline__ void tmem_st_32x1(uint32_t addr, uint32_t v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(addr), "r"(v) : "memory");
 }
 
-// Whether all 128 row threads say so (a barrier among them).
-__device__ __forceinline__ bool all_rows(bool mine) {
+// Whether all 128 threads of four warps say so (named barrier `id`).
+__device__ __forceinline__ bool all_four_warps(int id, bool mine) {
     uint32_t all;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(all) : "r"(mine ? 1u : 0u) : "memory");
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(all) : "r"(mine ? 1u : 0u), "r"(id) : "memory");
     return all != 0;
 }
 
@@ -75,16 +77,24 @@ __device__ __forceinline__ int first_key(int pos_first, int window) {
 }
 
 // requests[4 i ..]: first row, rows, first workspace token, workspace tokens (a multiple of 128) of request i.
-// 128 keys x one head: two accumulators of 128 x 128 (key, value) over C in steps of 64 columns.  Bound by the writes to the
-// workspace (1,664 bytes a token and head); two blocks an SM, so one's writes run beside the other's products.  The parts are laid
-// out in shared memory (the operands' stages are free then) and leave by TMA, whole 128-byte lines: 2,048 tokens of 16
-// heads 52 -> 21 us, 5,003 tokens 135 -> 57, against 16-byte stores of 32 rows at a time.
+// 128 keys x one head: two products of 128 x 128 (key, value) over C in steps of 64 columns.  A step's products start from nothing, in
+// one of two pairs of accumulators, and join the 128 sums that a thread holds in registers by rounded additions while the next step's
+// run: over C / 16 additions in one accumulator, each of which the tensor core cuts off, 0.06 % of the attention's results at
+// 128 to 512 keys rounded to another bfloat16 than the exact ones (general form 0.03 to 0.05 %), so 0.02 to 0.03 %.
+//   warp 0      producer, warp 1 products; warps 2 and 3 idle
+//   warps 4-7   the keys' sums, one thread a key; warps 8-11 the values'
+// The three parts of the sums are laid out in shared memory (the operands' stages are free then) and leave by TMA, whole 128-byte
+// lines.  Bound by the writes to the workspace (1,664 bytes a token and head), which one block an SM does not overlap with the next
+// one's products: 2,048 tokens of 16 heads 35 us, 5,003 tokens of 32 133 us (27 and 96 with one accumulator and two blocks an SM).
 constexpr int EXPAND_STAGE = 3 * ROWS * 128;                // 128 keys, 128 + 128 rows of the maps, 64 columns each
-constexpr int EXPAND_STAGES = 2;
-static_assert(EXPAND_STAGES * EXPAND_STAGE >= 6 * ROWS * 128, "the parts of 128 keys or values");
+constexpr int EXPAND_STAGES = 4;
+static_assert(EXPAND_STAGES * EXPAND_STAGE >= 2 * 6 * ROWS * 128, "the parts of 128 keys and values");
 constexpr int EXPAND_SMEM = EXPAND_STAGES * EXPAND_STAGE + 1024 + 256;
+// Launched with 3 x 128 x 168 registers; the first group gives back what the sums need: 40 + 232 + 232 = 3 x 168.
+constexpr int EXPAND_THREADS = 3 * 128, FEWER_REGISTERS = 40, MORE_REGISTERS = 232;
+static_assert(FEWER_REGISTERS + 2 * MORE_REGISTERS <= 3 * 168, "setmaxnreg draws on the block's registers at launch");
 
-__global__ void __launch_bounds__(PROMPT_THREADS, 2)
+__global__ void __launch_bounds__(EXPAND_THREADS, 1)
 latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid_constant__ CUtensorMap uk_map,
                      const __grid_constant__ CUtensorMap uv_map, const __grid_constant__ CUtensorMap expanded_map, const __nv_bfloat16* __restrict__ cache,
                      __nv_bfloat16* __restrict__ expanded, const int* __restrict__ requests,
@@ -95,8 +105,8 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = (uint64_t*)(smem + EXPAND_STAGES * EXPAND_STAGE);
     uint64_t* empty = full + EXPAND_STAGES;
-    uint64_t* done = empty + EXPAND_STAGES;
-    uint32_t* tmem_slot = (uint32_t*)(done + 1);
+    uint64_t *made = empty + EXPAND_STAGES, *taken = made + 2;          // [2] a step's products are complete / have joined the sums
+    uint32_t* tmem_slot = (uint32_t*)(taken + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -104,7 +114,10 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid
             tc::mbar_init(&full[i], 1);
             tc::mbar_init(&empty[i], 1);
         }
-        tc::mbar_init(done, 1);
+        for (int i = 0; i < 2; ++i) {
+            tc::mbar_init(&made[i], 1);
+            tc::mbar_init(&taken[i], 2 * ROW_WARPS);
+        }
         *abort_flag = 0;
         tc::fence_barrier_init();
         tc::tma_prefetch_desc(&cache_map);
@@ -112,7 +125,7 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid
         tc::tma_prefetch_desc(&uv_map);
     }
     if (warp == 1) {
-        tc::tmem_alloc(tmem_slot, 2 * D);
+        tc::tmem_alloc(tmem_slot, 4 * D);
         tc::tmem_relinquish();
     }
     tc::tc_fence_before();
@@ -132,96 +145,112 @@ latent_expand_kernel(const __grid_constant__ CUtensorMap cache_map, const __grid
     const int* table = block_tables + (size_t)row_request[row0] * table_stride;
     const int n_steps = C / 64;
 
-    if (active && warp == 0) {
-        // Lane l < 8: the sixteen keys from key0 + 16 l; a page that the window has given back (-1), or past the last key,
-        // is read from page 0 and written as zeros.
-        const int t = key0 + 16 * lane;
-        const int page = lane < 8 && t < end ? max(table[t / page_size], 0) : 0;
-        const int slot = page * page_size + t % page_size;
-        bool ok = true;
-        for (int s = 0; s < n_steps; ++s) {
-            const int st = s % EXPAND_STAGES;
-            ok = tc::mbar_wait_warp(&empty[st], ((s / EXPAND_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_LAT_EXPAND);
-            if (!ok) break;
-            uint8_t* base = smem + st * EXPAND_STAGE;
-            if (lane == 0) tc::mbar_expect_tx(&full[st], EXPAND_STAGE);
-            __syncwarp();
-            if (lane < 8) tc::tma_load_2d(base + lane * 16 * 128, &cache_map, s * 64, slot, &full[st]);
-            else if (lane == 8) tc::tma_load_2d(base + ROWS * 128, &uk_map, s * 64, head * D, &full[st]);
-            else if (lane == 9) tc::tma_load_2d(base + 2 * ROWS * 128, &uv_map, s * 64, head * D, &full[st]);
-        }
-    } else if (active && warp == 1) {
-        if (tc::elect_one()) {
-            bool ok = true;
-            for (int s = 0; s < n_steps && ok; ++s) {
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FEWER_REGISTERS));
+        if (active && warp == 0) {
+            // Lane l < 8: the sixteen keys from key0 + 16 l; a page that the window has given back (-1), or past the last key,
+            // is read from page 0 and written as zeros.
+            const int t = key0 + 16 * lane;
+            const int page = lane < 8 && t < end ? max(table[t / page_size], 0) : 0;
+            const int slot = page * page_size + t % page_size;
+            for (int s = 0; s < n_steps; ++s) {
                 const int st = s % EXPAND_STAGES;
-                ok = tc::mbar_wait(&full[st], (s / EXPAND_STAGES) & 1u, abort_flag, error_word, ERR_LAT_EXPAND);
+                if (!tc::mbar_wait_warp(&empty[st], ((s / EXPAND_STAGES) & 1u) ^ 1u, abort_flag, error_word, ERR_LAT_EXPAND)) break;
+                uint8_t* base = smem + st * EXPAND_STAGE;
+                if (lane == 0) tc::mbar_expect_tx(&full[st], EXPAND_STAGE);
+                __syncwarp();
+                if (lane < 8) tc::tma_load_2d(base + lane * 16 * 128, &cache_map, s * 64, slot, &full[st]);
+                else if (lane == 8) tc::tma_load_2d(base + ROWS * 128, &uk_map, s * 64, head * D, &full[st]);
+                else if (lane == 9) tc::tma_load_2d(base + 2 * ROWS * 128, &uv_map, s * 64, head * D, &full[st]);
+            }
+        } else if (active && warp == 1) {
+            if (tc::elect_one()) {
+                for (int s = 0; s < n_steps; ++s) {
+                    const int st = s % EXPAND_STAGES;
+                    if (!tc::mbar_wait(&taken[s & 1], ((s >> 1) & 1u) ^ 1u, abort_flag, error_word, ERR_LAT_EXPAND) ||
+                        !tc::mbar_wait(&full[st], (s / EXPAND_STAGES) & 1u, abort_flag, error_word, ERR_LAT_EXPAND))
+                        break;
+                    tc::tc_fence_after();
+                    const uint32_t a = tc::smem_u32(smem + st * EXPAND_STAGE);
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                        for (int w = 0; w < 2; ++w)
+                            tc::mma_bf16_ss(tmem_base + (2 * (s & 1) + w) * D, tc::smem_desc_k_sw128(a + kk * 32),
+                                            tc::smem_desc_k_sw128(a + (1 + w) * ROWS * 128 + kk * 32), IDESC_EXPAND, kk > 0 ? 1u : 0u);
+                    tc::mma_commit(&empty[st]);
+                    tc::mma_commit(&made[s & 1]);
+                }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(MORE_REGISTERS));
+        if (active) {
+            const int which = (warp - 4) / ROW_WARPS;          // 0: keys, 1: values
+            const int quarter = warp & 3, row = quarter * 32 + lane, t = key0 + row;
+            const bool real = t >= lo && t < end;
+            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+            if (which == 0) {
+                __nv_bfloat16* dst = expanded + ((size_t)blockIdx.y * tokens + rq[2] + blockIdx.x * ROWS + row) * (TOKEN_BLOCKS * 64);
+                uint4* rot = reinterpret_cast<uint4*>(dst + 3 * D);
+                const uint4* src = reinterpret_cast<const uint4*>(
+                    cache + ((size_t)(real ? table[t / page_size] : 0) * page_size + t % page_size) * (C + R) + C);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) rot[i] = real && i * 8 < R ? src[i] : zero;
+            }
+            float sum[D];
+#pragma unroll
+            for (int d = 0; d < D; ++d) sum[d] = 0.0f;
+            bool ok = true;
+            for (int s = 0; s < n_steps; ++s) {
+                ok = tc::mbar_wait_warp(&made[s & 1], (s >> 1) & 1u, abort_flag, error_word, ERR_LAT_EXPAND);
                 if (!ok) break;
                 tc::tc_fence_after();
-                const uint32_t a = tc::smem_u32(smem + st * EXPAND_STAGE);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-                    for (int w = 0; w < 2; ++w)
-                        tc::mma_bf16_ss(tmem_base + w * D, tc::smem_desc_k_sw128(a + kk * 32),
-                                        tc::smem_desc_k_sw128(a + (1 + w) * ROWS * 128 + kk * 32), IDESC_EXPAND, (s > 0 || kk > 0) ? 1u : 0u);
-                tc::mma_commit(&empty[st]);
-            }
-            if (ok) tc::mma_commit(done);
-        }
-    } else if (active) {
-        const int quarter = warp & 3, row = quarter * 32 + lane, t = key0 + row;
-        const bool real = t >= lo && t < end;
-        __nv_bfloat16* dst = expanded + ((size_t)blockIdx.y * tokens + rq[2] + blockIdx.x * ROWS + row) * (TOKEN_BLOCKS * 64);
-        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-        uint4* rot = reinterpret_cast<uint4*>(dst + 3 * D);
-        const uint4* src = reinterpret_cast<const uint4*>(
-            cache + ((size_t)(real ? table[t / page_size] : 0) * page_size + t % page_size) * (C + R) + C);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) rot[i] = real && i * 8 < R ? src[i] : zero;
-        // The four warps of rows go on together or not at all: they meet at barriers below.
-        if (all_rows(tc::mbar_wait(done, 0, abort_flag, error_word, ERR_LAT_EXPAND))) {
-            tc::tc_fence_after();
-#pragma unroll 1
-            for (int which = 0; which < 2; ++which) {          // the keys' parts, then the values'
-#pragma unroll 1
                 for (int c = 0; c < D; c += 32) {
                     uint32_t v[32];
-                    tc::tmem_ld_32x32(tmem_base + which * D + c + ((uint32_t)(quarter * 32) << 16), v);
+                    tc::tmem_ld_32x32(tmem_base + (2 * (s & 1) + which) * D + c + ((uint32_t)(quarter * 32) << 16), v);
                     tc::tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint32_t p[3][4];
+                    for (int k = 0; k < 32; ++k) sum[c + k] += __uint_as_float(v[k]);
+                }
+                tc::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&taken[s & 1]);
+            }
+            // The last step's products are complete, so all stages are free.  The four warps of keys, or of values, go on together or
+            // not at all: they meet at a barrier below.
+            uint8_t* parts = smem + which * 6 * ROWS * 128;
+            if (all_four_warps(1 + which, ok)) {
 #pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            attn::split3_pair(__uint_as_float(v[i + 2 * u]), __uint_as_float(v[i + 2 * u + 1]), p[0][u], p[1][u], p[2][u]);
+                for (int c = 0; c < D; c += 8) {
+                    uint32_t p[3][4];
 #pragma unroll
-                        for (int q = 0; q < 3; ++q)
-                            *reinterpret_cast<uint4*>(smem + (2 * q + (c >> 6)) * ROWS * 128 + attn::swz(row, ((c & 63) + i) >> 3)) =
-                                real ? make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]) : zero;
-                    }
+                    for (int u = 0; u < 4; ++u) attn::split3_pair(sum[c + 2 * u], sum[c + 2 * u + 1], p[0][u], p[1][u], p[2][u]);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q)
+                        *reinterpret_cast<uint4*>(parts + (2 * q + (c >> 6)) * ROWS * 128 + attn::swz(row, (c & 63) >> 3)) =
+                            real ? make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]) : zero;
                 }
                 tc::fence_proxy_async();
-                asm volatile("bar.sync 1, 128;" ::: "memory");                 // the four warps of rows
-                if (threadIdx.x == 64) {
+                all_four_warps(1 + which, true);
+                if (quarter == 0 && lane == 0) {
                     for (int b = 0; b < 12; ++b)
                         asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];"
-                                     ::"l"(&expanded_map), "r"(tc::smem_u32(smem + (b >> 1) * ROWS * 128 + (b & 1) * BLOCK_BYTES)), "r"(0),
+                                     ::"l"(&expanded_map), "r"(tc::smem_u32(parts + (b >> 1) * ROWS * 128 + (b & 1) * BLOCK_BYTES)), "r"(0),
                                      "r"(rq[2] + (int)blockIdx.x * ROWS + (b & 1) * KEYS), "r"((which ? K_BLOCKS : 0) + (b >> 1)), "r"((int)blockIdx.y),
                                      "r"(0) : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    if (which == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    else asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");                 // the copies have read what the next half overwrites
             }
+            tc::tc_fence_before();
         }
-        tc::tc_fence_before();
     }
     __syncthreads();
     if (warp == 1) {
         tc::tc_fence_after();
-        tc::tmem_dealloc(tmem_base, 2 * D);
+        tc::tmem_dealloc(tmem_base, 4 * D);
     }
 }
 
@@ -508,7 +537,7 @@ LLMX_EXPORT int llmx_latent_expand(const void* cache, long long pool_tokens, con
     if (int e = llmx_make_map_bf16_2d(&uk_map, w_uk, (uint64_t)all_heads * D, (uint64_t)C, D, 64)) return e;
     if (int e = llmx_make_map_bf16_2d(&uv_map, w_uv, (uint64_t)all_heads * D, (uint64_t)C, D, 64)) return e;
     if (int e = allow_smem(latent_expand_kernel, EXPAND_SMEM)) return e;
-    launch_kernel(latent_expand_kernel, dim3(max_tokens / ROWS, n_heads, n_req), dim3(PROMPT_THREADS), (size_t)EXPAND_SMEM, stream, cache_map,
+    launch_kernel(latent_expand_kernel, dim3(max_tokens / ROWS, n_heads, n_req), dim3(EXPAND_THREADS), (size_t)EXPAND_SMEM, stream, cache_map,
                   uk_map, uv_map, expanded_map, (const __nv_bfloat16*)cache, (__nv_bfloat16*)expanded, requests, row_request, positions, block_tables,
                   table_stride, tokens, head0, C, R, page_size, window, error_word);
     return launch_status();

@@ -1305,3 +1305,51 @@ def test_attention_over_many_keys_rounds_as_the_exact_one(keys, mean):
     nearest = want.float().bfloat16().view(rows, -1)
     share, before = ((x != nearest).double().mean().item() for x in (out, other))
     assert share <= (4e-4 if mean else max(before, 4e-4)), (share, before)
+
+
+@pytest.mark.parametrize("mean,spread", [(0.5, 0.1), (0.5, 1.0), (0.0, 1.0)])
+@pytest.mark.parametrize("history", [0, 512])
+def test_latent_prompts_round_as_the_exact_ones(mean, spread, history):
+    """How many results round to another bfloat16 than the 64-bit ones: no more in the form for many rows, whose keys, values, scores
+    and outputs pass through the tensor cores' accumulators, than in the general form.  Latents of one sign and of both, even
+    and peaked scores; a twentieth is left for chance (the counts are in the hundreds)."""
+    from llmx_b200 import ops
+    from llmx_b200.parts.base import Precision, StepShape
+    from llmx_b200.parts.latent_attention import LatentAttention
+    from llmx_b200.runtime import check_errors
+    g = torch.Generator(device="cuda").manual_seed(history)
+    rows, heads, latent, rot, page, scale = 512, 8, 512, 64, 16, 192 ** -0.5 * spread
+    part = LatentAttention(64, heads, 128, rot, 128, None, latent, scale, 1e4, rot, 1e-6, None)
+    part.precision, part._sms = Precision.of("bfloat16"), 148
+    part.w_uk, part.w_uv = (torch.randn(heads * 128, latent, device="cuda", generator=g).mul_(latent ** -0.5).bfloat16() for _ in range(2))
+    freq = torch.from_numpy(part.frequencies()[0]).cuda()
+    plan = part.plan_step(StepShape([rows], [history]))
+    ints = torch.tensor(plan.values, device="cuda")
+    keys = rows + history
+    cache = torch.randn(keys // page, 1, 1, page, latent + rot, device="cuda", generator=g)
+    cache[..., :latent] += mean
+    cache = cache.bfloat16()
+    q = torch.randn(rows, heads * (128 + rot), device="cuda", generator=g)
+    positions = torch.arange(history, keys, dtype=torch.int32, device="cuda")
+    meta = torch.zeros(rows, dtype=torch.int32, device="cuda"), positions, torch.arange(keys // page, dtype=torch.int32, device="cuda")[None].contiguous()
+    sizes = (heads, 128, rot, 128, latent, page, None, scale)
+    out, general = (torch.zeros(rows, heads * 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    first, n_req, share, tiles_at, n_tiles, tokens, group = plan.wide
+    ops.latent_attention_prompt(q, cache, part.w_uk, part.w_uv, out, freq, *meta, ints[first:], n_req, share, ints[tiles_at:], n_tiles, tokens, group, *sizes)
+    _, _, at, n_tiles, splits = plan.whole
+    ops.latent_attention_tiled(q, cache, part.w_uk, part.w_uv, general, freq, *meta, ints[at:], n_tiles, splits, *sizes)
+    check_errors()
+    c, pos = cache.view(-1, latent + rot).double(), positions.double()
+    angle = (positions[:, None].float() * freq[None]).double()
+    unseen = torch.arange(keys, device="cuda")[None] > positions[:, None]
+    want = torch.empty(rows, heads, 128, device="cuda", dtype=torch.float64)
+    for h in range(heads):
+        x = q.view(rows, heads, -1)[:, h].double()
+        a, b = x[:, 128::2], x[:, 129::2]
+        turned = torch.stack([a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()], 2).reshape(rows, rot)
+        uk, uv = (w[h * 128:(h + 1) * 128].double() for w in (part.w_uk, part.w_uv))
+        s = (x[:, :128] @ (uk @ c[:, :latent].T) + turned @ c[:, latent:].T) * scale
+        want[:, h] = torch.softmax(s.masked_fill(unseen, -math.inf), 1) @ (c[:, :latent] @ uv.T)
+    nearest = want.float().bfloat16().view(rows, -1)
+    made, before = ((o != nearest).double().mean().item() for o in (out, general))
+    assert made <= 1.05 * before, (made, before)
