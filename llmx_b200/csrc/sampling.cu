@@ -17,9 +17,12 @@
 // each scans its slice of the vocabulary, their counts and sums meet in the first block's shared memory, which
 // decides (one block alone issues instructions for 150,000 scores at about 25 us a pass, whatever its loads do).
 // The top-k threshold is found by radix selection over the 32-bit order-preserving image of the score (counting
-// tokens): the pass that finds the best token also counts the leading eight bits, the next one lists each block's tokens at or
-// above the bin that holds the k-th, and what follows reads that list (a few hundred tokens) instead of the row.  32 rows of
-// 151,936, top-k 40: 50 -> 35 us.  When the kept set then fits shared memory (top-k of at most 1,024, the usual case) it is gathered
+// tokens): the pass that finds the best token also counts the leading eight bits, and as soon as a block's own counts say that
+// its tokens at or above the bin that holds the k-th fit a list, the next pass writes it and what follows reads the list instead of
+// the row (the leading eight bits tell scores apart by a factor of four: usually that leaves a few hundred tokens; scores that all
+// lie within such a factor, or a thousand kept of a wide row, leave a quarter of the row and more, and sixteen bits are needed).
+// 32 rows of 151,936, us with full passes, with a list after eight bits that is given up when it overflows, and so: top-k 40 of
+// normal scores 57, 41, 42; of scores between 8 and 32 56, 60, 47; top-k 1,000 of those 231, 243, 216.  When the kept set then fits shared memory (top-k of at most 1,024, the usual case) it is gathered
 // there, ranked, and the nucleus, min-p and the draw are one thread's walk over it with double sums, exactly the
 // reference's walk.  Without top-k (or a larger one) nothing is gathered: thresholds by radix selection over the
 // vocabulary, summing weights.
@@ -135,7 +138,7 @@ struct Shared {
     uint32_t u32[4];
     double f64[4];
     int i32[8];
-    int n_hits, n_kept, walked, n_listed;
+    int n_hits, n_kept, walked, n_listed, n_above, n_reached;
     int hit_list[TIES];
     int c_id[KMAX], o_id[KMAX];
     uint32_t c_bits[KMAX], l_bits[KMAX];
@@ -394,8 +397,8 @@ __device__ __forceinline__ void find_count_bin(Shared& sh, int remaining) {
 // tokens with exactly those bits are among the k best, and the lowest id with those bits (the last round notes each
 // bin's, so that the usual case -- one token of the tie is taken -- needs no pass of its own).  A round: every block
 // counts its slice's tokens by the next eight bits, adds its bins to the leader's, and the leader finds the bin that
-// holds the k-th.  The first round was `best_token`'s.  The second lists the block's tokens at or above the first round's bin;
-// `listed` is their number, or -1 when they are more than the list holds (every block for itself).
+// holds the k-th.  The first round was `best_token`'s, whose counts the block still holds.  A round lists the block's tokens at or above
+// the bin found so far if they fit and no earlier round did; `listed` is their number, or -1 (every block for itself).
 __device__ void select_by_count(const Row& c, const Sets& sets, uint32_t& out_bits, int& out_equal_taken, int& out_first_id, int& listed) {
     Shared& sh = *c.sh;
     uint32_t prefix = lead_load(&sh.u32[0]) << 24, mask = 255u << 24;
@@ -403,20 +406,33 @@ __device__ void select_by_count(const Row& c, const Sets& sets, uint32_t& out_bi
     int* ids = reinterpret_cast<int*>(c.stripes);
     float* scores = reinterpret_cast<float*>(ids + LISTED);
     listed = -1;
+    if (threadIdx.x == 0) sh.n_above = 0;
     for (int shift = 16; shift >= 0; shift -= 8) {
+        if (threadIdx.x < 32) {
+            // The block's tokens above the bin found so far, and those in it with them.
+            const int bin = (int)(prefix >> (shift + 8) & 255u);
+            int above = 0;
+            for (int i = threadIdx.x; i < 256; i += 32) above += i > bin ? (int)sh.count[i] : 0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
+            if (threadIdx.x == 0) {
+                sh.n_above += above;
+                sh.n_reached = sh.n_above + (int)sh.count[bin];
+                sh.n_listed = 0;
+            }
+        }
+        __syncthreads();
+        const bool list = listed < 0 && sh.n_reached <= LISTED;
         for (int i = threadIdx.x; i < 256; i += THREADS) { sh.count[i] = 0; sh.min_id[i] = NO_ID; }
-        if (threadIdx.x == 0) sh.n_listed = 0;
         __syncthreads();
         RunCount run;
         scan_listed(c, listed, [&](int id, float s, bool ok) {
             const uint32_t b = order_bits(s);
             if (!ok || id == sets.skip || b < prefix) return;
-            if (shift == 16) {
-                const int slot = atomicAdd(&sh.n_listed, 1);
-                if (slot < LISTED) {
-                    ids[slot] = id;
-                    scores[slot] = s;
-                }
+            if (list) {
+                const int slot = atomicAdd(&sh.n_listed, 1);     // below n_reached
+                ids[slot] = id;
+                scores[slot] = s;
             }
             if ((b & mask) != prefix) return;
             const int bin = (b >> shift) & 255u;
@@ -425,7 +441,7 @@ __device__ void select_by_count(const Row& c, const Sets& sets, uint32_t& out_bi
         });
         run.flush(sh.count);
         __syncthreads();
-        if (shift == 16 && sh.n_listed <= LISTED) listed = sh.n_listed;
+        if (list) listed = sh.n_listed;
         if (threadIdx.x < 256 && sh.count[threadIdx.x]) {
             lead_add(&sh.gcount[threadIdx.x], sh.count[threadIdx.x]);
             if (shift == 0) lead_min(&sh.gmin_id[threadIdx.x], sh.min_id[threadIdx.x]);

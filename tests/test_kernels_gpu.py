@@ -578,6 +578,22 @@ def test_sampling_settings_at_random_against_the_plain_sampler(vocab, coarse):
     assert halves == expected
 
 
+@pytest.mark.parametrize("kind", ["one_binade", "wide", "two_values", "negative"])
+def test_sampling_of_rows_whose_best_tokens_outnumber_a_blocks_list(kind):
+    """Scores whose leading eight bits hardly tell them apart (all within a factor of two or four, of two values, a third of the row
+    above the threshold's leading bits): a block's tokens do not fit its list (8,192) after the first round, after the second,
+    or ever.  Against the plain sampler, with one row (eight blocks) and with sixteen (four)."""
+    rng = np.random.default_rng(len(kind))
+    vocab, rows = 151936, 16
+    logits = {"one_binade": 8 + 8 * rng.random((rows, vocab)), "wide": 3 * rng.standard_normal((rows, vocab)),
+              "two_values": 1.0 + 0.5 * (rng.random((rows, vocab)) < 0.4), "negative": -32 + 24 * rng.random((rows, vocab))}[kind].astype(np.float32)
+    settings = [dict(temp=float(t), top_k=int(k), top_p=float(p), seed=r + 1, masked=7 if r % 3 == 0 else -1)
+                for r, (t, k, p) in enumerate(zip(rng.choice([0.7, 1.0], rows), np.resize([1, 40, 1000, 1024, 1025, 3000, 100000, 62000], rows), rng.choice([1.0, 0.9], rows)))]
+    expected = [plain.sample(row, s["temp"], s["top_k"], s["top_p"], 0.0, plain.XorShift64(s["seed"]).unit(), masked=s["masked"]) for row, s in zip(logits, settings)]
+    assert _sample_rows(logits.copy(), settings)[0] == expected
+    assert [_sample_rows(logits[r:r + 1].copy(), settings[r:r + 1])[0][0] for r in range(8)] == expected[:8]
+
+
 def test_sampling_distribution_and_independence_of_the_batch():
     """Draws follow the softmax, and a request's draws do not depend on what shares its batch."""
     from llmx_b200.sampling import RequestSampling, SamplingParams, sample
