@@ -37,10 +37,22 @@ from .rope import blended_frequencies, power_frequencies
 
 
 # Requests that bring at least this many rows, and one for this many of the keys they see, have their keys and values made
-# (csrc/latent_prompt_tc.cu): making them costs the same for one row as for many.  Measured, us, that form / the general one, 16
-# heads of 128 + 64 over latents of 512: after nothing 16 rows 45 / 53, 32 rows 46 / 68, 512 rows 75 / 394; after 1,000 tokens 16
-# rows 98 / 80, 32 rows 102 / 131, 512 rows 137 / 840; after 8,000 tokens 32 rows 538 / 364, 64 rows 539 / 640, 512 rows 574 / 3,973.
-PROMPT_ROWS, PROMPT_KEYS_A_ROW = 32, 128
+# (csrc/latent_prompt_tc.cu): making them costs the same for one row as for many.  Their tiles walk all keys one stage after the
+# other, a block a tile and head, so when the step has few tiles its time is that of the longest walk, once for every group of
+# heads, while the general form cuts keys into ranges that fill the device: beyond PROMPT_FEW_KEYS keys the step's rows x heads (weighted by their
+# keys) must also reach `_rows_needed`.  Measured, us, that form / the general one:
+#   16 heads of 128 + 64 over latents of 512, one group: after nothing 32 rows 46 / 50, 512 rows 80 / 419; after 1,000 tokens 32 rows 93 / 106;
+#   after 2,000 32 rows 148 / 134, 40 148 / 175; after 4,000 32 rows 265 / 181, 40 269 / 259, 48 269 / 294; after 8,000 48 rows
+#   490 / 484, 64 490 / 607; two groups after 12,000 96 rows 1,291 / 1,236, 128 1,302 / 1,557
+#   32 heads: after 4,000 32 rows 310 / 359; two groups after 5,000 48 rows 644 / 550, 64 648 / 722; four after 16,000 128 rows 3,388 / 3,823
+PROMPT_ROWS, PROMPT_KEYS_A_ROW, PROMPT_FEW_KEYS = 32, 128, 1280
+
+
+def _rows_needed(keys: int, groups: int) -> int:
+    """Rows x heads from which making keys and values is the faster form, for walks of `keys` keys and heads in `groups`."""
+    return 480 + keys // 24 if groups == 1 else 900 * groups
+
+
 # The workspace of made keys and values: heads are taken in groups that fit these bytes, or what the general form's queries
 # and sums over the same rows would take if that is more.
 PROMPT_BYTES = 256 << 20
@@ -151,21 +163,22 @@ class LatentAttention(Part):
 
     def _wide(self, counts, contexts):
         """The requests whose keys and values are made: (ints of the requests, ints of their tiles, largest share of the
-        workspace, workspace tokens, heads a group), or None when there are none or their workspace would not fit."""
-        requests, tiles, start, tokens, rows = [], [], 0, 0, 0
+        workspace, workspace tokens, heads a group), or None when there are none, their workspace would not fit or the general
+        form is the faster one for them."""
+        requests, tiles, start, tokens, rows, longest, work = [], [], 0, 0, 0, 0, 0
         for n, context in zip(counts, contexts):
             keys = context if self.window is None else min(context, self.window + n - 1)
             if n >= PROMPT_ROWS and n * PROMPT_KEYS_A_ROW >= keys:
                 share = -(-(keys + 63) // 128) * 128             # the first key lies up to 63 tokens into its share
                 requests.append((start, n, tokens, share))
                 tiles += [(start + i, min(128, n - i), tokens, start) for i in reversed(range(0, n, 128))]
-                tokens, rows = tokens + share, rows + n
+                tokens, rows, longest, work = tokens + share, rows + n, max(longest, keys), work + n * self.heads * keys
             start += n
         if not requests:
             return None
         room = max(PROMPT_BYTES, rows * self.heads * (2 * self.kv_rank + self.rot_dim + 2) * 4)
         group = min(self.heads, room // (tokens * ops.LATENT_EXPANDED * 2))
-        if group < 1:
+        if group < 1 or (longest > PROMPT_FEW_KEYS and work < _rows_needed(longest, -(-self.heads // group)) * longest):
             return None
         return requests, tiles, max(r[3] for r in requests), tokens, group
 
