@@ -45,12 +45,14 @@ from .rope import blended_frequencies, power_frequencies
 #   after 2,000 32 rows 148 / 134, 40 148 / 175; after 4,000 32 rows 265 / 181, 40 269 / 259, 48 269 / 294; after 8,000 48 rows
 #   490 / 484, 64 490 / 607; two groups after 12,000 96 rows 1,291 / 1,236, 128 1,302 / 1,557
 #   32 heads: after 4,000 32 rows 310 / 359; two groups after 5,000 48 rows 644 / 550, 64 648 / 722; four after 16,000 128 rows 3,388 / 3,823
+#   several requests, 16 heads: 2 x 32 rows after 4,000 312 / 359, 4 x 33 after 2,000 228 / 433; in groups 2 x 32 after 8,000 974 / 609,
+#   8 x 32 after 4,000 (four groups) 1,231 / 1,123
 PROMPT_ROWS, PROMPT_KEYS_A_ROW, PROMPT_FEW_KEYS = 32, 128, 1280
 
 
 def _rows_needed(keys: int, groups: int) -> int:
     """Rows x heads from which making keys and values is the faster form, for walks of `keys` keys and heads in `groups`."""
-    return 480 + keys // 24 if groups == 1 else 900 * groups
+    return 480 + keys // 24 if groups == 1 else groups * (900 + 600000 // keys)
 
 
 # The workspace of made keys and values: heads are taken in groups that fit these bytes, or what the general form's queries

@@ -24,9 +24,10 @@ def test_few_rows_after_many_keys_take_the_form_that_is_faster_for_them(heads, r
 
 
 def test_several_requests_count_together():
-    """Eight requests of few rows fill the device as one of many does; a request beside them that brings one row stays with the
-    general form, and every row belongs to one of the two."""
-    plan = _wide(16, [32] * 8 + [1], [4000] * 9)
-    assert plan is not None and plan.wide[1] == 8 and plan.runs and sum(r[1] for r in plan.runs) == 1
+    """Requests of few rows add up while their heads fit one group; a request beside them that brings one row stays with the general
+    form, and every row belongs to one of the two.  In several groups every one walks all keys again."""
+    plan = _wide(16, [32, 1, 32], [4000, 4000, 4000])
+    assert plan is not None and plan.wide[1] == 2 and sum(r[1] for r in plan.runs) == 1
     assert _wide(16, [32, 1], [4000, 9]) is None
-    assert _wide(16, [32] * 8, None, room=4096) is not None
+    assert _wide(16, [33] * 4, [2000] * 4) is not None and _wide(16, [33] * 4, None, room=2048) is not None
+    assert _wide(16, [32] * 2, [8000] * 2) is None and _wide(16, [32] * 8, [4000] * 8) is None
