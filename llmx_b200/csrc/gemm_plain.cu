@@ -6,6 +6,10 @@
 // Each output's sum runs over k in increasing order whatever M is, so a row's result
 // does not depend on what else is in the batch (the reference's rule,
 // src/backends/backend.hpp:141-150; its kernels: f32.gpu:1034-1084).
+//
+// Three forms with the same bits: up to eight rows a thread an output column (`gemm_plain_few_kernel`, which reads its
+// first weights before it waits for the kernel before: W must not be that kernel's output), more than 64 rows 128 x 64 tiles with two
+// multiply-adds an instruction (`gemm_plain_many_kernel`), both for K in fours and aligned operands of one type; else 64 x 64 tiles.
 #include "common.cuh"
 
 namespace {

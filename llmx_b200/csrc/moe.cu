@@ -441,8 +441,9 @@ moe_few_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv_bfloat
 // The warps' number divides the ring's places, so that a place is always the same warp's: a waiter tells uses of a place
 // apart by parity only, and a warp that came to a place before its last use had landed would take it for the next.
 // Eight pairs that name six experts, gate and up of K 4,096 and N 3,072: 70 -> 57 us, down 38.7 -> 32; two pairs 38.8 -> 22
-// and 15.4 -> 12.6 us.  Bound by the dot products more than by the memory where an expert's rows meet several pairs: sixteen
-// pairs on twelve experts took 204 us (eight warps) against the kernel above's 118, so the line lies at eight.
+// and 15.4 -> 12.6 us.  Bound by the dot products more than by the memory where an expert's rows meet several pairs.  Eight is the most it
+// takes; beyond, stream / kernel above, gate and up, inputs out of the cache: K 4,096 nine pairs on nine experts 93 / 96 us, sixteen on
+// twelve 123 / 133, on two 78 / 123; K 2,048 sixteen on sixteen 53 / 51, on two 29 / 39; down products equal or up to 40 % faster.
 constexpr int FEW_PAIRS = 8, FEW_WARPS = 16, FEW_THREADS = 32 * FEW_WARPS + 32, FEW_PLACES = 32, FEW_K = 12288, FEW_RING = 192 * 1024;
 enum : int { ERR_FEW_PRODUCER = 451, ERR_FEW_CONSUMER = 452 };
 

@@ -883,7 +883,6 @@ int launch_recurrence(int D, bool wide, int requests, cudaStream_t stream, const
         if (D <= 256) LLMX_WIDE_COLS(8, 32, 2, 16);
         if (D <= 512) LLMX_WIDE_COLS(16, 32, 1, 16);
 #undef LLMX_WIDE_COLS
-#undef LLMX_WIDE_COLS
 #undef LLMX_WIDE
     } else {
         if (D <= 16) LLMX_REC(2, 8);
@@ -959,7 +958,7 @@ LLMX_EXPORT int llmx_conv_prepare(const float* proj, int stride, int first, int 
         (((uintptr_t)proj | (uintptr_t)ready | (uintptr_t)state | (uintptr_t)taps_b) & 15) == 0) {
         const int per = gate_kind == 2 ? heads * D : heads, block = CONV_THREADS * 4;
         const int conv_blocks = (channels + block - 1) / block, gate_blocks = (per + CONV_THREADS - 1) / CONV_THREADS;
-        // One row a block while that leaves the SMs' 296 places unfilled, longer runs of rows beyond.
+        // One row a block while there are fewer blocks than four to an SM, longer runs of rows beyond.
         int run = (int)((long long)rows * conv_blocks / 592);
         run = run < 1 ? 1 : run > CONV_RUN ? CONV_RUN : run;
         const int row_blocks = (rows + run - 1) / run;

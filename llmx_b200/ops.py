@@ -328,7 +328,8 @@ def swiglu(gu: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
 
 
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
-    """out (+)= a @ w.T on the CUDA cores; a [M, K], w [N, K] of one type, out float32 [M, N]."""
+    """out (+)= a @ w.T on the CUDA cores; a [M, K], w [N, K] of one type, out float32 [M, N].  `w` is a weight: with few rows it is read
+    before the kernel launched just before has ended, so it must not be what another of this module's kernels has just written."""
     _cuda(a, w, out)
     m, k = a.shape
     n = w.shape[0]
