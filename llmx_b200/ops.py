@@ -937,7 +937,7 @@ def attention_tiled(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, ste
           "attention: cache layout does not fit")
     _need(block_tables.dtype == torch.int32 and block_tables.dim() == 2 and rows == step.rows, "attention: metadata does not fit")
     if (key_dim == 128 and value_dim == 128 and cache.shape[3] % 16 == 0 and scale > 0 and heads // kv_heads <= 128 and (extras or NO_EXTRAS).plain
-            and cache.numel() // 256 < 2 ** 31):
+            and cache.numel() // 256 < 2 ** 31 and rows * heads < 2 ** 31):
         _check(_fn("attention_rows_tc", "llmx_attention_rows_tc")(
             _ptr(q), _ptr(cache), cache.numel() // 256, _ptr(out), _ptr(step.row_start), _ptr(step.row_count), _ptr(step.history),
             _ptr(block_tables), block_tables.shape[1], rows, step.requests, heads, kv_heads, cache.shape[3], int(window or 0),

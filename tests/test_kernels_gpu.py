@@ -1231,10 +1231,11 @@ def test_gated_unit_at_extreme_inputs():
 
 
 @pytest.mark.parametrize("heads,kv_heads,page,window,chunk", [(4, 1, 16, None, None), (3, 1, 32, 70, None), (32, 2, 48, None, 96), (2, 2, 16, 1, None), (10, 2, 16, 64, 200)])
-@pytest.mark.parametrize("counts,histories", [([5], [0]), ([128, 1, 33], [0, 63, 64]), ([65, 7], [700, 130]), ([300], [1])])
+@pytest.mark.parametrize("counts,histories", [([5], [0]), ([128, 1, 33], [0, 63, 64]), ([65, 7], [700, 130]), ([300], [1]),
+                                              ([1 + r % 3 for r in range(210)], [(37 * r) % 130 for r in range(210)])])
 def test_attention_of_rows_that_share_their_keys(heads, kv_heads, page, window, chunk, counts, histories):
-    """The tcgen05 form of the tiled attention against 64 bits: runs of rows below, at and above a tile, padded head groups, windows
-    and chunks that begin within a stage; every slot of the cache that no row may see holds NaN, pages below a window are
+    """The tcgen05 form of the tiled attention against 64 bits: runs of rows below, at and above a tile, as many requests as give
+    every SM a second tile and some a third (210 or 420 tiles on 148), padded head groups, windows and chunks that begin within a stage; every slot of the cache that no row may see holds NaN, pages below a window are
     given back.  Weights keep 24 bits, so the result's own rounding decides: twice its 2^-9 are allowed (how exactly the sums behind it
     are made, `test_attention_over_many_keys_rounds_as_the_exact_one` counts)."""
     import types
