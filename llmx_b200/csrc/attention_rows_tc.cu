@@ -19,8 +19,8 @@
 // 4,096 keys left 0.65 % of the results at another bfloat16 than the exact ones (values of mean 1; 0.28 % in the form on mma.sync, whose
 // accumulators run through too, 0.002 % so), 16,384 keys 2.6 % (1.4 %; 0.004 %).
 // With 48 keys a stage, scores, weights and output have tensor memory of their own: a stage's scores are made while the weights of
-// the one before are.  209 KB of shared memory and all of tensor memory a block.  What bounds it: the products of an SM's two tiles (80 %
-// of the tensor pipe's cycles on the SMs that have work to the end), and the causal edge: the last tiles of a prompt see all keys.
+// the one before are.  209 KB of shared memory and all of tensor memory a block.  What bounds it: the products of an SM's two tiles (with
+// two long ones on it the tensor pipe was busy 80 % of the cycles), and the causal edge: the last tiles of a prompt see all keys.
 // 2,048 rows of 16 heads over 4: 330 us on mma.sync, 70 so; 1,201 rows of 32 over 8: 240 -> 59 (72 and 50 with sums and weights that
 // were less exact); 64 rows of 16 over 4 16 us.
 //
@@ -352,6 +352,8 @@ LLMX_EXPORT int llmx_attention_rows_tc(const void* q, const void* cache, long lo
     if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || heads / kv_heads > ROWS || kv_heads > 65535 || page_size <= 0 || page_size % RUN ||
         pool_rows <= 0 || pool_rows >= (1ll << 31) || (long long)rows * heads >= (1ll << 31) || !(scale > 0.0f) || (((uintptr_t)q | (uintptr_t)cache | (uintptr_t)out) & 15))
         return LLMX_ERR_UNSUPPORTED;
+    static const bool enough = registers_reach(attention_rows_kernel, THREADS, FEWER_REGISTERS + PLACES * MORE_REGISTERS);
+    if (!enough) return LLMX_ERR_UNSUPPORTED;
     int r_pad = 1;
     while (r_pad < heads / kv_heads) r_pad *= 2;
     const int tok = ROWS / r_pad;

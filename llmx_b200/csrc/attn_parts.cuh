@@ -31,3 +31,11 @@ __device__ __forceinline__ void split3_pair(float a, float b, uint32_t& hi, uint
 }
 
 }  // namespace attn
+
+// Host: whether a kernel of `threads` threads a block was given at least `total` registers for 128 threads' worth of them each
+// (setmaxnreg hands the block's own registers around: asked for more than it was launched with, it would wait for good).
+template <typename K>
+static inline bool registers_reach(K kernel, int threads, int total) {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, kernel) == cudaSuccess && threads / 128 * a.numRegs >= total;
+}

@@ -531,6 +531,8 @@ LLMX_EXPORT int llmx_latent_expand(const void* cache, long long pool_tokens, con
         pool_tokens <= 0 || tokens <= 0 || tokens % ROWS || max_tokens <= 0 || max_tokens % ROWS || head0 < 0 || head0 + n_heads > all_heads ||
         (((uintptr_t)cache | (uintptr_t)w_uk | (uintptr_t)w_uv | (uintptr_t)expanded) & 15))
         return LLMX_ERR_UNSUPPORTED;
+    static const bool enough = registers_reach(latent_expand_kernel, EXPAND_THREADS, FEWER_REGISTERS + 2 * MORE_REGISTERS);
+    if (!enough) return LLMX_ERR_UNSUPPORTED;
     CUtensorMap cache_map, uk_map, uv_map, expanded_map;
     if (int e = make_expanded_map(&expanded_map, expanded, (uint64_t)tokens, (uint64_t)n_heads)) return e;
     if (int e = llmx_make_map_bf16_2d(&cache_map, cache, (uint64_t)pool_tokens, (uint64_t)(C + R), 16, 64)) return e;
