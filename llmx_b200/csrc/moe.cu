@@ -19,7 +19,7 @@
 // take), and on the tensor cores (tcgen05.mma, bfloat16 in, 32-bit sums) for bfloat16 with K a multiple of 32.
 // A third form serves steps of a few pairs (decoding), where the products are the experts' weights streamed once.
 // The CUDA-core form checks its tiles' size against what the routing wrote (tiles[1]).
-#include "tc_common.cuh"
+#include "tc_pair.cuh"
 #include <math.h>
 #include <type_traits>
 
@@ -187,195 +187,269 @@ moe_cores_kernel(const T* __restrict__ a, int a_div, const T* __restrict__ w, co
 }
 
 // ---- the product on the tensor cores -------------------------------------------------------------------------------
-// A block: a tile of up to 256 of an expert's pairs x 256 weight rows, as tcgen05.mma with the weights as the A operand
-// (M = 128, twice) and the gathered rows as B (N = the tile's pairs, rounded up to 16).  The two halves of 128 weight rows
-// are, gated, the gate rows and the up rows of the same 128 output columns, so that a thread holds both of an output and
-// writes the gated unit; else 256 output columns.  The halves' sums fill tensor memory (2 x 256 columns).
-//   warp 0       the weights: K in steps of 64 through three to five stages (as many as the tile's pairs leave room for), two
-//                TMA boxes a step
-//   warp 1       the products, issued by one thread
-//   warps 2-9    the pairs' rows of a step, gathered by cp.async in pieces of 16 bytes laid out as the 128-byte swizzle wants
-//                them (a TMA gather of four rows an instruction took three times as long as the products); then the epilogue: a
-//                thread has an output column (of each half) and half of the pairs, so that a warp writes 32 neighbouring
-//                columns of a pair at a time
-// An expert's list is cut into ceil(pairs / 256) equal tiles: its weights are read that often, and no tile is left with a few
-// pairs.  Of the routing's tiles of 128 pairs the expert's first ones stand for these, the others' blocks return.  Tiles are
-// the grid's fast dimension, so tiles of one expert read the same weights at the same time.
-// 2,048 rows x 2 of 16 experts, 2,048 -> 2 x 1,536 and back: 259 -> 99 us and 141 -> 51 us against tiles of 128 pairs on
-// mma.sync; 1,201 rows x 2 of 16, 4,096 -> 2 x 3,072 and back: 718 -> 189 us and 374 -> 87 us, where reading the weights
-// once takes 123 and 62 us: bound by how soon a step's rows and weights arrive and by the last wave's blocks.  (Handing the
-// rows over two steps late with three stages made every product wait for the one before: 134, 73, 253 and 121 us.)
+// The pairs' rows lie sorted by expert (`gather_kernel`, or as the gated product wrote them), so that both operands come by TMA.
+// Pairs of SMs (a cluster of two blocks, tcgen05 `cta_group::2`) walk units: 256 weight rows x up to 256 of an expert's pairs; a
+// block holds 128 of the weight rows and half of the pairs' rows, and its sums (128 x 256) twice in tensor memory, so that a unit is
+// written out beside the next one's products.
+//   warp 0 (both blocks)   TMA: K in steps of 64 through six stages; gated, the block's weight rows are runs of 16 gate rows and the
+//                          16 up rows of the same outputs, so that a warp's 32 sums of a pair are 16 whole outputs; of the pairs' rows
+//                          as many boxes of 32 as the unit's half has
+//   warp 1 (first block)   the products, and a commit that frees a stage in both blocks
+//   warps 2-5 (both)       sums to the output; gated, lanes i and i + 16 swap halves of their pairs, each makes 16 units of both
+// An expert's list is cut into ceil(pairs / 256) equal parts: its weights are read that often, and none is left with a few
+// pairs.  Units of one expert follow one another, its weight tiles fastest: what they share meets in the L2 cache.
 constexpr int TC_LIST_TILE = 128;                                            // pairs a tile of the routing holds for this form
-constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_MAX_STAGES = 5;
-constexpr int TC_W_BYTES = TC_M * TC_K * 2;                                  // one half's weights of a stage
-constexpr int TC_ROOM = 224 * 1024;                                          // shared memory of the stages
-constexpr int TC_ROW_WARPS = 8, TC_THREADS = 64 + TC_ROW_WARPS * 32;
-constexpr size_t TC_SMEM = TC_ROOM + 1024;
+constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_BOX = 32;
+constexpr int TC_W_BYTES = TC_M * TC_K * 2, TC_R_BYTES = TC_ROWS / 2 * TC_K * 2, TC_STAGE = TC_W_BYTES + TC_R_BYTES, TC_STAGES = 6;
+constexpr int TC_EPI_WARPS = 4, TC_THREADS = 64 + TC_EPI_WARPS * 32;
+constexpr int TC_MAX_EXPERTS = 8192;                                         // three numbers of each lie in shared memory, beside fewer stages if need be
+constexpr int tc_smem(int stages, int experts) { return stages * TC_STAGE + 1024 + 256 + 3 * experts * (int)sizeof(int); }
+constexpr int tc_stages(int experts) {
+    int stages = TC_STAGES;
+    while (tc_smem(stages, experts) > 227 * 1024) --stages;
+    return stages;
+}
+static_assert(tc_stages(TC_MAX_EXPERTS) >= 3, "a stage in use and two on their way");
 enum : int { ERR_MOE_PRODUCER = 441, ERR_MOE_MMA = 442, ERR_MOE_EPILOGUE = 443 };
 
-__device__ __forceinline__ void cp_async_16_or_zeros(uint32_t dst, const void* src, bool real) {
-    const int bytes = real ? 16 : 0;                 // fewer source bytes than 16: the rest of the piece is zeros
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+// rows[place] = a[pair / a_div] for the pair at that place of the sorted lists; a block a place.
+__global__ void __launch_bounds__(256)
+gather_kernel(const uint4* __restrict__ a, int a_div, const int* __restrict__ lists, const int* __restrict__ counts, int experts, int pairs,
+              uint4* __restrict__ rows, int per_row) {
+    pdl_trigger();
+    pdl_wait();
+    const int place = blockIdx.x;
+    __shared__ int found;
+    if (threadIdx.x < 32) {                          // the expert whose list holds the place
+        int base = 0, pair = -1;
+        for (int e0 = 0; e0 < experts && pair < 0; e0 += 32) {
+            const int mine = e0 + (int)threadIdx.x < experts ? counts[e0 + threadIdx.x] : 0;
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if ((int)threadIdx.x >= o) upto += below;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, place < base + upto);
+            if (hit) {
+                const int first = __ffs(hit) - 1;
+                const int at = place - base - __shfl_sync(0xffffffffu, upto - mine, first);
+                pair = lists[(size_t)(e0 + first) * pairs + at];
+            }
+            base += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (threadIdx.x == 0) found = pair;
+    }
+    __syncthreads();
+    if (found < 0) return;                           // past the lists: pairs of experts without weights
+    const uint4* src = a + (size_t)(found / a_div) * per_row;
+    for (int i = threadIdx.x; i < per_row; i += 256) rows[(size_t)place * per_row + i] = src[i];
 }
+
+// An expert's units and where its pairs' rows begin; filled by the block, read by its warps.
+struct Units {
+    const int* count;        // [experts]
+    const int* tile;         // [experts]: parts of lists up to and with the expert's
+    int experts, w_tiles, cur, step, e;
+    // Unit `cur`: expert e, pairs at .. at + n - 1 of its list, weight tile w.
+    __device__ bool next(int& at, int& n, int& w) {
+        const int t = cur / w_tiles;
+        while (e < experts && tile[e] <= t) ++e;
+        if (e >= experts) return false;
+        w = cur % w_tiles;
+        const int parts = (count[e] + TC_ROWS - 1) / TC_ROWS;
+        // Equal parts, multiples of 16 of at most 256 pairs: the last one is never empty, (parts - 1) * 256 being below the count.
+        const int size = ((count[e] + parts - 1) / parts + 15) & ~15;
+        at = (t - (tile[e] - parts)) * size;
+        n = min(size, count[e] - at);
+        cur += step;
+        return true;
+    }
+};
 
 template <bool GATED, typename OutT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-moe_tc_kernel(const __nv_bfloat16* __restrict__ a, const __grid_constant__ CUtensorMap w_map, int a_div,
-              const int* __restrict__ lists, const int* __restrict__ counts, const int* __restrict__ tiles, int pairs,
-              OutT* __restrict__ out, int N, int K, Glu glu, int* error_word) {
-    pdl_wait();
-    if ((int)blockIdx.x >= tiles[0] || tiles[1] != TC_LIST_TILE) return;
-    const int e = tiles[2 + 2 * blockIdx.x], count = counts[e];
-    const int parts = (count + TC_ROWS - 1) / TC_ROWS, part = tiles[3 + 2 * blockIdx.x] / TC_LIST_TILE;
-    if (part >= parts) return;
-    // Equal parts, multiples of 16 of at most 256 pairs: the last one is never empty, (parts - 1) * 256 being below the count.
-    const int step = ((count + parts - 1) / parts + 15) & ~15, at = part * step;
+moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap r_map, const int* __restrict__ lists,
+              const int* __restrict__ counts, int experts, int pairs, OutT* __restrict__ out, int out_sorted, int N, int K, Glu glu,
+              int stages, int* error_word) {
     extern __shared__ uint8_t tc_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES], done;
-    __shared__ uint32_t tmem_slot;
-    __shared__ int abort_word;
-    __shared__ int src_pair[TC_ROWS];
-    volatile int* abort_flag = &abort_word;
+    uint64_t* full = (uint64_t*)(smem + stages * TC_STAGE);          // used in the first block
+    uint64_t* empty = full + stages;                                // one in each block
+    uint64_t* acc_full = empty + stages;                            // [2], one in each block
+    uint64_t* acc_empty = acc_full + 2;                             // [2], used in the first block
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    int* count = (int*)(smem + stages * TC_STAGE + 256);
+    int* row = count + experts;                                     // rows before the expert's
+    int* tile = row + experts;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_here = min(step, count - at);
-    const int n16 = (n_here + 15) & ~15;
-    const int stage_bytes = 2 * TC_W_BYTES + n16 * TC_K * 2, stages = min(TC_MAX_STAGES, TC_ROOM / stage_bytes);
-    const int* list = lists + (size_t)e * pairs + at;
+    const uint32_t rank = cluster_rank();
+    const bool leader = rank == 0;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < TC_MAX_STAGES; ++i) {
-            tc::mbar_init(&full[i], 1 + TC_ROW_WARPS);
+        for (int i = 0; i < stages; ++i) {
+            tc::mbar_init(&full[i], 1);
             tc::mbar_init(&empty[i], 1);
         }
-        tc::mbar_init(&done, 1);
-        abort_word = 0;
+        for (int i = 0; i < 2; ++i) {
+            tc::mbar_init(&acc_full[i], 1);
+            tc::mbar_init(&acc_empty[i], 2 * TC_EPI_WARPS);
+        }
+        *abort_flag = 0;
         tc::fence_barrier_init();
         tc::tma_prefetch_desc(&w_map);
+        tc::tma_prefetch_desc(&r_map);
     }
     if (warp == 1) {
-        tc::tmem_alloc(&tmem_slot, 2 * TC_ROWS);
-        tc::tmem_relinquish();
+        tmem_alloc_pair(tmem_slot, 2 * TC_ROWS);
+        tmem_relinquish_pair();
     }
-    if (threadIdx.x < TC_ROWS) src_pair[threadIdx.x] = (int)threadIdx.x < n_here ? list[threadIdx.x] : -1;
     tc::tc_fence_before();
     __syncthreads();
+    cluster_sync();           // both blocks' barriers exist before either signals the other
     tc::tc_fence_after();
-    pdl_trigger();
-    const uint32_t tmem_base = tmem_slot;
-    const int col0 = blockIdx.y * (GATED ? TC_M : 2 * TC_M);
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();            // only now that this block holds its tensor memory (gemm_tc_pair.cu)
+    pdl_wait();
+    if (warp == 2) {
+        int rows_before = 0, tiles_before = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int e = e0 + lane, c = e < experts ? counts[e] : 0;
+            int rows_upto = c, tiles_upto = (c + TC_ROWS - 1) / TC_ROWS;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int r = __shfl_up_sync(0xffffffffu, rows_upto, o), t = __shfl_up_sync(0xffffffffu, tiles_upto, o);
+                if (lane >= o) rows_upto += r, tiles_upto += t;
+            }
+            if (e < experts) count[e] = c, row[e] = rows_before + rows_upto - c, tile[e] = tiles_before + tiles_upto;
+            rows_before += __shfl_sync(0xffffffffu, rows_upto, 31);
+            tiles_before += __shfl_sync(0xffffffffu, tiles_upto, 31);
+        }
+    }
+    __syncthreads();
+    const int w_cols = GATED ? TC_M : 2 * TC_M;      // output columns of a unit
     const int steps = (K + TC_K - 1) / TC_K;
+    Units units{count, tile, experts, (N + w_cols - 1) / w_cols, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, 0};
+    int at, n, w;
 
     if (warp == 0) {
-        const int w_row = e * (GATED ? 2 * N : N) + col0;
         if (tc::elect_one()) {
-            uint32_t st = 0, phase = 1;
-            for (int s = 0; s < steps; ++s) {
-                if (!tc::mbar_wait(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER)) break;
-                uint8_t* base = smem + st * stage_bytes;
-                tc::mbar_expect_tx(&full[st], 2 * TC_W_BYTES);
-                tc::tma_load_2d(base, &w_map, s * TC_K, w_row, &full[st]);
-                tc::tma_load_2d(base + TC_W_BYTES, &w_map, s * TC_K, w_row + (GATED ? N : TC_M), &full[st]);
-                if ((int)++st == stages) { st = 0; phase ^= 1; }
+            int st = 0;
+            uint32_t phase = 1;
+            bool ok = true;
+            while (ok && units.next(at, n, w)) {
+                const int half = ((n + 15) & ~15) / 2, boxes = (half + TC_BOX - 1) / TC_BOX;
+                const int first = row[units.e] + at + (int)rank * half;
+                const int col = w * w_cols + (int)rank * (GATED ? TC_M / 2 : TC_M);
+                for (int s = 0; s < steps; ++s) {
+                    ok = tc::mbar_wait(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER);
+                    if (!ok) break;
+                    if (leader) tc::mbar_expect_tx(&full[st], 2 * (TC_W_BYTES + boxes * TC_BOX * TC_K * 2));
+                    const uint32_t bar = peer_addr(&full[st], 0);
+                    uint8_t* base = smem + st * TC_STAGE;
+                    if (GATED) {
+#pragma unroll
+                        for (int i = 0; i < TC_M / 32; ++i) tma_load_3d_pair(base + i * 32 * TC_K * 2, &w_map, s * TC_K, col + 16 * i, 2 * units.e, bar);
+                    } else {
+                        tma_load_3d_pair(base, &w_map, s * TC_K, col, units.e, bar);
+                    }
+                    for (int i = 0; i < boxes; ++i)
+                        tma_load_2d_pair(base + TC_W_BYTES + i * TC_BOX * TC_K * 2, &r_map, s * TC_K, first + i * TC_BOX, bar);
+                    if (++st == stages) { st = 0; phase ^= 1; }
+                }
             }
         }
     } else if (warp == 1) {
-        if (tc::elect_one()) {
-            const uint32_t idesc = tc::instr_desc_bf16(TC_M, n16);
+        if (leader && tc::elect_one()) {
+            int st = 0;
+            uint32_t phase = 0, acc = 0, acc_phase = 1;
             bool ok = true;
-            uint32_t st = 0, phase = 0;
-            for (int s = 0; s < steps; ++s) {
-                ok = tc::mbar_wait(&full[st], phase, abort_flag, error_word, ERR_MOE_MMA);
+            while (ok && units.next(at, n, w)) {
+                ok = tc::mbar_wait(&acc_empty[acc], acc_phase, abort_flag, error_word, ERR_MOE_MMA);
                 if (!ok) break;
                 tc::tc_fence_after();
-                const uint32_t w_addr = tc::smem_u32(smem + st * stage_bytes), b_addr = w_addr + 2 * TC_W_BYTES;
+                const uint32_t idesc = tc::instr_desc_bf16(2 * TC_M, (n + 15) & ~15), tmem_d = tmem_base + acc * TC_ROWS;
+                for (int s = 0; s < steps; ++s) {
+                    ok = tc::mbar_wait(&full[st], phase, abort_flag, error_word, ERR_MOE_MMA);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    const uint32_t addr = tc::smem_u32(smem + st * TC_STAGE);
+                    const uint64_t desc_w = tc::smem_desc_k_sw128(addr), desc_r = tc::smem_desc_k_sw128(addr + TC_W_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < TC_K / 16; ++kk)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        tc::mma_bf16_ss(tmem_base + h * TC_ROWS, tc::smem_desc_k_sw128(w_addr + h * TC_W_BYTES + kk * 32),
-                                        tc::smem_desc_k_sw128(b_addr + kk * 32), idesc, (s > 0 || kk > 0) ? 1u : 0u);
-                tc::mma_commit(&empty[st]);
-                if ((int)++st == stages) { st = 0; phase ^= 1; }
+                    for (int k = 0; k < TC_K / 16; ++k)
+                        mma_bf16_pair(tmem_d, desc_w + 2 * k, desc_r + 2 * k, idesc, (s > 0 || k > 0) ? 1u : 0u);
+                    mma_commit_pair(&empty[st], 3);
+                    if (++st == stages) { st = 0; phase ^= 1; }
+                }
+                if (!ok) break;
+                mma_commit_pair(&acc_full[acc], 3);
+                if (++acc == 2) { acc = 0; acc_phase ^= 1; }
             }
-            if (ok) tc::mma_commit(&done);
         }
     } else {
-        // Piece `piece` of every 32nd of the pairs' rows; a place without a pair gets zeros.
-        const int piece = threadIdx.x & 7, first = (threadIdx.x - 64) >> 3;
-        long long at16[TC_ROWS / 32];                    // where the piece of the step 0 lies, in pieces of 16 bytes
-#pragma unroll
-        for (int i = 0; i < TC_ROWS / 32; ++i) {
-            const int p = src_pair[first + 32 * i];
-            at16[i] = p < 0 ? -1 : (long long)(p / a_div) * (K / 8) + piece;
-        }
-        const uint4* src = reinterpret_cast<const uint4*>(a);
-        const uint32_t place = tc::smem_u32(smem) + 2 * TC_W_BYTES + first * 128 + ((piece ^ (first & 7)) << 4);
-        // A stage's rows are handed over `stages` - 2 steps later, when they have landed (a fence makes them visible to the
-        // products): the stage whose turn it is then has been free for a step, so that no product waits for the one before.
-        const int lag = stages - 2;
-        uint32_t st = 0, phase = 1, ready = 0;
-        auto hand_over = [&]() {
-            tc::fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&full[ready]);
-            if ((int)++ready == stages) ready = 0;
-        };
+        const int quarter = warp & 3;                // the tensor-memory lanes that this warp may touch
+        uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
-        for (int s = 0; s < steps; ++s) {
-            ok = tc::mbar_wait_warp(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER);
+        while (ok && units.next(at, n, w)) {
+            ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_MOE_EPILOGUE);
             if (!ok) break;
-            const bool real = 64 * s + 8 * piece < K;
+            tc::tc_fence_after();
+            const uint32_t taddr = tmem_base + acc * TC_ROWS + ((uint32_t)(quarter * 32) << 16);
+            const int* list = lists + (size_t)units.e * pairs + at;
+            const int place = row[units.e] + at;
+            const int c = w * w_cols + (GATED ? (int)rank * (TC_M / 2) + quarter * 16 + (lane & 15) : (int)rank * TC_M + quarter * 32 + lane);
+#pragma unroll 1
+            for (int p0 = 0; p0 < n; p0 += 32) {
+                uint32_t r[32];
+                tc::tmem_ld_32x32(taddr + p0, r);
+                const int to = out_sorted ? place + p0 + lane : p0 + lane < n ? list[p0 + lane] : 0;         // the row that pair p0 + lane goes to
+                tc::tmem_wait_ld();
+                if constexpr (GATED) {
+                    const bool up = lane >= 16;      // this lane's sums are up rows; it makes the second half of the pairs
+                    OutT x[16];
 #pragma unroll
-            for (int i = 0; i < TC_ROWS / 32; ++i)
-                if (32 * i < n16 && first + 32 * i < n16)
-                    cp_async_16_or_zeros(place + st * stage_bytes + i * 32 * 128, src + (real && at16[i] >= 0 ? at16[i] + 8 * s : 0), real && at16[i] >= 0);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if ((int)++st == stages) { st = 0; phase ^= 1; }
-            if (s >= lag) {
-                if (lag == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                else if (lag == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
-                else asm volatile("cp.async.wait_group 3;" ::: "memory");
-                hand_over();
+                    for (int j = 0; j < 16; ++j) {
+                        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(up ? r[j] : r[16 + j]), 16);
+                        const float own = __uint_as_float(up ? r[16 + j] : r[j]);
+                        x[j] = from_float<OutT>(glu_f(glu, up ? got : own, up ? own : got));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const int p = j + (up ? 16 : 0);
+                        const size_t dst = (size_t)__shfl_sync(0xffffffffu, to, p);
+                        if (p0 + p < n && c < N) out[dst * N + c] = x[j];
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const size_t dst = (size_t)__shfl_sync(0xffffffffu, to, j);
+                        if (p0 + j < n && c < N) out[dst * N + c] = from_float<OutT>(__uint_as_float(r[j]));
+                    }
+                }
             }
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_at(peer_addr(&acc_empty[acc], 0));
+            if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (ok)
-            for (int s = max(0, steps - lag); s < steps; ++s) hand_over();
-        ok = ok && tc::mbar_wait_warp(&done, 0, abort_flag, error_word, ERR_MOE_EPILOGUE);
-        tc::tc_fence_after();
-        // A warp may touch the tensor-memory lanes 32 (warp % 4) .. + 31; of two warps with the same lanes each takes every
-        // other run of 16 pairs.
-        const int quarter = warp & 3, c = col0 + 32 * quarter + lane;
-        const uint32_t lanes = tmem_base + ((uint32_t)(32 * quarter) << 16);
-        for (int p0 = 16 * ((warp - 2) >> 2); ok && p0 < n16; p0 += 32) {
-            uint32_t v[2][16];
-            tc::tmem_ld_32x16(lanes + p0, v[0]);
-            tc::tmem_ld_32x16(lanes + TC_ROWS + p0, v[1]);
-            tc::tmem_wait_ld();
-            // All values are made before any is stored: with the conditions around each, their chains ran one after another.
-            OutT x0[16], x1[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float a0 = __uint_as_float(v[0][i]), a1 = __uint_as_float(v[1][i]);
-                x0[i] = from_float<OutT>(GATED ? glu_f(glu, a0, a1) : a0);
-                x1[i] = from_float<OutT>(a1);
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int p = src_pair[p0 + i];
-                if (p < 0) break;                            // the tile's pairs come first
-                OutT* row = out + (size_t)p * N;
-                if (c < N) row[c] = x0[i];
-                if (!GATED && c + TC_M < N) row[c + TC_M] = x1[i];
-            }
-        }
-        tc::tc_fence_before();
     }
+    tc::tc_fence_before();
     __syncthreads();
+    cluster_sync();           // the partner no longer reads this block's shared memory or signals its barriers
     if (warp == 1) {
         tc::tc_fence_after();
-        tc::tmem_dealloc(tmem_base, 2 * TC_ROWS);
+        tmem_dealloc_pair(tmem_base, 2 * TC_ROWS);
     }
+}
+
+// A tensor map of three dimensions of bfloat16 (x contiguous), 128-byte swizzle.
+static int make_map_3d(CUtensorMap* map, const void* base, uint64_t x, uint64_t y, uint64_t z, uint32_t bx, uint32_t by, uint32_t bz) {
+    llmx_encode_tiled_fn enc = llmx_encode_tiled();
+    if (!enc) return 10003;
+    const cuuint64_t dims[3] = {x, y, z}, strides[2] = {x * 2, x * y * 2};
+    const cuuint32_t box[3] = {bx, by, bz}, elem[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 10003;
 }
 
 // ---- steps of a few pairs -------------------------------------------------------------------------------------------
@@ -903,7 +977,7 @@ LLMX_EXPORT int llmx_moe_tile_rows(int tensor_cores) { return tensor_cores ? TC_
 LLMX_EXPORT int llmx_moe_tensor_cores_fit(int dtype, int K) { return dtype == LLMX_BF16 && K > 0 && K % 32 == 0; }
 
 // token_ids int32 [rows]; table int32 [vocab, top]; lists int32 [experts, rows * top]; counts int32 [experts]; tiles int32
-// [2 + 2 * (ceil(rows * top / tile_rows) + experts)].
+// [2 + 2 * (ceil(rows * top / tile_rows) + experts)], or null (the tensor cores' products read the counts alone).
 LLMX_EXPORT int llmx_moe_route(const int* token_ids, const int* table, int top, int rows, int experts, int vocab, int* lists,
                                int* counts, int* tiles, int tile_rows, cudaStream_t stream) {
     if (rows <= 0) return 0;
@@ -911,42 +985,21 @@ LLMX_EXPORT int llmx_moe_route(const int* token_ids, const int* table, int top, 
     launch_kernel(route_kernel, dim3(experts), dim3(ROUTE_THREADS), 0, stream, token_ids, table, top, rows, experts, vocab, lists, counts);
     int status = launch_status();
     if (status) return status;
+    if (tiles == nullptr) return 0;
     launch_kernel(tiles_kernel, dim3(1), dim3(32), 0, stream, (const int*)counts, experts, tiles, tile_rows);
     return launch_status();
 }
 
 // a [rows of `a_div` pairs each, K] and w [experts, (gated ? 2 : 1) * N, K] of `dtype`; out [pairs, N] of `out_dtype`
-// (gated: silu(gate) * up, or the clamped unit of `limit` and `alpha` if `clamped`; else the plain product, float32).  `tensor_cores`: the form to run; the routing must have cut
-// the lists into tiles of `llmx_moe_tile_rows(tensor_cores)` pairs.
+// (gated: silu(gate) * up, or the clamped unit of `limit` and `alpha` if `clamped`; else the plain product, float32).  The routing must have
+// cut the lists into tiles of `llmx_moe_tile_rows(0)` pairs.
 LLMX_EXPORT int llmx_moe_product(const void* a, int a_div, const void* w, int dtype, const int* lists, const int* counts,
                                  const int* tiles, int pairs, int experts, void* out, int out_dtype, int N, int K,
-                                 int gated, int clamped, float limit, float alpha, int tensor_cores, int* error_word,
-                                 cudaStream_t stream) {
+                                 int gated, int clamped, float limit, float alpha, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (N <= 0 || K <= 0 || a_div <= 0) return LLMX_ERR_BAD_ARGUMENT;
     if (!gated && out_dtype != LLMX_F32) return LLMX_ERR_UNSUPPORTED;
     const Glu glu = {clamped, limit, alpha};
-    if (tensor_cores) {
-        if (!llmx_moe_tensor_cores_fit(dtype, K) || ((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return LLMX_ERR_UNSUPPORTED;
-        const int out_cols = gated ? TC_M : 2 * TC_M;
-        const __nv_bfloat16* ab = (const __nv_bfloat16*)a;
-        const long long w_rows = (long long)experts * (gated ? 2 : 1) * N;
-        dim3 grid(max_tiles(pairs, experts, TC_LIST_TILE), (N + out_cols - 1) / out_cols);
-        if (grid.y > 65535 || w_rows >= (1ll << 31)) return LLMX_ERR_UNSUPPORTED;
-        CUtensorMap w_map;
-        if (int bad = llmx_make_map_bf16_2d(&w_map, w, (uint64_t)w_rows, (uint64_t)K, TC_M, TC_K)) return bad;
-#define LLMX_MOE_TC(G, O)                                                                                              \
-    do {                                                                                                                \
-        cudaFuncSetAttribute(moe_tc_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);          \
-        launch_kernel(moe_tc_kernel<G, O>, dim3(grid), dim3(TC_THREADS), TC_SMEM, stream, ab, w_map, a_div, lists,      \
-                      counts, tiles, pairs, (O*)out, N, K, glu, error_word);                                              \
-    } while (0)
-        if (gated && out_dtype == LLMX_BF16) LLMX_MOE_TC(true, __nv_bfloat16);
-        else if (gated) LLMX_MOE_TC(true, float);
-        else LLMX_MOE_TC(false, float);
-#undef LLMX_MOE_TC
-        return launch_status();
-    }
     dim3 grid(max_tiles(pairs, experts, TILE_ROWS), (N + CC_COLS - 1) / CC_COLS);
     if (grid.y > 65535) return LLMX_ERR_UNSUPPORTED;
 #define LLMX_MOE(T, G, O) \
@@ -958,6 +1011,64 @@ LLMX_EXPORT int llmx_moe_product(const void* a, int a_div, const void* w, int dt
     else if (dtype == LLMX_F32 && !gated) LLMX_MOE(float, false, float);
     else return LLMX_ERR_UNSUPPORTED;
 #undef LLMX_MOE
+    return launch_status();
+}
+
+// rows [pairs, K] = the lists' rows of a [rows of `a_div` pairs each, K], bfloat16, one expert's after the other's.
+LLMX_EXPORT int llmx_moe_gather(const void* a, int a_div, const int* lists, const int* counts, int experts, int pairs, void* rows, int K,
+                                cudaStream_t stream) {
+    if (pairs <= 0) return 0;
+    if (K <= 0 || a_div <= 0 || experts <= 0) return LLMX_ERR_BAD_ARGUMENT;
+    if (K % 8 || (((uintptr_t)a | (uintptr_t)rows) & 15)) return LLMX_ERR_UNSUPPORTED;
+    launch_kernel(gather_kernel, dim3(pairs), dim3(256), 0, stream, (const uint4*)a, a_div, lists, counts, experts, pairs, (uint4*)rows, K / 8);
+    return launch_status();
+}
+
+// The same products on the tensor cores: rows [pairs, K] and w bfloat16, the rows sorted as the lists are; out [pairs, N] by pair or,
+// `out_sorted`, in the rows' order.
+LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* lists, const int* counts, int pairs, int experts, void* out,
+                                    int out_dtype, int out_sorted, int N, int K, int gated, int clamped, float limit, float alpha,
+                                    int* error_word, cudaStream_t stream) {
+    if (pairs <= 0) return 0;
+    if (N <= 0 || K <= 0 || experts <= 0) return LLMX_ERR_BAD_ARGUMENT;
+    if (!gated && out_dtype != LLMX_F32) return LLMX_ERR_UNSUPPORTED;
+    if (!llmx_moe_tensor_cores_fit(LLMX_BF16, K) || experts > TC_MAX_EXPERTS || (((uintptr_t)rows | (uintptr_t)w) & 15)) return LLMX_ERR_UNSUPPORTED;
+    const Glu glu = {clamped, limit, alpha};
+    const int w_cols = gated ? TC_M : 2 * TC_M;
+    const long long most = ((long long)pairs / TC_ROWS + experts) * ((N + w_cols - 1) / w_cols);
+    if (most >= (1ll << 31)) return LLMX_ERR_UNSUPPORTED;
+    CUtensorMap w_map, r_map;
+    const int per = gated ? 2 : 1;                   // gate rows and up rows are planes of their own
+    if (int bad = make_map_3d(&w_map, w, K, N, (uint64_t)experts * per, TC_K, gated ? 16 : TC_M, per)) return bad;
+    if (int bad = llmx_make_map_bf16_2d(&r_map, rows, (uint64_t)pairs, (uint64_t)K, TC_BOX, TC_K)) return bad;
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 2) sms = 148;
+    const int stages = tc_stages(experts);
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)(2 * (most < sms / 2 ? most : sms / 2)));
+    lc.blockDim = dim3(TC_THREADS);
+    lc.dynamicSmemBytes = tc_smem(stages, experts);
+    lc.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = llmx_pdl_enabled() ? 2 : 1;
+#define LLMX_MOE_TC(G, O)                                                                                              \
+    do {                                                                                                                \
+        const cudaError_t e = cudaFuncSetAttribute(moe_tc_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lc.dynamicSmemBytes); \
+        if (e != cudaSuccess) return (int)e;                                                                            \
+        cudaLaunchKernelEx(&lc, moe_tc_kernel<G, O>, w_map, r_map, lists, counts, experts, pairs, (O*)out, out_sorted, N, K, glu, stages, error_word); \
+    } while (0)
+    if (gated && out_dtype == LLMX_BF16) LLMX_MOE_TC(true, __nv_bfloat16);
+    else if (gated) LLMX_MOE_TC(true, float);
+    else LLMX_MOE_TC(false, float);
+#undef LLMX_MOE_TC
     return launch_status();
 }
 

@@ -129,7 +129,9 @@ _SIGNATURES = {
     ("attention_rows_tc", "llmx_attention_rows_tc"): [_p, _p, ctypes.c_longlong, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p],
     ("moe", "llmx_moe_route"): [_p, _p, _i, _i, _i, _i, _p, _p, _p, _i, _p],
     ("moe", "llmx_moe_product_few"): [_p, _i, _p, _p, _p, _i, _i, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _p, _p],
-    ("moe", "llmx_moe_product"): [_p, _i, _p, _i, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _i, _p, _p],
+    ("moe", "llmx_moe_product"): [_p, _i, _p, _i, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _p],
+    ("moe", "llmx_moe_gather"): [_p, _i, _p, _p, _i, _i, _p, _i, _p],
+    ("moe", "llmx_moe_product_tc"): [_p, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _i, _f, _f, _p, _p],
     ("moe", "llmx_moe_combine"): [_p, _p, _i, _i, _i, _f, _p],
     ("moe", "llmx_moe_router"): [_p, _i, _p, _p, _i, _i, _i, _i, _i, _i, _p, _i, _i, _f, _p, _p, _p, _p],
     ("moe", "llmx_moe_combine_weighted"): [_p, _p, _p, _p, _i, _p, _i, _p, _p, _i, _i, _i, _f, _p],
@@ -956,6 +958,7 @@ def moe_tiles_len(pairs: int, experts: int) -> int:
 
 
 _moe_tile_rows = {}
+MOE_TC_EXPERTS = 8192            # experts that the tensor cores' products take (csrc/moe.cu)
 
 
 def moe_tensor_cores_fit(dtype: torch.dtype, *inner_widths: int) -> bool:
@@ -997,13 +1000,13 @@ def moe_route(token_ids: torch.Tensor, table: torch.Tensor, experts: int, lists:
               tiles: torch.Tensor, tensor_cores: bool = False) -> None:
     """Sort the step's (row, k) pairs by the expert the table gives them: lists int32 [experts, rows * top] (pairs in
     order), counts int32 [experts], tiles int32 [moe_tiles_len] (their number, their size, then (expert, first place) of
-    every tile).  `tensor_cores`: the form of `moe_product` that will run (it sets the tiles' size: 128 pairs, else 32)."""
+    every tile; None: not wanted, as `moe_product_sorted` reads none).  `tensor_cores`: the form of `moe_product` that will run (it sets the tiles' size: 128 pairs, else 32)."""
     _cuda(token_ids, table, lists, counts, tiles)
     vocab, top = table.shape
     rows = vocab if token_ids is None else token_ids.numel()      # no ids: the table has a row for each row of the step
     for t in (token_ids, table, lists, counts, tiles):
         _need(t is None or t.dtype == torch.int32, "moe_route: int32 tensors")
-    _need(lists.numel() >= experts * rows * top and counts.numel() >= experts and tiles.numel() >= moe_tiles_len(rows * top, experts),
+    _need(lists.numel() >= experts * rows * top and counts.numel() >= experts and (tiles is None or tiles.numel() >= moe_tiles_len(rows * top, experts)),
           "moe_route: outputs too small")
     tile_rows = _moe_tile_rows.get(bool(tensor_cores))
     if tile_rows is None:
@@ -1014,22 +1017,50 @@ def moe_route(token_ids: torch.Tensor, table: torch.Tensor, experts: int, lists:
                                         _ptr(tiles), tile_rows, _stream()), "moe_route", 2)
 
 
+def moe_gather(a: torch.Tensor, a_div: int, lists: torch.Tensor, counts: torch.Tensor, pairs: int) -> torch.Tensor:
+    """The lists' rows of `a`, [pairs, K] bfloat16, one expert's after the other's: what the tensor cores' products read.  Rows past
+    the lists (pairs of experts without weights) are not written."""
+    _cuda(a, lists, counts)
+    _need(a.dtype == torch.bfloat16 and a.dim() == 2 and a.shape[0] * a_div >= pairs and lists.dtype == torch.int32 and counts.dtype == torch.int32
+          and lists.numel() >= counts.numel() * pairs, "moe_gather: bfloat16 rows, int32 lists")
+    rows = torch.empty((pairs, a.shape[1]), dtype=torch.bfloat16, device=a.device)
+    _check(_fn("moe", "llmx_moe_gather")(_ptr(a), int(a_div), _ptr(lists), _ptr(counts), counts.numel(), pairs, _ptr(rows), a.shape[1], _stream()), "moe_gather")
+    return rows
+
+
+def moe_product_sorted(rows: torch.Tensor, w: torch.Tensor, lists: torch.Tensor, counts: torch.Tensor, pairs: int, out: torch.Tensor, gated: bool,
+                       out_sorted: bool = False, clamp=None) -> torch.Tensor:
+    """`moe_product` on the tensor cores over rows in the lists' order (`moe_gather`).  `out_sorted`: out's rows are in that order too
+    (what the next product reads), else by pair."""
+    from .runtime import error_word
+    clamped, limit, alpha = _clamp(clamp)
+    _cuda(rows, w, lists, counts, out)
+    experts, wn, K = w.shape
+    N = wn // 2 if gated else wn
+    _need(rows.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and tuple(rows.shape) == (pairs, K), "moe_product: rows do not fit the weights")
+    _need(tuple(out.shape) == (pairs, N), "moe_product: output shape does not fit")
+    _need(lists.dtype == torch.int32 and counts.dtype == torch.int32 and counts.numel() >= experts and lists.numel() >= experts * pairs, "moe_product: int32 lists")
+    _check(_fn("moe", "llmx_moe_product_tc")(_ptr(rows), _ptr(w), _ptr(lists), _ptr(counts), pairs, experts, _ptr(out), _code(out), 1 if out_sorted else 0,
+                                             N, K, 1 if gated else 0, clamped, limit, alpha, _ptr(error_word(rows.device)), _stream()), "moe_product")
+    return out
+
+
 def moe_product(a: torch.Tensor, a_div: int, w: torch.Tensor, lists: torch.Tensor, counts: torch.Tensor, tiles: torch.Tensor,
                 pairs: int, out: torch.Tensor, gated: bool, tensor_cores: bool = False, clamp=None) -> torch.Tensor:
     """out[pair] = a[pair // a_div] W_e^T for the expert e whose list holds the pair; w [experts, N (gated: 2 N, gate rows
     then up rows), K] of a's type.  gated: out = silu(gate) * up in out's type, or with `clamp` = (limit, alpha)
     min(gate, limit) sigmoid(alpha min(gate, limit)) (clamp(up, -limit, limit) + 1); else float32.  `tensor_cores` as the
     routing was told.  Pairs in no list (an expert without weights) keep what `out` held."""
-    from .runtime import error_word
     clamped, limit, alpha = _clamp(clamp)
     _cuda(a, w, lists, counts, tiles, out)
     experts, wn, K = w.shape
     N = wn // 2 if gated else wn
     _need(a.dtype == w.dtype and a.dim() == 2 and a.shape[1] == K and a.shape[0] * a_div >= pairs, "moe_product: rows do not fit the weights")
     _need(tuple(out.shape) == (pairs, N), "moe_product: output shape does not fit")
+    if tensor_cores:
+        return moe_product_sorted(moe_gather(a, a_div, lists, counts, pairs), w, lists, counts, pairs, out, gated, clamp=clamp)
     _check(_fn("moe", "llmx_moe_product")(_ptr(a), int(a_div), _ptr(w), _code(w), _ptr(lists), _ptr(counts), _ptr(tiles), pairs,
-                                          experts, _ptr(out), _code(out), N, K, 1 if gated else 0, clamped, limit, alpha,
-                                          1 if tensor_cores else 0, _ptr(error_word(a.device)), _stream()), "moe_product")
+                                          experts, _ptr(out), _code(out), N, K, 1 if gated else 0, clamped, limit, alpha, _stream()), "moe_product")
     return out
 
 

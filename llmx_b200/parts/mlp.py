@@ -177,7 +177,8 @@ class TableRoutedExperts(Part):
         self.w_gate_up = torch.stack([torch.cat([tensors[f"e{e}.{g}"], tensors[f"e{e}.{u}"]], dim=0) for e in range(self.experts)]).to(act).contiguous()
         self.w_down = torch.stack([tensors[f"e{e}.{d}"] for e in range(self.experts)]).to(act).contiguous()
         from .. import ops
-        self.tensor_cores = not precision.invariant and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate)
+        self.tensor_cores = (not precision.invariant and self.experts <= ops.MOE_TC_EXPERTS
+                             and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate))
 
     def forward(self, h: torch.Tensor, step: StepBatch, residual: torch.Tensor) -> None:
         from .. import ops
@@ -196,11 +197,16 @@ class TableRoutedExperts(Part):
         else:
             lists = torch.empty((self.experts, pairs), dtype=torch.int32, device=dev)
             counts = torch.empty((self.experts,), dtype=torch.int32, device=dev)
-            tiles = torch.empty((ops.moe_tiles_len(pairs, self.experts),), dtype=torch.int32, device=dev)
-            tc = self.tensor_cores
-            ops.moe_route(step.token_ids, self.table, self.experts, lists, counts, tiles, tensor_cores=tc)
-            ops.moe_product(h, self.top, self.w_gate_up, lists, counts, tiles, pairs, act, gated=True, tensor_cores=tc)
-            ops.moe_product(act, 1, self.w_down, lists, counts, tiles, pairs, y, gated=False, tensor_cores=tc)
+            if self.tensor_cores:               # rows and what the gated unit gives lie in the lists' order between the products
+                ops.moe_route(step.token_ids, self.table, self.experts, lists, counts, None, tensor_cores=True)
+                sorted_rows = ops.moe_gather(h, self.top, lists, counts, pairs)
+                ops.moe_product_sorted(sorted_rows, self.w_gate_up, lists, counts, pairs, act, gated=True, out_sorted=True)
+                ops.moe_product_sorted(act, self.w_down, lists, counts, pairs, y, gated=False)
+            else:
+                tiles = torch.empty((ops.moe_tiles_len(pairs, self.experts),), dtype=torch.int32, device=dev)
+                ops.moe_route(step.token_ids, self.table, self.experts, lists, counts, tiles)
+                ops.moe_product(h, self.top, self.w_gate_up, lists, counts, tiles, pairs, act, gated=True)
+                ops.moe_product(act, 1, self.w_down, lists, counts, tiles, pairs, y, gated=False)
         ops.moe_combine_(residual, y, self.top, 1.0 / self.top)
         if self.shared is not None:
             self.shared.forward(h, step, residual)
@@ -291,7 +297,8 @@ class RoutedExperts(Part):
         self.w_gate_up = torch.stack([torch.cat([tensors[f"e{e}.{g}"], tensors[f"e{e}.{u}"]], dim=0) for e in range(self.experts)]).to(act).contiguous()
         self.w_down = torch.stack([tensors[f"e{e}.{d}"] for e in range(self.experts)]).to(act).contiguous()
         from .. import ops
-        self.tensor_cores = not precision.invariant and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate)
+        self.tensor_cores = (not precision.invariant and self.experts <= ops.MOE_TC_EXPERTS
+                             and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate))
 
     def forward(self, h: torch.Tensor, step: StepBatch, residual: torch.Tensor) -> None:
         from .. import ops
@@ -315,11 +322,16 @@ class RoutedExperts(Part):
         else:
             lists = torch.empty((self.experts, pairs), dtype=torch.int32, device=dev)
             counts = torch.empty((self.experts,), dtype=torch.int32, device=dev)
-            tiles = torch.empty((ops.moe_tiles_len(pairs, self.experts),), dtype=torch.int32, device=dev)
-            tc = self.tensor_cores
-            ops.moe_route(None, choice, self.experts, lists, counts, tiles, tensor_cores=tc)
-            ops.moe_product(h, self.top, self.w_gate_up, lists, counts, tiles, pairs, act, gated=True, tensor_cores=tc, clamp=self.clamp)
-            ops.moe_product(act, 1, self.w_down, lists, counts, tiles, pairs, y, gated=False, tensor_cores=tc)
+            if self.tensor_cores:               # rows and what the gated unit gives lie in the lists' order between the products
+                ops.moe_route(None, choice, self.experts, lists, counts, None, tensor_cores=True)
+                sorted_rows = ops.moe_gather(h, self.top, lists, counts, pairs)
+                ops.moe_product_sorted(sorted_rows, self.w_gate_up, lists, counts, pairs, act, gated=True, out_sorted=True, clamp=self.clamp)
+                ops.moe_product_sorted(act, self.w_down, lists, counts, pairs, y, gated=False)
+            else:
+                tiles = torch.empty((ops.moe_tiles_len(pairs, self.experts),), dtype=torch.int32, device=dev)
+                ops.moe_route(None, choice, self.experts, lists, counts, tiles)
+                ops.moe_product(h, self.top, self.w_gate_up, lists, counts, tiles, pairs, act, gated=True, clamp=self.clamp)
+                ops.moe_product(act, 1, self.w_down, lists, counts, tiles, pairs, y, gated=False)
         shared_out = None
         if self.shared_gate:
             scratch, self.scratch = self.scratch, None

@@ -1395,3 +1395,31 @@ def test_latent_prompts_round_as_the_exact_ones(mean, spread, history):
     nearest = want.float().bfloat16().view(rows, -1)
     made, before = ((o != nearest).double().mean().item() for o in (out, general))
     assert made <= 1.05 * before, (made, before)
+
+
+@pytest.mark.parametrize("experts,top,rows,K,N", [(16, 2, 300, 576, 160), (1500, 1, 900, 32, 96), (6000, 2, 200, 96, 32), (3, 3, 700, 160, 416)])
+def test_expert_products_in_sorted_rows(experts, top, rows, K, N):
+    """The gated product leaves its rows in the lists' order and the plain one reads them there: every pair's result against 64 bits of
+    the same bfloat16 steps, experts so many that fewer stages fit beside their numbers, widths that end within a unit."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(experts + N)
+    table = torch.rand(rows, experts, generator=g).argsort(1)[:, :top].to(torch.int32).contiguous().to(DEV)
+    h = _bf16(torch.randn(rows, K, generator=g)).to(DEV)
+    w_gu = _bf16(torch.randn(experts, 2 * N, K, generator=g) * K ** -0.5).to(DEV)
+    w = _bf16(torch.randn(experts, K, N, generator=g) * N ** -0.5).to(DEV)
+    pairs = rows * top
+    lists = torch.empty((experts, pairs), dtype=torch.int32, device=DEV)
+    counts = torch.empty((experts,), dtype=torch.int32, device=DEV)
+    ops.moe_route(None, table, experts, lists, counts, None, tensor_cores=True)
+    act = torch.full((pairs, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.moe_product_sorted(ops.moe_gather(h, top, lists, counts, pairs), w_gu, lists, counts, pairs, act, gated=True, out_sorted=True)
+    y = torch.full((pairs, K), 7.0, device=DEV)
+    ops.moe_product_sorted(act, w, lists, counts, pairs, y, gated=False)
+    at = torch.cat([lists[e, :n] for e, n in enumerate(counts.tolist())]).long()
+    expert = table.reshape(-1)[at].long()
+    both = torch.einsum("pk,pnk->pn", h.double()[at // top], w_gu.double()[expert])
+    want = both[:, :N] * torch.sigmoid(both[:, :N]) * both[:, N:]
+    slack = K ** 0.5 * 2.0 ** -22
+    assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 8 * slack).all()
+    want = torch.einsum("pn,pkn->pk", act.double(), w.double()[expert])
+    assert (y[at].double() - want).abs().max() <= 4 * N ** 0.5 * 2.0 ** -22 * max(1.0, float(act.abs().max()))
