@@ -87,6 +87,77 @@ qk_write_kernel(const float* __restrict__ proj, int stride, const float* __restr
     }
 }
 
+// The same for heads of 32 PER values of which a multiple of 64 is rotated: a rotated value's partner is then in the same lane, and a
+// lane's angles are the same for every head of a row: they are made once a row (sines and cosines were most of the time).
+template <typename QT, typename KVT, int PER>
+__global__ void __launch_bounds__(128)
+qk_write_lane_kernel(const float* __restrict__ proj, int stride, const float* __restrict__ q_weight,
+                     const float* __restrict__ k_weight, float eps, const float* __restrict__ freq, int rot_half,
+                     const int* __restrict__ positions, const int* __restrict__ slots, QT* __restrict__ q_out,
+                     KVT* __restrict__ cache, int heads, int kv_heads, int V, int page_size) {
+    constexpr int D = 32 * PER;
+    pdl_trigger();
+    const int row = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int rots = rot_half / 32;                  // values i < rots of a lane turn with values i + rots
+    float qw[PER], kw[PER], f[PER / 2];              // written by no kernel
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        qw[i] = q_weight ? q_weight[lane + 32 * i] : 1.0f;
+        kw[i] = k_weight ? k_weight[lane + 32 * i] : 1.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < PER / 2; ++i) f[i] = i < rots ? freq[lane + 32 * i] : 0.0f;
+    pdl_wait();
+    const float pos = (float)positions[row];
+    const int slot = slots[row];
+    const float* src = proj + (size_t)row * stride;
+    const int v_off = (heads + kv_heads) * D;
+    float s[PER / 2], c[PER / 2];
+#pragma unroll
+    for (int i = 0; i < PER / 2; ++i)
+        if (i < rots) sincosf(pos * f[i], &s[i], &c[i]);
+    for (int item = (int)blockIdx.y * warps + warp; item < heads + kv_heads; item += warps * gridDim.y) {
+        const bool is_q = item < heads;
+        const float* x = src + (size_t)item * D;
+        float val[PER], ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) val[i] = x[lane + 32 * i];
+        if (!is_q && slot < 0) continue;             // a row whose cache write is skipped
+        if (q_weight != nullptr) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) ss = fmaf(val[i], val[i], ss);
+            const float rr = 1.0f / sqrtf(warp_sum(ss) / (float)D + eps);
+#pragma unroll
+            for (int i = 0; i < PER; ++i) val[i] = val[i] * rr * (is_q ? qw[i] : kw[i]);
+        }
+        float turned[PER];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) turned[i] = val[i];
+#pragma unroll
+        for (int n = 1; n <= PER / 2; ++n) {         // every distance the partner may have
+            if (n != rots) continue;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                turned[i] = val[i] * c[i] - val[i + n] * s[i];
+                turned[i + n] = val[i + n] * c[i] + val[i] * s[i];
+            }
+        }
+        if (is_q) {
+            QT* dst = q_out + ((size_t)row * heads + item) * D;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) dst[lane + 32 * i] = from_float<QT>(turned[i]);
+        } else {
+            const int g = item - heads;
+            KVT* dst = cache + (((size_t)(slot / page_size) * kv_heads + g) * page_size + slot % page_size) * (size_t)(D + V);
+            const float* vsrc = src + v_off + (size_t)g * V;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) dst[lane + 32 * i] = from_float<KVT>(turned[i]);
+            for (int d = lane; d < V; d += 32) dst[D + d] = from_float<KVT>(vsrc[d]);
+        }
+    }
+}
+
 // The general finishing of the rows of a q/k/v product, for designs that put more between the product and the attention:
 //   u = proj + bias                                   (bias may be null)
 //   y[t] = sum_j taps_w[c, j] u[t - taps + 1 + j]      a short causal filter per channel, zeros before the request's first
@@ -1049,15 +1120,30 @@ LLMX_EXPORT int llmx_qk_norm_rope_write(const float* proj, int stride, const flo
     if (D <= 0 || V <= 0 || D > 32 * MAX_PER_LANE || 2 * rot_half > D || rot_half < 0 || (rot_half > 0 && freq == nullptr) ||
         (q_weight == nullptr) != (k_weight == nullptr))
         return LLMX_ERR_UNSUPPORTED;
+    const dim3 grid(rows, rows <= 64 ? (heads + kv_heads + 3) / 4 : 1);
+#define LLMX_QKL(QT, KVT, P)                                                                                            \
+    if (D == 32 * P) {                                                                                                   \
+        launch_kernel(qk_write_lane_kernel<QT, KVT, P>, dim3(grid), dim3(128), 0, stream, proj, stride, q_weight, k_weight, eps, freq, \
+                      rot_half, positions, slots, (QT*)q_out, (KVT*)cache, heads, kv_heads, V, page_size);               \
+        return launch_status();                                                                                          \
+    }
 #define LLMX_QKW(QT, KVT)                                                                                              \
-    launch_kernel(qk_write_kernel<QT, KVT>, dim3(rows, rows <= 64 ? (heads + kv_heads + 3) / 4 : 1), dim3(128), 0, stream, proj, stride, q_weight, k_weight, eps, \
-                  freq, rot_half, positions, slots, (QT*)q_out, (KVT*)cache, heads, kv_heads, D, V, page_size)
+    do {                                                                                                                 \
+        if (rot_half % 32 == 0) {                                                                                        \
+            LLMX_QKL(QT, KVT, 2)                                                                                         \
+            LLMX_QKL(QT, KVT, 4)                                                                                         \
+            LLMX_QKL(QT, KVT, 8)                                                                                         \
+        }                                                                                                                \
+        launch_kernel(qk_write_kernel<QT, KVT>, dim3(grid), dim3(128), 0, stream, proj, stride, q_weight, k_weight, eps, \
+                      freq, rot_half, positions, slots, (QT*)q_out, (KVT*)cache, heads, kv_heads, D, V, page_size);      \
+    } while (0)
     if (q_dtype == LLMX_BF16 && cache_dtype == LLMX_BF16) LLMX_QKW(__nv_bfloat16, __nv_bfloat16);
     else if (q_dtype == LLMX_BF16 && cache_dtype == LLMX_F32) LLMX_QKW(__nv_bfloat16, float);
     else if (q_dtype == LLMX_F32 && cache_dtype == LLMX_BF16) LLMX_QKW(float, __nv_bfloat16);
     else if (q_dtype == LLMX_F32 && cache_dtype == LLMX_F32) LLMX_QKW(float, float);
     else return LLMX_ERR_UNSUPPORTED;
 #undef LLMX_QKW
+#undef LLMX_QKL
     return launch_status();
 }
 

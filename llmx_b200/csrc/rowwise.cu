@@ -26,9 +26,43 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
     for (int i = threadIdx.x; i < width; i += blockDim.x) dst[i] = to_float(src[i]);
 }
 
+// Eight values a thread (16 bytes of a bfloat16 table, 32 of a 32-bit one), blocks of 1,024 values of a row.
+template <typename T>
+__global__ void __launch_bounds__(128)
+embed_eight_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ x, int width, int table_rows) {
+    pdl_trigger();
+    pdl_wait();
+    const int r = blockIdx.x, i = (blockIdx.y * 128 + threadIdx.x) * 8;
+    if (i >= width) return;
+    const int id = ids[r];
+    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+    if (id >= 0 && id < table_rows) {
+        const T* src = table + (size_t)id * width + i;
+        if constexpr (sizeof(T) == 2) {
+            const uint4 v = *reinterpret_cast<const uint4*>(src);
+            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+            const float2 a = __bfloat1622float2(p[0]), b = __bfloat1622float2(p[1]), c = __bfloat1622float2(p[2]), d = __bfloat1622float2(p[3]);
+            lo = make_float4(a.x, a.y, b.x, b.y), hi = make_float4(c.x, c.y, d.x, d.y);
+        } else {
+            lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
+        }
+    }
+    float* dst = x + (size_t)r * width + i;
+    *reinterpret_cast<float4*>(dst) = lo;
+    *reinterpret_cast<float4*>(dst + 4) = hi;
+}
+
 LLMX_EXPORT int llmx_embed(const void* table, int table_dtype, const int* ids, float* x, int rows, int width,
                            int table_rows, cudaStream_t stream) {
     if (rows <= 0) return 0;
+    if (width % 8 == 0 && !(((uintptr_t)table | (uintptr_t)x) & 15) && width <= 1024 * 65535) {
+        const dim3 grid(rows, (width + 1023) / 1024);
+        if (table_dtype == LLMX_BF16)
+            launch_kernel(embed_eight_kernel<__nv_bfloat16>, dim3(grid), dim3(128), 0, stream, (const __nv_bfloat16*)table, ids, x, width, table_rows);
+        else
+            launch_kernel(embed_eight_kernel<float>, dim3(grid), dim3(128), 0, stream, (const float*)table, ids, x, width, table_rows);
+        return launch_status();
+    }
     if (table_dtype == LLMX_BF16)
         launch_kernel(embed_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, (const __nv_bfloat16*)table, ids, x, width, table_rows);
     else
