@@ -27,6 +27,7 @@
 // reference's walk.  Without top-k (or a larger one) nothing is gathered: thresholds by radix selection over the
 // vocabulary, summing weights.
 #include "common.cuh"
+#include <string.h>
 #include <math.h>
 
 namespace {
@@ -43,6 +44,12 @@ static_assert(LISTED * 8 <= STRIPES_BYTES, "the list lies in the stripes' memory
 struct RowParams {
     float temperature, top_p, min_p, r;
     int top_k, masked;
+};
+
+// The rows' settings as an argument of the launch: no buffer for them and no copy in front of the draw.
+constexpr int ARG_ROWS = 128;
+struct RowBatch {
+    RowParams rows[ARG_ROWS];
 };
 
 __device__ __forceinline__ uint32_t order_bits(float s) {
@@ -635,14 +642,15 @@ __device__ __forceinline__ Row row_of_block(const float* logits, int vocab, Shar
 }
 
 __global__ void __launch_bounds__(THREADS) sample_kernel(const float* __restrict__ logits, int vocab,
-                                                         const RowParams* __restrict__ params, int* __restrict__ out) {
+                                                         const RowParams* __restrict__ params, const __grid_constant__ RowBatch batch,
+                                                         int* __restrict__ out) {
     pdl_trigger();
     pdl_wait();
     __shared__ Shared sh;
     extern __shared__ double stripes[];       // STRIPES_BYTES
     const Row c = row_of_block(logits, vocab, &sh, stripes);
     const float* row = c.row;
-    const RowParams p = params[blockIdx.y];
+    const RowParams p = params ? params[blockIdx.y] : batch.rows[blockIdx.y];
     const int n = vocab;
     // What the blocks meet in starts empty (only the leader's copy is ever used).
     for (int i = threadIdx.x; i < 256; i += THREADS) { sh.gcount[i] = 0; sh.gweight[i] = 0.0; sh.gmin_id[i] = NO_ID; }
@@ -860,12 +868,13 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(const float* __restrict
 
 // Greedy rows only: the best token of every row.  Used when no row of the batch draws.
 __global__ void __launch_bounds__(THREADS) argmax_kernel(const float* __restrict__ logits, int vocab,
-                                                         const RowParams* __restrict__ params, int* __restrict__ out) {
+                                                         const RowParams* __restrict__ params, const __grid_constant__ RowBatch batch,
+                                                         int* __restrict__ out) {
     pdl_trigger();
     pdl_wait();
     __shared__ Shared sh;
     const Row c = row_of_block(logits, vocab, &sh, nullptr);
-    const int masked = params[blockIdx.y].masked;
+    const int masked = params ? params[blockIdx.y].masked : batch.rows[blockIdx.y].masked;
     const int skip = (masked >= 0 && masked < vocab && vocab > 1) ? masked : -1;
     const int best = best_token(c, skip);
     if (c.rank == 0 && threadIdx.x == 0) out[blockIdx.y] = best;
@@ -909,7 +918,7 @@ int blocks_for(int vocab, int rows) {
 }
 
 template <typename K>
-int launch_rows(K kernel, int dynamic_bytes, int rows, int vocab, const float* logits, const RowParams* params, int* out,
+int launch_rows(K kernel, int dynamic_bytes, int rows, int vocab, const float* logits, const RowParams* params, const RowBatch& batch, int* out,
                 cudaStream_t stream) {
     const int blocks = blocks_for(vocab, rows);
     cudaLaunchConfig_t lc = {};
@@ -926,8 +935,20 @@ int launch_rows(K kernel, int dynamic_bytes, int rows, int vocab, const float* l
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = llmx_pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&lc, kernel, logits, vocab, params, out);
+    cudaLaunchKernelEx(&lc, kernel, logits, vocab, params, batch, out);
     return launch_status();
+}
+
+int draw(const float* logits, int rows, int vocab, const RowParams* params, const RowBatch& batch, int* out, int all_greedy, cudaStream_t stream) {
+    if (vocab <= 0 || rows > 65535) return LLMX_ERR_BAD_ARGUMENT;
+    if (all_greedy) return launch_rows(argmax_kernel, 0, rows, vocab, logits, params, batch, out, stream);
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STRIPES_BYTES) != cudaSuccess)
+            return (int)cudaGetLastError();
+        configured = true;
+    }
+    return launch_rows(sample_kernel, STRIPES_BYTES, rows, vocab, logits, params, batch, out, stream);
 }
 
 }  // namespace
@@ -937,15 +958,18 @@ int launch_rows(K kernel, int dynamic_bytes, int rows, int vocab, const float* l
 LLMX_EXPORT int llmx_sample(const float* logits, int rows, int vocab, const void* params, int* out, int all_greedy,
                             cudaStream_t stream) {
     if (rows <= 0) return 0;
-    if (vocab <= 0 || rows > 65535) return LLMX_ERR_BAD_ARGUMENT;
-    if (all_greedy) return launch_rows(argmax_kernel, 0, rows, vocab, logits, (const RowParams*)params, out, stream);
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STRIPES_BYTES) != cudaSuccess)
-            return (int)cudaGetLastError();
-        configured = true;
-    }
-    return launch_rows(sample_kernel, STRIPES_BYTES, rows, vocab, logits, (const RowParams*)params, out, stream);
+    if (params == nullptr) return LLMX_ERR_BAD_ARGUMENT;
+    return draw(logits, rows, vocab, (const RowParams*)params, RowBatch{}, out, all_greedy, stream);
+}
+
+// The same for up to ARG_ROWS rows, `params` in host memory (read before the call returns).
+LLMX_EXPORT int llmx_sample_rows(const float* logits, int rows, int vocab, const void* params, int* out, int all_greedy,
+                                 cudaStream_t stream) {
+    if (rows <= 0) return 0;
+    if (params == nullptr || rows > ARG_ROWS) return LLMX_ERR_BAD_ARGUMENT;
+    RowBatch batch;
+    memcpy(batch.rows, params, (size_t)rows * sizeof(RowParams));
+    return draw(logits, rows, vocab, nullptr, batch, out, all_greedy, stream);
 }
 
 LLMX_EXPORT int llmx_penalize(float* logits, int vocab, const int* row_of, const int* token, const int* count,

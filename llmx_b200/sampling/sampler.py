@@ -9,6 +9,7 @@ are copied back.
 from __future__ import annotations
 
 import ctypes
+import functools
 import struct
 from typing import Dict, Hashable, List, Optional, Sequence
 
@@ -20,6 +21,7 @@ from .params import SamplingParams
 
 _i, _p = ctypes.c_int, ctypes.c_void_p
 register_signature("sampling", "llmx_sample", [_p, _i, _i, _p, _p, _i, _p])
+register_signature("sampling", "llmx_sample_rows", [_p, _i, _i, ctypes.c_char_p, _p, _i, _p])
 register_signature("sampling", "llmx_penalize", [_p, _i, _p, _p, _p, _p, _p, _p, _i, _p])
 
 _MASK = (1 << 64) - 1
@@ -40,8 +42,8 @@ class XorShift64:
         return x
 
     def unit(self) -> float:
-        """Uniform float in [0, 1): the top 24 bits."""
-        return float(np.float32((self.next() >> 40) * (1.0 / 16777216.0)))
+        """Uniform float in [0, 1): the top 24 bits (exact in 32-bit)."""
+        return (self.next() >> 40) * (1.0 / 16777216.0)
 
 
 class RequestSampling:
@@ -58,7 +60,13 @@ class RequestSampling:
             self.counts[token] = self.counts.get(token, 0) + 1
 
 
-_ROW = struct.Struct("<ffffii")
+_ROW = "ffffii"
+_ARG_ROWS = 128          # rows whose settings travel as an argument of the launch (csrc/sampling.cu)
+
+
+@functools.lru_cache(maxsize=256)
+def _packer(rows: int) -> struct.Struct:
+    return struct.Struct("<" + _ROW * rows)
 
 
 class PendingSample:
@@ -98,28 +106,32 @@ def sample_async(logits: torch.Tensor, states: Sequence[RequestSampling]) -> Pen
         _check(_fn("sampling", "llmx_penalize")(_ptr(logits), vocab, _ptr(arr[0]), _ptr(arr[1]), _ptr(arr[2]),
                                                 _ptr(pen[0]), _ptr(pen[1]), _ptr(pen[2]), len(items), _stream()),
                "penalize")
-    all_greedy = all(s.params.greedy for s in states)
-    key = None
-    if all_greedy:
-        # Greedy rows draw nothing: their parameters are the same from step to step and stay on the device.
-        key = (dev.index, tuple(s.masked for s in states))
-    params = _greedy_params.get(key) if key is not None else None
-    if params is None:
-        raw = bytearray(_ROW.size * rows)
-        for r, s in enumerate(states):
-            p = s.params
-            u = 0.0 if p.greedy else s.rng.unit()
-            _ROW.pack_into(raw, r * _ROW.size, p.temp, p.top_p, p.min_p, u, p.top_k, s.masked)
-        host = torch.empty(len(raw), dtype=torch.uint8, pin_memory=True)
-        host.numpy()[:] = np.frombuffer(raw, dtype=np.uint8)
-        params = host.to(dev, non_blocking=True)
-        if key is not None:
-            if len(_greedy_params) > 64:
-                _greedy_params.clear()
-            _greedy_params[key] = params
+    all_greedy = True
+    values = []
+    for s in states:
+        p = s.params
+        u = 0.0
+        if p.temp > 0.0:                # greedy rows draw nothing
+            all_greedy = False
+            u = s.rng.unit()
+        values += (p.temp, p.top_p, p.min_p, u, p.top_k, s.masked)
+    raw = _packer(rows).pack(*values)
     out = torch.empty(rows, dtype=torch.int32, device=dev)
-    _check(_fn("sampling", "llmx_sample")(_ptr(logits), rows, vocab, _ptr(params), _ptr(out), 1 if all_greedy else 0,
-                                          _stream()), "sample")
+    if rows <= _ARG_ROWS:
+        _check(_fn("sampling", "llmx_sample_rows")(_ptr(logits), rows, vocab, raw, _ptr(out), 1 if all_greedy else 0, _stream()), "sample")
+    else:
+        # Greedy rows' settings are the same from step to step and stay on the device.
+        key = (dev.index, tuple(s.masked for s in states)) if all_greedy else None
+        params = _greedy_params.get(key) if key is not None else None
+        if params is None:
+            host = torch.empty(len(raw), dtype=torch.uint8, pin_memory=True)
+            host.numpy()[:] = np.frombuffer(raw, dtype=np.uint8)
+            params = host.to(dev, non_blocking=True)
+            if key is not None:
+                if len(_greedy_params) > 64:
+                    _greedy_params.clear()
+                _greedy_params[key] = params
+        _check(_fn("sampling", "llmx_sample")(_ptr(logits), rows, vocab, _ptr(params), _ptr(out), 1 if all_greedy else 0, _stream()), "sample")
     host = torch.empty(rows, dtype=torch.int32, pin_memory=True)
     host.copy_(out, non_blocking=True)
     event = torch.cuda.Event()
