@@ -613,7 +613,7 @@ latent_merge_kernel(const float* __restrict__ part, const WT* __restrict__ w_uv,
 // it waits for the kernel before.  Eight rows, 16 heads of 128 over latents of 512: the query step 12.2 -> 4.6 us, the merge
 // step 34 -> 10 us (its 2-byte reads waited for one another).
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int MAP_THREADS = 256, MAP_AHEAD = 16;
+constexpr int MAP_THREADS = 256, MAP_AHEAD = 16, MERGE_AHEAD = 4;
 
 __device__ __forceinline__ void unpack8(const uint4& w, float (&f)[8]) {
     const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&w);
@@ -691,7 +691,8 @@ __global__ void __launch_bounds__(MAP_THREADS)
 latent_merge_few_kernel(const float* __restrict__ part, const __nv_bfloat16* __restrict__ w_uv, __nv_bfloat16* __restrict__ out,
                         int heads, int V, int C, int splits) {
     pdl_trigger();
-    extern __shared__ __align__(16) float lat[];     // C
+    extern __shared__ __align__(16) float lat[];     // C, then a weight for each range
+    float* share = lat + C;
     const int row = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int v0 = blockIdx.z * 32 + warp * 4;
     uint4 w[4][CH];
@@ -704,20 +705,39 @@ latent_merge_few_kernel(const float* __restrict__ part, const __nv_bfloat16* __r
         }
     pdl_wait();
     const float* src = part + ((size_t)row * heads + h) * splits * (C + 2);
-    float mm = -INFINITY;
-    for (int s = 0; s < splits; ++s) mm = fmaxf(mm, src[(size_t)s * (C + 2) + C]);
-    float sum[CH], ll = 0.0f;
+    // The ranges' weights first, every warp all of them, a lane a range: a range that none of the row's keys lie in weighs nothing and
+    // its sums, which were never made, are not read.  Then the sums of MERGE_AHEAD ranges at a time (one after the other, each
+    // waited for its own maximum).
+    float mm = -INFINITY, ll = 0.0f;
+    for (int s = lane; s < splits; s += 32) mm = fmaxf(mm, src[(size_t)s * (C + 2) + C]);
+    mm = warp_max(mm);
+    for (int s = lane; s < splits; s += 32) {
+        const float ms = src[(size_t)s * (C + 2) + C];
+        const float e = ms == -INFINITY ? 0.0f : expf(ms - mm);
+        if (ms != -INFINITY) ll = fmaf(src[(size_t)s * (C + 2) + C + 1], e, ll);
+        if (warp == 0) share[s] = ms == -INFINITY ? -1.0f : e;
+    }
+    ll = warp_sum(ll);
+    __syncthreads();
+    float sum[CH];
 #pragma unroll
     for (int i = 0; i < CH; ++i) sum[i] = 0.0f;
-    for (int s = 0; s < splits; ++s) {
-        const float* one = src + (size_t)s * (C + 2);
-        const float ms = one[C];
-        if (ms == -INFINITY) continue;               // a range that none of the row's keys lie in: its sums were never made
-        const float e = expf(ms - mm);
-        ll += one[C + 1] * e;
+    for (int s0 = 0; s0 < splits; s0 += MERGE_AHEAD) {
+        float x[MERGE_AHEAD][CH], e[MERGE_AHEAD];
 #pragma unroll
-        for (int i = 0; i < CH; ++i)
-            if ((int)threadIdx.x + MAP_THREADS * i < C) sum[i] = fmaf(one[threadIdx.x + MAP_THREADS * i], e, sum[i]);
+        for (int a = 0; a < MERGE_AHEAD; ++a) {
+            e[a] = s0 + a < splits ? share[s0 + a] : -1.0f;
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                const int c = threadIdx.x + MAP_THREADS * i;
+                x[a][i] = !(e[a] < 0.0f) && c < C ? src[(size_t)(s0 + a) * (C + 2) + c] : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < MERGE_AHEAD; ++a)
+#pragma unroll
+            for (int i = 0; i < CH; ++i)
+                if (!(e[a] < 0.0f)) sum[i] = fmaf(x[a][i], e[a], sum[i]);
     }
 #pragma unroll
     for (int i = 0; i < CH; ++i)
@@ -818,15 +838,6 @@ latent_scores_tc_kernel(const float* __restrict__ qk, const __nv_bfloat16* __res
         row_m[p] = -INFINITY;
         row_l[p] = 0.0f;
     }
-    for (int i = threadIdx.x; i < 16 * W; i += TILE_THREADS) {
-        const int p = i / W, e = i % W, ri = p / HT, h = blockIdx.y * HT + p % HT;
-        const float x = (ri < tile_rows && h < heads) ? qk[((size_t)(row0 + ri) * heads + h) * W + e] : 0.0f;
-        __nv_bfloat16 a, b, c;
-        split3(x, a, b, c);
-        qs[(size_t)(0 * 16 + p) * WS + e] = a;
-        qs[(size_t)(1 * 16 + p) * WS + e] = b;
-        qs[(size_t)(2 * 16 + p) * WS + e] = c;
-    }
     const int per_row = W / 8;                      // 16-byte pieces a key has
     auto issue = [&](int t0, int which) {
         const uint32_t base = (uint32_t)__cvta_generic_to_shared(keys + (size_t)which * TC_KT * WS);
@@ -839,14 +850,40 @@ latent_scores_tc_kernel(const float* __restrict__ qk, const __nv_bfloat16* __res
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    const int n_tiles = end > begin ? (end - begin + TC_KT - 1) / TC_KT : 0;
+    if (n_tiles > 0) issue(begin, 0);
+    // The queries in fours, QS_AHEAD of them asked for before the first is cut into its parts, while the first keys are on their way.
+    constexpr int QS_AHEAD = 5;
+    const int fours = W / 4;
+    for (int i0 = threadIdx.x; i0 < 16 * fours; i0 += QS_AHEAD * TILE_THREADS) {
+        float4 x[QS_AHEAD];
+#pragma unroll
+        for (int u = 0; u < QS_AHEAD; ++u) {
+            const int i = i0 + u * TILE_THREADS, p = i / fours, ri = p / HT, h = blockIdx.y * HT + p % HT;
+            x[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (i < 16 * fours && ri < tile_rows && h < heads)
+                x[u] = *reinterpret_cast<const float4*>(qk + ((size_t)(row0 + ri) * heads + h) * W + 4 * (i % fours));
+        }
+#pragma unroll
+        for (int u = 0; u < QS_AHEAD; ++u) {
+            const int i = i0 + u * TILE_THREADS, p = i / fours;
+            if (i >= 16 * fours) break;
+            __align__(8) __nv_bfloat16 parts[3][4];
+            split3(x[u].x, parts[0][0], parts[1][0], parts[2][0]);
+            split3(x[u].y, parts[0][1], parts[1][1], parts[2][1]);
+            split3(x[u].z, parts[0][2], parts[1][2], parts[2][2]);
+            split3(x[u].w, parts[0][3], parts[1][3], parts[2][3]);
+#pragma unroll
+            for (int sp = 0; sp < 3; ++sp)
+                *reinterpret_cast<uint2*>(qs + (size_t)(sp * 16 + p) * WS + 4 * (i % fours)) = *reinterpret_cast<const uint2*>(parts[sp]);
+        }
+    }
     float o[NB][4];
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
         for (int i = 0; i < 4; ++i) o[nb][i] = 0.0f;
 
-    const int n_tiles = end > begin ? (end - begin + TC_KT - 1) / TC_KT : 0;
-    if (n_tiles > 0) issue(begin, 0);
     const uint32_t qs_addr = (uint32_t)__cvta_generic_to_shared(qs);
     const uint32_t ps_addr = (uint32_t)__cvta_generic_to_shared(ps);
     for (int it = 0; it < n_tiles; ++it) {
@@ -1102,10 +1139,10 @@ LLMX_EXPORT int llmx_latent_merge(const float* part, const void* w_uv, int w_dty
     const int rq = rows > 64 ? 8 : 1;
     const size_t smem = (size_t)rq * C * sizeof(float);
     if (smem > 48 * 1024) return LLMX_ERR_UNSUPPORTED;
-    if (rq == 1 && w_dtype == LLMX_BF16 && C % 8 == 0 && C <= 768 && !((uintptr_t)w_uv & 15)) {
+    if (rq == 1 && w_dtype == LLMX_BF16 && C % 8 == 0 && C <= 768 && splits <= 4096 && !((uintptr_t)w_uv & 15)) {
         const dim3 few(rows, heads, (V + 31) / 32);
 #define LLMX_MF(CH)                                                                                                        \
-    launch_kernel(latent_merge_few_kernel<CH>, few, dim3(MAP_THREADS), (size_t)C * sizeof(float), stream, part,            \
+    launch_kernel(latent_merge_few_kernel<CH>, few, dim3(MAP_THREADS), (size_t)(C + splits) * sizeof(float), stream, part, \
                   (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, heads, V, C, splits)
         if (C <= 256) LLMX_MF(1);
         else if (C <= 512) LLMX_MF(2);
