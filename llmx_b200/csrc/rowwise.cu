@@ -983,10 +983,37 @@ __global__ void clamped_glu_kernel(const float* __restrict__ gu, OutT* __restric
     act[i] = from_float<OutT>(g / (1.0f + expf(-alpha * g)) * (u + 1.0f));
 }
 
+__device__ __forceinline__ float clamped_f(float g, float u, float limit, float alpha) {
+    g = fminf(g, limit);
+    u = fminf(fmaxf(u, -limit), limit);
+    return quotient(g, 1.0f + expf(-alpha * g)) * (u + 1.0f);
+}
+
+// The same for widths in fours: a block a row and 1,024 of its values, four a thread, no division by the width (a 64-bit division and a
+// remainder a value were a quarter of a decoding step's launch: eight rows of 6,144, 3.3 -> 2.3 us between the products beside it).
+template <typename OutT>
+__global__ void __launch_bounds__(256)
+clamped_glu_four_kernel(const float* __restrict__ gu, OutT* __restrict__ act, int width, float limit, float alpha) {
+    pdl_trigger();
+    pdl_wait();
+    const size_t r = blockIdx.x;
+    const int c = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (c >= width) return;
+    const float4 g = *reinterpret_cast<const float4*>(gu + r * 2 * width + c), u = *reinterpret_cast<const float4*>(gu + r * 2 * width + width + c);
+    store4(act + r * width + c, clamped_f(g.x, u.x, limit, alpha), clamped_f(g.y, u.y, limit, alpha), clamped_f(g.z, u.z, limit, alpha),
+           clamped_f(g.w, u.w, limit, alpha));
+}
+
 LLMX_EXPORT int llmx_clamped_glu(const float* gu, void* act, int out_dtype, int rows, int width, float limit, float alpha,
                                  cudaStream_t stream) {
     const long long total = (long long)rows * width;
     if (total <= 0) return 0;
+    if (width % 4 == 0 && width <= 1024 * 65535 && !(((uintptr_t)gu | (uintptr_t)act) & 15)) {
+        const dim3 grid(rows, (width + 1023) / 1024);
+        if (out_dtype == LLMX_BF16) launch_kernel(clamped_glu_four_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, gu, (__nv_bfloat16*)act, width, limit, alpha);
+        else launch_kernel(clamped_glu_four_kernel<float>, dim3(grid), dim3(256), 0, stream, gu, (float*)act, width, limit, alpha);
+        return launch_status();
+    }
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (out_dtype == LLMX_BF16) launch_kernel(clamped_glu_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, gu, (__nv_bfloat16*)act, total, width, limit, alpha);
     else launch_kernel(clamped_glu_kernel<float>, dim3(blocks), dim3(256), 0, stream, gu, (float*)act, total, width, limit, alpha);
