@@ -7,7 +7,7 @@
 // does not depend on what else is in the batch (the reference's rule,
 // src/backends/backend.hpp:141-150; its kernels: f32.gpu:1034-1084).
 //
-// Three forms with the same bits: up to eight rows a thread an output column (`gemm_plain_few_kernel`, which reads its
+// Forms with the same bits: up to eight rows a thread an output column (`gemm_plain_few_kernel`, which reads its
 // first weights before it waits for the kernel before: W must not be that kernel's output), more than 64 rows 128 x 64 tiles with two
 // multiply-adds an instruction (`gemm_plain_many_kernel`), both for K in fours and aligned operands of one type; else 64 x 64 tiles.
 #include "common.cuh"
@@ -208,6 +208,51 @@ __global__ void __launch_bounds__(FEW_COLS) gemm_plain_few_kernel(const AT* __re
         *c = accumulate ? *c + acc[m] : acc[m];
     }
 }
+
+// A few rows over a short K (the second half of a low-rank pair): 32 columns a block, whose weight rows the block copies to shared
+// memory before it waits for the kernel before (a thread reading its own row asked for 16 bytes of 32 rows at a time); a thread
+// then has a column of up to two rows.  The same order of k, the same bits.
+constexpr int SHORT_COLS = 32, SHORT_THREADS = 128, SHORT_K = 512;
+
+__global__ void __launch_bounds__(SHORT_THREADS) gemm_plain_short_kernel(const float* __restrict__ A, const float* __restrict__ W,
+                                                                         float* __restrict__ C, int M, int N, int K, int accumulate) {
+    pdl_trigger();
+    extern __shared__ __align__(16) float short_mem[];   // weights [32][K + 4], then A's rows [M][K]
+    const int n0 = blockIdx.x * SHORT_COLS, pieces = K / 4, stride = K + 4;
+    float* rows = short_mem + SHORT_COLS * stride;
+    for (int i = threadIdx.x; i < SHORT_COLS * pieces; i += SHORT_THREADS) {
+        const int r = i / pieces, c = 4 * (i - r * pieces);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(short_mem + r * stride + c)),
+                     "l"(W + (size_t)min(n0 + r, N - 1) * K + c) : "memory");
+    }
+    pdl_wait();
+    for (int i = threadIdx.x; i < M * pieces; i += SHORT_THREADS)
+        *reinterpret_cast<float4*>(rows + 4 * i) = *reinterpret_cast<const float4*>(A + 4 * i);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int col = threadIdx.x & 31, m0 = threadIdx.x >> 5, n = n0 + col;
+    const float* w = short_mem + col * stride;
+    const float* a0 = rows + min(m0, M - 1) * K;
+    const float* a1 = rows + min(m0 + 4, M - 1) * K;
+    float acc0 = 0.0f, acc1 = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < K; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(w + k), y = *reinterpret_cast<const float4*>(a0 + k), z = *reinterpret_cast<const float4*>(a1 + k);
+        acc0 = fmaf(y.x, x.x, acc0), acc1 = fmaf(z.x, x.x, acc1);
+        acc0 = fmaf(y.y, x.y, acc0), acc1 = fmaf(z.y, x.y, acc1);
+        acc0 = fmaf(y.z, x.z, acc0), acc1 = fmaf(z.z, x.z, acc1);
+        acc0 = fmaf(y.w, x.w, acc0), acc1 = fmaf(z.w, x.w, acc1);
+    }
+    if (n >= N) return;
+    if (m0 < M) {
+        float* c = C + (size_t)m0 * N + n;
+        *c = accumulate ? *c + acc0 : acc0;
+    }
+    if (m0 + 4 < M) {
+        float* c = C + (size_t)(m0 + 4) * N + n;
+        *c = accumulate ? *c + acc1 : acc1;
+    }
+}
 }  // namespace
 
 LLMX_EXPORT int llmx_gemm_plain(const void* A, int a_dtype, const void* W, int w_dtype, float* C, int M, int N, int K,
@@ -215,6 +260,16 @@ LLMX_EXPORT int llmx_gemm_plain(const void* A, int a_dtype, const void* W, int w
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return LLMX_ERR_BAD_ARGUMENT;
     const size_t few_bytes = (size_t)M * K * sizeof(float);
+    if (M <= FEW_ROWS && K % 4 == 0 && K <= SHORT_K && a_dtype == LLMX_F32 && w_dtype == LLMX_F32 && !(((uintptr_t)A | (uintptr_t)W) & 15)) {
+        const size_t bytes = ((size_t)SHORT_COLS * (K + 4) + (size_t)M * K) * sizeof(float);
+        if (bytes > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(gemm_plain_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (e != cudaSuccess) return (int)e;
+        }
+        launch_kernel(gemm_plain_short_kernel, dim3((N + SHORT_COLS - 1) / SHORT_COLS), dim3(SHORT_THREADS), bytes, stream, (const float*)A,
+                      (const float*)W, C, M, N, K, accumulate);
+        return launch_status();
+    }
     if (M <= FEW_ROWS && K % 4 == 0 && few_bytes <= FEW_BYTES && !((uintptr_t)W & 15) && a_dtype == w_dtype) {
         const dim3 few((N + FEW_COLS - 1) / FEW_COLS);
         if (a_dtype == LLMX_F32)

@@ -544,7 +544,10 @@ moe_few_stream_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv
         tc::fence_barrier_init();
     }
     pdl_trigger();
-    pdl_wait();
+    // The step's tokens and a table that came with the weights are written by no kernel of the step: the stream of weights starts
+    // while the kernel before still runs (a router's choice is such a kernel's output).
+    const bool early = token_ids != nullptr;
+    if (!early) pdl_wait();
     if (warp == 0) {
         int mine = -1;
         if (lane < pairs) {
@@ -589,6 +592,7 @@ moe_few_stream_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv
         }
         return;
     }
+    if (early) pdl_wait();       // the rows, and the output's earlier readers
     for (int n = warp; n < count; n += workers) {
         const int st = n % places;
         if (!tc::mbar_wait_warp(&full[st], (n / places) & 1u, abort_flag, error_word, ERR_FEW_CONSUMER)) break;
