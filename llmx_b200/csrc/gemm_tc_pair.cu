@@ -12,8 +12,8 @@
 //                          without multicast: `cp.async.bulk.tensor...cta_group::2` only names whose barrier counts)
 //   warp 1 (first block)   waits for a stage of both blocks, issues the products, and frees the stage in both blocks
 //                          with one commit (`tcgen05.commit...multicast::cluster`, an arrival on each block's barrier)
-//   warps 2-5 (both)       epilogue: tensor memory -> float32 output (stored, or added with float atomics), then an
-//                          arrival on the first block's accumulator-empty barrier
+//   warps 2-9 (both)       epilogue: tensor memory -> float32 output (stored, or added with float atomics), two warps for a
+//                          quarter of the lanes (HEADS: one, warps 2-5), then an arrival on the first block's accumulator-empty barrier
 //
 // Work: the pair walks tiles pair, pair + pairs, ... (token tiles vary fastest), optionally with K cut into `splits`
 // ranges that are added with atomics, or (`splits` 0) with only the last, partial round's tiles cut.  Every wait
@@ -38,8 +38,6 @@ namespace {
 constexpr int BM = 128;      // weight rows per block (half of the pair's 256)
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int EPI_WARPS = 4;
-constexpr int THREADS = 64 + EPI_WARPS * 32;
 enum : int { MODE_STORE = 0, MODE_ACCUMULATE = 1, MODE_ACT = 2 };
 enum : int { ERR_PAIR_PRODUCER = 111, ERR_PAIR_MMA_FULL = 112, ERR_PAIR_MMA_ACC = 113, ERR_PAIR_EPILOGUE = 114 };
 
@@ -49,6 +47,11 @@ enum : int { PLAIN = 0, DUAL = 1, HEADS = 2 };
 // "narrow" one (BN / 2 rows a block).
 template <int BN, int FORM>
 struct PairCfg {
+    // Two warps for each quarter of the accumulator's lanes, every other 32 of its columns each: over a short inner width the write-out
+    // takes longer than the products (1,833 tokens: 1,024 outputs over 2,048 or 3,072 28.0 -> 25.9 us, gated 3,072 over 1,024 27.6 ->
+    // 26.8).  A thread of the HEADS form would read its token's angles for one head in place of two: 27 -> 31 us with two warps.
+    static constexpr int EPI_WARPS = FORM == HEADS ? 4 : 8;
+    static constexpr int THREADS = 64 + EPI_WARPS * 32;
     static constexpr int A_TILES = FORM == DUAL ? 2 : 1;
     static constexpr int A_BYTES = BM * BK * 2;                 // one tile of the block's wide rows
     static constexpr int B_BYTES = (BN / 2) * BK * 2;           // the block's half of the narrow tile
@@ -119,7 +122,7 @@ struct PairScheduler {
 // extents.  PLAIN: wide = weight [N, K], narrow = tokens [M, K], C float32 [M, N].  DUAL: the weight has 2 N rows,
 // C bfloat16 [M, N].  HEADS: wide = tokens, narrow = weight; the outputs are `hp`'s.
 template <int BN, int FORM>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__((PairCfg<BN, FORM>::THREADS), 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_constant__ CUtensorMap map_narrow,
                     void* __restrict__ C_, int wide_rows, int narrow_rows, int K, int mode, int splits, int group,
                     int tail, int* error_word, const HeadsEpilogue hp, const ActEpilogue ae) {
@@ -148,7 +151,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
         }
         for (int b = 0; b < 2; ++b) {
             tc::mbar_init(&acc_full[b], 1);
-            tc::mbar_init(&acc_empty[b], 2 * EPI_WARPS);        // the epilogue warps of both blocks
+            tc::mbar_init(&acc_empty[b], 2 * cfg::EPI_WARPS);        // the epilogue warps of both blocks
         }
         *abort_flag = 0;
         tc::fence_barrier_init();
@@ -234,7 +237,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
             }
         }
     } else {
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, share = (warp - 2) >> 2;     // with two warps a quarter: whose columns
         PairScheduler sched(w_tiles, m_tiles, k_blocks, splits, group, tail);
         Work w;
         uint32_t acc = 0, acc_phase = 0;
@@ -251,7 +254,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
                 heads_epilogue<BN>(hp, norm_w, taddr, n, wide_rows, w.mt * BN, narrow_rows);
             } else if (w.kb1 > w.kb0) {
 #pragma unroll 1
-                for (int c = 0; c < BN; c += 32) {
+                for (int c = 32 * share; c < BN; c += 64) {
                     uint32_t r[32];
                     tc::tmem_ld_32x32(taddr + c, r);
                     if constexpr (FORM == DUAL) {
@@ -349,7 +352,7 @@ int launch_pair(const CUtensorMap& wide, const CUtensorMap& narrow, void* C, int
     }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(2 * pairs));
-    lc.blockDim = dim3(THREADS);
+    lc.blockDim = dim3(cfg::THREADS);
     lc.dynamicSmemBytes = cfg::SMEM_BYTES;
     lc.stream = stream;
     cudaLaunchAttribute attr[2];
