@@ -195,13 +195,18 @@ moe_cores_kernel(const T* __restrict__ a, int a_div, const T* __restrict__ w, co
 //                          16 up rows of the same outputs, so that a warp's 32 sums of a pair are 16 whole outputs; of the pairs' rows
 //                          as many boxes of 32 as the unit's half has
 //   warp 1 (first block)   the products, and a commit that frees a stage in both blocks
-//   warps 2-5 (both)       sums to the output; gated, lanes i and i + 16 swap halves of their pairs, each makes 16 units of both
+//   warps 2-9 (both)       sums to the output, of two warps with the same lanes each every other run of 32 pairs; gated, lanes i and
+//                          i + 16 swap halves of their pairs, each makes 16 units of both
 // An expert's list is cut into ceil(pairs / 256) equal parts: its weights are read that often, and none is left with a few
 // pairs.  Units of one expert follow one another, its weight tiles fastest: what they share meets in the L2 cache.
+// Bound, at a few dozen to a few hundred pairs an expert, by the experts' weights from memory and by the write-out: with one warp for a
+// quarter of the lanes the tensor cores were busy a third of the time.  Measured against the mma.sync form over gathered rows, 16 experts,
+// two a token: 2,048 tokens, 2,048 -> 1,536 gated 98 us, one warp 80, two 71; back 51, 34 and 34; 1,201 tokens, 4,096 -> 3,072 gated
+// 188 us -> 167 (one warp), back 87 -> 80.
 constexpr int TC_LIST_TILE = 128;                                            // pairs a tile of the routing holds for this form
 constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_BOX = 32;
 constexpr int TC_W_BYTES = TC_M * TC_K * 2, TC_R_BYTES = TC_ROWS / 2 * TC_K * 2, TC_STAGE = TC_W_BYTES + TC_R_BYTES, TC_STAGES = 6;
-constexpr int TC_EPI_WARPS = 4, TC_THREADS = 64 + TC_EPI_WARPS * 32;
+constexpr int TC_EPI_WARPS = 8, TC_THREADS = 64 + TC_EPI_WARPS * 32;
 constexpr int TC_MAX_EXPERTS = 8192;                                         // three numbers of each lie in shared memory, beside fewer stages if need be
 constexpr int tc_smem(int stages, int experts) { return stages * TC_STAGE + 1024 + 256 + 3 * experts * (int)sizeof(int); }
 constexpr int tc_stages(int experts) {
@@ -213,7 +218,8 @@ static_assert(tc_stages(TC_MAX_EXPERTS) >= 3, "a stage in use and two on their w
 enum : int { ERR_MOE_PRODUCER = 441, ERR_MOE_MMA = 442, ERR_MOE_EPILOGUE = 443 };
 
 // rows[place] = a[pair / a_div] for the pair at that place of the sorted lists; a block a place.
-__global__ void __launch_bounds__(256)
+constexpr int GATHER_THREADS = 128;                  // many blocks an SM: a block waits for one read after the other
+__global__ void __launch_bounds__(GATHER_THREADS)
 gather_kernel(const uint4* __restrict__ a, int a_div, const int* __restrict__ lists, const int* __restrict__ counts, int experts, int pairs,
               uint4* __restrict__ rows, int per_row) {
     pdl_trigger();
@@ -243,7 +249,7 @@ gather_kernel(const uint4* __restrict__ a, int a_div, const int* __restrict__ li
     __syncthreads();
     if (found < 0) return;                           // past the lists: pairs of experts without weights
     const uint4* src = a + (size_t)(found / a_div) * per_row;
-    for (int i = threadIdx.x; i < per_row; i += 256) rows[(size_t)place * per_row + i] = src[i];
+    for (int i = threadIdx.x; i < per_row; i += GATHER_THREADS) rows[(size_t)place * per_row + i] = src[i];
 }
 
 // An expert's units and where its pairs' rows begin; filled by the block, read by its warps.
@@ -387,22 +393,29 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
             }
         }
     } else {
-        const int quarter = warp & 3;                // the tensor-memory lanes that this warp may touch
+        const int quarter = warp & 3, share = (warp - 2) >> 2;        // the tensor-memory lanes that this warp may touch, and which pairs it has
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
         while (ok && units.next(at, n, w)) {
+            const int* list = lists + (size_t)units.e * pairs + at;
+            const int place = row[units.e] + at;
+            const int c = w * w_cols + (GATED ? (int)rank * (TC_M / 2) + quarter * 16 + (lane & 15) : (int)rank * TC_M + quarter * 32 + lane);
+            int dest[TC_ROWS / 64];                  // the rows that the lane's pairs go to: read while the products run
+#pragma unroll
+            for (int i = 0; i < TC_ROWS / 64; ++i) {
+                const int p = 32 * share + 64 * i + lane;
+                dest[i] = out_sorted ? place + p : p < n ? list[p] : 0;
+            }
             ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_MOE_EPILOGUE);
             if (!ok) break;
             tc::tc_fence_after();
             const uint32_t taddr = tmem_base + acc * TC_ROWS + ((uint32_t)(quarter * 32) << 16);
-            const int* list = lists + (size_t)units.e * pairs + at;
-            const int place = row[units.e] + at;
-            const int c = w * w_cols + (GATED ? (int)rank * (TC_M / 2) + quarter * 16 + (lane & 15) : (int)rank * TC_M + quarter * 32 + lane);
-#pragma unroll 1
-            for (int p0 = 0; p0 < n; p0 += 32) {
+#pragma unroll
+            for (int i = 0; i < TC_ROWS / 64; ++i) {
+                const int p0 = 32 * share + 64 * i, to = dest[i];
+                if (p0 >= n) break;
                 uint32_t r[32];
                 tc::tmem_ld_32x32(taddr + p0, r);
-                const int to = out_sorted ? place + p0 + lane : p0 + lane < n ? list[p0 + lane] : 0;         // the row that pair p0 + lane goes to
                 tc::tmem_wait_ld();
                 if constexpr (GATED) {
                     const bool up = lane >= 16;      // this lane's sums are up rows; it makes the second half of the pairs
@@ -413,11 +426,18 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
                         const float own = __uint_as_float(up ? r[16 + j] : r[j]);
                         x[j] = from_float<OutT>(glu_f(glu, up ? got : own, up ? own : got));
                     }
+                    const int half = up ? 16 : 0;
+                    if (out_sorted && p0 + 32 <= n) {            // no condition a value: neighbouring rows
+                        OutT* to_row = out + (size_t)(place + p0 + half) * N + c;
+                        if (c < N)
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int p = j + (up ? 16 : 0);
-                        const size_t dst = (size_t)__shfl_sync(0xffffffffu, to, p);
-                        if (p0 + p < n && c < N) out[dst * N + c] = x[j];
+                            for (int j = 0; j < 16; ++j) to_row[(size_t)j * N] = x[j];
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const size_t dst = (size_t)__shfl_sync(0xffffffffu, to, half + j);
+                            if (p0 + half + j < n && c < N) out[dst * N + c] = x[j];
+                        }
                     }
                 } else {
 #pragma unroll
@@ -1024,7 +1044,7 @@ LLMX_EXPORT int llmx_moe_gather(const void* a, int a_div, const int* lists, cons
     if (pairs <= 0) return 0;
     if (K <= 0 || a_div <= 0 || experts <= 0) return LLMX_ERR_BAD_ARGUMENT;
     if (K % 8 || (((uintptr_t)a | (uintptr_t)rows) & 15)) return LLMX_ERR_UNSUPPORTED;
-    launch_kernel(gather_kernel, dim3(pairs), dim3(256), 0, stream, (const uint4*)a, a_div, lists, counts, experts, pairs, (uint4*)rows, K / 8);
+    launch_kernel(gather_kernel, dim3(pairs), dim3(GATHER_THREADS), 0, stream, (const uint4*)a, a_div, lists, counts, experts, pairs, (uint4*)rows, K / 8);
     return launch_status();
 }
 
