@@ -504,8 +504,47 @@ attention_split_kernel(const QT* __restrict__ q, const KVT* __restrict__ cache, 
     }
 }
 
-// The ranges' partial states of one (row, head), merged in range order.  One warp a (row, head).
-template <typename QT>
+// A warp's merge of the ranges' partial states of one (row, map head): the largest score, the sum and the outputs, not yet divided.
+// A lane has a range's maximum and sum, 32 ranges at a time; then the ranges' outputs are added in range order, their factors passed
+// around by shuffles.  Bound by the reads' latency: those of AHEAD ranges are issued without a condition (a range without keys
+// of the row made no output; what lies there is read and not used) before the first is added.
+template <int PER_LANE>
+__device__ __forceinline__ void merge_ranges(const float* __restrict__ p, int V, int splits, int lane, float& mm, float& ll, float (&o)[PER_LANE]) {
+    constexpr int AHEAD = PER_LANE <= 4 ? 8 : 4;
+    mm = -INFINITY, ll = 0.0f;
+    for (int s = lane; s < splits; s += 32) mm = fmaxf(mm, p[(size_t)s * (V + 2) + V]);
+    mm = warp_max(mm);
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) o[i] = 0.0f;
+    for (int s0 = 0; s0 < splits; s0 += 32) {
+        const float* mine = p + (size_t)(s0 + lane) * (V + 2);
+        const float ms = s0 + lane < splits ? mine[V] : -INFINITY;
+        const float e = ms == -INFINITY ? 0.0f : expf(ms - mm);
+        if (ms != -INFINITY) ll += mine[V + 1] * e;
+        const unsigned made = __ballot_sync(0xffffffffu, ms != -INFINITY);
+        const int count = min(32, splits - s0);
+        for (int j = 0; j < count; j += AHEAD) {
+            float x[AHEAD][PER_LANE];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const float* one = p + (size_t)(s0 + min(j + u, count - 1)) * (V + 2);
+#pragma unroll
+                for (int i = 0; i < PER_LANE; ++i) x[u][i] = lane + 32 * i < V ? one[lane + 32 * i] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const float f = __shfl_sync(0xffffffffu, e, (j + u) & 31);
+                const bool counts = j + u < count && (made >> ((j + u) & 31) & 1);
+#pragma unroll
+                for (int i = 0; i < PER_LANE; ++i) o[i] = counts ? fmaf(x[u][i], f, o[i]) : o[i];
+            }
+        }
+    }
+    ll = warp_sum(ll);
+}
+
+// The ranges' partial states of one (row, head), merged in range order.  One warp a (row, head); V <= 32 * PER_LANE.
+template <typename QT, int PER_LANE>
 __global__ void __launch_bounds__(128)
 attention_merge_kernel(const float* __restrict__ partial, QT* __restrict__ out, int items, int V, int splits, int heads,
                        const int* __restrict__ positions, AttnExtras extras) {
@@ -515,36 +554,11 @@ attention_merge_kernel(const float* __restrict__ partial, QT* __restrict__ out, 
     const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= items) return;
     float* turned = merge_smem + (threadIdx.x >> 5) * V;
-    const float* p = partial + (size_t)item * splits * (V + 2);
-    // A lane has a range's maximum and sum, 32 ranges at a time; then the ranges' outputs are added in order, their factors
-    // passed around by shuffles, four ranges' reads in flight.
-    float mm = -INFINITY;
-    for (int s = lane; s < splits; s += 32) mm = fmaxf(mm, p[(size_t)s * (V + 2) + V]);
-    mm = warp_max(mm);
-    float ll = 0.0f, o[MAX_PER_LANE];
-#pragma unroll
-    for (int i = 0; i < MAX_PER_LANE; ++i) o[i] = 0.0f;
-    for (int s0 = 0; s0 < splits; s0 += 32) {
-        const float* mine = p + (size_t)(s0 + lane) * (V + 2);
-        const float ms = s0 + lane < splits ? mine[V] : -INFINITY;
-        const float e = ms == -INFINITY ? 0.0f : expf(ms - mm);
-        if (ms != -INFINITY) ll += mine[V + 1] * e;
-        const unsigned made = __ballot_sync(0xffffffffu, ms != -INFINITY);       // a range without keys of the row made no output
-        const int count = min(32, splits - s0);
-#pragma unroll 4
-        for (int j = 0; j < count; ++j) {
-            const float f = __shfl_sync(0xffffffffu, e, j);
-            if (!(made >> j & 1)) continue;
-            const float* one = p + (size_t)(s0 + j) * (V + 2);
-#pragma unroll
-            for (int i = 0; i < MAX_PER_LANE; ++i)
-                if (lane + 32 * i < V) o[i] += one[lane + 32 * i] * f;
-        }
-    }
-    ll = warp_sum(ll);
+    float mm, ll, o[PER_LANE];
+    merge_ranges(partial + (size_t)item * splits * (V + 2), V, splits, lane, mm, ll, o);
     const float inv = finish_softmax(mm, ll, extras, item % heads) * head_gate(extras, item / heads, item % heads);
 #pragma unroll
-    for (int i = 0; i < MAX_PER_LANE; ++i) {
+    for (int i = 0; i < PER_LANE; ++i) {
         const int d = lane + 32 * i;
         if (d >= V) continue;
         if (extras.vfreq) turned[d] = o[i] * inv;
@@ -557,65 +571,54 @@ attention_merge_kernel(const float* __restrict__ partial, QT* __restrict__ out, 
 }
 
 // The two maps of one (row, head) merged and combined (see `AttnExtras`).  One warp a (row, head); `heads` counts heads.
-template <typename QT>
+template <typename QT, int PER_LANE>
 __global__ void __launch_bounds__(128)
 attention_merge_maps_kernel(const float* __restrict__ partial, QT* __restrict__ out, int items, int V, int splits, int heads,
-                            AttnExtras extras) {
+                            const int* __restrict__, AttnExtras extras) {
     pdl_trigger();
     pdl_wait();
     const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= items) return;
-    float o[MAX_PER_LANE];
+    float o[PER_LANE];
 #pragma unroll
-    for (int i = 0; i < MAX_PER_LANE; ++i) o[i] = 0.0f;
+    for (int i = 0; i < PER_LANE; ++i) o[i] = 0.0f;
+#pragma unroll 1
     for (int map = 0; map < 2; ++map) {
-        const float* p = partial + ((size_t)item * 2 + map) * splits * (V + 2);
-        float mm = -INFINITY;
-        for (int s = 0; s < splits; ++s) mm = fmaxf(mm, p[(size_t)s * (V + 2) + V]);
-        float ll = 0.0f;
-        for (int s = 0; s < splits; ++s) {
-            const float ms = p[(size_t)s * (V + 2) + V];
-            ll += ms == -INFINITY ? 0.0f : p[(size_t)s * (V + 2) + V + 1] * expf(ms - mm);
-        }
+        float mm, ll, one[PER_LANE];
+        merge_ranges(partial + ((size_t)item * 2 + map) * splits * (V + 2), V, splits, lane, mm, ll, one);
         const float inv = (map == 0 ? 1.0f : -extras.factor) / ll;
-        for (int s = 0; s < splits; ++s) {
-            const float ms = p[(size_t)s * (V + 2) + V];
-            if (ms == -INFINITY) continue;
-            const float f = expf(ms - mm) * inv;
 #pragma unroll
-            for (int i = 0; i < MAX_PER_LANE; ++i) {
-                const int d = lane + 32 * i;
-                if (d < V) o[i] = fmaf(p[(size_t)s * (V + 2) + d], f, o[i]);
-            }
-        }
+        for (int i = 0; i < PER_LANE; ++i) o[i] = fmaf(one[i], inv, o[i]);
     }
     float ss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < MAX_PER_LANE; ++i) ss = fmaf(o[i], o[i], ss);
+    for (int i = 0; i < PER_LANE; ++i) ss = fmaf(o[i], o[i], ss);
     const float f = extras.out_factor / sqrtf(warp_sum(ss) / (float)V + extras.eps) * head_gate(extras, item / heads, item % heads);
     QT* orow = out + (size_t)item * V;
 #pragma unroll
-    for (int i = 0; i < MAX_PER_LANE; ++i) {
+    for (int i = 0; i < PER_LANE; ++i) {
         const int d = lane + 32 * i;
         if (d < V) orow[d] = from_float<QT>(o[i] * f);
     }
 }
 
 // The merge of `heads` map heads' ranges, whichever form left them.
+template <typename QT, int PER_LANE>
+static int launch_merge_as(const float* partial, QT* out, int items, int heads, int V, int splits, const int* positions, const AttnExtras& extras,
+                           cudaStream_t stream) {
+    const bool maps = extras.maps == 2;
+    launch_kernel(maps ? attention_merge_maps_kernel<QT, PER_LANE> : attention_merge_kernel<QT, PER_LANE>, dim3((items + 3) / 4), dim3(128),
+                  maps ? 0 : (size_t)4 * V * sizeof(float), stream, partial, out, items, V, splits, maps ? heads / 2 : heads, positions, extras);
+    return launch_status();
+}
 static int launch_merge(const float* partial, void* out, int q_dtype, int rows, int heads, int V, int splits, const int* positions,
                         const AttnExtras& extras, cudaStream_t stream) {
     const int items = rows * heads / extras.maps;
-    const dim3 grid((items + 3) / 4);
-    const size_t smem = (size_t)4 * V * sizeof(float);
-    if (extras.maps == 2) {
-        if (q_dtype == LLMX_BF16) launch_kernel(attention_merge_maps_kernel<__nv_bfloat16>, grid, dim3(128), 0, stream, partial, (__nv_bfloat16*)out, items, V, splits, heads / 2, extras);
-        else launch_kernel(attention_merge_maps_kernel<float>, grid, dim3(128), 0, stream, partial, (float*)out, items, V, splits, heads / 2, extras);
-    } else if (q_dtype == LLMX_BF16) {
-        launch_kernel(attention_merge_kernel<__nv_bfloat16>, grid, dim3(128), smem, stream, partial, (__nv_bfloat16*)out, items, V, splits, heads, positions, extras);
-    } else {
-        launch_kernel(attention_merge_kernel<float>, grid, dim3(128), smem, stream, partial, (float*)out, items, V, splits, heads, positions, extras);
-    }
-    return launch_status();
+    if (q_dtype == LLMX_BF16)
+        return V <= 128 ? launch_merge_as<__nv_bfloat16, 4>(partial, (__nv_bfloat16*)out, items, heads, V, splits, positions, extras, stream)
+                        : launch_merge_as<__nv_bfloat16, MAX_PER_LANE>(partial, (__nv_bfloat16*)out, items, heads, V, splits, positions, extras, stream);
+    return V <= 128 ? launch_merge_as<float, 4>(partial, (float*)out, items, heads, V, splits, positions, extras, stream)
+                    : launch_merge_as<float, MAX_PER_LANE>(partial, (float*)out, items, heads, V, splits, positions, extras, stream);
 }
 
 // ---- the staged form, for rows that are few -------------------------------------------------------------------------------

@@ -1423,3 +1423,34 @@ def test_expert_products_in_sorted_rows(experts, top, rows, K, N):
     assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 8 * slack).all()
     want = torch.einsum("pn,pkn->pk", act.double(), w.double()[expert])
     assert (y[at].double() - want).abs().max() <= 4 * N ** 0.5 * 2.0 ** -22 * max(1.0, float(act.abs().max()))
+
+
+@pytest.mark.parametrize("maps", [1, 2])
+@pytest.mark.parametrize("value_dim", [40, 128, 192])
+@pytest.mark.parametrize("splits", [1, 7, 9, 33, 64])
+def test_ranges_without_keys_are_left_out_of_the_merge(maps, value_dim, splits):
+    """More ranges than keys: rows of 1, 3, 40 and 200 keys against the same in one range.  A range without keys leaves what lay in the
+    scratch memory.  Bound: 32-bit sums in another order, 64 terms of at most 4 each, with the difference's norm behind them."""
+    from llmx_b200 import ops
+    heads, kv_heads, key_dim, page = 4, 2, 64, 16
+    g = torch.Generator().manual_seed(splits)
+    lengths = [1, 3, 40, 200]
+    pages = [(x + page - 1) // page for x in lengths]
+    table = torch.zeros(4, max(pages), dtype=torch.int32)
+    at = 0
+    for r, p in enumerate(pages):
+        table[r, :p] = torch.arange(at, at + p)
+        at += p
+    cache = torch.randn(at, 1, kv_heads, page, maps * key_dim + value_dim, generator=g).to(DEV)
+    q = torch.randn(4, heads * maps * key_dim, generator=g).to(DEV)
+    req, pos = torch.arange(4, dtype=torch.int32, device=DEV), torch.tensor([x - 1 for x in lengths], dtype=torch.int32, device=DEV)
+    extras = ops.SoftmaxExtras(difference=(0.4, 0.8, 1e-6)) if maps == 2 else None
+    outs = []
+    for n in (1, splits):
+        torch.full((1 << 22,), float("nan"), device=DEV)           # what the scratch memory may then hold
+        out = torch.empty(4, heads * value_dim, device=DEV)
+        ops.attention_split(q, cache, out, req, pos, table.to(DEV), heads, kv_heads, key_dim, value_dim, None, None, key_dim ** -0.5, splits=n,
+                            extras=extras)
+        outs.append(out)
+    assert bool(torch.isfinite(outs[1]).all())
+    assert torch.allclose(outs[0], outs[1], rtol=2e-5, atol=2e-5)
