@@ -106,6 +106,7 @@ _SIGNATURES = {
     ("rowwise", "llmx_add_bias"): [_p, _p, _i, _i, _p],
     ("rowwise", "llmx_clamped_glu"): [_p, _p, _i, _i, _i, _f, _f, _p],
     ("rowwise", "llmx_silu_columns"): [_p, _i, _i, _i, _i, _p],
+    ("rowwise", "llmx_split_rows"): [_p, ctypes.c_longlong, _i, _p, _i, _i, _p],
     ("rowwise", "llmx_gated_rmsnorm"): [_p, _p, _i, _p, _i, _p, _i, _i, _i, _i, _f, _i, _i, _p],
     ("rowwise", "llmx_rmsnorm_add"): [_p, _p, _p, _p, _p, _i, _i, _i, _f, _p, ctypes.c_longlong, _p],
     ("recurrence", "llmx_channel_decay"): [_p, _i, _i, _i, _i, _p, _p, _f, _p, _i, _i, _f, _p],
@@ -514,6 +515,17 @@ def silu_columns_(x: torch.Tensor, first: int, count: int) -> torch.Tensor:
     _need(x.dtype == torch.float32 and x.dim() == 2 and 0 <= first and first + count <= x.shape[1], "silu_columns: range does not fit")
     _check(_fn("rowwise", "llmx_silu_columns")(_ptr(x), x.shape[0], x.shape[1], int(first), int(count), _stream()), "silu_columns")
     return x
+
+
+def split_rows(x: torch.Tensor, weight: bool = False) -> torch.Tensor:
+    """float32 rows [rows, n] (a view whose rows may be strided) as bfloat16 parts [rows, 6 n], so that split_rows(a) @
+    split_rows(w, weight=True).T is a @ w.T as close as a 32-bit product (csrc/rowwise.cu); n a multiple of 4."""
+    _need(x.is_cuda, "kernel arguments must be CUDA tensors (there is no CPU path)")
+    _need(x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] % 4 == 0, "split_rows: float32 rows of a multiple of four values")
+    out = torch.empty((x.shape[0], 6 * x.shape[1]), dtype=torch.bfloat16, device=x.device)
+    _check(_fn("rowwise", "llmx_split_rows")(_ptr(x), _row_stride(x), 1 if weight else 0, _ptr(out), x.shape[0], x.shape[1], _stream()),
+           "split_rows")
+    return out
 
 
 def gated_rmsnorm(o: torch.Tensor, gate: torch.Tensor, weight: Optional[torch.Tensor], eps: float, group: int, gate_kind: str,

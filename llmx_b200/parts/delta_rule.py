@@ -33,7 +33,7 @@ from .. import ops, runtime
 from ..cache.manager import StateSpec
 from ..weights.spec import TensorSpec
 from .base import Part, Precision, StepBatch
-from .linear import Linear, stored_product
+from .linear import Linear, SplitLinear, stored_product
 
 
 class GatedDeltaRule(Part):
@@ -96,9 +96,8 @@ class GatedDeltaRule(Part):
         self.decay_in = self.decay_rank or self.heads
         self.inputs = Linear(torch.cat([t["q"], t["k"], t["v"], t["g1" if self.gate_rank else "g"], t["b"],
                                         t["a1" if self.decay_rank else "a"]], dim=0), precision)
-        full = Precision("float32", torch.float32, precision.invariant)
-        self.a2 = Linear(t["a2"].to(torch.float32), full) if self.decay_rank else None
-        self.g2 = Linear(t["g2"].to(torch.float32), full) if self.gate_rank else None
+        self.a2 = SplitLinear(t["a2"], precision) if self.decay_rank else None
+        self.g2 = SplitLinear(t["g2"], precision) if self.gate_rank else None
         self.o = Linear(t["o"], precision)
         self.taps_w = torch.cat([t["q.conv"], t["k.conv"], t["v.conv"]], dim=0).to(torch.float32).contiguous()
         self.a_log = t["A_log"].to(torch.float32).contiguous()
@@ -119,7 +118,7 @@ class GatedDeltaRule(Part):
         ready = torch.empty((rows, self.channels), dtype=torch.float32, device=h.device)
         o = torch.empty((rows, vw), dtype=torch.float32, device=h.device)
         if self.decay_rank:
-            decay_in = self.a2(proj[:, a_off:a_off + self.decay_rank].contiguous())          # [rows, heads * D], 32-bit
+            decay_in = self.a2.of_rows(proj[:, a_off:a_off + self.decay_rank])          # [rows, heads * D], 32-bit
             gates = torch.empty((rows, H + H * self.key_dim), dtype=torch.float32, device=h.device)
             ops.conv_prepare(proj, self.channels, qk, qk, self.taps_w, ready, self.a_log, self.dt_bias, b_off, a_off, gates, H,
                              self.key_dim, self.key_dim ** -0.5, state, self.state_floats, step, gate_kind="delta_channel",
@@ -132,7 +131,7 @@ class GatedDeltaRule(Part):
                              self.key_dim, self.key_dim ** -0.5, state, self.state_floats, step)
             ops.linear_recurrence(ready[:, :qk], ready[:, qk:2 * qk], ready[:, 2 * qk:], state, step, o, H, self.kv_heads,
                                   self.key_dim, self.value_dim, gate=gates[:, :H], beta=gates[:, H:], invariant=self.precision.invariant)
-        gate = self.g2(proj[:, g_off:g_off + self.gate_rank].contiguous()) if self.gate_rank else proj[:, g_off:g_off + vw]
+        gate = self.g2.of_rows(proj[:, g_off:g_off + self.gate_rank]) if self.gate_rank else proj[:, g_off:g_off + vw]
         y = torch.empty((rows, vw), dtype=self.precision.act, device=h.device)
         ops.gated_rmsnorm(o, gate, self.norm_weight, self.norm_eps, self.value_dim, self.gate, y)
         self.o(y, out=residual, accumulate=True)

@@ -1425,6 +1425,29 @@ def test_expert_products_in_sorted_rows(experts, top, rows, K, N):
     assert (y[at].double() - want).abs().max() <= 4 * N ** 0.5 * 2.0 ** -22 * max(1.0, float(act.abs().max()))
 
 
+@pytest.mark.parametrize("rows,n,k,offset", [(65, 128, 4, 0), (66, 2, 20, 1), (130, 200, 64, 3), (300, 4096, 256, 4), (777, 514, 132, 2)])
+def test_product_in_parts(rows, n, k, offset):
+    """A 32-bit product whose factors are cut into three bfloat16 parts, over strided rows at any offset, against 64 bits.  Bound: the
+    parts' products left out and the last parts' rounding, 4 * 2^-24 of the terms' absolute sum; and 6 k / 16 additions on the tensor
+    cores, which cut sums off at 2^-23 of it.  Numbers that are not finite, and the largest one, come out as from the plain product."""
+    from llmx_b200.parts.base import Precision
+    from llmx_b200.parts.linear import SplitLinear
+    g = torch.Generator().manual_seed(rows)
+    wide = torch.randn(rows, k + 8, generator=g).to(DEV)
+    w = (0.1 * torch.randn(n, k, generator=g)).to(DEV)
+    lin = SplitLinear(w, Precision.of("bfloat16"))
+    assert lin.parts is not None
+    torch.cuda.synchronize()
+    a = wide[:, offset:offset + k]
+    got = lin.of_rows(a).double()
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert bool(((got - want).abs() <= (4 * 2.0 ** -24 + 6 * k / 16 * 2.0 ** -23) * size).all())
+    wide[0, offset], wide[1, offset + 1], wide[2, offset + 2] = float("inf"), float("nan"), torch.finfo(torch.float32).max
+    got, plain = lin.of_rows(a), lin(a.contiguous())
+    assert torch.equal(torch.isnan(got), torch.isnan(plain)) and torch.equal(torch.isinf(got), torch.isinf(plain))
+    assert torch.allclose(got[2], plain[2], rtol=1e-5)
+
+
 @pytest.mark.parametrize("maps", [1, 2])
 @pytest.mark.parametrize("value_dim", [40, 128, 192])
 @pytest.mark.parametrize("splits", [1, 7, 9, 33, 64])
