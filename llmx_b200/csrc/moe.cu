@@ -200,8 +200,8 @@ moe_cores_kernel(const T* __restrict__ a, int a_div, const T* __restrict__ w, co
 // An expert's list is cut into ceil(pairs / 256) equal parts: its weights are read that often, and none is left with a few
 // pairs.  Units of one expert follow one another, its weight tiles fastest: what they share meets in the L2 cache.
 // Bound, at a few dozen to a few hundred pairs an expert, by the experts' weights from memory and by the write-out: with one warp for a
-// quarter of the lanes the tensor cores were busy a third of the time.  Measured against the mma.sync form over gathered rows, 16 experts,
-// two a token: 2,048 tokens, 2,048 -> 1,536 gated 98 us, one warp 80, two 71; back 51, 34 and 34; 1,201 tokens, 4,096 -> 3,072 gated
+// quarter of the lanes the tensor cores were busy a third of the time.  Measured against one SM a tile with rows gathered by cp.async, 16
+// experts, two a token: 2,048 tokens, 2,048 -> 1,536 gated 98 us, one warp 80, two 71; back 51, 34 and 34; 1,201 tokens, 4,096 -> 3,072 gated
 // 188 us -> 167 (one warp), back 87 -> 80.
 constexpr int TC_LIST_TILE = 128;                                            // pairs a tile of the routing holds for this form
 constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_BOX = 32;
