@@ -243,6 +243,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
         const bool atomic = mode == MODE_ACCUMULATE || splits > 1;
+        // Additions of several rounds of wide tiles leave the first warp of a quarter all of its columns: they end before the next
+        // tile's products anyway, and twice the warps' bursts get in the way of its loads (5,003 x 4,096 over 4,096: 111 us, 115 with two).
+        // One round and a rest has the two (1,201 x 4,096 over 4,096: 55 us, 58 with one).
+        const bool alone = FORM == PLAIN && BN == 256 && atomic && w_tiles * m_tiles >= (int)gridDim.x;
+        const int first = alone ? (share ? BN : 0) : 32 * share, stride = alone ? 32 : 64;
         while (ok && sched.next(w)) {
             ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_PAIR_EPILOGUE);
             if (!ok) break;
@@ -254,7 +259,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
                 heads_epilogue<BN>(hp, norm_w, taddr, n, wide_rows, w.mt * BN, narrow_rows);
             } else if (w.kb1 > w.kb0) {
 #pragma unroll 1
-                for (int c = 32 * share; c < BN; c += 64) {
+                for (int c = first; c < BN; c += stride) {
                     uint32_t r[32];
                     tc::tmem_ld_32x32(taddr + c, r);
                     if constexpr (FORM == DUAL) {
