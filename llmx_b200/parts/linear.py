@@ -139,6 +139,9 @@ class SplitLinear(Linear):
                 and self.in_features % 4 == 0 and self.in_features <= SPLIT_WIDTH):
             from .. import ops
             self.parts = Linear(ops.split_rows(self.weight, weight=True), precision)
+            # A product asks for its weights before it waits for the kernel before, and its wait covers that kernel alone: what a
+            # kernel of this package made must be there before the first one is launched, on whichever stream.
+            torch.cuda.current_stream().synchronize()
 
     def of_rows(self, a: torch.Tensor) -> torch.Tensor:
         """a @ W.T; a float32 [rows, in], a view whose rows may be strided."""

@@ -1437,7 +1437,6 @@ def test_product_in_parts(rows, n, k, offset):
     w = (0.1 * torch.randn(n, k, generator=g)).to(DEV)
     lin = SplitLinear(w, Precision.of("bfloat16"))
     assert lin.parts is not None
-    torch.cuda.synchronize()
     a = wide[:, offset:offset + k]
     got = lin.of_rows(a).double()
     want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T

@@ -192,3 +192,26 @@ def test_data_off_its_element_size_is_read_all_the_same(tmp_path):
     write_safetensors(path, {"a": a, "b": b, "c": torch.tensor([3.0])})
     entries, _ = read_header(path)
     assert entries["b"].begin < entries["a"].begin and all((e.begin - entries["b"].begin) % 2 == 0 for e in entries.values())
+
+
+class _OnTheDevice(torch.Tensor):
+    """A tensor that says it is on a GPU: what is launched for it is only recorded."""
+    is_cuda = property(lambda self: True)
+
+
+def test_weights_that_a_kernel_lays_out_are_there_before_the_first_product(monkeypatch):
+    """Products ask for their weights before they wait for the kernel before (csrc/common.cuh): the parts that a kernel makes of a
+    weight must have been waited for when the part that keeps them can first be called."""
+    from llmx_b200 import ops
+    from llmx_b200.parts.base import Precision
+    from llmx_b200.parts.linear import SplitLinear
+    order = []
+
+    class Stream:
+        def synchronize(self):
+            order.append("waited")
+
+    monkeypatch.setattr(ops, "split_rows", lambda x, weight=False: order.append("made") or torch.zeros(x.shape[0], 6 * x.shape[1], dtype=torch.bfloat16))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: Stream())
+    lin = SplitLinear(torch.ones(8, 16).as_subclass(_OnTheDevice), Precision.of("bfloat16"))
+    assert lin.parts is not None and order == ["made", "waited"]
