@@ -586,7 +586,8 @@ attention_merge_maps_kernel(const float* __restrict__ partial, QT* __restrict__ 
     for (int map = 0; map < 2; ++map) {
         float mm, ll, one[PER_LANE];
         merge_ranges(partial + ((size_t)item * 2 + map) * splits * (V + 2), V, splits, lane, mm, ll, one);
-        const float inv = (map == 0 ? 1.0f : -extras.factor) / ll;
+        // A row without any key (nothing was summed: the range with the largest score alone sums to at least one) gives zeros.
+        const float inv = ll == 0.0f ? 0.0f : (map == 0 ? 1.0f : -extras.factor) / ll;
 #pragma unroll
         for (int i = 0; i < PER_LANE; ++i) o[i] = fmaf(one[i], inv, o[i]);
     }

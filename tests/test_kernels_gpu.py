@@ -1476,3 +1476,19 @@ def test_ranges_without_keys_are_left_out_of_the_merge(maps, value_dim, splits):
         outs.append(out)
     assert bool(torch.isfinite(outs[1]).all())
     assert torch.allclose(outs[0], outs[1], rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("splits", [1, 7])
+def test_two_maps_of_a_row_without_keys_give_zeros(splits):
+    """A position of -1 sees no key: both maps' sums are empty, and the row's output is zero, as is their difference's norm (the row
+    beside it has keys)."""
+    from llmx_b200 import ops
+    heads, kv_heads, key_dim, value_dim, page = 4, 2, 64, 64, 16
+    g = torch.Generator().manual_seed(5)
+    cache = torch.randn(2, 1, kv_heads, page, 2 * key_dim + value_dim, generator=g).to(DEV)
+    q = torch.randn(2, heads * 2 * key_dim, generator=g).to(DEV)
+    req, table = torch.arange(2, dtype=torch.int32, device=DEV), torch.tensor([[0], [1]], dtype=torch.int32, device=DEV)
+    out = torch.full((2, heads * value_dim), 7.0, device=DEV)
+    ops.attention_split(q, cache, out, req, torch.tensor([-1, 11], dtype=torch.int32, device=DEV), table, heads, kv_heads, key_dim, value_dim,
+                        None, None, key_dim ** -0.5, splits=splits, extras=ops.SoftmaxExtras(difference=(0.4, 0.8, 1e-6)))
+    assert bool((out[0] == 0).all()) and bool(torch.isfinite(out[1]).all()) and bool((out[1] != 0).any())
