@@ -21,12 +21,17 @@
 // after its barriers are initialised (before any block signals the other) and before either block exits (a block's
 // shared memory and barriers are read and signalled by its partner until then).
 //
-// Three forms share the kernel.  PLAIN: float32 output, stored or added.  DUAL: two products that share the token
+// Four forms share the kernel.  PLAIN: float32 output, stored or added.  DUAL: two products that share the token
 // tile -- weight rows n and n + N (gate and up of a gated feed-forward), two tiles of 128 rows a block and two
 // accumulators -- written as silu(gate) * up (or another gated unit, gemm_act_epilogue.cuh) in bfloat16.  HEADS: the q/k/v product of heads of 128; the operands
 // change sides (the pair's 256 rows are tokens, 128 a block; the narrow side is 256 weight rows = two heads, of which
 // each block loads one), so a thread of the epilogue holds two whole heads of one token, norms and rotates them and
-// writes queries and cache rows as bfloat16 (gemm_heads_epilogue.cuh).
+// writes queries and cache rows as bfloat16 (gemm_heads_epilogue.cuh).  PARTS: a 32-bit product whose factors are cut into bfloat16
+// parts (`llmx_split_rows`).  The tensor cores cut sums off where 32-bit additions round, so each sum of 64 values' parts starts from
+// nothing in the other accumulator and the epilogue's threads add it to the 64 outputs that each keeps in registers: one order of
+// sums, no pieces in memory.  Bound by the operands' way from L2 (24 KB a block and k block).  2,048 rows x 256 -> 4,096, cutting
+// included: 47 us, 33 as one sum over all 1,536 columns, whose error against 64 bits was 3.5e-7 of the result's norm for terms of one
+// sign (0.9e-7 joined, 2.3e-7 the plain product); tiles of 256 tokens keep 128 outputs a thread, spill, and took 74.
 //
 // The reference has no tensor-core path for this product (its kernels: f32.gpu:1034-1084).
 #include "tc_pair.cuh"
@@ -41,7 +46,8 @@ constexpr int UMMA_K = 16;
 enum : int { MODE_STORE = 0, MODE_ACCUMULATE = 1, MODE_ACT = 2 };
 enum : int { ERR_PAIR_PRODUCER = 111, ERR_PAIR_MMA_FULL = 112, ERR_PAIR_MMA_ACC = 113, ERR_PAIR_EPILOGUE = 114 };
 
-enum : int { PLAIN = 0, DUAL = 1, HEADS = 2 };
+enum : int { PLAIN = 0, DUAL = 1, HEADS = 2, PARTS = 3 };
+constexpr int PARTS_BLOCKS = 6;     // k blocks of a group: 64 values in six runs (rowwise.cu)
 
 // The instruction's 256-row side is the "wide" operand (128 rows a block; DUAL: two such tiles), its BN-row side the
 // "narrow" one (BN / 2 rows a block).
@@ -207,12 +213,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
             Work w;
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
-            while (ok && sched.next(w)) {
+            bool have = sched.next(w);
+            while (ok && have) {
                 ok = tc::mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, error_word, ERR_PAIR_MMA_ACC);
                 if (!ok) break;
                 tc::tc_fence_after();
                 const uint32_t tmem_d = tmem_base + acc * cfg::ACC_COLS;
-                for (int kb = w.kb0; kb < w.kb1; ++kb) {
+                const int kb1 = FORM == PARTS ? w.kb0 + PARTS_BLOCKS : w.kb1;      // PARTS: a group's sum starts from nothing
+                for (int kb = w.kb0; kb < kb1; ++kb) {
                     ok = tc::mbar_wait(&full_bar[stage], phase, abort_flag, error_word, ERR_PAIR_MMA_FULL);
                     if (!ok) break;
                     tc::tc_fence_after();
@@ -234,6 +242,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
                 if (!ok) break;
                 mma_commit_pair(&acc_full[acc], 3);             // both blocks' accumulators are complete
                 if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+                if (FORM == PARTS && kb1 < w.kb1) w.kb0 = kb1;
+                else have = sched.next(w);
             }
         }
     } else {
@@ -248,7 +258,42 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
         // One round and a rest has the two (1,201 x 4,096 over 4,096: 55 us, 58 with one).
         const bool alone = FORM == PLAIN && BN == 256 && atomic && w_tiles * m_tiles >= (int)gridDim.x;
         const int first = alone ? (share ? BN : 0) : 32 * share, stride = alone ? 32 : 64;
+        float sum[FORM == PARTS ? BN / 2 : 1];              // PARTS: the thread's outputs of the tile, group by group
         while (ok && sched.next(w)) {
+            if constexpr (FORM == PARTS) {
+                const int n = (w.wt * 2 + (int)rank) * BM + quarter * 32 + lane;
+#pragma unroll 1
+                for (int kb = w.kb0; kb < w.kb1; kb += PARTS_BLOCKS) {
+                    ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_PAIR_EPILOGUE);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    const uint32_t taddr = tmem_base + acc * cfg::ACC_COLS + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+                    for (int i = 0; i < BN / 64; ++i) {
+                        uint32_t r[32];
+                        tc::tmem_ld_32x32(taddr + 32 * share + 64 * i, r);
+                        tc::tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            sum[32 * i + j] = kb > w.kb0 ? __fadd_rn(sum[32 * i + j], __uint_as_float(r[j])) : __uint_as_float(r[j]);
+                    }
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) arrive_at(peer_addr(&acc_empty[acc], 0));
+                    if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+                }
+                if (ok && n < N) {
+#pragma unroll
+                    for (int i = 0; i < BN / 64; ++i) {
+                        const int m0 = w.mt * BN + 32 * share + 64 * i, m_left = M - m0;
+                        float* out = (float*)C_ + (size_t)m0 * N + n;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            if (j < m_left) out[(size_t)j * N] = sum[32 * i + j];
+                    }
+                }
+                continue;
+            }
             ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_PAIR_EPILOGUE);
             if (!ok) break;
             tc::tc_fence_after();
@@ -395,6 +440,19 @@ LLMX_EXPORT int llmx_gemm_tc_pair(const void* weight_map, const void* A, float* 
     if (int e = llmx_make_map_bf16_2d(&map_a, A, (uint64_t)M, (uint64_t)K, token_tile / 2, BK)) return e;
     if (token_tile == 128) return launch_pair<128, PLAIN>(map_w, map_a, C, N, M, K, mode, splits, HeadsEpilogue{}, error_word, stream);
     return launch_pair<256, PLAIN>(map_w, map_a, C, N, M, K, mode, splits, HeadsEpilogue{}, error_word, stream);
+}
+
+// C = A W^T, both factors cut into bfloat16 parts by `llmx_split_rows`: K columns, 384 a group of 64 values.  C float32 [M, N], stored;
+// one order of sums.
+LLMX_EXPORT int llmx_gemm_tc_pair_parts(const void* weight_map, const void* A, float* C, int M, int N, int K, int* error_word,
+                                        cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (((uintptr_t)A & 15) || ((uintptr_t)C & 3)) return LLMX_ERR_UNSUPPORTED;
+    if (K <= 0 || K % (PARTS_BLOCKS * BK)) return LLMX_ERR_BAD_ARGUMENT;
+    ensure_sm_count();
+    CUtensorMap map_a;
+    if (int e = llmx_make_map_bf16_2d(&map_a, A, (uint64_t)M, (uint64_t)K, 64, BK)) return e;
+    return launch_pair<128, PARTS>(*(const CUtensorMap*)weight_map, map_a, C, N, M, K, MODE_STORE, 1, HeadsEpilogue{}, error_word, stream);
 }
 
 // out = act(A W^T) as bfloat16 [M, N] on pairs of SMs; `weight_map` with boxes of 128 rows; activations as in

@@ -1139,28 +1139,33 @@ LLMX_EXPORT int llmx_silu_columns(float* x, int rows, int stride, int c0, int n,
 
 // ---------------------------------------------------------------------------
 // Float32 rows as bfloat16 parts, for a 32-bit product on the tensor cores: x = hi + mid + lo, 8 bits each, and x w is the six
-// parts' products that reach 2^-24 of it.  They are laid along the product's inner width, so that an ordinary bfloat16 product
-// over 6 n values adds them, the small ones first:
+// parts' products that reach 2^-24 of it.  They are laid along the product's inner width, the small ones first:
 //   rows    lo | mid | hi | mid | hi | hi
 //   weight  hi | mid | lo | hi  | mid | hi
+// A run is a group of SPLIT_GROUP values (the last one filled up with zeros), one group's six runs after the other's: the tensor cores
+// cut their sums off, so the product starts anew with each group and joins the groups' sums by rounded additions (gemm_tc_pair.cu, PARTS).
 // A number that is not finite stands in the last run alone: the product then has what the 32-bit one has.  Four values a thread.
 // ---------------------------------------------------------------------------
+constexpr int SPLIT_GROUP = 64, RUN4 = SPLIT_GROUP / 4;
+
 __global__ void __launch_bounds__(256)
-split_rows_kernel(const float* __restrict__ x, long long stride, bool aligned, bool weight, uint2* __restrict__ out, int n4, long long total) {
+split_rows_kernel(const float* __restrict__ x, long long stride, bool aligned, bool weight, uint2* __restrict__ out, int n4, int groups, long long total) {
     pdl_trigger();
     pdl_wait();
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= total) return;
-    const long long r = i / n4;
-    const int c = (int)(i - r * n4);
+    const long long r = i / (RUN4 * groups);
+    const int c = (int)(i - r * (RUN4 * groups)), group = c / RUN4, at = c % RUN4;
     const float* src = x + r * stride + 4 * c;
-    float v[4];
-    if (aligned) {
-        const float4 q = *reinterpret_cast<const float4*>(src);
-        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-    } else {
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (c < n4) {
+        if (aligned) {
+            const float4 q = *reinterpret_cast<const float4*>(src);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = src[j];
+            for (int j = 0; j < 4; ++j) v[j] = src[j];
+        }
     }
     unsigned short hi[4], mid[4], lo[4], last[4];
 #pragma unroll
@@ -1174,7 +1179,7 @@ split_rows_kernel(const float* __restrict__ x, long long stride, bool aligned, b
         lo[j] = __bfloat16_as_ushort(__float2bfloat16_rn(rest - __uint_as_float((unsigned)mid[j] << 16)));
     }
     auto put = [&](int run, const unsigned short (&p)[4]) {
-        out[(r * 6 + run) * n4 + c] = make_uint2(p[0] | (unsigned)p[1] << 16, p[2] | (unsigned)p[3] << 16);
+        out[((r * groups + group) * 6 + run) * RUN4 + at] = make_uint2(p[0] | (unsigned)p[1] << 16, p[2] | (unsigned)p[3] << 16);
     };
     put(0, weight ? hi : lo);
     put(1, mid);
@@ -1184,14 +1189,15 @@ split_rows_kernel(const float* __restrict__ x, long long stride, bool aligned, b
     put(5, last);
 }
 
-// x [rows, n] float32, rows `stride` floats apart; out bfloat16 [rows, 6 n]; n a multiple of 4.
+// x [rows, n] float32, rows `stride` floats apart; out bfloat16 [rows, 6 times n rounded up to whole groups]; n a multiple of 4.
 LLMX_EXPORT int llmx_split_rows(const float* x, long long stride, int weight, void* out, int rows, int n, cudaStream_t stream) {
     if (rows <= 0 || n <= 0) return 0;
     if (stride < n) return LLMX_ERR_BAD_ARGUMENT;
-    const long long total = (long long)rows * (n / 4);
+    const int groups = (n + SPLIT_GROUP - 1) / SPLIT_GROUP;
+    const long long total = (long long)rows * groups * RUN4;
     if (n % 4 || ((uintptr_t)out & 7) || (total + 255) / 256 > 0x7fffffff) return LLMX_ERR_UNSUPPORTED;
     launch_kernel(split_rows_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, x, stride,
-                  stride % 4 == 0 && !((uintptr_t)x & 15), weight != 0, (uint2*)out, n / 4, total);
+                  stride % 4 == 0 && !((uintptr_t)x & 15), weight != 0, (uint2*)out, n / 4, groups, total);
     return launch_status();
 }
 

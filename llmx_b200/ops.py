@@ -517,12 +517,16 @@ def silu_columns_(x: torch.Tensor, first: int, count: int) -> torch.Tensor:
     return x
 
 
+SPLIT_GROUP = 64                 # values a group of parts (csrc/rowwise.cu)
+
+
 def split_rows(x: torch.Tensor, weight: bool = False) -> torch.Tensor:
-    """float32 rows [rows, n] (a view whose rows may be strided) as bfloat16 parts [rows, 6 n], so that split_rows(a) @
-    split_rows(w, weight=True).T is a @ w.T as close as a 32-bit product (csrc/rowwise.cu); n a multiple of 4."""
+    """float32 rows [rows, n] (a view whose rows may be strided) as bfloat16 parts [rows, 6 times n rounded up to whole groups of
+    `SPLIT_GROUP` values] (csrc/rowwise.cu); n a multiple of 4.  The product of split_rows(a) and split_rows(w, weight=True) is
+    a @ w.T (`ops_tc.gemm_tc_pair_parts`)."""
     _need(x.is_cuda, "kernel arguments must be CUDA tensors (there is no CPU path)")
     _need(x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] % 4 == 0, "split_rows: float32 rows of a multiple of four values")
-    out = torch.empty((x.shape[0], 6 * x.shape[1]), dtype=torch.bfloat16, device=x.device)
+    out = torch.empty((x.shape[0], 6 * -(-x.shape[1] // SPLIT_GROUP) * SPLIT_GROUP), dtype=torch.bfloat16, device=x.device)
     _check(_fn("rowwise", "llmx_split_rows")(_ptr(x), _row_stride(x), 1 if weight else 0, _ptr(out), x.shape[0], x.shape[1], _stream()),
            "split_rows")
     return out

@@ -14,6 +14,7 @@ _i, _p = ctypes.c_int, ctypes.c_void_p
 register_signature("gemm_tc", "llmx_gemm_tc_weight_map", [_p, _p, _i, _i])
 register_signature("gemm_tc", "llmx_gemm_tc", [_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p, _p])
 register_signature("gemm_tc_pair", "llmx_gemm_tc_pair", [_p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _p])
+register_signature("gemm_tc_pair", "llmx_gemm_tc_pair_parts", [_p, _p, _p, _i, _i, _i, _p, _p])
 register_signature("gemm_tc", "llmx_gemm_tc_act", [_p, _p, _p, _i, _i, _i, _i, ctypes.c_float, ctypes.c_float, _i, _p, _p])
 register_signature("gemm_tc_pair", "llmx_gemm_tc_pair_act", [_p, _p, _p, _i, _i, _i, _i, ctypes.c_float, ctypes.c_float, _i, _p, _p])
 register_signature("gemm_tc_pair", "llmx_gemm_tc_pair_swiglu", [_p, _p, _p, _i, _i, _i, _p, _p])
@@ -236,4 +237,17 @@ def gemm_tc_pair(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate
     _check(_fn("gemm_tc_pair", "llmx_gemm_tc_pair")(ctypes.c_void_p(wmap.address), _ptr(a), _ptr(out), m, n, k,
                                                     1 if accumulate else 0, splits, token_tile, _ptr(error_word(a.device)),
                                                     _stream()), "gemm_tc_pair")
+    return out
+
+
+def gemm_tc_pair_parts(a: torch.Tensor, wmap: WeightMap) -> torch.Tensor:
+    """The 32-bit product whose factors `ops.split_rows` cut into bfloat16 parts: a [M, K] the rows' parts, `wmap` over the weight's;
+    float32 [M, N].  Each group's sum is joined by rounded additions in one order (csrc/gemm_tc_pair.cu, PARTS)."""
+    _cuda(a, wmap.weight)
+    m, k = a.shape
+    n = wmap.weight.shape[0]
+    _need(a.dtype is torch.bfloat16 and wmap.weight.shape[1] == k and wmap.box_rows == 128, "gemm_tc_pair_parts: the parts do not fit")
+    out = torch.empty((m, n), dtype=torch.float32, device=a.device)
+    _check(_fn("gemm_tc_pair", "llmx_gemm_tc_pair_parts")(ctypes.c_void_p(wmap.address), _ptr(a), _ptr(out), m, n, k,
+                                                          _ptr(error_word(a.device)), _stream()), "gemm_tc_pair_parts")
     return out

@@ -121,24 +121,25 @@ class Linear:
         return torch.empty((rows, self.out_features), dtype=torch.float32, device=device)
 
 
-# Where the product in parts beats the plain one: beyond 64 rows (65 rows x 128 -> 2,048: 17 us against 13 and the cutting; 2,048 rows x
-# 256 -> 4,096: 118 us against 32) and up to 256 values, where its error against 64 bits is the smaller one too (2.3e-7 of the result's
-# norm against 2.9e-7; 1.3e-7 against 2.0e-7 at 128; it grows with the width, the plain form's with the width's root).
-SPLIT_ROWS, SPLIT_WIDTH = 64, 256
+# Where the product in parts, cutting included, is the faster one: beyond 64 rows (65 rows x 128 -> 2,048: 14 us against 18; 2,048 rows x
+# 256 -> 4,096: 47 against 121; x 64 -> 1,024: 16 against 18) of at least 64 values (300 rows x 32 -> 512: 14 us against 12; 2,048 x 16 ->
+# 2,048: 18 against 16).  Its error against 64 bits is the smaller one from 12 values on (64: 0.8e-7 of the result's norm against 1.4e-7,
+# terms of one sign 0.9e-7 against 1.2e-7; 256: 0.9e-7 against 2.9e-7 and 2.3e-7), measured up to 256.
+SPLIT_ROWS, SPLIT_LEAST, SPLIT_WIDTH = 64, 64, 256
 
 
 class SplitLinear(Linear):
     """A short 32-bit product that stays 32-bit on the bfloat16 path.  There many rows run on the tensor cores, both factors in
-    three bfloat16 parts (`ops.split_rows`; the weight's are laid out once); few rows, the float32 path and `Precision.invariant`
-    have the plain product."""
+    three bfloat16 parts (`ops.split_rows`; the weight's are laid out once, 12 bytes a value beside the 32-bit ones), their sums joined
+    in 32-bit every 64 values; few rows, other widths, the float32 path and `Precision.invariant` have the plain product."""
 
     def __init__(self, weight: torch.Tensor, precision: Precision):
         super().__init__(weight.to(torch.float32), Precision("float32", torch.float32, precision.invariant))
-        self.parts: Optional[Linear] = None
+        self.parts = None                # the tensor map of the weight's parts
         if (precision.act is torch.bfloat16 and not precision.invariant and self.weight.is_cuda
-                and self.in_features % 4 == 0 and self.in_features <= SPLIT_WIDTH):
-            from .. import ops
-            self.parts = Linear(ops.split_rows(self.weight, weight=True), precision)
+                and self.in_features % 4 == 0 and SPLIT_LEAST <= self.in_features <= SPLIT_WIDTH):
+            from .. import ops, ops_tc
+            self.parts = ops_tc.WeightMap(ops.split_rows(self.weight, weight=True))
             # A product asks for its weights before it waits for the kernel before, and its wait covers that kernel alone: what a
             # kernel of this package made must be there before the first one is launched, on whichever stream.
             torch.cuda.current_stream().synchronize()
@@ -146,8 +147,8 @@ class SplitLinear(Linear):
     def of_rows(self, a: torch.Tensor) -> torch.Tensor:
         """a @ W.T; a float32 [rows, in], a view whose rows may be strided."""
         if self.parts is not None and a.shape[0] > SPLIT_ROWS:
-            from .. import ops
-            return self.parts(ops.split_rows(a))
+            from .. import ops, ops_tc
+            return ops_tc.gemm_tc_pair_parts(ops.split_rows(a), self.parts)
         return self(a.contiguous())
 
 

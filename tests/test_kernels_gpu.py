@@ -1427,24 +1427,49 @@ def test_expert_products_in_sorted_rows(experts, top, rows, K, N):
 
 @pytest.mark.parametrize("rows,n,k,offset", [(65, 128, 4, 0), (66, 2, 20, 1), (130, 200, 64, 3), (300, 4096, 256, 4), (777, 514, 132, 2)])
 def test_product_in_parts(rows, n, k, offset):
-    """A 32-bit product whose factors are cut into three bfloat16 parts, over strided rows at any offset, against 64 bits.  Bound: the
-    parts' products left out and the last parts' rounding, 4 * 2^-24 of the terms' absolute sum; and 6 k / 16 additions on the tensor
-    cores, which cut sums off at 2^-23 of it.  Numbers that are not finite, and the largest one, come out as from the plain product."""
+    """A 32-bit product whose factors are cut into three bfloat16 parts, over strided rows at any offset, against 64 bits.  Bound, in
+    2^-24 of the terms' absolute sum: 4 for the parts' products left out and the last parts' rounding; 8 for a group's additions on the
+    tensor cores, which cut sums off (four whose sums are of full size and one between the runs, the smaller runs' a 256th of
+    that); one for each group's addition.  (Leaving out a product of parts that counts is further off at every width here.)  Numbers that are not finite, and the largest one, come out as from the plain product."""
     from llmx_b200.parts.base import Precision
     from llmx_b200.parts.linear import SplitLinear
     g = torch.Generator().manual_seed(rows)
     wide = torch.randn(rows, k + 8, generator=g).to(DEV)
     w = (0.1 * torch.randn(n, k, generator=g)).to(DEV)
     lin = SplitLinear(w, Precision.of("bfloat16"))
-    assert lin.parts is not None
+    assert (lin.parts is not None) == (k >= 64)          # narrower ones run the plain product
     a = wide[:, offset:offset + k]
     got = lin.of_rows(a).double()
     want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
-    assert bool(((got - want).abs() <= (4 * 2.0 ** -24 + 6 * k / 16 * 2.0 ** -23) * size).all())
+    groups = -(-k // 64)
+    assert bool(((got - want).abs() <= (12 + groups if lin.parts is not None else k + 1) * 2.0 ** -24 * size).all())
     wide[0, offset], wide[1, offset + 1], wide[2, offset + 2] = float("inf"), float("nan"), torch.finfo(torch.float32).max
     got, plain = lin.of_rows(a), lin(a.contiguous())
     assert torch.equal(torch.isnan(got), torch.isnan(plain)) and torch.equal(torch.isinf(got), torch.isinf(plain))
     assert torch.allclose(got[2], plain[2], rtol=1e-5)
+
+
+@pytest.mark.parametrize("signs", ["both", "one", "mean"])
+@pytest.mark.parametrize("k", [64, 68, 100, 128, 132, 192, 252, 256])
+def test_product_in_parts_is_no_further_off_than_the_plain_one(k, signs):
+    """Error norms against 64 bits: the product in parts' is at most the plain product's, for terms of both signs, of one sign and
+    with a mean, at the narrowest width that it takes (one group of 64 values), with parts of groups and at the widest.  (Sums that the
+    tensor cores cut off over the whole width are further off from 128 values of one sign on.)"""
+    from llmx_b200.parts.base import Precision
+    from llmx_b200.parts.linear import Linear, SplitLinear
+    g = torch.Generator().manual_seed(k)
+    a, w = torch.randn(300, k, generator=g), 0.1 * torch.randn(515, k, generator=g)
+    if signs == "one":
+        a, w = a.abs(), w.abs()
+    if signs == "mean":
+        a, w = a + 1.0, w + 0.1
+    a, w = a.to(DEV), w.to(DEV)
+    lin = SplitLinear(w, Precision.of("bfloat16"))
+    assert lin.parts is not None
+    got, plain, want = lin.of_rows(a), Linear.__call__(lin, a), a.double() @ w.double().T
+    assert not torch.equal(got, plain)
+    assert (got.double() - want).norm() <= (plain.double() - want).norm()
+    assert torch.equal(got, lin.of_rows(a))              # one order of sums
 
 
 @pytest.mark.parametrize("maps", [1, 2])

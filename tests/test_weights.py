@@ -202,7 +202,7 @@ class _OnTheDevice(torch.Tensor):
 def test_weights_that_a_kernel_lays_out_are_there_before_the_first_product(monkeypatch):
     """Products ask for their weights before they wait for the kernel before (csrc/common.cuh): the parts that a kernel makes of a
     weight must have been waited for when the part that keeps them can first be called."""
-    from llmx_b200 import ops
+    from llmx_b200 import ops, ops_tc
     from llmx_b200.parts.base import Precision
     from llmx_b200.parts.linear import SplitLinear
     order = []
@@ -212,6 +212,7 @@ def test_weights_that_a_kernel_lays_out_are_there_before_the_first_product(monke
             order.append("waited")
 
     monkeypatch.setattr(ops, "split_rows", lambda x, weight=False: order.append("made") or torch.zeros(x.shape[0], 6 * x.shape[1], dtype=torch.bfloat16))
+    monkeypatch.setattr(ops_tc, "WeightMap", lambda parts: parts)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: Stream())
-    lin = SplitLinear(torch.ones(8, 16).as_subclass(_OnTheDevice), Precision.of("bfloat16"))
+    lin = SplitLinear(torch.ones(8, 64).as_subclass(_OnTheDevice), Precision.of("bfloat16"))
     assert lin.parts is not None and order == ["made", "waited"]
