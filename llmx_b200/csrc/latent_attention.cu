@@ -799,7 +799,7 @@ static inline size_t tc_smem_bytes(int W) {
 
 template <int NB>                              // n-blocks of 8 columns a warp owns: C = 64 * NB
 __global__ void __launch_bounds__(TILE_THREADS, 1)
-latent_scores_tc_kernel(const float* __restrict__ qk, const __nv_bfloat16* __restrict__ cache, float* __restrict__ part,
+latent_scores_tc_kernel(const float* __restrict__ qk, bool aligned, const __nv_bfloat16* __restrict__ cache, float* __restrict__ part,
                         const int* __restrict__ tiles, const int* __restrict__ row_request,
                         const int* __restrict__ positions, const int* __restrict__ block_tables, int table_stride,
                         int heads, int C, int R, int HT, int splits, int page_size, int window) {
@@ -861,8 +861,10 @@ latent_scores_tc_kernel(const float* __restrict__ qk, const __nv_bfloat16* __res
         for (int u = 0; u < QS_AHEAD; ++u) {
             const int i = i0 + u * TILE_THREADS, p = i / fours, ri = p / HT, h = blockIdx.y * HT + p % HT;
             x[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (i < 16 * fours && ri < tile_rows && h < heads)
-                x[u] = *reinterpret_cast<const float4*>(qk + ((size_t)(row0 + ri) * heads + h) * W + 4 * (i % fours));
+            if (i < 16 * fours && ri < tile_rows && h < heads) {
+                const float* src = qk + ((size_t)(row0 + ri) * heads + h) * W + 4 * (i % fours);
+                x[u] = aligned ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+            }
         }
 #pragma unroll
         for (int u = 0; u < QS_AHEAD; ++u) {
@@ -1115,8 +1117,8 @@ LLMX_EXPORT int llmx_latent_scores(const float* qk, const void* cache, int cache
 #define LLMX_TC(NB)                                                                                                       \
         do {                                                                                                              \
             cudaFuncSetAttribute(latent_scores_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);     \
-            launch_kernel(latent_scores_tc_kernel<NB>, grid, dim3(TILE_THREADS), tsm, stream, qk, (const __nv_bfloat16*)cache, \
-                          part, tiles, row_request, positions, block_tables, table_stride, heads, C, R, HT, splits,     \
+            launch_kernel(latent_scores_tc_kernel<NB>, grid, dim3(TILE_THREADS), tsm, stream, qk, !((uintptr_t)qk & 15), \
+                          (const __nv_bfloat16*)cache, part, tiles, row_request, positions, block_tables, table_stride, heads, C, R, HT, splits,     \
                           page_size, window);                                                                             \
         } while (0)
         if (C == 128) LLMX_TC(2);

@@ -1517,3 +1517,26 @@ def test_two_maps_of_a_row_without_keys_give_zeros(splits):
     ops.attention_split(q, cache, out, req, torch.tensor([-1, 11], dtype=torch.int32, device=DEV), table, heads, kv_heads, key_dim, value_dim,
                         None, None, key_dim ** -0.5, splits=splits, extras=ops.SoftmaxExtras(difference=(0.4, 0.8, 1e-6)))
     assert bool((out[0] == 0).all()) and bool(torch.isfinite(out[1]).all()) and bool((out[1] != 0).any())
+
+
+def test_latent_scores_take_queries_at_any_offset():
+    """Rows of queries at the start of an allocation and a float further (not on 16 bytes): the same partial states, bit for bit."""
+    from llmx_b200 import ops
+    rows, heads, C, R, page, keys = 3, 4, 128, 32, 16, 70
+    g = torch.Generator().manual_seed(9)
+    cache = _bf16(torch.randn(5, 1, 1, page, C + R, generator=g)).to(DEV)
+    whole = torch.randn(rows * heads * (C + R) + 1, generator=g).to(DEV)
+    further = whole[1:]
+    start = further.clone()
+    assert further.data_ptr() % 16 == 4 and start.data_ptr() % 16 == 0
+    tiles = torch.tensor([[0, rows]], dtype=torch.int32, device=DEV)
+    req, pos = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.arange(keys - rows, keys, dtype=torch.int32, device=DEV)
+    table = torch.arange(5, dtype=torch.int32, device=DEV).view(1, 5)
+    parts = []
+    for qk in (start, further):
+        part = torch.zeros(rows, heads, 1, C + 2, device=DEV)
+        ops._check(ops._fn("latent_attention", "llmx_latent_scores")(ops._ptr(qk), ops._ptr(cache), ops._code(cache), ops._ptr(part), ops._ptr(tiles), 1, 1,
+                                                                     ops._ptr(req), ops._ptr(pos), ops._ptr(table), 5, heads, C, R, page, 0, 0,
+                                                                     ops._stream()), "scores")
+        parts.append(part)
+    assert bool((parts[0] != 0).any()) and torch.equal(parts[0], parts[1])
