@@ -545,7 +545,7 @@ template <bool GATED, typename OutT>
 __global__ void __launch_bounds__(FEW_THREADS, 1)
 moe_few_stream_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv_bfloat16* __restrict__ w,
                       const int* __restrict__ token_ids, const int* __restrict__ table, int top, int vocab, int experts, int pairs,
-                      OutT* __restrict__ out, int N, int K, Glu glu, int places, int* error_word) {
+                      OutT* __restrict__ out, int N, int K, Glu glu, int places, bool early, int* error_word) {
     const int workers = (int)blockDim.x / 32 - 1;
     extern __shared__ __align__(128) unsigned char ring[];
     __shared__ uint64_t full[FEW_PLACES], empty[FEW_PLACES];
@@ -564,9 +564,8 @@ moe_few_stream_kernel(const __nv_bfloat16* __restrict__ a, int a_div, const __nv
         tc::fence_barrier_init();
     }
     pdl_trigger();
-    // The step's tokens and a table that came with the weights are written by no kernel of the step: the stream of weights starts
-    // while the kernel before still runs (a router's choice is such a kernel's output).
-    const bool early = token_ids != nullptr;
+    // `early`: no kernel that may still run writes the ids or the table (the caller says so: a step's tokens that a copy brought, a
+    // table that came with the weights).  The stream of weights then starts while the kernel before still runs.
     if (!early) pdl_wait();
     if (warp == 0) {
         int mine = -1;
@@ -1097,10 +1096,11 @@ LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* 
 }
 
 // The same products for steps of a few pairs, without lists: a [rows of `a_div` pairs each, K] and w bfloat16 with K a
-// multiple of 8; the pair's expert is read from the table.
+// multiple of 8; the pair's expert is read from the table.  `settled`: ids and table are written by none of the kernels launched since
+// the stream was last waited for in full (a copy does): they may be read before the kernel before has ended.
 LLMX_EXPORT int llmx_moe_product_few(const void* a, int a_div, const void* w, const int* token_ids, const int* table,
                                      int top, int vocab, int pairs, int experts, void* out, int out_dtype, int N, int K,
-                                     int gated, int clamped, float limit, float alpha, int* error_word, cudaStream_t stream) {
+                                     int gated, int clamped, float limit, float alpha, int settled, int* error_word, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (N <= 0 || K <= 0 || K % 8 || a_div <= 0 || top <= 0 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return LLMX_ERR_UNSUPPORTED;
     if (!gated && out_dtype != LLMX_F32) return LLMX_ERR_UNSUPPORTED;
@@ -1120,7 +1120,7 @@ LLMX_EXPORT int llmx_moe_product_few(const void* a, int a_div, const void* w, co
     do {                                                                                                                \
         cudaFuncSetAttribute(moe_few_stream_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_RING);        \
         launch_kernel(moe_few_stream_kernel<G, O>, stream_grid, dim3(32 * workers + 32), ring, stream, (const __nv_bfloat16*)a, a_div, \
-                      (const __nv_bfloat16*)w, token_ids, table, top, vocab, experts, pairs, (O*)out, N, K, glu, places, error_word); \
+                      (const __nv_bfloat16*)w, token_ids, table, top, vocab, experts, pairs, (O*)out, N, K, glu, places, settled != 0, error_word); \
     } while (0)
         if (gated && out_dtype == LLMX_BF16) LLMX_FEW(true, __nv_bfloat16);
         else if (gated) LLMX_FEW(true, float);

@@ -129,7 +129,7 @@ _SIGNATURES = {
                                                   _f, _p, _i, _p, _i, _i, _f, _f, _f, _p, _i, _p],
     ("attention_rows_tc", "llmx_attention_rows_tc"): [_p, _p, ctypes.c_longlong, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p],
     ("moe", "llmx_moe_route"): [_p, _p, _i, _i, _i, _i, _p, _p, _p, _i, _p],
-    ("moe", "llmx_moe_product_few"): [_p, _i, _p, _p, _p, _i, _i, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _p, _p],
+    ("moe", "llmx_moe_product_few"): [_p, _i, _p, _p, _p, _i, _i, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _i, _p, _p],
     ("moe", "llmx_moe_product"): [_p, _i, _p, _i, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _p],
     ("moe", "llmx_moe_gather"): [_p, _i, _p, _p, _i, _i, _p, _i, _p],
     ("moe", "llmx_moe_product_tc"): [_p, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _i, _f, _f, _p, _p],
@@ -990,9 +990,11 @@ def _clamp(clamp):
 
 
 def moe_product_few(a: torch.Tensor, a_div: int, w: torch.Tensor, token_ids: torch.Tensor, table: torch.Tensor, pairs: int,
-                    out: torch.Tensor, gated: bool, clamp=None) -> torch.Tensor:
+                    out: torch.Tensor, gated: bool, clamp=None, settled: bool = False) -> torch.Tensor:
     """`moe_product` for steps of a few pairs (bfloat16, inner width a multiple of 8): the pairs' experts are read
-    from the table, no lists.  Up to eight pairs the named experts' rows are one stream, else a block takes a pair and 16 columns."""
+    from the table, no lists.  Up to eight pairs the named experts' rows are one stream, else a block takes a pair and 16 columns.
+    `settled`: ids and table are there already -- a copy brought the ids, or the stream was waited for; none of this module's kernels
+    has written them since -- so that the stream of weights may start before the kernel just before has ended."""
     from .runtime import error_word
     clamped, limit, alpha = _clamp(clamp)
     _cuda(a, w, token_ids, table, out)
@@ -1007,7 +1009,8 @@ def moe_product_few(a: torch.Tensor, a_div: int, w: torch.Tensor, token_ids: tor
           "moe_product_few: int32 ids and table")
     _need(tuple(out.shape) == (pairs, N), "moe_product_few: output shape does not fit")
     _check(_fn("moe", "llmx_moe_product_few")(_ptr(a), int(a_div), _ptr(w), _ptr(token_ids), _ptr(table), top, vocab, pairs, experts,
-                                              _ptr(out), _code(out), N, K, 1 if gated else 0, clamped, limit, alpha, _ptr(error_word(a.device)), _stream()),
+                                              _ptr(out), _code(out), N, K, 1 if gated else 0, clamped, limit, alpha, 1 if settled else 0,
+                                              _ptr(error_word(a.device)), _stream()),
            "moe_product_few")
     return out
 

@@ -192,8 +192,9 @@ class TableRoutedExperts(Part):
         y = torch.empty((pairs, self.hidden), dtype=torch.float32, device=dev)
         if self.tensor_cores and pairs <= self.few_pairs:
             # A few pairs (decoding): the experts' weights streamed once a pair; which form runs follows the step's rows alone.
-            ops.moe_product_few(h, self.top, self.w_gate_up, step.token_ids, self.table, pairs, act, gated=True)
-            ops.moe_product_few(act, 1, self.w_down, step.token_ids, self.table, pairs, y, gated=False)
+            # A step's token ids come by a copy in front of its first kernel, the table came with the weights.
+            ops.moe_product_few(h, self.top, self.w_gate_up, step.token_ids, self.table, pairs, act, gated=True, settled=True)
+            ops.moe_product_few(act, 1, self.w_down, step.token_ids, self.table, pairs, y, gated=False, settled=True)
         else:
             lists = torch.empty((self.experts, pairs), dtype=torch.int32, device=dev)
             counts = torch.empty((self.experts,), dtype=torch.int32, device=dev)

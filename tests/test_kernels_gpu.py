@@ -1540,3 +1540,28 @@ def test_latent_scores_take_queries_at_any_offset():
                                                                      ops._stream()), "scores")
         parts.append(part)
     assert bool((parts[0] != 0).any()) and torch.equal(parts[0], parts[1])
+
+
+def test_expert_products_of_a_few_pairs_wait_for_ids_that_a_draw_has_just_written():
+    """Ids handed over straight from a draw (a kernel that lets its followers start early): without `settled` the product reads them only
+    when they are there, and gives what it gives for the same ids once everything has ended; so does `settled` then."""
+    from llmx_b200 import ops
+    from llmx_b200.sampling import sampler
+    rows, top, experts, vocab, K, N = 4, 2, 16, 32768, 64, 48
+    g = torch.Generator().manual_seed(3)
+    table = torch.rand(vocab, experts, generator=g).argsort(1)[:, :top].to(torch.int32).contiguous().to(DEV)
+    h = _bf16(torch.randn(rows, K, generator=g)).to(DEV)
+    w = _bf16(torch.randn(experts, 2 * N, K, generator=g)).to(DEV)
+    settings = sampler._packer(rows).pack(*(rows * (0.0, 1.0, 0.0, 0.0, 0, -1)))
+    ids, seen = torch.zeros(rows, dtype=torch.int32, device=DEV), set()
+    product = lambda **kw: ops.moe_product_few(h, top, w, ids, table, rows * top, torch.full((rows * top, N), 7.0, dtype=torch.bfloat16, device=DEV), gated=True, **kw)
+    first = product()
+    for i in range(20):
+        logits, out = torch.randn(rows, vocab, generator=g).to(DEV), torch.full_like(first, 7.0)
+        torch.cuda.synchronize()
+        ops._check(ops._fn("sampling", "llmx_sample_rows")(ops._ptr(logits), rows, vocab, settings, ops._ptr(ids), 1, ops._stream()), "sample")
+        ops.moe_product_few(h, top, w, ids, table, rows * top, out, gated=True)
+        torch.cuda.synchronize()
+        assert torch.equal(ids.long(), logits.argmax(1)) and torch.equal(out, product()) and torch.equal(out, product(settled=True)), i
+        seen.add(tuple(ids.tolist()))
+    assert len(seen) > 1
