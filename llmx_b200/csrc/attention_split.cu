@@ -1252,7 +1252,7 @@ LLMX_EXPORT int llmx_attention_tiled(const void* q, const void* cache, void* out
     const size_t smem = tiled_smem(D, V, maps);
 #define LLMX_TILED(VN, M)                                                                                                   \
     do {                                                                                                                  \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(attention_tiled_kernel<VN, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (smem > 48 * 1024) LLMX_ALLOW_SMEM(attention_tiled_kernel<VN, M>);                                             \
         launch_kernel(attention_tiled_kernel<VN, M>, dim3(grid), dim3(128), smem, stream, (const __nv_bfloat16*)q,          \
                       (const __nv_bfloat16*)cache, (__nv_bfloat16*)out, row_start, row_count, history, block_tables,    \
                       table_stride, requests, heads, kv_heads, D, V, page_size, window, chunk, scale, r_pad, extras);   \
@@ -1293,7 +1293,7 @@ LLMX_EXPORT int llmx_attention_staged(const void* q, int q_dtype, const void* ca
     const int hpw = (heads / kv_heads + 3) / 4;
 #define LLMX_STAGED(T, H, VL)                                                                                              \
     do {                                                                                                                    \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(attention_staged_kernel<T, H, VL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (smem > 48 * 1024) LLMX_ALLOW_SMEM(attention_staged_kernel<T, H, VL>);                                           \
         launch_kernel(attention_staged_kernel<T, H, VL>, grid, dim3(128), smem, stream, (const T*)q, (const T*)cache, row_request, \
                       positions, block_tables, table_stride, heads, kv_heads, D, V, page_size, window, chunk, scale, splits, tk, \
                       softcap, maps, partial);                                                                                    \

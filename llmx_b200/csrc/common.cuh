@@ -70,6 +70,22 @@ __device__ __forceinline__ float quotient(float a, float b) {
 
 static inline int launch_status() { return (int)cudaGetLastError(); }
 
+// Dynamic shared memory beyond 48 KB has to be allowed for a kernel, by a limit that belongs to the function and not to the thread
+// or stream that sets it.  So every call allows the same: all that a block can have beside what the kernel declares.  (A call
+// that set its own size would lower the limit under a launch that another thread had just made room for.)
+template <auto KERNEL>
+static inline cudaError_t allow_all_smem() {
+    static const int most = [] {
+        cudaFuncAttributes a = {};
+        return cudaFuncGetAttributes(&a, KERNEL) == cudaSuccess ? 227 * 1024 - (int)a.sharedSizeBytes : 0;
+    }();
+    return cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+#define LLMX_ALLOW_SMEM(...)                                                          \
+    do {                                                                              \
+        if (const cudaError_t allowed = allow_all_smem<__VA_ARGS__>()) return (int)allowed; \
+    } while (0)
+
 // ---- programmatic dependent launch --------------------------------------------------------------
 // Kernels of a step run one after another on one stream.  Launched with the "programmatic stream
 // serialization" attribute, a kernel's blocks may be placed on the SMs and run their prologue (barriers,

@@ -262,10 +262,7 @@ LLMX_EXPORT int llmx_gemm_plain(const void* A, int a_dtype, const void* W, int w
     const size_t few_bytes = (size_t)M * K * sizeof(float);
     if (M <= FEW_ROWS && K % 4 == 0 && K <= SHORT_K && a_dtype == LLMX_F32 && w_dtype == LLMX_F32 && !(((uintptr_t)A | (uintptr_t)W) & 15)) {
         const size_t bytes = ((size_t)SHORT_COLS * (K + 4) + (size_t)M * K) * sizeof(float);
-        if (bytes > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(gemm_plain_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e != cudaSuccess) return (int)e;
-        }
+        if (bytes > 48 * 1024) LLMX_ALLOW_SMEM(gemm_plain_short_kernel);
         launch_kernel(gemm_plain_short_kernel, dim3((N + SHORT_COLS - 1) / SHORT_COLS), dim3(SHORT_THREADS), bytes, stream, (const float*)A,
                       (const float*)W, C, M, N, K, accumulate);
         return launch_status();

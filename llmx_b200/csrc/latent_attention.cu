@@ -243,8 +243,7 @@ int launch_attention(int pl, dim3 grid, size_t smem, cudaStream_t stream, const 
                      int page_size, int window, float scale) {
 #define LLMX_LAT(P)                                                                                                       \
     do {                                                                                                                  \
-        if (smem > 48 * 1024)                                                                                             \
-            cudaFuncSetAttribute(latent_attention_kernel<WT, KVT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (smem > 48 * 1024) LLMX_ALLOW_SMEM(latent_attention_kernel<WT, KVT, P>);                                       \
         launch_kernel(latent_attention_kernel<WT, KVT, P>, grid, dim3(WARPS * 32), smem, stream, q, q_stride,             \
                       (const KVT*)cache, (const WT*)w_uk, (const WT*)w_uv, (WT*)out, freq, rot_pairs, rot_halves, rot_mag, row_request, \
                       positions, block_tables, table_stride, heads, D, R, V, C, page_size, window, scale);               \
@@ -1032,14 +1031,12 @@ int launch_scores(int plp, dim3 grid, size_t smem, cudaStream_t stream, const fl
 #define LLMX_SC(P)                                                                                                        \
     do {                                                                                                                  \
         if (C + R == 64 * P) {                                                                                            \
-            if (smem > 48 * 1024)                                                                                         \
-                cudaFuncSetAttribute(latent_scores_kernel<KVT, P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            if (smem > 48 * 1024) LLMX_ALLOW_SMEM(latent_scores_kernel<KVT, P, true>);                                    \
             launch_kernel(latent_scores_kernel<KVT, P, true>, grid, dim3(TILE_THREADS), smem, stream, qk, (const KVT*)cache, \
                           part, tiles, row_request, positions, block_tables, table_stride, heads, C, R, HT, splits,     \
                           page_size, window);                                                                             \
         } else {                                                                                                          \
-            if (smem > 48 * 1024)                                                                                         \
-                cudaFuncSetAttribute(latent_scores_kernel<KVT, P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            if (smem > 48 * 1024) LLMX_ALLOW_SMEM(latent_scores_kernel<KVT, P, false>);                                   \
             launch_kernel(latent_scores_kernel<KVT, P, false>, grid, dim3(TILE_THREADS), smem, stream, qk, (const KVT*)cache, \
                           part, tiles, row_request, positions, block_tables, table_stride, heads, C, R, HT, splits,     \
                           page_size, window);                                                                             \
@@ -1116,7 +1113,7 @@ LLMX_EXPORT int llmx_latent_scores(const float* qk, const void* cache, int cache
         const size_t tsm = tc_smem_bytes(W);
 #define LLMX_TC(NB)                                                                                                       \
         do {                                                                                                              \
-            cudaFuncSetAttribute(latent_scores_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);     \
+            LLMX_ALLOW_SMEM(latent_scores_tc_kernel<NB>);                                                                 \
             launch_kernel(latent_scores_tc_kernel<NB>, grid, dim3(TILE_THREADS), tsm, stream, qk, !((uintptr_t)qk & 15), \
                           (const __nv_bfloat16*)cache, part, tiles, row_request, positions, block_tables, table_stride, heads, C, R, HT, splits,     \
                           page_size, window);                                                                             \

@@ -512,11 +512,6 @@ int make_expanded_map(CUtensorMap* map, const void* base, uint64_t tokens, uint6
     return r == CUDA_SUCCESS ? 0 : 10003;
 }
 
-template <typename K>
-int allow_smem(K kernel, int bytes) {
-    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 }  // namespace
 
 // Keys and values of heads head0 .. head0 + n_heads for the tokens that the requests' rows see.  cache [pool_tokens, C + R]
@@ -538,7 +533,7 @@ LLMX_EXPORT int llmx_latent_expand(const void* cache, long long pool_tokens, con
     if (int e = llmx_make_map_bf16_2d(&cache_map, cache, (uint64_t)pool_tokens, (uint64_t)(C + R), 16, 64)) return e;
     if (int e = llmx_make_map_bf16_2d(&uk_map, w_uk, (uint64_t)all_heads * D, (uint64_t)C, D, 64)) return e;
     if (int e = llmx_make_map_bf16_2d(&uv_map, w_uv, (uint64_t)all_heads * D, (uint64_t)C, D, 64)) return e;
-    if (int e = allow_smem(latent_expand_kernel, EXPAND_SMEM)) return e;
+    LLMX_ALLOW_SMEM(latent_expand_kernel);
     launch_kernel(latent_expand_kernel, dim3(max_tokens / ROWS, n_heads, n_req), dim3(EXPAND_THREADS), (size_t)EXPAND_SMEM, stream, cache_map,
                   uk_map, uv_map, expanded_map, (const __nv_bfloat16*)cache, (__nv_bfloat16*)expanded, requests, row_request, positions, block_tables,
                   table_stride, tokens, head0, C, R, page_size, window, error_word);
@@ -557,7 +552,7 @@ LLMX_EXPORT int llmx_latent_prompt(const void* expanded, int tokens, const float
         return LLMX_ERR_UNSUPPORTED;
     CUtensorMap map;
     if (int e = make_expanded_map(&map, expanded, (uint64_t)tokens, (uint64_t)n_heads)) return e;
-    if (int e = allow_smem(latent_prompt_kernel, PROMPT_SMEM)) return e;
+    LLMX_ALLOW_SMEM(latent_prompt_kernel);
     launch_kernel(latent_prompt_kernel, dim3(n_tiles, n_heads), dim3(PROMPT_THREADS), (size_t)PROMPT_SMEM, stream, map, q, q_stride,
                   (__nv_bfloat16*)out, tiles, freq, rot_pairs, rot_halves, rot_mag, positions, heads, head0, R, window,
                   scale * attn::LOG2E, error_word);

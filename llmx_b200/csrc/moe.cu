@@ -1084,8 +1084,7 @@ LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* 
     lc.numAttrs = llmx_pdl_enabled() ? 2 : 1;
 #define LLMX_MOE_TC(G, O)                                                                                              \
     do {                                                                                                                \
-        const cudaError_t e = cudaFuncSetAttribute(moe_tc_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lc.dynamicSmemBytes); \
-        if (e != cudaSuccess) return (int)e;                                                                            \
+        LLMX_ALLOW_SMEM(moe_tc_kernel<G, O>);                                                                           \
         cudaLaunchKernelEx(&lc, moe_tc_kernel<G, O>, w_map, r_map, lists, counts, experts, pairs, (O*)out, out_sorted, N, K, glu, stages, error_word); \
     } while (0)
     if (gated && out_dtype == LLMX_BF16) LLMX_MOE_TC(true, __nv_bfloat16);
@@ -1118,7 +1117,7 @@ LLMX_EXPORT int llmx_moe_product_few(const void* a, int a_div, const void* w, co
         const dim3 stream_grid((unsigned)(items < 148 ? items : 148));
 #define LLMX_FEW(G, O)                                                                                                  \
     do {                                                                                                                \
-        cudaFuncSetAttribute(moe_few_stream_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_RING);        \
+        LLMX_ALLOW_SMEM(moe_few_stream_kernel<G, O>);                                                                   \
         launch_kernel(moe_few_stream_kernel<G, O>, stream_grid, dim3(32 * workers + 32), ring, stream, (const __nv_bfloat16*)a, a_div, \
                       (const __nv_bfloat16*)w, token_ids, table, top, vocab, experts, pairs, (O*)out, N, K, glu, places, settled != 0, error_word); \
     } while (0)
@@ -1132,7 +1131,7 @@ LLMX_EXPORT int llmx_moe_product_few(const void* a, int a_div, const void* w, co
     if (grid.y > 65535) return LLMX_ERR_UNSUPPORTED;
 #define LLMX_FEW(G, O)                                                                                                  \
     do {                                                                                                                \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(moe_few_kernel<G, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (smem > 48 * 1024) LLMX_ALLOW_SMEM(moe_few_kernel<G, O>);                                                    \
         launch_kernel(moe_few_kernel<G, O>, dim3(grid), dim3(256), smem, stream, (const __nv_bfloat16*)a, a_div,       \
                       (const __nv_bfloat16*)w, token_ids, table, top, vocab, experts, (O*)out, N, K, glu);              \
     } while (0)

@@ -859,8 +859,7 @@ int launch_recurrence(int D, bool wide, int requests, cudaStream_t stream, const
         const int stages = 3 * buffer <= 200 * 1024 ? 3 : 2;                                                              \
         const size_t smem = stages * buffer;                                                                              \
         if (smem > 200 * 1024) return LLMX_ERR_UNSUPPORTED;                                                               \
-        if (smem > 48 * 1024)                                                                                             \
-            cudaFuncSetAttribute(recurrence_wide_kernel<P, L, W, C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (smem > 48 * 1024) LLMX_ALLOW_SMEM(recurrence_wide_kernel<P, L, W, C, MODE>);                                  \
         launch_kernel(recurrence_wide_kernel<P, L, W, C, MODE>, dim3(requests, (unsigned)by), dim3(C / W * L + 32 * WIDE_COPY_WARPS), \
                       smem, stream, q, k, v, q_stride, k_stride, v_stride, decay, gate, beta, gate_stride, beta_stride, skip, state, \
                       slot_floats, row_start, row_count, history, slot_in, slot_out, out, heads, qk_heads, D, V, stages); \
@@ -968,7 +967,7 @@ LLMX_EXPORT int llmx_conv_prepare(const float* proj, int stride, int first, int 
                       row_request, row_start, row_count, history, slot_in, slot_out, rows, run, row_blocks, gate_blocks);
         return launch_status();
     }
-    if (smem > 48 * 1024) cudaFuncSetAttribute(conv_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) LLMX_ALLOW_SMEM(conv_prepare_kernel);
     launch_kernel(conv_prepare_kernel, dim3(rows + requests), dim3(256), smem, stream, proj, stride, first, channels,
                   q_channels, k_channels, taps_w, taps_b, taps, ready, a_log, dt_bias, b_off, a_off, gate_kind, decay_in,
                   decay_stride, gates, gates_stride, heads, D, q_factor, state, slot_floats, conv_off, row_request,

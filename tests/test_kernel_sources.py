@@ -18,3 +18,16 @@ def test_whole_warps_wait_with_a_vote():
             if m:
                 found.append((os.path.basename(path), number, m.group(1)))
     assert not found, found
+
+
+def test_no_call_lowers_a_kernels_limit_of_shared_memory():
+    """The limit belongs to the function: a call that sets it to its own size can lower it under another thread's launch.  It is set to
+    a constant (or, `allow_all_smem`, to all that there is)."""
+    found = []
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        text = open(path, encoding="utf-8").read()
+        for m in re.finditer(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*?)\)\s*(?:;|!=|==|\)|\|\|)", text):
+            value = m.group(1).strip()
+            if not re.fullmatch(r"(?:\w+(?:<[^>]*>)?::)?[A-Z][A-Z_0-9]*", value) and os.path.basename(path) != "common.cuh":
+                found.append((os.path.basename(path), text.count("\n", 0, m.start()) + 1, value))
+    assert not found, found
