@@ -1077,6 +1077,7 @@ def moe_product(a: torch.Tensor, a_div: int, w: torch.Tensor, lists: torch.Tenso
     _need(a.dtype == w.dtype and a.dim() == 2 and a.shape[1] == K and a.shape[0] * a_div >= pairs, "moe_product: rows do not fit the weights")
     _need(tuple(out.shape) == (pairs, N), "moe_product: output shape does not fit")
     if tensor_cores:
+        counts = counts.reshape(-1)[:experts]           # may be longer: the routing wrote `experts` of them
         return moe_product_sorted(moe_gather(a, a_div, lists, counts, pairs), w, lists, counts, pairs, out, gated, clamp=clamp)
     _check(_fn("moe", "llmx_moe_product")(_ptr(a), int(a_div), _ptr(w), _code(w), _ptr(lists), _ptr(counts), _ptr(tiles), pairs,
                                           experts, _ptr(out), _code(out), N, K, 1 if gated else 0, clamped, limit, alpha, _stream()), "moe_product")

@@ -1565,3 +1565,19 @@ def test_expert_products_of_a_few_pairs_wait_for_ids_that_a_draw_has_just_writte
         assert torch.equal(ids.long(), logits.argmax(1)) and torch.equal(out, product()) and torch.equal(out, product(settled=True)), i
         seen.add(tuple(ids.tolist()))
     assert len(seen) > 1
+
+
+@pytest.mark.parametrize("tensor_cores", [False, True])
+def test_expert_products_read_the_counts_that_the_routing_wrote(tensor_cores):
+    """A buffer of counts longer than the experts: what lies behind theirs is nobody's count."""
+    from llmx_b200 import ops
+    experts, rows, K, N = 3, 40, 64, 96
+    g = torch.Generator().manual_seed(2)
+    choice = torch.randint(0, experts, (rows, 1), generator=g, dtype=torch.int32)
+    h, w = _bf16(torch.randn(rows, K, generator=g)).to(DEV), _bf16(torch.randn(experts, N, K, generator=g)).to(DEV)
+    lists, tiles = torch.empty((experts, rows), dtype=torch.int32, device=DEV), torch.empty((ops.moe_tiles_len(rows, experts),), dtype=torch.int32, device=DEV)
+    counts = torch.full((experts + 5,), 1 << 20, dtype=torch.int32, device=DEV)
+    ops.moe_route(None, choice.to(DEV), experts, lists, counts, tiles, tensor_cores=tensor_cores)
+    out = ops.moe_product(h, 1, w, lists, counts, tiles, rows, torch.zeros(rows, N, device=DEV), gated=False, tensor_cores=tensor_cores)
+    want = torch.einsum("rk,rnk->rn", h.double(), w.double()[choice[:, 0].long().to(DEV)])
+    assert (out.double() - want).abs().max() <= 4 * K ** 0.5 * 2.0 ** -22 * 8
