@@ -217,39 +217,51 @@ constexpr int tc_stages(int experts) {
 static_assert(tc_stages(TC_MAX_EXPERTS) >= 3, "a stage in use and two on their way");
 enum : int { ERR_MOE_PRODUCER = 441, ERR_MOE_MMA = 442, ERR_MOE_EPILOGUE = 443 };
 
-// rows[place] = a[pair / a_div] for the pair at that place of the sorted lists; a block a place.
-constexpr int GATHER_THREADS = 128;                  // many blocks an SM: a block waits for one read after the other
+// rows[place] = a[pair / a_div] for the pair at that place of the sorted lists; a warp a place, four to a block.  The block's threads add up
+// the counts of equal runs of experts (reads that wait for nothing), and the thread whose run holds a place walks it: a warp that
+// added up 32 experts after the other made a chain of reads as long as there are experts.  Bound by three reads that follow one
+// another (counts, list, row).
+constexpr int GATHER_PLACES = 4, GATHER_THREADS = 32 * GATHER_PLACES, GATHER_AHEAD = 8;
 __global__ void __launch_bounds__(GATHER_THREADS)
 gather_kernel(const uint4* __restrict__ a, int a_div, const int* __restrict__ lists, const int* __restrict__ counts, int experts, int pairs,
               uint4* __restrict__ rows, int per_row) {
     pdl_trigger();
     pdl_wait();
-    const int place = blockIdx.x;
-    __shared__ int found;
-    if (threadIdx.x < 32) {                          // the expert whose list holds the place
-        int base = 0, pair = -1;
-        for (int e0 = 0; e0 < experts && pair < 0; e0 += 32) {
-            const int mine = e0 + (int)threadIdx.x < experts ? counts[e0 + threadIdx.x] : 0;
-            int upto = mine;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, first = blockIdx.x * GATHER_PLACES;
+    __shared__ int carry[GATHER_PLACES], found[GATHER_PLACES];
+    const int run = (experts + GATHER_THREADS - 1) / GATHER_THREADS, e0 = threadIdx.x * run, e1 = min(e0 + run, experts);
+    int mine = 0;
+    for (int e = e0; e < e1; ++e) mine += counts[e];
+    int upto = mine;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int below = __shfl_up_sync(0xffffffffu, upto, o);
-                if ((int)threadIdx.x >= o) upto += below;
-            }
-            const unsigned hit = __ballot_sync(0xffffffffu, place < base + upto);
-            if (hit) {
-                const int first = __ffs(hit) - 1;
-                const int at = place - base - __shfl_sync(0xffffffffu, upto - mine, first);
-                pair = lists[(size_t)(e0 + first) * pairs + at];
-            }
-            base += __shfl_sync(0xffffffffu, upto, 31);
-        }
-        if (threadIdx.x == 0) found = pair;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += below;
+    }
+    if (lane == 31) carry[warp] = upto;
+    if (threadIdx.x < GATHER_PLACES) found[threadIdx.x] = -1;
+    __syncthreads();
+    int before = upto - mine;
+    for (int w = 0; w < warp; ++w) before += carry[w];
+    for (int i = 0; i < GATHER_PLACES; ++i) {
+        int at = first + i - before, e = e0;
+        if (at < 0 || at >= mine) continue;
+        while (at >= counts[e]) at -= counts[e++];
+        found[i] = lists[(size_t)e * pairs + at];
     }
     __syncthreads();
-    if (found < 0) return;                           // past the lists: pairs of experts without weights
-    const uint4* src = a + (size_t)(found / a_div) * per_row;
-    for (int i = threadIdx.x; i < per_row; i += GATHER_THREADS) rows[(size_t)place * per_row + i] = src[i];
+    const int pair = found[warp];
+    if (pair < 0) return;                            // past the lists: pairs of experts without weights
+    const uint4* src = a + (size_t)(pair / a_div) * per_row;
+    uint4* dst = rows + (size_t)(first + warp) * per_row;
+    for (int i0 = lane; i0 < per_row; i0 += 32 * GATHER_AHEAD) {
+        uint4 x[GATHER_AHEAD];
+#pragma unroll
+        for (int u = 0; u < GATHER_AHEAD; ++u) x[u] = src[min(i0 + 32 * u, per_row - 1)];
+#pragma unroll
+        for (int u = 0; u < GATHER_AHEAD; ++u)
+            if (i0 + 32 * u < per_row) dst[i0 + 32 * u] = x[u];
+    }
 }
 
 // An expert's units and where its pairs' rows begin; filled by the block, read by its warps.
@@ -1043,7 +1055,7 @@ LLMX_EXPORT int llmx_moe_gather(const void* a, int a_div, const int* lists, cons
     if (pairs <= 0) return 0;
     if (K <= 0 || a_div <= 0 || experts <= 0) return LLMX_ERR_BAD_ARGUMENT;
     if (K % 8 || (((uintptr_t)a | (uintptr_t)rows) & 15)) return LLMX_ERR_UNSUPPORTED;
-    launch_kernel(gather_kernel, dim3(pairs), dim3(GATHER_THREADS), 0, stream, (const uint4*)a, a_div, lists, counts, experts, pairs, (uint4*)rows, K / 8);
+    launch_kernel(gather_kernel, dim3((pairs + GATHER_PLACES - 1) / GATHER_PLACES), dim3(GATHER_THREADS), 0, stream, (const uint4*)a, a_div, lists, counts, experts, pairs, (uint4*)rows, K / 8);
     return launch_status();
 }
 
