@@ -207,89 +207,165 @@ constexpr int TC_LIST_TILE = 128;                                            // 
 constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_BOX = 32;
 constexpr int TC_W_BYTES = TC_M * TC_K * 2, TC_R_BYTES = TC_ROWS / 2 * TC_K * 2, TC_STAGE = TC_W_BYTES + TC_R_BYTES, TC_STAGES = 6;
 constexpr int TC_EPI_WARPS = 8, TC_THREADS = 64 + TC_EPI_WARPS * 32;
-constexpr int TC_MAX_EXPERTS = 8192;                                         // three numbers of each lie in shared memory, beside fewer stages if need be
-constexpr int tc_smem(int stages, int experts) { return stages * TC_STAGE + 1024 + 256 + 3 * experts * (int)sizeof(int); }
-constexpr int tc_stages(int experts) {
+constexpr int TC_MAX_EXPERTS = 8192;
+// Four numbers of each expert that has pairs lie in shared memory, beside fewer stages if need be.
+constexpr int TC_MAX_LISTED = 8192, TC_BARS = 512;                           // barriers, what the block's scan carries from warp to warp
+constexpr int tc_smem(int stages, int listed) { return stages * TC_STAGE + 1024 + TC_BARS + 4 * listed * (int)sizeof(int); }
+constexpr int tc_stages(int listed) {
     int stages = TC_STAGES;
-    while (tc_smem(stages, experts) > 227 * 1024) --stages;
+    while (tc_smem(stages, listed) > 227 * 1024) --stages;
     return stages;
 }
-static_assert(tc_stages(TC_MAX_EXPERTS) >= 3, "a stage in use and two on their way");
+static_assert(tc_stages(TC_MAX_LISTED) >= 3, "a stage in use and two on their way");
 enum : int { ERR_MOE_PRODUCER = 441, ERR_MOE_MMA = 442, ERR_MOE_EPILOGUE = 443 };
 
-// rows[place] = a[pair / a_div] for the pair at that place of the sorted lists; a warp a place, four to a block.  The block's threads add up
-// the counts of equal runs of experts (reads that wait for nothing), and the thread whose run holds a place walks it: a warp that
-// added up 32 experts after the other made a chain of reads as long as there are experts.  Bound by three reads that follow one
-// another (counts, list, row).
-constexpr int GATHER_PLACES = 4, GATHER_THREADS = 32 * GATHER_PLACES, GATHER_AHEAD = 8;
+// rows[place] = a[pair / a_div] for the pair at that place of the sorted lists; a block a place.  Bound by three reads that follow one
+// another, from memory (counts, list, row).  Few experts: the first warp adds up their counts, 32 at a time.  MANY: the block's threads
+// add up equal runs of experts side by side and the one whose run holds the place walks it (32 at a time the chain of reads is as long
+// as there are experts: 1,024 of them, 80 pairs, 19 us and 8,192 105 us, between the kernels beside it, against 7 and 28).
+constexpr int GATHER_THREADS = 128;                  // many blocks an SM: a block waits for one read after the other
+template <bool MANY>
 __global__ void __launch_bounds__(GATHER_THREADS)
 gather_kernel(const uint4* __restrict__ a, int a_div, const int* __restrict__ lists, const int* __restrict__ counts, int experts, int pairs,
               uint4* __restrict__ rows, int per_row) {
     pdl_trigger();
     pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, first = blockIdx.x * GATHER_PLACES;
-    __shared__ int carry[GATHER_PLACES], found[GATHER_PLACES];
-    const int run = (experts + GATHER_THREADS - 1) / GATHER_THREADS, e0 = threadIdx.x * run, e1 = min(e0 + run, experts);
-    int mine = 0;
-    for (int e = e0; e < e1; ++e) mine += counts[e];
-    int upto = mine;
+    const int place = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int found, carry[GATHER_THREADS / 32];
+    if (MANY) {
+        const int run = (experts + GATHER_THREADS - 1) / GATHER_THREADS, e0 = threadIdx.x * run, e1 = min(e0 + run, experts);
+        int mine = 0;
+        for (int e = e0; e < e1; ++e) mine += counts[e];
+        int upto = mine;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int below = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += below;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int below = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += below;
+        }
+        if (lane == 31) carry[warp] = upto;
+        if (threadIdx.x == 0) found = -1;
+        __syncthreads();
+        int at = place - (upto - mine);
+        for (int w = 0; w < warp; ++w) at -= carry[w];
+        if (at >= 0 && at < mine) {
+            int e = e0;
+            while (at >= counts[e]) at -= counts[e++];
+            found = lists[(size_t)e * pairs + at];
+        }
+    } else if (warp == 0) {                          // the expert whose list holds the place
+        int base = 0, pair = -1;
+        for (int e0 = 0; e0 < experts && pair < 0; e0 += 32) {
+            const int mine = e0 + lane < experts ? counts[e0 + lane] : 0;
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, place < base + upto);
+            if (hit) {
+                const int first = __ffs(hit) - 1;
+                const int at = place - base - __shfl_sync(0xffffffffu, upto - mine, first);
+                pair = lists[(size_t)(e0 + first) * pairs + at];
+            }
+            base += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (lane == 0) found = pair;
     }
-    if (lane == 31) carry[warp] = upto;
-    if (threadIdx.x < GATHER_PLACES) found[threadIdx.x] = -1;
     __syncthreads();
-    int before = upto - mine;
-    for (int w = 0; w < warp; ++w) before += carry[w];
-    for (int i = 0; i < GATHER_PLACES; ++i) {
-        int at = first + i - before, e = e0;
-        if (at < 0 || at >= mine) continue;
-        while (at >= counts[e]) at -= counts[e++];
-        found[i] = lists[(size_t)e * pairs + at];
-    }
-    __syncthreads();
-    const int pair = found[warp];
-    if (pair < 0) return;                            // past the lists: pairs of experts without weights
-    const uint4* src = a + (size_t)(pair / a_div) * per_row;
-    uint4* dst = rows + (size_t)(first + warp) * per_row;
-    for (int i0 = lane; i0 < per_row; i0 += 32 * GATHER_AHEAD) {
-        uint4 x[GATHER_AHEAD];
-#pragma unroll
-        for (int u = 0; u < GATHER_AHEAD; ++u) x[u] = src[min(i0 + 32 * u, per_row - 1)];
-#pragma unroll
-        for (int u = 0; u < GATHER_AHEAD; ++u)
-            if (i0 + 32 * u < per_row) dst[i0 + 32 * u] = x[u];
-    }
+    if (found < 0) return;                           // past the lists: pairs of experts without weights
+    const uint4* src = a + (size_t)(found / a_div) * per_row;
+    for (int i = threadIdx.x; i < per_row; i += GATHER_THREADS) rows[(size_t)place * per_row + i] = src[i];
 }
 
-// An expert's units and where its pairs' rows begin; filled by the block, read by its warps.
+// What the block's warps read of the experts, made by the block at its start: numbers [4][room] = how many pairs; rows before its own;
+// parts of lists up to and with its own; and, MANY, which expert (only those with pairs are listed: when every role of every block walked
+// the others, 8,192 experts, 80 pairs were 600 us of a product).  Few experts keep a place each and one warp's scan, 32 at a time: less
+// code, which comes from memory too, and for 16 experts 1 to 2 us a launch less than the list.
+constexpr int MANY_EXPERTS = 128;
+__device__ __forceinline__ void number_experts(const int* __restrict__ counts, int experts, int* numbers, int lane) {
+    int rows_before = 0, tiles_before = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+        const int e = e0 + lane, c = e < experts ? counts[e] : 0;
+        int rows_upto = c, tiles_upto = (c + TC_ROWS - 1) / TC_ROWS;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int r = __shfl_up_sync(0xffffffffu, rows_upto, o), t = __shfl_up_sync(0xffffffffu, tiles_upto, o);
+            if (lane >= o) rows_upto += r, tiles_upto += t;
+        }
+        if (e < experts) numbers[e] = c, numbers[experts + e] = rows_before + rows_upto - c, numbers[2 * experts + e] = tiles_before + tiles_upto;
+        rows_before += __shfl_sync(0xffffffffu, rows_upto, 31);
+        tiles_before += __shfl_sync(0xffffffffu, tiles_upto, 31);
+    }
+}
+// All threads of the block, each an equal run of the experts, so that counts are read side by side; `carry`: 3 ints a warp.  Returns how
+// many are listed, `room` at most (counts that add up to more than the pairs are nobody's routing).
+__device__ __forceinline__ int list_experts(const int* __restrict__ counts, int experts, int* numbers, int room, int* carry) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)blockDim.x >> 5;
+    const int run = (experts + (int)blockDim.x - 1) / (int)blockDim.x, e0 = (int)threadIdx.x * run, e1 = min(e0 + run, experts);
+    int mine[3] = {0, 0, 0}, upto[3];
+    for (int e = e0; e < e1; ++e) {
+        const int c = counts[e];
+        mine[0] += c > 0, mine[1] += c, mine[2] += (c + TC_ROWS - 1) / TC_ROWS;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        upto[i] = mine[i];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int below = __shfl_up_sync(0xffffffffu, upto[i], o);
+            if (lane >= o) upto[i] += below;
+        }
+        if (lane == 31) carry[3 * warp + i] = upto[i];
+    }
+    __syncthreads();
+    int total = 0;
+    for (int w = 0; w < warps; ++w) {
+        if (w < warp) upto[0] += carry[3 * w], upto[1] += carry[3 * w + 1], upto[2] += carry[3 * w + 2];
+        total += carry[3 * w];
+    }
+    int at = upto[0] - mine[0], row = upto[1] - mine[1], tile = upto[2] - mine[2];
+    for (int e = e0; e < e1; ++e) {
+        const int c = counts[e];
+        if (c <= 0 || at >= room) continue;
+        tile += (c + TC_ROWS - 1) / TC_ROWS;
+        numbers[at] = c, numbers[room + at] = row, numbers[2 * room + at] = tile, numbers[3 * room + at] = e;
+        row += c, ++at;
+    }
+    return min(total, room);
+}
+
+// A pair of blocks' units.
+template <bool MANY>
 struct Units {
-    const int* count;        // [experts]
-    const int* tile;         // [experts]: parts of lists up to and with the expert's
-    int experts, w_tiles, cur, step, e;
-    // Unit `cur`: expert e, pairs at .. at + n - 1 of its list, weight tile w.
-    __device__ bool next(int& at, int& n, int& w) {
+    const int* numbers;      // as above
+    int room, listed, w_tiles, cur, step, place;
+    // Unit `cur`: expert e, pairs at .. at + n - 1 of its list, rows from `row` on, weight tile w.
+    __device__ __forceinline__ bool next(int& e, int& at, int& n, int& row, int& w) {
+        const int* tile = numbers + 2 * room;
         const int t = cur / w_tiles;
-        while (e < experts && tile[e] <= t) ++e;
-        if (e >= experts) return false;
+        if (MANY)
+            while (place + 8 <= listed && tile[place + 7] <= t) place += 8;
+        while (place < listed && tile[place] <= t) ++place;
+        if (place >= listed) return false;
+        e = MANY ? numbers[3 * room + place] : place;
         w = cur % w_tiles;
-        const int parts = (count[e] + TC_ROWS - 1) / TC_ROWS;
+        const int count = numbers[place], parts = (count + TC_ROWS - 1) / TC_ROWS;
         // Equal parts, multiples of 16 of at most 256 pairs: the last one is never empty, (parts - 1) * 256 being below the count.
-        const int size = ((count[e] + parts - 1) / parts + 15) & ~15;
-        at = (t - (tile[e] - parts)) * size;
-        n = min(size, count[e] - at);
+        const int size = ((count + parts - 1) / parts + 15) & ~15;
+        at = (t - (tile[place] - parts)) * size;
+        n = min(size, count - at);
+        row = numbers[room + place] + at;
         cur += step;
         return true;
     }
 };
 
-template <bool GATED, typename OutT>
+template <bool GATED, typename OutT, bool MANY>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap r_map, const int* __restrict__ lists,
               const int* __restrict__ counts, int experts, int pairs, OutT* __restrict__ out, int out_sorted, int N, int K, Glu glu,
-              int stages, int* error_word) {
+              int stages, int room, int* error_word) {
     extern __shared__ uint8_t tc_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = (uint64_t*)(smem + stages * TC_STAGE);          // used in the first block
@@ -298,9 +374,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
     uint64_t* acc_empty = acc_full + 2;                             // [2], used in the first block
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    int* count = (int*)(smem + stages * TC_STAGE + 256);
-    int* row = count + experts;                                     // rows before the expert's
-    int* tile = row + experts;
+    int* carry = (int*)(smem + stages * TC_STAGE + 256);
+    int* numbers = (int*)(smem + stages * TC_STAGE + TC_BARS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const bool leader = rank == 0;
@@ -329,35 +404,23 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
     const uint32_t tmem_base = *tmem_slot;
     pdl_trigger();            // only now that this block holds its tensor memory (gemm_tc_pair.cu)
     pdl_wait();
-    if (warp == 2) {
-        int rows_before = 0, tiles_before = 0;
-        for (int e0 = 0; e0 < experts; e0 += 32) {
-            const int e = e0 + lane, c = e < experts ? counts[e] : 0;
-            int rows_upto = c, tiles_upto = (c + TC_ROWS - 1) / TC_ROWS;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int r = __shfl_up_sync(0xffffffffu, rows_upto, o), t = __shfl_up_sync(0xffffffffu, tiles_upto, o);
-                if (lane >= o) rows_upto += r, tiles_upto += t;
-            }
-            if (e < experts) count[e] = c, row[e] = rows_before + rows_upto - c, tile[e] = tiles_before + tiles_upto;
-            rows_before += __shfl_sync(0xffffffffu, rows_upto, 31);
-            tiles_before += __shfl_sync(0xffffffffu, tiles_upto, 31);
-        }
-    }
+    int listed = experts;
+    if (MANY) listed = list_experts(counts, experts, numbers, room, carry);
+    else if (warp == 2) number_experts(counts, experts, numbers, lane);
     __syncthreads();
     const int w_cols = GATED ? TC_M : 2 * TC_M;      // output columns of a unit
     const int steps = (K + TC_K - 1) / TC_K;
-    Units units{count, tile, experts, (N + w_cols - 1) / w_cols, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, 0};
-    int at, n, w;
+    Units<MANY> units{numbers, MANY ? room : experts, listed, (N + w_cols - 1) / w_cols, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, 0};
+    int e, at, n, row, w;
 
     if (warp == 0) {
         if (tc::elect_one()) {
             int st = 0;
             uint32_t phase = 1;
             bool ok = true;
-            while (ok && units.next(at, n, w)) {
+            while (ok && units.next(e, at, n, row, w)) {
                 const int half = ((n + 15) & ~15) / 2, boxes = (half + TC_BOX - 1) / TC_BOX;
-                const int first = row[units.e] + at + (int)rank * half;
+                const int first = row + (int)rank * half;
                 const int col = w * w_cols + (int)rank * (GATED ? TC_M / 2 : TC_M);
                 for (int s = 0; s < steps; ++s) {
                     ok = tc::mbar_wait(&empty[st], phase, abort_flag, error_word, ERR_MOE_PRODUCER);
@@ -367,9 +430,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
                     uint8_t* base = smem + st * TC_STAGE;
                     if (GATED) {
 #pragma unroll
-                        for (int i = 0; i < TC_M / 32; ++i) tma_load_3d_pair(base + i * 32 * TC_K * 2, &w_map, s * TC_K, col + 16 * i, 2 * units.e, bar);
+                        for (int i = 0; i < TC_M / 32; ++i) tma_load_3d_pair(base + i * 32 * TC_K * 2, &w_map, s * TC_K, col + 16 * i, 2 * e, bar);
                     } else {
-                        tma_load_3d_pair(base, &w_map, s * TC_K, col, units.e, bar);
+                        tma_load_3d_pair(base, &w_map, s * TC_K, col, e, bar);
                     }
                     for (int i = 0; i < boxes; ++i)
                         tma_load_2d_pair(base + TC_W_BYTES + i * TC_BOX * TC_K * 2, &r_map, s * TC_K, first + i * TC_BOX, bar);
@@ -382,7 +445,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
             int st = 0;
             uint32_t phase = 0, acc = 0, acc_phase = 1;
             bool ok = true;
-            while (ok && units.next(at, n, w)) {
+            while (ok && units.next(e, at, n, row, w)) {
                 ok = tc::mbar_wait(&acc_empty[acc], acc_phase, abort_flag, error_word, ERR_MOE_MMA);
                 if (!ok) break;
                 tc::tc_fence_after();
@@ -408,15 +471,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
         const int quarter = warp & 3, share = (warp - 2) >> 2;        // the tensor-memory lanes that this warp may touch, and which pairs it has
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
-        while (ok && units.next(at, n, w)) {
-            const int* list = lists + (size_t)units.e * pairs + at;
-            const int place = row[units.e] + at;
+        while (ok && units.next(e, at, n, row, w)) {
+            const int* list = lists + (size_t)e * pairs + at;
             const int c = w * w_cols + (GATED ? (int)rank * (TC_M / 2) + quarter * 16 + (lane & 15) : (int)rank * TC_M + quarter * 32 + lane);
             int dest[TC_ROWS / 64];                  // the rows that the lane's pairs go to: read while the products run
 #pragma unroll
             for (int i = 0; i < TC_ROWS / 64; ++i) {
                 const int p = 32 * share + 64 * i + lane;
-                dest[i] = out_sorted ? place + p : p < n ? list[p] : 0;
+                dest[i] = out_sorted ? row + p : p < n ? list[p] : 0;
             }
             ok = tc::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, error_word, ERR_MOE_EPILOGUE);
             if (!ok) break;
@@ -440,7 +502,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
                     }
                     const int half = up ? 16 : 0;
                     if (out_sorted && p0 + 32 <= n) {            // no condition a value: neighbouring rows
-                        OutT* to_row = out + (size_t)(place + p0 + half) * N + c;
+                        OutT* to_row = out + (size_t)(row + p0 + half) * N + c;
                         if (c < N)
 #pragma unroll
                             for (int j = 0; j < 16; ++j) to_row[(size_t)j * N] = x[j];
@@ -1055,7 +1117,8 @@ LLMX_EXPORT int llmx_moe_gather(const void* a, int a_div, const int* lists, cons
     if (pairs <= 0) return 0;
     if (K <= 0 || a_div <= 0 || experts <= 0) return LLMX_ERR_BAD_ARGUMENT;
     if (K % 8 || (((uintptr_t)a | (uintptr_t)rows) & 15)) return LLMX_ERR_UNSUPPORTED;
-    launch_kernel(gather_kernel, dim3((pairs + GATHER_PLACES - 1) / GATHER_PLACES), dim3(GATHER_THREADS), 0, stream, (const uint4*)a, a_div, lists, counts, experts, pairs, (uint4*)rows, K / 8);
+    launch_kernel(experts > MANY_EXPERTS ? gather_kernel<true> : gather_kernel<false>, dim3(pairs), dim3(GATHER_THREADS), 0, stream, (const uint4*)a,
+                  a_div, lists, counts, experts, pairs, (uint4*)rows, K / 8);
     return launch_status();
 }
 
@@ -1070,7 +1133,9 @@ LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* 
     if (!llmx_moe_tensor_cores_fit(LLMX_BF16, K) || experts > TC_MAX_EXPERTS || (((uintptr_t)rows | (uintptr_t)w) & 15)) return LLMX_ERR_UNSUPPORTED;
     const Glu glu = {clamped, limit, alpha};
     const int w_cols = gated ? TC_M : 2 * TC_M;
-    const long long most = ((long long)pairs / TC_ROWS + experts) * ((N + w_cols - 1) / w_cols);
+    const bool many = experts > MANY_EXPERTS;
+    const int room = many && pairs < experts ? pairs : experts;   // experts that have a place
+    const long long most = ((long long)pairs / TC_ROWS + room) * ((N + w_cols - 1) / w_cols);
     if (most >= (1ll << 31)) return LLMX_ERR_UNSUPPORTED;
     CUtensorMap w_map, r_map;
     const int per = gated ? 2 : 1;                   // gate rows and up rows are planes of their own
@@ -1079,11 +1144,11 @@ LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* 
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 2) sms = 148;
-    const int stages = tc_stages(experts);
+    const int stages = tc_stages(room);
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(2 * (most < sms / 2 ? most : sms / 2)));
     lc.blockDim = dim3(TC_THREADS);
-    lc.dynamicSmemBytes = tc_smem(stages, experts);
+    lc.dynamicSmemBytes = tc_smem(stages, room);
     lc.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1094,14 +1159,20 @@ LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = llmx_pdl_enabled() ? 2 : 1;
-#define LLMX_MOE_TC(G, O)                                                                                              \
+#define LLMX_MOE_TC_AS(G, O, M)                                                                                        \
     do {                                                                                                                \
-        LLMX_ALLOW_SMEM(moe_tc_kernel<G, O>);                                                                           \
-        cudaLaunchKernelEx(&lc, moe_tc_kernel<G, O>, w_map, r_map, lists, counts, experts, pairs, (O*)out, out_sorted, N, K, glu, stages, error_word); \
+        LLMX_ALLOW_SMEM(moe_tc_kernel<G, O, M>);                                                                        \
+        cudaLaunchKernelEx(&lc, moe_tc_kernel<G, O, M>, w_map, r_map, lists, counts, experts, pairs, (O*)out, out_sorted, N, K, glu, stages, room, error_word); \
+    } while (0)
+#define LLMX_MOE_TC(G, O)                          \
+    do {                                           \
+        if (many) LLMX_MOE_TC_AS(G, O, true);      \
+        else LLMX_MOE_TC_AS(G, O, false);          \
     } while (0)
     if (gated && out_dtype == LLMX_BF16) LLMX_MOE_TC(true, __nv_bfloat16);
     else if (gated) LLMX_MOE_TC(true, float);
     else LLMX_MOE_TC(false, float);
+#undef LLMX_MOE_TC_AS
 #undef LLMX_MOE_TC
     return launch_status();
 }
