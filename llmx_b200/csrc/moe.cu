@@ -207,8 +207,7 @@ constexpr int TC_LIST_TILE = 128;                                            // 
 constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_BOX = 32;
 constexpr int TC_W_BYTES = TC_M * TC_K * 2, TC_R_BYTES = TC_ROWS / 2 * TC_K * 2, TC_STAGE = TC_W_BYTES + TC_R_BYTES, TC_STAGES = 6;
 constexpr int TC_EPI_WARPS = 8, TC_THREADS = 64 + TC_EPI_WARPS * 32;
-constexpr int TC_MAX_EXPERTS = 8192;
-// Four numbers of each expert that has pairs lie in shared memory, beside fewer stages if need be.
+// Four numbers of each expert that has pairs lie in shared memory, beside fewer stages if need be; of more than TC_MAX_LISTED, in memory.
 constexpr int TC_MAX_LISTED = 8192, TC_BARS = 512;                           // barriers, what the block's scan carries from warp to warp
 constexpr int tc_smem(int stages, int listed) { return stages * TC_STAGE + 1024 + TC_BARS + 4 * listed * (int)sizeof(int); }
 constexpr int tc_stages(int listed) {
@@ -335,6 +334,16 @@ __device__ __forceinline__ int list_experts(const int* __restrict__ counts, int 
     return min(total, room);
 }
 
+// More experts with pairs than shared memory has room for: their numbers, then how many they are, in memory; one block.
+constexpr int LIST_THREADS = 1024;
+__global__ void __launch_bounds__(LIST_THREADS) list_experts_kernel(const int* __restrict__ counts, int experts, int* __restrict__ numbers, int room) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ int carry[3 * LIST_THREADS / 32];
+    const int listed = list_experts(counts, experts, numbers, room, carry);
+    if (threadIdx.x == 0) numbers[4 * (size_t)room] = listed;
+}
+
 // A pair of blocks' units.
 template <bool MANY>
 struct Units {
@@ -365,7 +374,7 @@ template <bool GATED, typename OutT, bool MANY>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap r_map, const int* __restrict__ lists,
               const int* __restrict__ counts, int experts, int pairs, OutT* __restrict__ out, int out_sorted, int N, int K, Glu glu,
-              int stages, int room, int* error_word) {
+              int stages, int room, const int* __restrict__ made, int* error_word) {
     extern __shared__ uint8_t tc_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = (uint64_t*)(smem + stages * TC_STAGE);          // used in the first block
@@ -405,12 +414,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__
     pdl_trigger();            // only now that this block holds its tensor memory (gemm_tc_pair.cu)
     pdl_wait();
     int listed = experts;
-    if (MANY) listed = list_experts(counts, experts, numbers, room, carry);
+    if (MANY) listed = made ? made[4 * (size_t)room] : list_experts(counts, experts, numbers, room, carry);
     else if (warp == 2) number_experts(counts, experts, numbers, lane);
     __syncthreads();
     const int w_cols = GATED ? TC_M : 2 * TC_M;      // output columns of a unit
     const int steps = (K + TC_K - 1) / TC_K;
-    Units<MANY> units{numbers, MANY ? room : experts, listed, (N + w_cols - 1) / w_cols, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, 0};
+    Units<MANY> units{MANY && made ? made : numbers, MANY ? room : experts, listed, (N + w_cols - 1) / w_cols, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, 0};
     int e, at, n, row, w;
 
     if (warp == 0) {
@@ -1123,14 +1132,14 @@ LLMX_EXPORT int llmx_moe_gather(const void* a, int a_div, const int* lists, cons
 }
 
 // The same products on the tensor cores: rows [pairs, K] and w bfloat16, the rows sorted as the lists are; out [pairs, N] by pair or,
-// `out_sorted`, in the rows' order.
+// `out_sorted`, in the rows' order.  `numbers`: int32 [4 m + 1] where m = min(pairs, experts) is more than TC_MAX_LISTED, else null.
 LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* lists, const int* counts, int pairs, int experts, void* out,
                                     int out_dtype, int out_sorted, int N, int K, int gated, int clamped, float limit, float alpha,
-                                    int* error_word, cudaStream_t stream) {
+                                    int* numbers, int* error_word, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (N <= 0 || K <= 0 || experts <= 0) return LLMX_ERR_BAD_ARGUMENT;
     if (!gated && out_dtype != LLMX_F32) return LLMX_ERR_UNSUPPORTED;
-    if (!llmx_moe_tensor_cores_fit(LLMX_BF16, K) || experts > TC_MAX_EXPERTS || (((uintptr_t)rows | (uintptr_t)w) & 15)) return LLMX_ERR_UNSUPPORTED;
+    if (!llmx_moe_tensor_cores_fit(LLMX_BF16, K) || (((uintptr_t)rows | (uintptr_t)w) & 15)) return LLMX_ERR_UNSUPPORTED;
     const Glu glu = {clamped, limit, alpha};
     const int w_cols = gated ? TC_M : 2 * TC_M;
     const bool many = experts > MANY_EXPERTS;
@@ -1144,11 +1153,18 @@ LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* 
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 2) sms = 148;
-    const int stages = tc_stages(room);
+    const bool apart = room > TC_MAX_LISTED;
+    if (apart) {
+        if (numbers == nullptr) return LLMX_ERR_BAD_ARGUMENT;
+        launch_kernel(list_experts_kernel, dim3(1), dim3(LIST_THREADS), 0, stream, counts, experts, numbers, room);
+        if (const int status = launch_status()) return status;
+    }
+    const int* made = apart ? numbers : nullptr;
+    const int stages = tc_stages(apart ? 0 : room);
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(2 * (most < sms / 2 ? most : sms / 2)));
     lc.blockDim = dim3(TC_THREADS);
-    lc.dynamicSmemBytes = tc_smem(stages, room);
+    lc.dynamicSmemBytes = tc_smem(stages, apart ? 0 : room);
     lc.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1162,7 +1178,7 @@ LLMX_EXPORT int llmx_moe_product_tc(const void* rows, const void* w, const int* 
 #define LLMX_MOE_TC_AS(G, O, M)                                                                                        \
     do {                                                                                                                \
         LLMX_ALLOW_SMEM(moe_tc_kernel<G, O, M>);                                                                        \
-        cudaLaunchKernelEx(&lc, moe_tc_kernel<G, O, M>, w_map, r_map, lists, counts, experts, pairs, (O*)out, out_sorted, N, K, glu, stages, room, error_word); \
+        cudaLaunchKernelEx(&lc, moe_tc_kernel<G, O, M>, w_map, r_map, lists, counts, experts, pairs, (O*)out, out_sorted, N, K, glu, stages, room, made, error_word); \
     } while (0)
 #define LLMX_MOE_TC(G, O)                          \
     do {                                           \

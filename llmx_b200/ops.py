@@ -132,7 +132,7 @@ _SIGNATURES = {
     ("moe", "llmx_moe_product_few"): [_p, _i, _p, _p, _p, _i, _i, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _i, _p, _p],
     ("moe", "llmx_moe_product"): [_p, _i, _p, _i, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _f, _f, _p],
     ("moe", "llmx_moe_gather"): [_p, _i, _p, _p, _i, _i, _p, _i, _p],
-    ("moe", "llmx_moe_product_tc"): [_p, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _i, _f, _f, _p, _p],
+    ("moe", "llmx_moe_product_tc"): [_p, _p, _p, _p, _i, _i, _p, _i, _i, _i, _i, _i, _i, _f, _f, _p, _p, _p],
     ("moe", "llmx_moe_combine"): [_p, _p, _i, _i, _i, _f, _p],
     ("moe", "llmx_moe_router"): [_p, _i, _p, _p, _i, _i, _i, _i, _i, _i, _p, _i, _i, _f, _p, _p, _p, _p],
     ("moe", "llmx_moe_combine_weighted"): [_p, _p, _p, _p, _i, _p, _i, _p, _p, _i, _i, _i, _f, _p],
@@ -974,7 +974,7 @@ def moe_tiles_len(pairs: int, experts: int) -> int:
 
 
 _moe_tile_rows = {}
-MOE_TC_EXPERTS = 8192            # experts that the tensor cores' products take (csrc/moe.cu)
+MOE_LISTED_EXPERTS = 8192        # experts with pairs whose numbers fit beside the tensor cores' products (csrc/moe.cu)
 
 
 def moe_tensor_cores_fit(dtype: torch.dtype, *inner_widths: int) -> bool:
@@ -1059,8 +1059,11 @@ def moe_product_sorted(rows: torch.Tensor, w: torch.Tensor, lists: torch.Tensor,
     _need(rows.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and tuple(rows.shape) == (pairs, K), "moe_product: rows do not fit the weights")
     _need(tuple(out.shape) == (pairs, N), "moe_product: output shape does not fit")
     _need(lists.dtype == torch.int32 and counts.dtype == torch.int32 and counts.numel() >= experts and lists.numel() >= experts * pairs, "moe_product: int32 lists")
+    listed = min(pairs, experts)
+    numbers = torch.empty((4 * listed + 1,), dtype=torch.int32, device=rows.device) if listed > MOE_LISTED_EXPERTS else None
     _check(_fn("moe", "llmx_moe_product_tc")(_ptr(rows), _ptr(w), _ptr(lists), _ptr(counts), pairs, experts, _ptr(out), _code(out), 1 if out_sorted else 0,
-                                             N, K, 1 if gated else 0, clamped, limit, alpha, _ptr(error_word(rows.device)), _stream()), "moe_product")
+                                             N, K, 1 if gated else 0, clamped, limit, alpha, _ptr(numbers), _ptr(error_word(rows.device)), _stream()),
+           "moe_product", 1 if numbers is None else 2)
     return out
 
 

@@ -177,8 +177,7 @@ class TableRoutedExperts(Part):
         self.w_gate_up = torch.stack([torch.cat([tensors[f"e{e}.{g}"], tensors[f"e{e}.{u}"]], dim=0) for e in range(self.experts)]).to(act).contiguous()
         self.w_down = torch.stack([tensors[f"e{e}.{d}"] for e in range(self.experts)]).to(act).contiguous()
         from .. import ops
-        self.tensor_cores = (not precision.invariant and self.experts <= ops.MOE_TC_EXPERTS
-                             and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate))
+        self.tensor_cores = not precision.invariant and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate)
 
     def forward(self, h: torch.Tensor, step: StepBatch, residual: torch.Tensor) -> None:
         from .. import ops
@@ -298,8 +297,7 @@ class RoutedExperts(Part):
         self.w_gate_up = torch.stack([torch.cat([tensors[f"e{e}.{g}"], tensors[f"e{e}.{u}"]], dim=0) for e in range(self.experts)]).to(act).contiguous()
         self.w_down = torch.stack([tensors[f"e{e}.{d}"] for e in range(self.experts)]).to(act).contiguous()
         from .. import ops
-        self.tensor_cores = (not precision.invariant and self.experts <= ops.MOE_TC_EXPERTS
-                             and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate))
+        self.tensor_cores = not precision.invariant and ops.moe_tensor_cores_fit(act, self.hidden, self.intermediate)
 
     def forward(self, h: torch.Tensor, step: StepBatch, residual: torch.Tensor) -> None:
         from .. import ops

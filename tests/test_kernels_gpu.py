@@ -1397,10 +1397,13 @@ def test_latent_prompts_round_as_the_exact_ones(mean, spread, history):
     assert made <= 1.05 * before, (made, before)
 
 
-@pytest.mark.parametrize("experts,top,rows,K,N", [(16, 2, 300, 576, 160), (1500, 1, 900, 32, 96), (6000, 2, 200, 96, 32), (3, 3, 700, 160, 416)])
+@pytest.mark.parametrize("experts,top,rows,K,N", [(16, 2, 300, 576, 160), (1500, 1, 900, 32, 96), (6000, 2, 200, 96, 32), (3, 3, 700, 160, 416),
+                                                  (128, 2, 300, 64, 96), (129, 2, 300, 64, 96), (8193, 1, 300, 32, 64), (9000, 2, 5000, 32, 32),
+                                                  (8192, 1, 8300, 32, 32)])
 def test_expert_products_in_sorted_rows(experts, top, rows, K, N):
     """The gated product leaves its rows in the lists' order and the plain one reads them there: every pair's result against 64 bits of
-    the same bfloat16 steps, experts so many that fewer stages fit beside their numbers, widths that end within a unit."""
+    the same bfloat16 steps, experts so many that fewer stages fit beside their numbers or that the numbers lie apart, the last number of
+    experts that all have a place and the first that are listed, widths that end within a unit."""
     from llmx_b200 import ops
     g = torch.Generator().manual_seed(experts + N)
     table = torch.rand(rows, experts, generator=g).argsort(1)[:, :top].to(torch.int32).contiguous().to(DEV)
