@@ -211,8 +211,14 @@ __global__ void __launch_bounds__(FEW_COLS) gemm_plain_few_kernel(const AT* __re
 
 // A few rows over a short K (the second half of a low-rank pair): 32 columns a block, whose weight rows the block copies to shared
 // memory before it waits for the kernel before (a thread reading its own row asked for 16 bytes of 32 rows at a time); a thread
-// then has a column of up to two rows.  The same order of k, the same bits.
-constexpr int SHORT_COLS = 32, SHORT_THREADS = 128, SHORT_K = 512;
+// then has a column of up to two rows (with one row three of the four warps repeat the first one's: the reads decide, not the
+// multiply-adds).  The same order of k, the same bits.  Eight weights in a row, 1 to 8 rows, us against a column a thread:
+//   4,096 columns    K 32 2.2/3.3   128 3.4/6.1   256 5.0/9.9   512 8.3/17.5
+//   32,768 columns   K 32 3.9/5.2   128 8.9/13.7  256 17.8/23.9  512 33.8/42.7
+//   65,536 columns   K 32 5.1/6.3   128 15.7/15.9  256 24.7/28.0  384 40.5/39.7  512 59.8/51.2
+// The blocks' copies of more than 256 values a row leave room for two or three of them on an SM, and so many columns are more rounds of
+// such blocks: there a column a thread is the faster one (at 128 values of 65,536 columns the two are equal).
+constexpr int SHORT_COLS = 32, SHORT_THREADS = 128, SHORT_K = 512, SHORT_WIDE_K = 256, SHORT_MANY_COLS = 32768;
 
 __global__ void __launch_bounds__(SHORT_THREADS) gemm_plain_short_kernel(const float* __restrict__ A, const float* __restrict__ W,
                                                                          float* __restrict__ C, int M, int N, int K, int accumulate) {
@@ -260,7 +266,7 @@ LLMX_EXPORT int llmx_gemm_plain(const void* A, int a_dtype, const void* W, int w
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return LLMX_ERR_BAD_ARGUMENT;
     const size_t few_bytes = (size_t)M * K * sizeof(float);
-    if (M <= FEW_ROWS && K % 4 == 0 && K <= SHORT_K && a_dtype == LLMX_F32 && w_dtype == LLMX_F32 && !(((uintptr_t)A | (uintptr_t)W) & 15)) {
+    if (M <= FEW_ROWS && K % 4 == 0 && K <= (N > SHORT_MANY_COLS ? SHORT_WIDE_K : SHORT_K) && a_dtype == LLMX_F32 && w_dtype == LLMX_F32 && !(((uintptr_t)A | (uintptr_t)W) & 15)) {
         const size_t bytes = ((size_t)SHORT_COLS * (K + 4) + (size_t)M * K) * sizeof(float);
         if (bytes > 48 * 1024) LLMX_ALLOW_SMEM(gemm_plain_short_kernel);
         launch_kernel(gemm_plain_short_kernel, dim3((N + SHORT_COLS - 1) / SHORT_COLS), dim3(SHORT_THREADS), bytes, stream, (const float*)A,

@@ -1124,7 +1124,7 @@ def test_a_row_of_a_gated_norm_is_the_same_alone_and_among_others(groups, group,
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 65, 36), (4, 4096, 256), (3, 130, 1000), (8, 65, 512), (8, 33, 508)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 65, 36), (4, 4096, 256), (3, 130, 1000), (8, 65, 512), (8, 33, 508), (2, 32768, 260), (3, 32769, 260), (3, 32769, 256)])
 def test_plain_products_of_few_and_many_rows_are_the_tiled_one_bit_for_bit(dtype, M, N, K):
     from llmx_b200 import ops
     g = torch.Generator().manual_seed(K)
