@@ -1033,7 +1033,7 @@ def moe_route(token_ids: torch.Tensor, table: torch.Tensor, experts: int, lists:
         f.argtypes, f.restype = [_i], _i
         tile_rows = _moe_tile_rows[bool(tensor_cores)] = f(1 if tensor_cores else 0)
     _check(_fn("moe", "llmx_moe_route")(_ptr(token_ids), _ptr(table), top, rows, experts, vocab, _ptr(lists), _ptr(counts),
-                                        _ptr(tiles), tile_rows, _stream()), "moe_route", 2)
+                                        _ptr(tiles), tile_rows, _stream()), "moe_route", 1 if tiles is None else 2)
 
 
 def moe_gather(a: torch.Tensor, a_div: int, lists: torch.Tensor, counts: torch.Tensor, pairs: int) -> torch.Tensor:

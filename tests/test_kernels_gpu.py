@@ -1584,3 +1584,14 @@ def test_expert_products_read_the_counts_that_the_routing_wrote(tensor_cores):
     out = ops.moe_product(h, 1, w, lists, counts, tiles, rows, torch.zeros(rows, N, device=DEV), gated=False, tensor_cores=tensor_cores)
     want = torch.einsum("rk,rnk->rn", h.double(), w.double()[choice[:, 0].long().to(DEV)])
     assert (out.double() - want).abs().max() <= 4 * K ** 0.5 * 2.0 ** -22 * 8
+
+
+def test_launches_of_a_routing_are_counted_as_they_are():
+    """One kernel lists the pairs; the second one, which cuts tiles, runs only where tiles are wanted."""
+    from llmx_b200 import ops
+    choice = torch.zeros(5, 1, dtype=torch.int32, device=DEV)
+    lists, counts = torch.empty((2, 5), dtype=torch.int32, device=DEV), torch.empty((2,), dtype=torch.int32, device=DEV)
+    for tiles, launches in ((None, 1), (torch.empty((ops.moe_tiles_len(5, 2),), dtype=torch.int32, device=DEV), 2)):
+        before = ops.launch_count()
+        ops.moe_route(None, choice, 2, lists, counts, tiles, tensor_cores=True)
+        assert ops.launch_count() - before == launches
