@@ -507,7 +507,7 @@ attention_split_kernel(const QT* __restrict__ q, const KVT* __restrict__ cache, 
 // A warp's merge of the ranges' partial states of one (row, map head): the largest score, the sum and the outputs, not yet divided.
 // A lane has a range's maximum and sum, 32 ranges at a time; then the ranges' outputs are added in range order, their factors passed
 // around by shuffles.  Bound by the reads' latency: those of AHEAD ranges are issued without a condition (a range without keys
-// of the row made no output; what lies there is read and not used) before the first is added.
+// of the row left zeros and a largest score of -infinity; they are read and not used) before the first is added.
 template <int PER_LANE>
 __device__ __forceinline__ void merge_ranges(const float* __restrict__ p, int V, int splits, int lane, float& mm, float& ll, float (&o)[PER_LANE]) {
     constexpr int AHEAD = PER_LANE <= 4 ? 8 : 4;

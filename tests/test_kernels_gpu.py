@@ -1479,8 +1479,9 @@ def test_product_in_parts_is_no_further_off_than_the_plain_one(k, signs):
 @pytest.mark.parametrize("value_dim", [40, 128, 192])
 @pytest.mark.parametrize("splits", [1, 7, 9, 33, 64])
 def test_ranges_without_keys_are_left_out_of_the_merge(maps, value_dim, splits):
-    """More ranges than keys: rows of 1, 3, 40 and 200 keys against the same in one range.  A range without keys leaves what lay in the
-    scratch memory.  Bound: 32-bit sums in another order, 64 terms of at most 4 each, with the difference's norm behind them."""
+    """More ranges than keys: rows of 1, 3, 40 and 200 keys against the same in one range, in both forms that leave ranges, over scratch
+    memory full of NaN: what no range has written is not used.  Bound: 32-bit sums in another order, 64 terms of at most 4 each, with
+    the difference's norm behind them."""
     from llmx_b200 import ops
     heads, kv_heads, key_dim, page = 4, 2, 64, 16
     g = torch.Generator().manual_seed(splits)
@@ -1495,15 +1496,18 @@ def test_ranges_without_keys_are_left_out_of_the_merge(maps, value_dim, splits):
     q = torch.randn(4, heads * maps * key_dim, generator=g).to(DEV)
     req, pos = torch.arange(4, dtype=torch.int32, device=DEV), torch.tensor([x - 1 for x in lengths], dtype=torch.int32, device=DEV)
     extras = ops.SoftmaxExtras(difference=(0.4, 0.8, 1e-6)) if maps == 2 else None
-    outs = []
-    for n in (1, splits):
-        torch.full((1 << 22,), float("nan"), device=DEV)           # what the scratch memory may then hold
+    want = torch.empty(4, heads * value_dim, device=DEV)
+    ops.attention_split(q, cache, want, req, pos, table.to(DEV), heads, kv_heads, key_dim, value_dim, None, None, key_dim ** -0.5, extras=extras)
+    table = table.to(DEV)
+    x = (extras or ops.NO_EXTRAS).checked(heads, value_dim, 4)
+    for form in ("llmx_attention_split", "llmx_attention_staged"):
         out = torch.empty(4, heads * value_dim, device=DEV)
-        ops.attention_split(q, cache, out, req, pos, table.to(DEV), heads, kv_heads, key_dim, value_dim, None, None, key_dim ** -0.5, splits=n,
-                            extras=extras)
-        outs.append(out)
-    assert bool(torch.isfinite(outs[1]).all())
-    assert torch.allclose(outs[0], outs[1], rtol=2e-5, atol=2e-5)
+        partial = torch.full((4, heads * maps, splits, value_dim + 2), float("nan"), device=DEV)
+        ops._check(ops._fn("attention_split", form)(
+            ops._ptr(q), ops._code(q), ops._ptr(cache), ops._code(cache), ops._ptr(out), ops._ptr(req), ops._ptr(pos), ops._ptr(table), table.shape[1], 4,
+            heads * maps, kv_heads, key_dim, value_dim, page, 0, 0, key_dim ** -0.5, splits, ops._ptr(partial), *x, ops._stream()), form)
+        assert bool(torch.isfinite(out).all()), form
+        assert torch.allclose(out, want, rtol=2e-5, atol=2e-5), form
 
 
 @pytest.mark.parametrize("splits", [1, 7])
@@ -1595,3 +1599,121 @@ def test_launches_of_a_routing_are_counted_as_they_are():
         before = ops.launch_count()
         ops.moe_route(None, choice, 2, lists, counts, tiles, tensor_cores=True)
         assert ops.launch_count() - before == launches
+
+
+@pytest.mark.parametrize("rows", [1, 64, 65])
+@pytest.mark.parametrize("D,V,half", [(64, 64, 0), (64, 40, 32), (128, 128, 32), (128, 96, 64), (256, 256, 32), (256, 64, 96), (256, 128, 128), (128, 128, 24)])
+def test_queries_and_keys_of_lanes_that_turn_their_own_pairs(rows, D, V, half):
+    """Norm, rotation and write of heads of 64, 128 and 256 with nothing, a part and all of a head turned (a lane then holds both values of
+    a pair; 24 pairs take the general kernel), steps on both sides of the line by rows, skipped slots, all types: against 64 bits of the
+    same 32-bit angles.  Bound: sums of D squares and the norm's division, the sine's two units, a product and a sum: 2^-19 of the
+    row's largest value (which the norm leaves below 16), and the type's rounding."""
+    from llmx_b200 import ops
+    heads, kv_heads, page = 5, 3, 16
+    g = torch.Generator().manual_seed(D + V + half + rows)
+    proj = torch.randn(rows, (heads + kv_heads) * D + kv_heads * V, generator=g)
+    pos = torch.randint(0, 3000, (rows,), generator=g, dtype=torch.int32)
+    slots = torch.randperm(6 * page, generator=g)[:rows].to(torch.int32)
+    slots[rows // 2] = -1
+    freq = torch.rand(half, generator=g) if half else None
+    for norm in (False, True):
+        qw, kw = (torch.rand(2, D, generator=g) + 0.5) if norm else (None, None)
+        x = proj[:, :(heads + kv_heads) * D].double().view(rows, heads + kv_heads, D)
+        if norm:
+            x = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * torch.cat([qw.expand(heads, D), kw.expand(kv_heads, D)]).double()
+        want = x.clone()
+        if half:
+            angle = (pos.float()[:, None] * freq[None]).double()[:, None]
+            lo, hi = x[..., :half], x[..., half:2 * half]
+            want[..., :half], want[..., half:2 * half] = lo * angle.cos() - hi * angle.sin(), hi * angle.cos() + lo * angle.sin()
+        values = proj[:, (heads + kv_heads) * D:].double().view(rows, kv_heads, V)
+        for q_type in (torch.float32, torch.bfloat16):
+            for c_type in (torch.float32, torch.bfloat16):
+                q_out = torch.full((rows, heads * D), 7.0, dtype=q_type, device=DEV)
+                cache = torch.full((6, 1, kv_heads, page, D + V), 7.0, dtype=c_type, device=DEV)
+                ops.qk_norm_rope_write(proj.to(DEV), heads, kv_heads, D, V, None if qw is None else qw.to(DEV), None if kw is None else kw.to(DEV), 1e-6,
+                                       None if freq is None else freq.to(DEV), pos.to(DEV), slots.to(DEV), q_out, cache)
+                near = lambda got, ref, kind: bool(((got - ref).abs() <= 16 * 2.0 ** -19 + (2.0 ** -8 if kind is torch.bfloat16 else 0.0) * ref.abs()).all())
+                assert near(q_out.cpu().double().view(rows, heads, D), want[:, :heads], q_type)
+                held = cache.cpu().double()[:, 0].permute(0, 2, 1, 3).reshape(6 * page, kv_heads, D + V)
+                kept = slots >= 0
+                at = slots[kept].long()
+                assert near(held[at][..., :D], want[kept][:, heads:], c_type) and near(held[at][..., D:], values[kept], c_type)
+                rest = torch.ones(6 * page, dtype=torch.bool)
+                rest[at] = False
+                assert bool((held[rest] == 7.0).all())
+
+
+@pytest.mark.parametrize("rows,width", [(1, 4), (3, 1020), (2, 1024), (5, 1028), (2, 4100), (3, 1022)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_clamped_unit_in_fours(rows, width, out_dtype):
+    """Widths of one thread, below, at and above a block of 1,024 values, several blocks, and one that is not in fours: against 64 bits,
+    values on both sides of the limits.  Bound: the exponential's two units, a sum, a division and two products, below 2^-20 of the
+    result; its argument alpha g, rounded once from a rounded alpha, moves it by 2^-23 of alpha g; and the type's rounding."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(width)
+    gu = 4 * torch.randn(rows, 2 * width, generator=g)
+    gu[0, 0], gu[0, width] = -90.0, 50.0
+    out = ops.clamped_glu(gu.to(DEV), torch.empty(rows, width, dtype=out_dtype, device=DEV), 1.5, 1.702).cpu().double()
+    gate, up = gu[:, :width].double().clamp(max=1.5), gu[:, width:].double().clamp(-1.5, 1.5)
+    want = gate / (1.0 + torch.exp(-1.702 * gate)) * (up + 1.0)
+    bound = 2.0 ** -20 + 2.0 ** -23 * (1.702 * gate).abs() + (2.0 ** -8 if out_dtype is torch.bfloat16 else 0.0)
+    assert bool(((out - want).abs() <= bound * want.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("rows", [128, 129, 200])
+def test_sampling_of_more_rows_than_a_launch_carries(rows):
+    """Up to 128 rows' settings travel with the launch, more in a buffer on the device, kept where all rows are greedy: both against the
+    plain sampler, greedy rows twice with the same masked ids and once with others."""
+    rng = np.random.default_rng(rows)
+    vocab = 3001
+    logits = (3 * rng.standard_normal((rows, vocab))).astype(np.float32)
+    settings = [dict(temp=float(rng.choice([0.0, 0.7, 1.2])), top_k=int(rng.choice([0, 5, 40])), top_p=float(rng.choice([1.0, 0.9])), seed=r + 1,
+                     masked=int(rng.integers(-1, 5))) for r in range(rows)]
+    plainly = lambda some: [plain.sample(row, s["temp"], s["top_k"], s["top_p"], 0.0, 0.0 if s["temp"] <= 0 else plain.XorShift64(s["seed"]).unit(),
+                                         masked=s["masked"]) for row, s in zip(logits, some)]
+    assert _sample_rows(logits.copy(), settings)[0] == plainly(settings)
+    greedy = [dict(s, temp=0.0) for s in settings]
+    best = logits.argmax(1)
+    other = [dict(s, masked=int(best[r])) for r, s in enumerate(greedy)]
+    for some in (greedy, greedy, other, greedy):
+        assert _sample_rows(logits.copy(), some)[0] == plainly(some)
+
+
+@pytest.mark.parametrize("counts", [[1, 0, 15, 16, 17], [255, 256, 257], [127, 128, 129, 512, 513], [272, 3]])
+@pytest.mark.parametrize("K,N,clamp", [(32, 32, None), (160, 96, (1.5, 1.7)), (96, 256, (1.5, 1.7))])
+def test_expert_products_at_the_edges_of_their_parts_as_steps_run_them(counts, K, N, clamp):
+    """Gathered rows, the gated product left in their order and the product back by pair: experts whose pairs end just below, at and
+    above a part or in several equal ones, two pairs a row, every seventh row naming an expert without weights (its pairs lie past the
+    lists and keep what they held).  Bounds as in the test of the tiles' edges."""
+    from llmx_b200 import ops
+    g = torch.Generator().manual_seed(K + N)
+    experts, named = len(counts), sum(counts)
+    lost = named // 7 + (named + named // 7) % 2
+    pairs = named + lost
+    choice = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(counts + [lost])])
+    choice[choice == experts] = experts + 5
+    choice = choice[torch.randperm(pairs, generator=g)]
+    h = _bf16(torch.randn(pairs // 2, K, generator=g)).to(DEV)
+    w_gu, w = (_bf16(torch.randn(experts, a, b, generator=g) * b ** -0.5).to(DEV) for a, b in ((2 * N, K), (K, N)))
+    lists, held = torch.empty((experts, pairs), dtype=torch.int32, device=DEV), torch.empty((experts,), dtype=torch.int32, device=DEV)
+    ops.moe_route(None, choice.view(-1, 2).to(DEV), experts, lists, held, None, tensor_cores=True)
+    assert held.tolist() == counts
+    act, y = torch.full((pairs, N), 7.0, dtype=torch.bfloat16, device=DEV), torch.full((pairs, K), 7.0, device=DEV)
+    ops.moe_product_sorted(ops.moe_gather(h, 2, lists, held, pairs), w_gu, lists, held, pairs, act, gated=True, out_sorted=True, clamp=clamp)
+    ops.moe_product_sorted(act, w, lists, held, pairs, y, gated=False)
+    at = torch.cat([lists[e, :n] for e, n in enumerate(counts)]).long()
+    e = choice.to(DEV)[at].long()
+    both = torch.einsum("pk,pnk->pn", h.double()[at // 2], w_gu.double()[e])
+    gate, up = both[:, :N], both[:, N:]
+    if clamp is None:
+        want = gate * torch.sigmoid(gate) * up
+    else:
+        gate, up = gate.clamp(max=clamp[0]), up.clamp(-clamp[0], clamp[0])
+        want = gate * torch.sigmoid(clamp[1] * gate) * (up + 1.0)
+    assert ((act[:named].double() - want).abs() <= 2.0 ** -8 * want.abs() + 8 * K ** 0.5 * 2.0 ** -22).all() and bool((act[named:] == 7.0).all())
+    want = torch.einsum("pn,pkn->pk", act[:named].double(), w.double()[e])
+    assert (y[at].double() - want).abs().max() <= 4 * N ** 0.5 * 2.0 ** -22 * max(1.0, float(act.abs().max()))
+    gone = torch.ones(pairs, dtype=torch.bool, device=DEV)
+    gone[at] = False
+    assert int(gone.sum()) == lost and bool((y[gone] == 7.0).all())
