@@ -253,9 +253,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_wide, const __grid_c
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
         const bool atomic = mode == MODE_ACCUMULATE || splits > 1;
-        // Additions of several rounds of wide tiles leave the first warp of a quarter all of its columns: they end before the next
-        // tile's products anyway, and twice the warps' bursts get in the way of its loads (5,003 x 4,096 over 4,096: 111 us, 115 with two).
-        // One round and a rest has the two (1,201 x 4,096 over 4,096: 55 us, 58 with one).
+        // Additions of two and more rounds of wide tiles leave the first warp of a quarter all of its columns: they end before the next tile's
+        // products anyway, and twice the warps' bursts get in the way of its loads.  Measured in turn, one warp / two: 3,072 x 4,096 over
+        // 4,096 79.9 / 82.0 us, 4,096 rows 94.2 / 98.2, 5,003 rows 112.7 / 116.8; 5,003 x 5,120 over 5,120 196.9 / 215.1; 3,072 x 8,192 over
+        // 8,192 297 / 303; at 2,048 rows (160 tiles of 5,120 outputs) equal within 1 %.  So it is for steps of more than 2,048 rows.
+        // Narrow tiles and fewer than two rounds keep both: 1,201 x 4,096 over 4,096, token tile 128, 58 -> 55 us with them.
         const bool alone = FORM == PLAIN && BN == 256 && atomic && w_tiles * m_tiles >= (int)gridDim.x;
         const int first = alone ? (share ? BN : 0) : 32 * share, stride = alone ? 32 : 64;
         float sum[FORM == PARTS ? BN / 2 : 1];              // PARTS: the thread's outputs of the tile, group by group

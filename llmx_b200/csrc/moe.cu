@@ -4,21 +4,21 @@
 // A step's rows are sorted by expert on the device, so that nothing about the routing is read on the host and a step
 // can be recorded and replayed.  A *pair* is (row, k): row r with the k-th expert of its token, numbered r * top + k.
 //   llmx_moe_route       one block an expert walks the pairs in order and lists those that name it (so a list is in
-//                        row order, whatever else the launch holds); then one block cuts the lists into tiles of
-//                        32 or 128 pairs (as the products' form wants): (expert, first place in the list), compactly,
-//                        with their number.
+//                        row order, whatever else the launch holds); for the products on the CUDA cores one more block cuts
+//                        the lists into tiles of 32 pairs: (expert, first place in the list), compactly, with their number.
 //   llmx_moe_product     gated: act[pair, f] = glu(h[row] . Wg_e[f], h[row] . Wu_e[f])       (gate and up rows stacked per expert;
 //                        glu(g, u) = silu(g) u, or the clamped unit min(g, L) sigmoid(alpha min(g, L)) (clamp(u, -L, L) + 1));
 //                        else y[pair, c] = act[pair] . Wd_e[c]                               (32-bit)
+//   llmx_moe_gather      the pairs' rows, one expert's after the other's, for the next:
+//   llmx_moe_product_tc  the same products on the tensor cores over sorted rows; the gated one leaves its rows sorted for the second
 //   llmx_moe_combine     x[row]      += weight * sum_k y[row * top + k]                      (k in order: one order of sums)
 // A pair may name an expert beyond those that have weights (an identity expert): it is in no list, the products leave its
 // rows alone, and `llmx_moe_combine_weighted` takes the row's input in its place.
-// The products run one block a (tile of an expert's pairs, tile of output columns): rows are gathered through the
-// list, the expert's weights are read once a tile.  Two forms: on the CUDA cores with explicit fmaf and k in
-// increasing order (32-bit weights and rows: the true 32-bit path; also bfloat16 shapes the tensor-core form does not
-// take), and on the tensor cores (tcgen05.mma, bfloat16 in, 32-bit sums) for bfloat16 with K a multiple of 32.
-// A third form serves steps of a few pairs (decoding), where the products are the experts' weights streamed once.
-// The CUDA-core form checks its tiles' size against what the routing wrote (tiles[1]).
+// Three forms of the products.  On the CUDA cores (32-bit weights and rows: the true 32-bit path; also bfloat16 shapes the tensor-core form
+// does not take) a block has a tile of an expert's pairs and a tile of output columns, gathers its rows through the list and reads
+// the expert's weights once a tile, explicit fmaf, k in increasing order; it checks its tiles' size against what the routing wrote
+// (tiles[1]).  On the tensor cores (tcgen05.mma, bfloat16 in, 32-bit sums; K a multiple of 32) pairs of SMs walk parts of the lists.
+// Steps of a few pairs (decoding) need no lists: their products are the experts' weights streamed once.
 #include "tc_pair.cuh"
 #include <math.h>
 #include <type_traits>
@@ -203,7 +203,7 @@ moe_cores_kernel(const T* __restrict__ a, int a_div, const T* __restrict__ w, co
 // quarter of the lanes the tensor cores were busy a third of the time.  Measured against one SM a tile with rows gathered by cp.async, 16
 // experts, two a token: 2,048 tokens, 2,048 -> 1,536 gated 98 us, one warp 80, two 71; back 51, 34 and 34; 1,201 tokens, 4,096 -> 3,072 gated
 // 188 us -> 167 (one warp), back 87 -> 80.
-constexpr int TC_LIST_TILE = 128;                                            // pairs a tile of the routing holds for this form
+constexpr int TC_LIST_TILE = 128;                                            // pairs a tile holds where tiles are asked for beside this form, which reads none
 constexpr int TC_ROWS = 256, TC_K = 64, TC_M = 128, TC_BOX = 32;
 constexpr int TC_W_BYTES = TC_M * TC_K * 2, TC_R_BYTES = TC_ROWS / 2 * TC_K * 2, TC_STAGE = TC_W_BYTES + TC_R_BYTES, TC_STAGES = 6;
 constexpr int TC_EPI_WARPS = 8, TC_THREADS = 64 + TC_EPI_WARPS * 32;
@@ -1076,7 +1076,7 @@ LLMX_EXPORT int llmx_moe_combine_weighted(const float* y, float* x, const float*
     return launch_status();
 }
 
-// The pairs a tile holds for the products' two forms: the routing cuts the lists for the form that will run.
+// The pairs a tile holds for the products on the CUDA cores, or of the tiles that go with the other form (it reads the counts alone).
 LLMX_EXPORT int llmx_moe_tile_rows(int tensor_cores) { return tensor_cores ? TC_LIST_TILE : TILE_ROWS; }
 
 // Whether the tensor-core form takes a product of these sizes and type.

@@ -761,7 +761,8 @@ def qk_norm_rope_write(proj: torch.Tensor, heads: int, kv_heads: int, key_dim: i
     """Rows of the stacked product [q (heads * D) | k (kv_heads * D) | v (kv_heads * V)], float32: per-head RMS norm of q
     and k (weights [D] or None), rotation of the first 2 * len(freq) values of each q and k head (value i with value
     i + len(freq), angle position * freq[i]), queries to q_out [rows, heads * D], [k ; v] to cache [pages, 1, kv_heads,
-    page, D + V] at the rows' slots."""
+    page, D + V] at the rows' slots.  The weights and `freq` are read before the kernel launched just before has ended, so they must not be
+    what another of this module's kernels has just written."""
     _cuda(proj, q_weight, k_weight, freq, positions, slots, q_out, cache)
     rows = proj.shape[0]
     _need(proj.dtype == torch.float32 and proj.shape[1] == (heads + kv_heads) * key_dim + kv_heads * value_dim, "qk_write: product width does not fit")
@@ -1019,7 +1020,8 @@ def moe_route(token_ids: torch.Tensor, table: torch.Tensor, experts: int, lists:
               tiles: torch.Tensor, tensor_cores: bool = False) -> None:
     """Sort the step's (row, k) pairs by the expert the table gives them: lists int32 [experts, rows * top] (pairs in
     order), counts int32 [experts], tiles int32 [moe_tiles_len] (their number, their size, then (expert, first place) of
-    every tile; None: not wanted, as `moe_product_sorted` reads none).  `tensor_cores`: the form of `moe_product` that will run (it sets the tiles' size: 128 pairs, else 32)."""
+    every tile; None: not wanted, as the tensor cores' products read none).  `tensor_cores` sets the tiles' size: 128 pairs, else the 32 that
+    `moe_product` on the CUDA cores needs."""
     _cuda(token_ids, table, lists, counts, tiles)
     vocab, top = table.shape
     rows = vocab if token_ids is None else token_ids.numel()      # no ids: the table has a row for each row of the step
@@ -1071,8 +1073,9 @@ def moe_product(a: torch.Tensor, a_div: int, w: torch.Tensor, lists: torch.Tenso
                 pairs: int, out: torch.Tensor, gated: bool, tensor_cores: bool = False, clamp=None) -> torch.Tensor:
     """out[pair] = a[pair // a_div] W_e^T for the expert e whose list holds the pair; w [experts, N (gated: 2 N, gate rows
     then up rows), K] of a's type.  gated: out = silu(gate) * up in out's type, or with `clamp` = (limit, alpha)
-    min(gate, limit) sigmoid(alpha min(gate, limit)) (clamp(up, -limit, limit) + 1); else float32.  `tensor_cores` as the
-    routing was told.  Pairs in no list (an expert without weights) keep what `out` held."""
+    min(gate, limit) sigmoid(alpha min(gate, limit)) (clamp(up, -limit, limit) + 1); else float32.  `tensor_cores` gathers the
+    rows and runs `moe_product_sorted` (a step that needs both products keeps the rows sorted between them); else the tiles must be of
+    32 pairs.  Pairs in no list (an expert without weights) keep what `out` held."""
     clamped, limit, alpha = _clamp(clamp)
     _cuda(a, w, lists, counts, tiles, out)
     experts, wn, K = w.shape
