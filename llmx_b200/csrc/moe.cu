@@ -221,7 +221,7 @@ enum : int { ERR_MOE_PRODUCER = 441, ERR_MOE_MMA = 442, ERR_MOE_EPILOGUE = 443 }
 // rows[place] = a[pair / a_div] for the pair at that place of the sorted lists; a block a place.  Bound by three reads that follow one
 // another, from memory (counts, list, row).  Few experts: the first warp adds up their counts, 32 at a time.  MANY: the block's threads
 // add up equal runs of experts side by side and the one whose run holds the place walks it (32 at a time the chain of reads is as long
-// as there are experts: 1,024 of them, 80 pairs, 19 us and 8,192 105 us, between the kernels beside it, against 7 and 28).
+// as there are experts: 80 pairs of 1,024 of them 19 us and of 8,192 105 us, the wait for the routing included, against 5 and 57).
 constexpr int GATHER_THREADS = 128;                  // many blocks an SM: a block waits for one read after the other
 template <bool MANY>
 __global__ void __launch_bounds__(GATHER_THREADS)
